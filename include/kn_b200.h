@@ -140,6 +140,15 @@ KN_API int kn_executor_io_info(const kn_executor* exec, int is_output, int index
  * the executor's own staging pointer (kn_executor_host_buffer) for an entry skips the extra host
  * copy for it.  Bool outputs are validated to be 0/1 (executor.rs:181-189). */
 KN_API int kn_executor_evaluate(kn_executor* exec, const void* const* inputs, void* const* outputs);
+/* Pinned result buffers for the next `kn_executor_evaluate`: fills `outputs` with one pointer per output and `*set` with
+ * a handle that keeps them, also beyond the executor's life.  An evaluation that is given exactly these pointers
+ * downloads straight into them (no second host copy).  They stay the caller's until `kn_outputs_release`, which any thread
+ * may call; the executor then uses them again.  `*set` is NULL, and nothing is filled in, when the outputs are
+ * too small for it to pay or all of the executor's (few) sets are held: evaluate into buffers of your own then.
+ * The reference hands out borrowed tensors instead (kn-cuda-eval/src/executor.rs:194). */
+typedef struct kn_outputs kn_outputs;
+KN_API int kn_executor_outputs_acquire(kn_executor* exec, void** outputs, kn_outputs** set);
+KN_API void kn_outputs_release(kn_outputs* set);
 /* `evaluate` in two halves, for hosts that keep several executors of one device busy at once (the
  * reference's self-play and server loops run several executor threads per GPU; here one thread can do it):
  * `begin` stages the inputs and enqueues upload, steps and download on the executor's stream without waiting,

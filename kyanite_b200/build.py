@@ -24,11 +24,13 @@ SOURCES = [
     "strided.cpp",
     "plan.cpp",
     "comm.cpp",
+    "host_copy.cpp",
     "executor.cu",
     "kernels/elementwise.cu",
     "kernels/rows.cu",
     "kernels/rows_f16.cu",
     "kernels/gather.cu",
+    "kernels/host_copy.cu",
     "kernels/contract_simt.cu",
     "kernels/contract_tc.cu",
     "kernels/conv_chain.cu",
@@ -56,7 +58,7 @@ def _headers():
     for d, _, files in os.walk(CSRC):
         if os.path.basename(d) == "build":
             continue
-        out += [os.path.join(d, f) for f in files if f.endswith(".h")]
+        out += [os.path.join(d, f) for f in files if f.endswith((".h", ".cuh"))]
     return out
 
 

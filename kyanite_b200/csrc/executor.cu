@@ -3,14 +3,18 @@
 // captured CUDA graph of the step list.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <sstream>
 #include <string>
 #include <vector>
 
 #include "comm.h"
+#include "host_copy.h"
 #include "ir.h"
 #include "kernels.h"
 #include "kn_b200.h"
@@ -62,6 +66,24 @@ struct DeviceGuard {
 
 void set_last_error(const std::string& message) { g_last_error = message; }
 
+// Pinned result buffers, one per output, that one evaluation downloads into and that then belong to whoever holds the
+// set: the results reach the caller without a second copy into fresh pages (which took longer than the download
+// itself: 4.8 MB of policies are 94 us over the link and 265 us of memcpy and page faults).
+struct OutputSet {
+    std::vector<void*> ptr;
+    ~OutputSet() {
+        for (void* p : ptr) if (p) cudaFreeHost(p);
+    }
+};
+// An executor owns at most this many sets, and at most this many bytes of them (but two whatever their size); a caller
+// that keeps more results than that gets them copied instead.
+constexpr size_t kMaxOutputSets = 4;
+constexpr size_t kMaxOutputSetBytes = 512ull << 20;
+// Outputs smaller than this in all are copied: the copy costs less than handing a set over.
+constexpr size_t kMinOutputSetBytes = 64 << 10;
+// Inputs of up to this many bytes in all go up, and outputs of up to as many come down, by a kernel (host_copy.cu).
+constexpr size_t kKernelTransferBytes = 64 << 10;
+
 struct Executor {
     int device = 0;
     std::unique_ptr<Plan> plan;
@@ -74,7 +96,11 @@ struct Executor {
     std::vector<size_t> bytes_in, bytes_out;
     std::vector<DType> dtype_in, dtype_out;
     cudaGraphExec_t graph_exec = nullptr;        // the step list
-    cudaGraphExec_t eval_graph_exec = nullptr;   // uploads + step list + downloads (see capture_evaluate)
+    // uploads + step list + downloads (see capture_evaluate), per destination: [0] the staging, [1 + i] output_sets[i]
+    std::vector<cudaGraphExec_t> eval_graphs;
+    std::vector<std::shared_ptr<OutputSet>> output_sets;
+    std::shared_ptr<CopyPool> copy_pool;         // helpers for large host copies, made on first use
+    bool staging_busy = false;                   // transfers to or from the pinned buffers may be in flight
     cudaStream_t side_stream = nullptr;          // capture-time fork for early output copies
     bool profile = false;
     std::vector<float> step_us;
@@ -88,7 +114,7 @@ struct Executor {
         cudaSetDevice(device);
         if (stream) cudaStreamSynchronize(stream);
         if (graph_exec) cudaGraphExecDestroy(graph_exec);
-        if (eval_graph_exec) cudaGraphExecDestroy(eval_graph_exec);
+        drop_eval_graphs();
         if (side_stream) cudaStreamDestroy(side_stream);
         for (void* p : pinned_in) if (p) cudaFreeHost(p);
         for (void* p : pinned_out) if (p) cudaFreeHost(p);
@@ -98,6 +124,11 @@ struct Executor {
         if (status_host) cudaFreeHost(status_host);
         if (stream) cudaStreamDestroy(stream);
         if (prev >= 0) cudaSetDevice(prev);
+    }
+
+    void drop_eval_graphs() {
+        for (cudaGraphExec_t g : eval_graphs) if (g) cudaGraphExecDestroy(g);
+        eval_graphs.clear();
     }
 
     uint8_t* device_ptr(const PlanTensor& t) const {
@@ -266,16 +297,30 @@ struct Executor {
     bool use_graph() const { return plan->opts.use_cuda_graph && !(plan->collectives > 0 && comm != nullptr && comm->world > 1); }
 
     void upload_inputs() {
+        staging_busy = true;
         for (size_t i = 0; i < pinned_in.size(); i++)
             if (bytes_in[i])
                 KN_CUDA(cudaMemcpyAsync(device_ptr(plan->inputs[i]), pinned_in[i], bytes_in[i], cudaMemcpyHostToDevice, stream));
     }
-    void download_outputs() {
-        for (size_t i = 0; i < pinned_out.size(); i++)
+    void download_outputs(const std::vector<void*>& to) {
+        staging_busy = true;
+        for (size_t i = 0; i < to.size(); i++)
             if (bytes_out[i])
-                KN_CUDA(cudaMemcpyAsync(pinned_out[i], device_ptr(plan->outputs[i]), bytes_out[i], cudaMemcpyDeviceToHost, stream));
+                KN_CUDA(cudaMemcpyAsync(to[i], device_ptr(plan->outputs[i]), bytes_out[i], cudaMemcpyDeviceToHost, stream));
         KN_CUDA(cudaMemcpyAsync(status_host, status_dev, 4, cudaMemcpyDeviceToHost, stream));
     }
+    void settle() {   // the pinned buffers are the host's again
+        if (!staging_busy) return;
+        KN_CUDA(cudaStreamSynchronize(stream));
+        staging_busy = false;
+    }
+    static size_t sum(const std::vector<size_t>& v) {
+        size_t n = 0;
+        for (size_t x : v) n += x;
+        return n;
+    }
+    // Inputs too large for the upload kernel are uploaded as they are staged, in front of the graph.
+    bool upload_in_graph() const { return sum(bytes_in) <= kKernelTransferBytes && pinned_in.size() <= (size_t)kMaxHostCopies; }
     void check_status() {
         if (*status_host != 0) {
             uint32_t code = *status_host;
@@ -285,11 +330,11 @@ struct Executor {
         }
     }
 
-    // One graph for a whole `evaluate`: input copies, the steps, output copies.  An output that is complete
-    // before the last step (the large policy tensor of a two-headed network, say) starts its way back to
-    // the host on a forked branch right after the step that produces it, so the copy overlaps the rest
-    // of the step list instead of following it.
-    void capture_evaluate() {
+    // One graph for a whole `evaluate`: small inputs up, the steps, outputs down into `to`.  A large output that is
+    // complete before the last step (the policy tensor of a two-headed network, say) starts its way back to the host on
+    // a forked branch right after the step that produces it, so the copy overlaps the rest of the step list instead
+    // of following it.  Small ones, and the status word, share one kernel at the end (host_copy.cu).
+    cudaGraphExec_t capture_evaluate(const std::vector<void*>& to) {
         const size_t n_steps = plan->steps.size();
         // last step that writes each output's buffer (-1: none, e.g. an output that is an input or a constant)
         std::vector<int> producer(plan->outputs.size(), -1);
@@ -306,19 +351,42 @@ struct Executor {
             return e;
         };
         auto copy_out = [&](size_t o, cudaStream_t st) {
-            if (bytes_out[o])
-                KN_CUDA(cudaMemcpyAsync(pinned_out[o], device_ptr(plan->outputs[o]), bytes_out[o], cudaMemcpyDeviceToHost, st));
+            KN_CUDA(cudaMemcpyAsync(to[o], device_ptr(plan->outputs[o]), bytes_out[o], cudaMemcpyDeviceToHost, st));
+        };
+        HostCopyParams up{}, down{};
+        if (upload_in_graph())
+            for (size_t i = 0; i < pinned_in.size(); i++)
+                if (bytes_in[i]) {
+                    up.src[up.n] = pinned_in[i];
+                    up.dst[up.n] = device_ptr(plan->inputs[i]);
+                    up.bytes[up.n++] = (int64_t)bytes_in[i];
+                }
+        down.src[0] = status_dev;
+        down.dst[0] = status_host;
+        down.bytes[0] = 4;
+        down.n = 1;
+        std::vector<uint8_t> by_kernel(to.size(), 0);
+        for (size_t o = 0; o < to.size(); o++)
+            if (bytes_out[o] && bytes_out[o] <= kKernelTransferBytes && down.n < kMaxHostCopies) {
+                by_kernel[o] = 1;
+                down.src[down.n] = device_ptr(plan->outputs[o]);
+                down.dst[down.n] = to[o];
+                down.bytes[down.n++] = (int64_t)bytes_out[o];
+            }
+        auto launch_copies = [&](const HostCopyParams& c) {
+            int err = c.n ? launch_host_copy(c, stream) : 0;
+            if (err != 0) fail(KN_ERR_CUDA, std::string("launch of a host copy failed: ") + cudaGetErrorString((cudaError_t)err));
         };
         cudaGraph_t graph = nullptr;
         KN_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
-            upload_inputs();
+            launch_copies(up);
             bool forked = false;
             for (size_t i = 0; i < n_steps; i++) {
                 launch_step(plan->steps[i]);
                 if (i + 1 == n_steps) break;
                 for (size_t o = 0; o < producer.size(); o++) {
-                    if (producer[o] != (int)i || bytes_out[o] == 0) continue;
+                    if (producer[o] != (int)i || bytes_out[o] == 0 || by_kernel[o]) continue;
                     cudaEvent_t e = new_event();
                     KN_CUDA(cudaEventRecord(e, stream));
                     KN_CUDA(cudaStreamWaitEvent(side_stream, e, 0));
@@ -326,9 +394,9 @@ struct Executor {
                     forked = true;
                 }
             }
+            launch_copies(down);
             for (size_t o = 0; o < producer.size(); o++)
-                if (n_steps == 0 || producer[o] < 0 || producer[o] == (int)n_steps - 1) copy_out(o, stream);
-            KN_CUDA(cudaMemcpyAsync(status_host, status_dev, 4, cudaMemcpyDeviceToHost, stream));
+                if (bytes_out[o] && !by_kernel[o] && (n_steps == 0 || producer[o] < 0 || producer[o] == (int)n_steps - 1)) copy_out(o, stream);
             if (forked) {
                 cudaEvent_t e = new_event();
                 KN_CUDA(cudaEventRecord(e, side_stream));
@@ -343,33 +411,94 @@ struct Executor {
         cudaError_t end = cudaStreamEndCapture(stream, &graph);
         for (cudaEvent_t e : events) cudaEventDestroy(e);
         KN_CUDA(end);
-        cudaError_t err = cudaGraphInstantiate(&eval_graph_exec, graph, 0);
+        cudaGraphExec_t exec = nullptr;
+        cudaError_t err = cudaGraphInstantiate(&exec, graph, 0);
         cudaGraphDestroy(graph);
         KN_CUDA(err);
+        return exec;
     }
 
+    // A set of result buffers nobody holds, or null: outputs too small for it to pay, or the executor's sets all held.
+    std::shared_ptr<OutputSet> acquire_outputs() {
+        const size_t bytes = sum(bytes_out);
+        if (bytes < kMinOutputSetBytes) return nullptr;
+        for (auto& s : output_sets)
+            if (s.use_count() == 1) {
+                std::atomic_thread_fence(std::memory_order_acquire);   // the last holder's reads are over
+                return s;
+            }
+        if (output_sets.size() >= kMaxOutputSets || (output_sets.size() >= 2 && (output_sets.size() + 1) * bytes > kMaxOutputSetBytes)) return nullptr;
+        auto set = std::make_shared<OutputSet>();
+        for (size_t n : bytes_out) {
+            void* p = nullptr;
+            if (cudaHostAlloc(&p, std::max<size_t>(n, 16), cudaHostAllocDefault) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            set->ptr.push_back(p);
+        }
+        output_sets.push_back(set);
+        return set;
+    }
+    // The pinned buffers an evaluation with these output pointers downloads into: 0 the staging, 1 + i output set i
+    size_t destination_of(void* const* outputs) const {
+        if (outputs == nullptr || pinned_out.empty()) return 0;
+        for (size_t i = 0; i < output_sets.size(); i++)
+            if (std::equal(output_sets[i]->ptr.begin(), output_sets[i]->ptr.end(), outputs)) return 1 + i;
+        return 0;
+    }
+    const std::vector<void*>& destination(size_t d) const { return d == 0 ? pinned_out : output_sets[d - 1]->ptr; }
+
     void evaluate(const void* const* inputs, void* const* outputs) {
-        evaluate_begin(inputs);
+        evaluate_begin(inputs, destination_of(outputs));
         evaluate_end(outputs);
     }
 
     bool in_flight = false;   // evaluate_begin without its evaluate_end
+    size_t target = 0;        // where that evaluation downloads to (destination_of)
 
-    void evaluate_begin(const void* const* inputs) {
+    // Host copy `dst` <- `src`, large ones shared out over helper threads
+    void copy_host(void* dst, const void* src, size_t bytes, const std::function<void(size_t, size_t)>& ready = nullptr) {
+        if (bytes < kParallelCopyBytes) {
+            memcpy(dst, src, bytes);
+            if (ready) ready(0, bytes);
+            return;
+        }
+        if (!copy_pool) copy_pool = CopyPool::shared();
+        copy_pool->copy(dst, src, bytes, ready);
+    }
+
+    void evaluate_begin(const void* const* inputs, size_t to = 0) {
         KN_CHECK(!in_flight, KN_ERR_INVALID_ARG, "evaluate_begin while an evaluation is in flight");
-        KN_CUDA(cudaStreamSynchronize(stream));
-        for (size_t i = 0; i < pinned_in.size(); i++) {
+        for (size_t i = 0; i < pinned_in.size(); i++)
             KN_CHECK(inputs != nullptr && (inputs[i] != nullptr || bytes_in[i] == 0), KN_ERR_INVALID_ARG, "null input buffer");
-            if (bytes_in[i] && inputs[i] != pinned_in[i]) memcpy(pinned_in[i], inputs[i], bytes_in[i]);
+        settle();
+        staging_busy = true;
+        const bool graph = use_graph() && !profile;
+        const bool later = graph && upload_in_graph();   // the graph's first node uploads
+        for (size_t i = 0; i < pinned_in.size(); i++) {
+            if (!bytes_in[i]) continue;
+            uint8_t* dev = device_ptr(plan->inputs[i]);
+            auto upload = [&](size_t from, size_t until) {
+                KN_CUDA(cudaMemcpyAsync(dev + from, (uint8_t*)pinned_in[i] + from, until - from, cudaMemcpyHostToDevice, stream));
+            };
+            if (inputs[i] == pinned_in[i]) {
+                if (!later) upload(0, bytes_in[i]);
+            } else if (later) {
+                memcpy(pinned_in[i], inputs[i], bytes_in[i]);
+            } else {
+                copy_host(pinned_in[i], inputs[i], bytes_in[i], upload);
+            }
         }
-        if (use_graph() && !profile) {
-            if (!eval_graph_exec) capture_evaluate();
-            KN_CUDA(cudaGraphLaunch(eval_graph_exec, stream));
+        if (graph) {
+            if (eval_graphs.size() <= to) eval_graphs.resize(to + 1, nullptr);
+            if (!eval_graphs[to]) eval_graphs[to] = capture_evaluate(destination(to));
+            KN_CUDA(cudaGraphLaunch(eval_graphs[to], stream));
         } else {
-            upload_inputs();
             run_async();
-            download_outputs();
+            download_outputs(destination(to));
         }
+        target = to;
         in_flight = true;
     }
 
@@ -385,15 +514,17 @@ struct Executor {
             }
             KN_CUDA(done);
         }
+        staging_busy = false;
         check_status();
-        for (size_t i = 0; i < pinned_out.size(); i++) {
+        const std::vector<void*>& from = destination(target);
+        for (size_t i = 0; i < from.size(); i++) {
             KN_CHECK(outputs != nullptr && (outputs[i] != nullptr || bytes_out[i] == 0), KN_ERR_INVALID_ARG, "null output buffer");
             if (dtype_out[i] == DType::Bool) {
-                const uint8_t* b = (const uint8_t*)pinned_out[i];
+                const uint8_t* b = (const uint8_t*)from[i];
                 for (size_t k = 0; k < bytes_out[i]; k++)
                     KN_CHECK(b[k] <= 1, KN_ERR_INTERNAL, "bool output holds a value other than 0 or 1");
             }
-            if (bytes_out[i] && outputs[i] != pinned_out[i]) memcpy(outputs[i], pinned_out[i], bytes_out[i]);
+            if (bytes_out[i] && outputs[i] != from[i]) copy_host(outputs[i], from[i], bytes_out[i]);
         }
     }
 };
@@ -462,6 +593,9 @@ struct kn_graph {
 };
 struct kn_executor {
     std::unique_ptr<kn::Executor> e;
+};
+struct kn_outputs {
+    std::shared_ptr<kn::OutputSet> set;
 };
 struct kn_comm {
     kn::Comm* c = nullptr;
@@ -614,6 +748,22 @@ int kn_executor_evaluate(kn_executor* exec, const void* const* inputs, void* con
     });
 }
 
+int kn_executor_outputs_acquire(kn_executor* exec, void** outputs, kn_outputs** set) {
+    return guarded([&] {
+        KN_CHECK(exec != nullptr && set != nullptr, KN_ERR_INVALID_ARG, "null argument");
+        *set = nullptr;
+        KN_CHECK(!exec->e->in_flight, KN_ERR_INVALID_ARG, "an evaluation is in flight");
+        kn::DeviceGuard guard(exec->e->device);
+        auto s = exec->e->acquire_outputs();
+        if (!s) return;
+        KN_CHECK(outputs != nullptr, KN_ERR_INVALID_ARG, "null outputs");
+        std::copy(s->ptr.begin(), s->ptr.end(), outputs);
+        *set = new kn_outputs{std::move(s)};
+    });
+}
+
+void kn_outputs_release(kn_outputs* set) { delete set; }
+
 int kn_executor_evaluate_begin(kn_executor* exec, const void* const* inputs) {
     return guarded([&] {
         KN_CHECK(exec != nullptr, KN_ERR_INVALID_ARG, "null executor");
@@ -683,7 +833,7 @@ int kn_executor_download_outputs(kn_executor* exec) {
     return guarded([&] {
         KN_CHECK(exec != nullptr, KN_ERR_INVALID_ARG, "null executor");
         kn::DeviceGuard guard(exec->e->device);
-        exec->e->download_outputs();
+        exec->e->download_outputs(exec->e->pinned_out);
     });
 }
 
@@ -797,7 +947,7 @@ int kn_executor_set_comm(kn_executor* exec, kn_comm* comm) {
         KN_CUDA(cudaStreamSynchronize(e.stream));
         // graphs captured under the previous setting would replay the wrong kind of step
         if (e.graph_exec) { cudaGraphExecDestroy(e.graph_exec); e.graph_exec = nullptr; }
-        if (e.eval_graph_exec) { cudaGraphExecDestroy(e.eval_graph_exec); e.eval_graph_exec = nullptr; }
+        e.drop_eval_graphs();
         e.comm = comm ? comm->c : nullptr;
     });
 }

@@ -1,0 +1,123 @@
+// One core copies 18 GB/s into pinned memory, a third of what the link to the GPU takes: a 1.4 MB batch of boards was
+// 75 us on the caller's thread before its 35 us upload could start.  Four threads and an upload per finished range
+// bring the two to about 45 us together.
+#include "host_copy.h"
+
+#include <algorithm>
+#include <atomic>
+#include <condition_variable>
+#include <cstdint>
+#include <cstring>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace kn {
+
+namespace {
+
+constexpr int kHelpers = 3;
+constexpr size_t kChunk = 128 << 10;   // 7 us of one core: small enough to share out 1 MB, large against a wake
+
+class Pool : public CopyPool {
+   public:
+    ~Pool() override {
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            stop_ = true;
+        }
+        wake_.notify_all();
+        for (auto& t : threads_) t.join();
+    }
+
+    void copy(void* dst, const void* src, size_t bytes, const std::function<void(size_t, size_t)>& ready) override {
+        const size_t chunks = (bytes + kChunk - 1) / kChunk;
+        std::unique_lock<std::mutex> mine(user_, std::try_to_lock);
+        if (!mine.owns_lock() || bytes < kParallelCopyBytes) {
+            for (size_t c = 0; c < chunks; c++) {
+                const size_t from = c * kChunk, to = std::min(bytes, from + kChunk);
+                memcpy((uint8_t*)dst + from, (const uint8_t*)src + from, to - from);
+                if (ready) ready(from, to);
+            }
+            return;
+        }
+        auto job = std::make_shared<Job>(dst, src, bytes, chunks);
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            if (threads_.empty())
+                for (int i = 0; i < kHelpers; i++) threads_.emplace_back([this] { help(); });
+            job_ = job;
+            generation_++;
+        }
+        wake_.notify_all();
+        size_t done = 0;
+        auto advance = [&] {
+            size_t upto = done;
+            while (upto < chunks && job->complete[upto].load(std::memory_order_acquire)) upto++;
+            if (upto == done) return;
+            if (ready) ready(done * kChunk, std::min(bytes, upto * kChunk));
+            done = upto;
+        };
+        while (job->one()) advance();
+        while (done < chunks) {   // what the helpers still have in hand: a few microseconds
+            advance();
+            if (done < chunks) std::this_thread::yield();
+        }
+    }
+
+   private:
+    struct Job {
+        uint8_t* dst;
+        const uint8_t* src;
+        size_t bytes, chunks;
+        std::atomic<size_t> next{0};
+        std::vector<std::atomic<uint8_t>> complete;
+        Job(void* d, const void* s, size_t b, size_t c) : dst((uint8_t*)d), src((const uint8_t*)s), bytes(b), chunks(c), complete(c) {}
+        bool one() {
+            const size_t c = next.fetch_add(1, std::memory_order_relaxed);
+            if (c >= chunks) return false;
+            const size_t from = c * kChunk;
+            memcpy(dst + from, src + from, std::min(bytes, from + kChunk) - from);
+            complete[c].store(1, std::memory_order_release);
+            return true;
+        }
+    };
+
+    void help() {
+        uint64_t seen = 0;
+        for (;;) {
+            std::shared_ptr<Job> job;
+            {
+                std::unique_lock<std::mutex> lock(mu_);
+                wake_.wait(lock, [&] { return stop_ || generation_ != seen; });
+                if (stop_) return;
+                seen = generation_;
+                job = job_;
+            }
+            // (a job that is over hands out no more chunks: its buffers are not touched by a helper that wakes late)
+            while (job->one()) {
+            }
+        }
+    }
+
+    std::mutex user_;   // held by the caller whose job the helpers work on
+    std::mutex mu_;
+    std::condition_variable wake_;
+    std::vector<std::thread> threads_;
+    std::shared_ptr<Job> job_;
+    uint64_t generation_ = 0;
+    bool stop_ = false;
+};
+
+}  // namespace
+
+std::shared_ptr<CopyPool> CopyPool::shared() {
+    static std::mutex mu;
+    static std::weak_ptr<CopyPool> existing;
+    std::lock_guard<std::mutex> lock(mu);
+    std::shared_ptr<CopyPool> p = existing.lock();
+    if (!p) existing = p = std::make_shared<Pool>();
+    return p;
+}
+
+}  // namespace kn

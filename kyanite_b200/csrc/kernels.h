@@ -233,6 +233,15 @@ struct AllReduceParams {
     uint8_t dtype;     // DType: F32 or F16
 };
 
+// ---- small transfers between device memory and pinned host memory (kernels/host_copy.cu)
+constexpr int kMaxHostCopies = 8;
+struct HostCopyParams {
+    int32_t n;
+    const void* src[kMaxHostCopies];
+    void* dst[kMaxHostCopies];
+    int64_t bytes[kMaxHostCopies];
+};
+
 // All launchers enqueue on `stream` and return the cudaError_t of the launch as int.
 int launch_scalar(const ScalarParams& p, cudaStream_t stream);
 int launch_reduce(const ReduceParams& p, cudaStream_t stream);
@@ -245,5 +254,6 @@ int launch_gather(const GatherParams& p, cudaStream_t stream);
 int launch_im2col(const Im2colParams& p, cudaStream_t stream);
 int launch_gemm_simt(const GemmParams& p, cudaStream_t stream);
 int launch_conv_simt(const ConvParams& p, cudaStream_t stream);
+int launch_host_copy(const HostCopyParams& p, cudaStream_t stream);
 
 }  // namespace kn

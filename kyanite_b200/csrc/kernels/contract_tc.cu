@@ -779,7 +779,7 @@ static bool prepare_conv_channels_last(const ConvParams& c, uint32_t* status_wor
         return ((uintptr_t)ptr & 15) == 0 && st[1] == 1 && tma_stride_ok_host(c.ow, st[3]) && tma_stride_ok_host(c.oh, st[2]) &&
                tma_stride_ok_host(c.n, st[0]);
     };
-    auto per_channel = [&](const int64_t* st) { return st[0] == 0 && st[2] == 0 && st[3] == 0; };
+    auto per_channel = [&](const int64_t* st) { return (st[0] == 0 || c.n == 1) && (st[2] == 0 || c.oh == 1) && (st[3] == 0 || c.ow == 1); };
     const float* bias = nullptr;
     const float* res = nullptr;
     const int64_t* res_strides = nullptr;

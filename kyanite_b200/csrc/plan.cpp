@@ -1977,11 +1977,18 @@ class Planner {
         return g;
     }
 
+    // A tile of the tensor-core kernels is 128 output positions.  With fewer than that a part of it is idle, which still
+    // beats the exact-f32 kernel (one board of 8 x 8 positions, 128 -> 128 channels: 9 us a layer in a chain against 320)
+    // unless the whole convolution is a few hundred thousand multiply-adds, where either is a launch and little more.
+    static bool conv_worth_tensor_core(const std::vector<int64_t>& out, const std::vector<int64_t>& filter) {
+        const int64_t positions = out[0] * out[2] * out[3];
+        return positions >= 128 || (positions >= 32 && positions * out[1] * filter[1] * filter[2] * filter[3] >= 200000);
+    }
+
     bool conv_fits_tensor_core(const ValueInfo& ci, const PlanTensor& x, const PlanTensor& w, const std::vector<int64_t>& out) const {
         if (ci.stride_y != 1 || ci.stride_x != 1) return false;
         if (x.ss.rank() != 4 || w.ss.rank() != 4) return false;
-        const int64_t positions = out[0] * out[2] * out[3];
-        if (positions < 128 || out[1] < 4 || x.ss.shape[1] < 1) return false;
+        if (!conv_worth_tensor_core(out, w.ss.shape) || out[1] < 4 || x.ss.shape[1] < 1) return false;
         if (out[2] > 32768 || out[3] > 32768 || out[0] > (1 << 24) || w.ss.shape[2] * w.ss.shape[3] > 1024) return false;
         return true;
     }
@@ -1991,7 +1998,7 @@ class Planner {
         if (ci.op != OpKind::Conv || ci.inputs[0] != input || ci.dtype != DType::F32) return false;
         if (ci.stride_y != 1 || ci.stride_x != 1) return false;
         std::vector<int64_t> o = shape_of(conv);
-        return o[0] * o[2] * o[3] >= 128 && o[1] >= 4;
+        return conv_worth_tensor_core(o, shape_of(ci.inputs[1])) && o[1] >= 4;
     }
     bool feeds_tensor_core_conv(int v) {
         for (int u : users_[v])
@@ -2271,6 +2278,13 @@ class Planner {
             if (o != 1 || stored) s.alg_bytes += touched_bytes(s.operands[o]);
     }
 
+    // one value per channel, whatever the image and position (the stride of an axis of one entry says nothing)
+    static bool per_channel(const PlanTensor& t) {
+        for (int d : {0, 2, 3})
+            if (t.ss.shape[d] != 1 && t.ss.strides[d] != 0) return false;
+        return true;
+    }
+
     bool chain_candidate(const Step& s, ChainLayer& l) const {
         if (s.kind != StepKind::Conv || !s.tensor_core) return false;
         const ConvParams& c = s.conv;
@@ -2289,8 +2303,7 @@ class Planner {
         for (size_t o = 3; o < s.operands.size(); o++) {
             const PlanTensor& a = s.operands[o];
             const BufferInfo& ab = plan_.buffers[a.buf];
-            const auto& st = a.ss.strides;
-            if (st[0] == 0 && st[2] == 0 && st[3] == 0 && ab.kind == BufKind::Const && ab.host_data != nullptr && l.bias_operand < 0)
+            if (per_channel(a) && ab.kind == BufKind::Const && ab.host_data != nullptr && l.bias_operand < 0)
                 l.bias_operand = (int)o;
             else if (l.res_operand < 0)
                 l.res_operand = (int)o;
@@ -2315,8 +2328,7 @@ class Planner {
         if (s.operands.size() == 4) {
             const PlanTensor& a = s.operands[3];
             const BufferInfo& ab = plan_.buffers[a.buf];
-            const auto& st = a.ss.strides;
-            if (!(st[0] == 0 && st[2] == 0 && st[3] == 0 && ab.kind == BufKind::Const && ab.host_data != nullptr)) return false;
+            if (!(per_channel(a) && ab.kind == BufKind::Const && ab.host_data != nullptr)) return false;
             bias_operand = 3;
         }
         return true;

@@ -39,7 +39,10 @@ struct PlanTensor {
     PlanTensor slice(int axis, int64_t start, int64_t end, int64_t step) const;
     PlanTensor flip(int axis) const;
     bool same_storage(const PlanTensor& o) const {
-        return buf == o.buf && offset == o.offset && dtype == o.dtype && ss == o.ss;
+        if (buf != o.buf || offset != o.offset || dtype != o.dtype || ss.shape != o.ss.shape) return false;
+        for (size_t d = 0; d < ss.shape.size(); d++)   // (the stride of an axis of one entry says nothing)
+            if (ss.shape[d] != 1 && ss.strides[d] != o.ss.strides[d]) return false;
+        return true;
     }
     std::string str() const;
 };

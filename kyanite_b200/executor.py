@@ -32,6 +32,11 @@ FLAG_NO_CONV_CHAIN = _lib.KN_FLAG_NO_CONV_CHAIN
 FLAG_NO_PERSISTENT_GEMM = _lib.KN_FLAG_NO_PERSISTENT_GEMM
 
 
+# results smaller than this in all are copied into ordinary arrays: handing pinned memory out costs more than the copy
+# (the library refuses below 64 KB too)
+_HAND_OUT_BYTES = 64 << 10
+
+
 class CudaDeviceNotAvailable(RuntimeError):
     pass
 
@@ -164,6 +169,18 @@ class Communicator:
             pass
 
 
+class _HeldOutputs:
+    """A set of pinned result buffers (kn_executor_outputs_acquire): goes back to its executor when the last array that
+    views it is gone."""
+    __slots__ = ("_release", "_set")
+
+    def __init__(self, lib, handle: int):
+        self._release, self._set = lib.kn_outputs_release, handle
+
+    def __del__(self):
+        self._release(self._set)
+
+
 class CudaExecutor:
     def __init__(self, device, graph, batch_size: int, math_mode: Optional[int] = None,
                  use_cuda_graph: Optional[bool] = None, flags: int = 0):
@@ -187,6 +204,14 @@ class CudaExecutor:
         self._out_info = [self._io_info(1, i) for i in range(n_out.value)]
         self.host_inputs = [self._host_array(0, i) for i in range(n_in.value)]
         self.host_outputs = [self._host_array(1, i) for i in range(n_out.value)]
+        # what `evaluate` needs per call, looked up once: a small network's call is 10 us of GPU, so every microsecond
+        # of Python counts
+        self._in_spec = [(s, np.dtype(d.np)) for s, d, _ in self._in_info]
+        self._out_spec = [(s, np.dtype(d.np)) for s, d, _ in self._out_info]
+        self._in_ptrs_type = c_void_p * max(1, n_in.value)
+        self._out_ptrs_type = c_void_p * max(1, n_out.value)
+        self._out_bytes_types = [ctypes.c_uint8 * n for _, _, n in self._out_info]
+        self._hand_out = sum(n for _, _, n in self._out_info) >= _HAND_OUT_BYTES
 
     # ---------------------------------------------------------------- info
     def _io_info(self, is_output: int, index: int):
@@ -236,22 +261,40 @@ class CudaExecutor:
 
     # ---------------------------------------------------------------- running
     def evaluate(self, inputs: Sequence[np.ndarray]) -> List[np.ndarray]:
-        """Copies inputs to the device, runs the graph, returns fresh host arrays."""
-        if len(inputs) != len(self._in_info):
-            raise ValueError(f"Wrong input count, expected {len(self._in_info)} but got {len(inputs)}")
+        """Copies inputs to the device, runs the graph, returns fresh host arrays.  Large results are views of pinned
+        memory that the download went to directly; it is theirs as long as any of them lives."""
+        if len(inputs) != len(self._in_spec):
+            raise ValueError(f"Wrong input count, expected {len(self._in_spec)} but got {len(inputs)}")
         arrays = []
-        for i, (x, (shape, dtype, _)) in enumerate(zip(inputs, self._in_info)):
-            x = np.asarray(x)
-            if tuple(x.shape) != shape:
+        for i, (shape, dtype) in enumerate(self._in_spec):
+            x = inputs[i]
+            if type(x) is not np.ndarray:
+                x = np.asarray(x)
+            if x.shape != shape:
                 raise ValueError(f"Wrong shape for input {i}: expected {shape}, got {tuple(x.shape)}")
-            if x.dtype != dtype.np:
-                raise ValueError(f"Wrong dtype for input {i}: expected {dtype.np}, got {x.dtype}")
+            if x.dtype != dtype:
+                raise ValueError(f"Wrong dtype for input {i}: expected {dtype}, got {x.dtype}")
             if not x.flags.c_contiguous:
                 x = x.copy(order="C")   # `as_standard_layout` (executor.rs:135)
             arrays.append(x)
-        outs = [np.empty(shape, dtype=dtype.np) for shape, dtype, _ in self._out_info]
-        in_ptrs = (c_void_p * max(1, len(arrays)))(*[a.ctypes.data for a in arrays])
-        out_ptrs = (c_void_p * max(1, len(outs)))(*[o.ctypes.data for o in outs])
+        in_ptrs = self._in_ptrs_type(*[a.__array_interface__["data"][0] for a in arrays])
+        if self._hand_out:
+            out_ptrs, handle = self._out_ptrs_type(), c_void_p()
+            check(self._lib.kn_executor_outputs_acquire(self._ptr, out_ptrs, byref(handle)))
+            if handle.value:
+                held = _HeldOutputs(self._lib, handle.value)
+                check(self._lib.kn_executor_evaluate(self._ptr, in_ptrs, out_ptrs))
+                outs = []
+                for (shape, dtype), raw_type, ptr in zip(self._out_spec, self._out_bytes_types, out_ptrs):
+                    if raw_type._length_ == 0:
+                        outs.append(np.empty(shape, dtype=dtype))
+                        continue
+                    raw = raw_type.from_address(ptr)
+                    raw.held = held         # the array views `raw`, which keeps the set
+                    outs.append(np.frombuffer(raw, dtype=dtype).reshape(shape))
+                return outs
+        outs = [np.empty(shape, dtype=dtype) for shape, dtype in self._out_spec]
+        out_ptrs = self._out_ptrs_type(*[o.__array_interface__["data"][0] for o in outs])
         check(self._lib.kn_executor_evaluate(self._ptr, in_ptrs, out_ptrs))
         return outs
 

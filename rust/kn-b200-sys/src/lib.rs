@@ -66,6 +66,10 @@ pub struct kn_executor {
 pub struct kn_comm {
     _private: [u8; 0],
 }
+#[repr(C)]
+pub struct kn_outputs {
+    _private: [u8; 0],
+}
 
 extern "C" {
     pub fn kn_last_error() -> *const c_char;
@@ -86,6 +90,8 @@ extern "C" {
     pub fn kn_executor_io_info(exec: *const kn_executor, is_output: c_int, index: c_int, info: *mut kn_tensor_info) -> c_int;
 
     pub fn kn_executor_evaluate(exec: *mut kn_executor, inputs: *const *const c_void, outputs: *const *mut c_void) -> c_int;
+    pub fn kn_executor_outputs_acquire(exec: *mut kn_executor, outputs: *mut *mut c_void, set: *mut *mut kn_outputs) -> c_int;
+    pub fn kn_outputs_release(set: *mut kn_outputs);
     pub fn kn_executor_evaluate_begin(exec: *mut kn_executor, inputs: *const *const c_void) -> c_int;
     pub fn kn_executor_evaluate_end(exec: *mut kn_executor, outputs: *const *mut c_void) -> c_int;
     pub fn kn_executor_run_async(exec: *mut kn_executor) -> c_int;
