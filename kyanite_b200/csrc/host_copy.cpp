@@ -12,12 +12,41 @@
 #include <thread>
 #include <vector>
 
+#ifdef __SSE2__
+#include <emmintrin.h>
+#endif
+
 namespace kn {
 
 namespace {
 
+// memcpy whose stores bypass the caches.  The helpers' part of a staging buffer would otherwise sit modified in the
+// caches of cores that go to sleep right after, and the GPU's read of it took four times as long (1.4 MB: 140 us
+// against 35).
+void copy_past_caches(uint8_t* dst, const uint8_t* src, size_t bytes) {
+#ifdef __SSE2__
+    size_t i = 0;
+    if (((uintptr_t)dst & 15) == 0) {
+        for (; i + 64 <= bytes; i += 64) {
+            const __m128i a = _mm_loadu_si128((const __m128i*)(src + i)), b = _mm_loadu_si128((const __m128i*)(src + i + 16));
+            const __m128i c = _mm_loadu_si128((const __m128i*)(src + i + 32)), d = _mm_loadu_si128((const __m128i*)(src + i + 48));
+            _mm_stream_si128((__m128i*)(dst + i), a);
+            _mm_stream_si128((__m128i*)(dst + i + 16), b);
+            _mm_stream_si128((__m128i*)(dst + i + 32), c);
+            _mm_stream_si128((__m128i*)(dst + i + 48), d);
+        }
+        _mm_sfence();
+    }
+    memcpy(dst + i, src + i, bytes - i);
+#else
+    memcpy(dst, src, bytes);
+#endif
+}
+
 constexpr int kHelpers = 3;
 constexpr size_t kChunk = 128 << 10;   // 7 us of one core: small enough to share out 1 MB, large against a wake
+
+constexpr size_t kReadyBytes = 512 << 10;   // least range handed on before the end: an upload costs some 4 us on its own
 
 class Pool : public CopyPool {
    public:
@@ -54,7 +83,7 @@ class Pool : public CopyPool {
         auto advance = [&] {
             size_t upto = done;
             while (upto < chunks && job->complete[upto].load(std::memory_order_acquire)) upto++;
-            if (upto == done) return;
+            if (upto == done || (upto < chunks && (upto - done) * kChunk < kReadyBytes)) return;
             if (ready) ready(done * kChunk, std::min(bytes, upto * kChunk));
             done = upto;
         };
@@ -77,7 +106,7 @@ class Pool : public CopyPool {
             const size_t c = next.fetch_add(1, std::memory_order_relaxed);
             if (c >= chunks) return false;
             const size_t from = c * kChunk;
-            memcpy(dst + from, src + from, std::min(bytes, from + kChunk) - from);
+            copy_past_caches(dst + from, src + from, std::min(bytes, from + kChunk) - from);
             complete[c].store(1, std::memory_order_release);
             return true;
         }

@@ -7,8 +7,11 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
-#include "../kernels.h"
+#include <initializer_list>
+#include <mutex>
 #include <utility>
+
+#include "../kernels.h"
 
 #include "epilogue.cuh"
 #include "launch.cuh"
@@ -16,8 +19,6 @@
 namespace kn {
 
 namespace {
-
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 
 __device__ __forceinline__ float apply_epilogue(float v, int act, int round_tf32) {
     v = apply_activation(v, act);
@@ -29,19 +30,36 @@ __device__ __forceinline__ float apply_epilogue(float v, int act, int round_tf32
     return v;
 }
 
+// ---------------------------------------------------------------- problems
+// A problem tells the kernel where its operands are.  The reduction runs over `taps()` taps of `inner()` elements each
+// (a matmul: one tap of k; a convolution: one tap per filter position, over the channels), so that inside a tap an
+// operand is a pointer and a stride.  A `Tap` is what all rows and columns share about the current one.
+
+struct OneTap {};
+
 struct GemmProblem {
     GemmParams p;
-    __device__ int64_t M() const { return p.m; }
-    __device__ int64_t N() const { return p.n; }
-    __device__ int64_t K() const { return p.k; }
-    __device__ bool a_k_fast() const { return p.sa[2] == 1; }
-    __device__ bool b_k_fast() const { return p.sb[1] == 1; }
-    __device__ float load_a(int64_t b, int64_t m, int64_t k) const { return p.a[b * p.sa[0] + m * p.sa[1] + k * p.sa[2]]; }
-    __device__ float load_b(int64_t b, int64_t k, int64_t n) const { return p.b[b * p.sb[0] + k * p.sb[1] + n * p.sb[2]]; }
-    __device__ void store(int64_t b, int64_t m, int64_t n, float acc) const {
-        if (p.add1) acc += p.add1[b * p.s1[0] + m * p.s1[1] + n * p.s1[2]];
-        if (p.add2) acc += p.add2[b * p.s2[0] + m * p.s2[1] + n * p.s2[2]];
-        p.c[b * p.sc[0] + m * p.sc[1] + n * p.sc[2]] = apply_epilogue(acc, p.act, p.round_tf32);
+    using Element = float;
+    using Tap = OneTap;
+    __device__ int taps() const { return 1; }
+    __device__ Tap tap(int) const { return Tap{}; }
+    __device__ void next(Tap&) const {}
+    __device__ int64_t inner() const { return p.k; }
+    __device__ int64_t rows() const { return p.m; }
+    __device__ int64_t cols() const { return p.n; }
+    struct Row { const float* at; };
+    __device__ Row row(int64_t b, int64_t m) const { return Row{p.a + b * p.sa[0] + m * p.sa[1]}; }
+    __device__ const float* a_at(const Row& r, const Tap&) const { return r.at; }
+    __device__ int64_t a_stride() const { return p.sa[2]; }
+    __device__ const float* col(int64_t b, int64_t n) const { return p.b + b * p.sb[0] + n * p.sb[2]; }
+    __device__ const float* b_at(const float* col, const Tap&) const { return col; }
+    __device__ int64_t b_stride() const { return p.sb[1]; }
+    struct Out { int64_t b, m; };
+    __device__ Out out(int64_t b, int64_t m) const { return Out{b, m}; }
+    __device__ void store(const Out& o, int64_t n, float acc) const {
+        if (p.add1) acc += p.add1[o.b * p.s1[0] + o.m * p.s1[1] + n * p.s1[2]];
+        if (p.add2) acc += p.add2[o.b * p.s2[0] + o.m * p.s2[1] + n * p.s2[2]];
+        p.c[o.b * p.sc[0] + o.m * p.sc[1] + n * p.sc[2]] = apply_epilogue(acc, p.act, p.round_tf32);
     }
 };
 
@@ -49,133 +67,400 @@ struct GemmProblem {
 // the result is rounded to f16 once.
 struct GemmProblemHalf {
     GemmParams p;
-    __device__ int64_t M() const { return p.m; }
-    __device__ int64_t N() const { return p.n; }
-    __device__ int64_t K() const { return p.k; }
-    __device__ bool a_k_fast() const { return p.sa[2] == 1; }
-    __device__ bool b_k_fast() const { return p.sb[1] == 1; }
-    __device__ float load_a(int64_t b, int64_t m, int64_t k) const {
-        return __half2float(((const __half*)p.a)[b * p.sa[0] + m * p.sa[1] + k * p.sa[2]]);
-    }
-    __device__ float load_b(int64_t b, int64_t k, int64_t n) const {
-        return __half2float(((const __half*)p.b)[b * p.sb[0] + k * p.sb[1] + n * p.sb[2]]);
-    }
-    __device__ void store(int64_t b, int64_t m, int64_t n, float acc) const {
-        if (p.add1) acc += __half2float(((const __half*)p.add1)[b * p.s1[0] + m * p.s1[1] + n * p.s1[2]]);
-        if (p.add2) acc += __half2float(((const __half*)p.add2)[b * p.s2[0] + m * p.s2[1] + n * p.s2[2]]);
-        ((__half*)p.c)[b * p.sc[0] + m * p.sc[1] + n * p.sc[2]] = __float2half_rn(apply_activation(acc, p.act));
+    using Element = __half;
+    using Tap = OneTap;
+    __device__ int taps() const { return 1; }
+    __device__ Tap tap(int) const { return Tap{}; }
+    __device__ void next(Tap&) const {}
+    __device__ int64_t inner() const { return p.k; }
+    __device__ int64_t rows() const { return p.m; }
+    __device__ int64_t cols() const { return p.n; }
+    struct Row { const __half* at; };
+    __device__ Row row(int64_t b, int64_t m) const { return Row{(const __half*)p.a + b * p.sa[0] + m * p.sa[1]}; }
+    __device__ const __half* a_at(const Row& r, const Tap&) const { return r.at; }
+    __device__ int64_t a_stride() const { return p.sa[2]; }
+    __device__ const __half* col(int64_t b, int64_t n) const { return (const __half*)p.b + b * p.sb[0] + n * p.sb[2]; }
+    __device__ const __half* b_at(const __half* col, const Tap&) const { return col; }
+    __device__ int64_t b_stride() const { return p.sb[1]; }
+    struct Out { int64_t b, m; };
+    __device__ Out out(int64_t b, int64_t m) const { return Out{b, m}; }
+    __device__ void store(const Out& o, int64_t n, float acc) const {
+        if (p.add1) acc += __half2float(((const __half*)p.add1)[o.b * p.s1[0] + o.m * p.s1[1] + n * p.s1[2]]);
+        if (p.add2) acc += __half2float(((const __half*)p.add2)[o.b * p.s2[0] + o.m * p.s2[1] + n * p.s2[2]]);
+        ((__half*)p.c)[o.b * p.sc[0] + o.m * p.sc[1] + n * p.sc[2]] = __float2half_rn(apply_activation(acc, p.act));
     }
 };
 
 struct ConvProblem {
     ConvParams p;
-    __device__ int64_t M() const { return (int64_t)p.n * p.oh * p.ow; }
-    __device__ int64_t N() const { return p.k; }
-    __device__ int64_t K() const { return (int64_t)p.c * p.r * p.s; }
-    __device__ bool a_k_fast() const { return false; }
-    __device__ bool b_k_fast() const { return true; }
-    __device__ float load_a(int64_t, int64_t m, int64_t kk) const {
-        const int ox = (int)(m % p.ow);
-        const int64_t t = m / p.ow;
-        const int oy = (int)(t % p.oh);
-        const int64_t img = t / p.oh;
-        const int fx = (int)(kk % p.s);
-        const int64_t u = kk / p.s;
-        const int fy = (int)(u % p.r);
-        const int64_t ci = u / p.r;
-        const int iy = oy * p.stride_y + fy - p.pad_y;
-        const int ix = ox * p.stride_x + fx - p.pad_x;
-        if (iy < 0 || iy >= p.h || ix < 0 || ix >= p.w) return 0.0f;
-        return p.in[img * p.s_in[0] + ci * p.s_in[1] + iy * p.s_in[2] + ix * p.s_in[3]];
+    using Element = float;
+    struct Tap { int fy, fx; int64_t a, b; };
+    __device__ int taps() const { return p.r * p.s; }
+    __device__ Tap tap(int t) const {
+        const int fy = t / p.s, fx = t - fy * p.s;
+        return Tap{fy, fx, fy * p.s_in[2] + fx * p.s_in[3], fy * p.s_f[2] + fx * p.s_f[3]};
     }
-    __device__ float load_b(int64_t, int64_t kk, int64_t n) const {
-        const int fx = (int)(kk % p.s);
-        const int64_t u = kk / p.s;
-        const int fy = (int)(u % p.r);
-        const int64_t ci = u / p.r;
-        return p.filter[n * p.s_f[0] + ci * p.s_f[1] + fy * p.s_f[2] + fx * p.s_f[3]];
+    __device__ void next(Tap& t) const {
+        t.fx++, t.a += p.s_in[3], t.b += p.s_f[3];
+        if (t.fx == p.s) t.fx = 0, t.fy++, t.a += p.s_in[2] - p.s * p.s_in[3], t.b += p.s_f[2] - p.s * p.s_f[3];
     }
-    __device__ void store(int64_t, int64_t m, int64_t n, float acc) const {
-        const int64_t ox = m % p.ow;
-        const int64_t t = m / p.ow;
-        const int64_t oy = t % p.oh;
-        const int64_t img = t / p.oh;
-        if (p.add1) acc += p.add1[img * p.s1[0] + n * p.s1[1] + oy * p.s1[2] + ox * p.s1[3]];
-        if (p.add2) acc += p.add2[img * p.s2[0] + n * p.s2[1] + oy * p.s2[2] + ox * p.s2[3]];
-        p.out[img * p.s_out[0] + n * p.s_out[1] + oy * p.s_out[2] + ox * p.s_out[3]] = apply_epilogue(acc, p.act, p.round_tf32);
+    __device__ int64_t inner() const { return p.c; }
+    __device__ int64_t rows() const { return (int64_t)p.n * p.oh * p.ow; }
+    __device__ int64_t cols() const { return p.k; }
+    struct Row { const float* at; int iy, ix; };   // of the window's first tap, which may lie outside the image
+    __device__ Row row(int64_t, int64_t m) const {
+        const int64_t t = m / p.ow, img = t / p.oh;
+        const int iy = (int)(t - img * p.oh) * p.stride_y - p.pad_y, ix = (int)(m - t * p.ow) * p.stride_x - p.pad_x;
+        return Row{p.in + img * p.s_in[0] + iy * p.s_in[2] + ix * p.s_in[3], iy, ix};
+    }
+    __device__ const float* a_at(const Row& r, const Tap& t) const {   // null outside the image
+        return (unsigned)(r.iy + t.fy) < (unsigned)p.h && (unsigned)(r.ix + t.fx) < (unsigned)p.w ? r.at + t.a : nullptr;
+    }
+    __device__ int64_t a_stride() const { return p.s_in[1]; }
+    __device__ const float* col(int64_t, int64_t n) const { return p.filter + n * p.s_f[0]; }
+    __device__ const float* b_at(const float* col, const Tap& t) const { return col + t.b; }
+    __device__ int64_t b_stride() const { return p.s_f[1]; }
+    struct Out { int64_t o, a1, a2; };
+    __device__ Out out(int64_t, int64_t m) const {
+        const int64_t t = m / p.ow, img = t / p.oh, ox = m - t * p.ow, oy = t - img * p.oh;
+        return Out{img * p.s_out[0] + oy * p.s_out[2] + ox * p.s_out[3], img * p.s1[0] + oy * p.s1[2] + ox * p.s1[3],
+                   img * p.s2[0] + oy * p.s2[2] + ox * p.s2[3]};
+    }
+    __device__ void store(const Out& o, int64_t n, float acc) const {
+        if (p.add1) acc += p.add1[o.a1 + n * p.s1[1]];
+        if (p.add2) acc += p.add2[o.a2 + n * p.s2[1]];
+        p.out[o.o + n * p.s_out[1]] = apply_epilogue(acc, p.act, p.round_tf32);
     }
 };
 
-template <class Problem>
-__global__ void __launch_bounds__(256) contract_simt_kernel(const __grid_constant__ Problem prob) {
+// ---------------------------------------------------------------- the kernel
+constexpr int kThreads = 256, BK = 32, kStages = 3;
+constexpr int TM = 8;            // rows per thread
+constexpr int kTilePad = 4;      // row padding of the partial result tile
+
+// Shared tiles are [row][K], K contiguous, rows padded by 16 bytes: the 128-bit reads of eight neighbouring rows then
+// cover all banks once.
+template <class E> constexpr int row_elements = BK + 16 / (int)sizeof(E);
+template <class E, int BM, int BN> constexpr int stage_bytes = (BM + BN) * row_elements<E> * (int)sizeof(E);
+template <int BM, int BN, int KG> constexpr int tile_bytes = KG * BM * (BN + kTilePad) * 4;
+template <class E, int BM, int BN, int KG>
+constexpr int smem_bytes = kStages * stage_bytes<E, BM, BN> > tile_bytes<BM, BN, KG> ? kStages * stage_bytes<E, BM, BN> : tile_bytes<BM, BN, KG>;
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// `bytes` (0 .. 16) bytes of global memory, zeros up to 16
+__device__ __forceinline__ void fetch16(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// one element, or a zero (`src` is a valid address either way)
+__device__ __forceinline__ void fetch1(float* dst, const float* src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void fetch1(__half* dst, const __half* src, bool in) { *dst = in ? *src : __float2half_rn(0.f); }
+
+// four K elements of a row
+__device__ __forceinline__ float4 read4(const float* p) { return *(const float4*)p; }
+__device__ __forceinline__ float4 read4(const __half* p) {
+    const uint2 h = *(const uint2*)p;
+    const float2 lo = __half22float2(*(const __half2*)&h.x), hi = __half22float2(*(const __half2*)&h.y);
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+
+enum class Load : int { Wide, AlongK, AlongRows };   // how an operand is fetched: 16 bytes along K; one element along K / along its rows
+struct TileArgs {
+    int slices;              // of K, one cluster
+    Load load_a, load_b;
+    bool rows_fast;          // the result's rows, not its columns, are contiguous
+};
+
+// C tile of BM x BN per CTA, 8 x TN per thread, KG thread groups taking alternate halves of a K block (summed in shared
+// memory at the end).  `gridDim.z` = batch x slices of K; the slices of a tile are one cluster and sum their tiles
+// through distributed shared memory, so a problem with few tiles still fills the chip and needs no second launch.
+//
+// What bounds it is instruction issue.  Operands arrive 16 bytes at a time and stay along K in shared memory; four K
+// elements cost a thread 32 TN multiply-adds next to 8 + TN 128-bit reads.  (With the tiles along their rows, as the
+// classic layout has it, elements arrived by 4-byte copies, whose addresses were most of the instructions: 127 us
+// for 4096 positions x 128 channels x 1152, against 345 us of the kernel before it.)
+//   128 x 128, 8 x 8 per thread       the fewest reads per multiply-add; for problems that fill the chip with such tiles
+//    64 x  64, 8 x 4 per thread, KG 2  four times the tiles
+// Plain multiply-adds: the packed form (fma.rn.f32x2) issues at half the rate and measured 5 % slower, K blocks of 64
+// spilled registers.  4096 positions x 128 channels x 1152: 48 us; 19200 x 256 x 2304: 800 us (two tiles a SM, three
+// rounds of 148 for 300 tiles).
+template <class Problem, int BM, int BN, int TN, int KG>
+__global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __grid_constant__ Problem prob, const __grid_constant__ TileArgs args) {
+    constexpr int TX = BN / TN, TY = BM / TM;
+    static_assert(TX * TY * KG == kThreads, "one output tile per CTA");
+    using E = typename Problem::Element;
+    constexpr int LR = row_elements<E>, kWide = 16 / (int)sizeof(E);
+    extern __shared__ __align__(16) uint8_t smem[];
     pdl_enter();
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Bs[BK][BN + 4];
-    const int64_t M = prob.M(), N = prob.N(), K = prob.K();
-    const int64_t batch = blockIdx.z;
+    const int slices = args.slices;
+    const int64_t M = prob.rows(), N = prob.cols();
+    const int inner = (int)prob.inner(), taps = prob.taps();
+    const int slice = (int)(blockIdx.z % (unsigned)slices);
+    const int64_t batch = blockIdx.z / (unsigned)slices;
     const int64_t m0 = (int64_t)blockIdx.x * BM, n0 = (int64_t)blockIdx.y * BN;
     const int tid = threadIdx.x;
-    const int tx = tid % (BN / TN), ty = tid / (BN / TN);
-    const bool a_k_fast = prob.a_k_fast(), b_k_fast = prob.b_k_fast();
+    const int group = tid / (TX * TY), rank = tid % (TX * TY);
+    // Which rows and columns a lane takes decides what its 128-bit shared reads cost: half a warp's are served in one pass
+    // if lanes i and i ^ 1 (or i and i ^ 2) all read the same address, else in two.  Bit 0 and bit 4 of the lane pick the
+    // column, bits 1 to 3 the row: both operands' reads qualify (with rows along bits 0 to 2 an operand's did not:
+    // 40 passes per four K elements instead of 24, and the reads, not the multiply-adds, were the limit).
+    const int warp = rank >> 5, lane = rank & 31;
+    const int ty = ((lane >> 1) & 7) + 8 * (warp % (TY / 8)), tx = ((lane & 1) | ((lane >> 4) << 1)) + 4 * (warp / (TY / 8));
+
+    // K blocks of this slice: block kb is elements (kb % per_tap) * BK .. of tap kb / per_tap
+    const int per_tap = (inner + BK - 1) / BK;
+    const int total = taps * per_tap, per_slice = (total + slices - 1) / slices;
+    const int kb_first = min(slice * per_slice, total), blocks = min(kb_first + per_slice, total) - kb_first;
+
+    // 16-byte fetches: chunk tid % (BK / kWide) of rows tid / (BK / kWide) + i * kRowStep
+    constexpr int kChunks = BK / kWide, kRowStep = kThreads / kChunks;
+    constexpr int A_ROWS = BM / kRowStep > 0 ? BM / kRowStep : 1, B_ROWS = BN / kRowStep > 0 ? BN / kRowStep : 1;
+    const int chunk = tid % kChunks, chunk_row = tid / kChunks;
+    typename Problem::Row a_rows[A_ROWS];
+    uint32_t a_valid = 0;
+    if (args.load_a == Load::Wide) {
+#pragma unroll
+        for (int i = 0; i < A_ROWS; i++) {
+            const int mm = chunk_row + i * kRowStep;
+            const bool in = mm < BM && m0 + mm < M;
+            a_valid |= (uint32_t)in << i;
+            a_rows[i] = prob.row(batch, in ? m0 + mm : 0);
+        }
+    }
+    const E* any = prob.col(0, 0);   // an address to name where nothing is read
+    int load_tap = kb_first / per_tap, load_block = kb_first - load_tap * per_tap;
+    typename Problem::Tap tap = prob.tap(load_tap);
+    const E* a_at[A_ROWS];
+    const E* b_at[B_ROWS];
+    const E* b_col[B_ROWS];
+    uint32_t a_read = 0, b_read = 0;   // rows and columns that exist (and, for a row, whose window is inside the image)
+#pragma unroll
+    for (int i = 0; i < B_ROWS; i++) {
+        const int nn = chunk_row + i * kRowStep;
+        const bool in = args.load_b == Load::Wide && nn < BN && n0 + nn < N;
+        b_col[i] = in ? prob.col(batch, n0 + nn) : any;
+        b_read |= (uint32_t)in << i;
+    }
+    auto enter_tap = [&] {
+        a_read = 0;
+        const int k0 = load_block * BK + chunk * kWide;
+        if (args.load_a == Load::Wide) {
+#pragma unroll
+            for (int i = 0; i < A_ROWS; i++) {
+                const E* at = ((a_valid >> i) & 1) ? prob.a_at(a_rows[i], tap) : nullptr;
+                a_read |= (uint32_t)(at != nullptr) << i;
+                a_at[i] = at ? at + k0 : any;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < B_ROWS; i++) b_at[i] = ((b_read >> i) & 1) ? prob.b_at(b_col[i], tap) + k0 : any;
+    };
+    enter_tap();
+    const uint32_t fetch_to = smem_addr(smem) + (uint32_t)(chunk_row * LR + chunk * kWide) * (uint32_t)sizeof(E);
+    auto load_stage = [&](int stage) {
+        const uint32_t to = fetch_to + (uint32_t)stage * stage_bytes<E, BM, BN>;
+        const int k0 = load_block * BK;
+        const int left = (inner - k0 - chunk * kWide) * (int)sizeof(E);
+        const int bytes = min(16, max(0, left));
+        if (args.load_a == Load::Wide) {
+#pragma unroll
+            for (int i = 0; i < A_ROWS; i++) {
+                if (BM % kRowStep == 0 || chunk_row + i * kRowStep < BM)
+                    fetch16(to + i * kRowStep * LR * (int)sizeof(E), left > 0 ? a_at[i] : any, ((a_read >> i) & 1) ? bytes : 0);
+                a_at[i] += ((a_read >> i) & 1) ? BK : 0;
+            }
+        } else {
+            E* As = (E*)(smem + stage * stage_bytes<E, BM, BN>);
+            const bool along_k = args.load_a == Load::AlongK;
+#pragma unroll 1
+            for (int e = tid; e < BM * BK; e += kThreads) {
+                const int mm = along_k ? e / BK : e % BM, kk = along_k ? e % BK : e / BM;
+                const E* src = nullptr;
+                if (m0 + mm < M && k0 + kk < inner) src = prob.a_at(prob.row(batch, m0 + mm), tap);
+                fetch1(As + mm * LR + kk, src ? src + (k0 + kk) * prob.a_stride() : any, src != nullptr);
+            }
+        }
+        if (args.load_b == Load::Wide) {
+#pragma unroll
+            for (int i = 0; i < B_ROWS; i++) {
+                if (BN % kRowStep == 0 || chunk_row + i * kRowStep < BN)
+                    fetch16(to + (BM + i * kRowStep) * LR * (int)sizeof(E), left > 0 ? b_at[i] : any, ((b_read >> i) & 1) ? bytes : 0);
+                b_at[i] += ((b_read >> i) & 1) ? BK : 0;
+            }
+        } else {
+            E* Bs = (E*)(smem + stage * stage_bytes<E, BM, BN>) + BM * LR;
+            const bool along_k = args.load_b == Load::AlongK;
+#pragma unroll 1
+            for (int e = tid; e < BN * BK; e += kThreads) {
+                const int nn = along_k ? e / BK : e % BN, kk = along_k ? e % BK : e / BN;
+                const bool in = n0 + nn < N && k0 + kk < inner;
+                fetch1(Bs + nn * LR + kk, in ? prob.b_at(prob.col(batch, n0 + nn), tap) + (k0 + kk) * prob.b_stride() : any, in);
+            }
+        }
+        if (++load_block == per_tap) {
+            load_block = 0;
+            if (++load_tap < taps) {
+                prob.next(tap);
+                enter_tap();
+            }
+        }
+    };
 
     float acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; i++)
 #pragma unroll
-        for (int j = 0; j < TN; j++) acc[i][j] = 0.0f;
+        for (int j = 0; j < TN; j++) acc[i][j] = 0.f;
 
-    for (int64_t k0 = 0; k0 < K; k0 += BK) {
 #pragma unroll
-        for (int i = 0; i < (BM * BK) / 256; i++) {
-            const int e = tid + i * 256;
-            const int mm = a_k_fast ? e / BK : e % BM;
-            const int kk = a_k_fast ? e % BK : e / BM;
-            const int64_t m = m0 + mm, k = k0 + kk;
-            As[kk][mm] = (m < M && k < K) ? prob.load_a(batch, m, k) : 0.0f;
+    for (int s = 0; s < kStages - 1; s++) {
+        if (s < blocks) load_stage(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int stage = 0, next = kStages - 1;
+#pragma unroll 1
+    for (int b = 0; b < blocks; b++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+        __syncthreads();   // stage `b` is complete, and everybody has read stage `b - 1`, which is filled next
+        if (b + kStages - 1 < blocks) load_stage(next);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        // a thread's rows are TY (its columns TX) apart: neighbouring lanes read neighbouring rows
+        const E* As = (const E*)(smem + stage * stage_bytes<E, BM, BN>) + ty * LR + group * (BK / KG);
+        const E* Bs = (const E*)(smem + stage * stage_bytes<E, BM, BN>) + (BM + tx) * LR + group * (BK / KG);
+#pragma unroll
+        for (int k = 0; k < BK / KG; k += 4) {
+            float4 w[TN];
+#pragma unroll
+            for (int j = 0; j < TN; j++) w[j] = read4(Bs + j * TX * LR + k);
+#pragma unroll
+            for (int i = 0; i < TM; i++) {
+                const float4 a = read4(As + i * TY * LR + k);
+#pragma unroll
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a.x, w[j].x, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a.y, w[j].y, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a.z, w[j].z, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a.w, w[j].w, acc[i][j]);
+            }
         }
+        if (++stage == kStages) stage = 0;
+        if (++next == kStages) next = 0;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+
+    // the tile (one per thread group) in shared memory, [KG][BM][BN + pad]; read back along the result's contiguous axis
+    constexpr int LC = BN + kTilePad, kTile = BM * LC;
+    float* tile = (float*)smem;
 #pragma unroll
-        for (int i = 0; i < (BN * BK) / 256; i++) {
-            const int e = tid + i * 256;
-            const int nn = b_k_fast ? e / BK : e % BN;
-            const int kk = b_k_fast ? e % BK : e / BN;
-            const int64_t n = n0 + nn, k = k0 + kk;
-            Bs[kk][nn] = (n < N && k < K) ? prob.load_b(batch, k, n) : 0.0f;
-        }
-        __syncthreads();
+    for (int i = 0; i < TM; i++)
 #pragma unroll
-        for (int kk = 0; kk < BK; kk++) {
-            float a[TM], b[TN];
-#pragma unroll
-            for (int i = 0; i < TM; i++) a[i] = As[kk][ty * TM + i];
-#pragma unroll
-            for (int j = 0; j < TN; j++) b[j] = Bs[kk][tx * TN + j];
-#pragma unroll
-            for (int i = 0; i < TM; i++)
-#pragma unroll
-                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
+        for (int j = 0; j < TN; j++) tile[group * kTile + (ty + i * TY) * LC + tx + j * TX] = acc[i][j];
+    if (slices > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
         __syncthreads();
     }
+    const uint32_t own = smem_addr(tile);
+    for (int e = slice * kThreads + tid; e < BM * BN; e += slices * kThreads) {
+        const int mm = args.rows_fast ? e % BM : e / BN, nn = args.rows_fast ? e / BM : e % BN;
+        const int64_t m = m0 + mm, n = n0 + nn;
+        if (m >= M || n >= N) continue;
+        float v = 0.f;
+        for (int q = 0; q < slices; q++) {
+            uint32_t from = own;
+            if (slices > 1) asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(from) : "r"(own), "r"(q));
 #pragma unroll
-    for (int i = 0; i < TM; i++) {
-        const int64_t m = m0 + ty * TM + i;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < TN; j++) {
-            const int64_t n = n0 + tx * TN + j;
-            if (n < N) prob.store(batch, m, n, acc[i][j]);
+            for (int g = 0; g < KG; g++) {
+                float x;
+                const uint32_t at = from + 4u * (uint32_t)(g * kTile + mm * LC + nn);
+                if (slices > 1) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(at));
+                else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(at));
+                v += x;
+            }
         }
+        prob.store(prob.out(batch, m), n, v);
+    }
+    if (slices > 1) {   // nobody leaves while a peer still reads its tile
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
 }
 
+template <class Problem, int BM, int BN, int TN, int KG>
+int launch_tile(const Problem& prob, int64_t gx, int64_t gy, int64_t batch, const TileArgs& args, cudaStream_t stream) {
+    auto kernel = contract_simt_kernel<Problem, BM, BN, TN, KG>;
+    constexpr int smem = smem_bytes<typename Problem::Element, BM, BN, KG>;
+    // (the opt-in to more than 48 KB is per device)
+    static std::mutex mu;
+    static bool done[64] = {false};
+    int device = 0;
+    cudaGetDevice(&device);
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (device >= 0 && device < 64 && !done[device]) {
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (e != cudaSuccess) return (int)e;
+            done[device] = true;
+        }
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)gx, (unsigned)gy, (unsigned)(batch * args.slices));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = (unsigned)args.slices;
+    cfg.attrs = attr;
+    cfg.numAttrs = args.slices > 1 ? 2 : 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, prob, args);
+}
+
+// `taps` x `inner`: the reduction
 template <class Problem>
-int launch(const Problem& prob, int64_t M, int64_t N, int64_t batch, cudaStream_t stream) {
+int launch(const Problem& prob, int64_t M, int64_t N, int64_t batch, int64_t taps, int64_t inner, TileArgs args, cudaStream_t stream) {
     if (M == 0 || N == 0 || batch == 0) return 0;
-    const int64_t gx = (M + BM - 1) / BM, gy = (N + BN - 1) / BN;
+    if (inner > (1ll << 30)) return (int)cudaErrorInvalidValue;
+    const int64_t k_blocks = taps * ((inner + BK - 1) / BK);
+    const int64_t large = ((M + 127) / 128) * ((N + 127) / 128) * batch, small = ((M + 63) / 64) * ((N + 63) / 64) * batch;
+    // Rounds of tiles over the chip, times the time of a round: a 128 x 128 tile alone on its SM runs at 0.56 of the
+    // multiply-add rate, two 64 x 64 tiles sharing one at 0.45 (both measured), and the last round may be nearly empty.
+    const double rounds_large = (double)((large + 147) / 148) * 4 / 0.56, rounds_small = (double)((small + 295) / 296) * 2 / 0.45;
+    const bool wide = rounds_large < rounds_small;
+    const int64_t gx = (M + (wide ? 127 : 63)) / (wide ? 128 : 64), gy = (N + (wide ? 127 : 63)) / (wide ? 128 : 64);
     if (gy > 65535 || batch > 65535 || gx > 0x7FFFFFFFll) return (int)cudaErrorInvalidValue;
-    dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)batch);
-    launch_pdl(contract_simt_kernel<Problem>, dim3(grid), dim3(256), (size_t)(0), stream, prob);
-    return (int)cudaGetLastError();
+    args.slices = 1;
+    if (wide) return launch_tile<Problem, 128, 128, 8, 1>(prob, gx, gy, batch, args, stream);
+    // slices of K until the chip has two CTAs per SM (one alone leaves the schedulers two warps each, which cover neither
+    // the shared reads nor the multiply-adds' latency), at least four blocks each (a slice pays the pipeline's fill and
+    // two cluster barriers, some 3 us), eight at most (the portable cluster size)
+    while (args.slices < 8 && gx * gy * batch * args.slices * 2 <= 296 && k_blocks >= 4 * 2 * args.slices && batch * args.slices * 2 <= 65535)
+        args.slices *= 2;
+    return launch_tile<Problem, 64, 64, 4, 2>(prob, gx, gy, batch, args, stream);
+}
+
+// 16-byte fetches along K: K contiguous, everything else a multiple of 16 bytes apart
+Load load_of(const void* base, int64_t k_stride, std::initializer_list<int64_t> other_strides, int element) {
+    if (k_stride != 1) return Load::AlongRows;
+    bool aligned = ((uintptr_t)base & 15) == 0;
+    for (int64_t s : other_strides) aligned = aligned && (s * element) % 16 == 0;
+    return aligned ? Load::Wide : Load::AlongK;
+}
+
+int launch_gemm(const GemmParams& p, cudaStream_t stream) {
+    const int element = p.half ? 2 : 4;
+    TileArgs args{1, load_of(p.a, p.sa[2], {p.sa[0], p.sa[1]}, element), load_of(p.b, p.sb[1], {p.sb[0], p.sb[2]}, element), p.sc[1] == 1 && p.sc[2] != 1};
+    if (p.half) return launch(GemmProblemHalf{p}, p.m, p.n, p.batch, 1, p.k, args, stream);
+    return launch(GemmProblem{p}, p.m, p.n, p.batch, 1, p.k, args, stream);
 }
 
 // Matrix multiply with very few output columns (a classifier head, n <= 8): a 64 x 64 tile would leave
@@ -236,7 +521,7 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(const __grid_constant_
 }  // namespace
 
 int launch_gemm_simt(const GemmParams& p, cudaStream_t stream) {
-    if (p.half) return launch(GemmProblemHalf{p}, p.m, p.n, p.batch, stream);
+    if (p.half) return launch_gemm(p, stream);
     if (p.n >= 1 && p.n <= kSkinnyMaxN && p.k >= 32 && p.batch * p.m > 0) {
         const int64_t rows = p.batch * p.m;
         launch_pdl(gemm_skinny_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), (size_t)(0), stream, p);
@@ -262,11 +547,13 @@ int launch_gemm_simt(const GemmParams& p, cudaStream_t stream) {
         launch_pdl(gemm_skinny_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), (size_t)(0), stream, t);
         return (int)cudaGetLastError();
     }
-    return launch(GemmProblem{p}, p.m, p.n, p.batch, stream);
+    return launch_gemm(p, stream);
 }
 
 int launch_conv_simt(const ConvParams& p, cudaStream_t stream) {
-    return launch(ConvProblem{p}, (int64_t)p.n * p.oh * p.ow, p.k, 1, stream);
+    TileArgs args{1, load_of(p.in, p.s_in[1], {p.s_in[0], p.s_in[2], p.s_in[3]}, 4), load_of(p.filter, p.s_f[1], {p.s_f[0], p.s_f[2], p.s_f[3]}, 4),
+                  p.s_out[1] != 1};
+    return launch(ConvProblem{p}, (int64_t)p.n * p.oh * p.ow, p.k, 1, (int64_t)p.r * p.s, p.c, args, stream);
 }
 
 }  // namespace kn

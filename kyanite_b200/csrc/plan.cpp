@@ -1386,6 +1386,18 @@ class Planner {
                 out = out.with(out.ss.permute({0, 3, 1, 2}));
             }
         }
+        if (!tensor_core && ci.op == OpKind::Conv && g_.values[ci.inputs[1]].op == OpKind::Constant) {
+            // the exact-f32 kernel, too, reads both operands along the channels when it can
+            w = tap_major_filter(w, ci.inputs[1], false);
+            if (exact_conv_products(m->contraction) >= 20e6) x = channels_last(x, ci.inputs[0]);   // (a copy is a launch: 3 us)
+            bool chained = false;
+            for (int u : users_[root])
+                chained = chained || (g_.values[u].op == OpKind::Conv && g_.values[u].inputs[0] == root && exact_conv_products(u) >= 200e3);
+            if (chained && root_shape == native && native[1] % 4 == 0) {
+                out = alloc_shared({native[0], native[2], native[3], native[1]}, DType::F32, root);
+                out = out.with(out.ss.permute({0, 3, 1, 2}));
+            }
+        }
         if (out.buf < 0) out = alloc_shared(native, DType::F32, root);
 
         Step s;
@@ -2006,6 +2018,14 @@ class Planner {
         return false;
     }
 
+    // multiply-adds of a convolution that the exact-f32 kernel computes under KN_MATH_F32, 0 for any other value
+    double exact_conv_products(int conv) {
+        const ValueInfo& ci = g_.values[conv];
+        if (opts_.math_mode != KN_MATH_F32 || ci.dtype != DType::F32 || g_.values[ci.inputs[1]].op != OpKind::Constant) return 0;
+        const std::vector<int64_t> o = shape_of(conv), f = shape_of(ci.inputs[1]);
+        return (double)o[0] * o[2] * o[3] * o[1] * f[1] * f[2] * f[3];
+    }
+
     // The convolution kernel reads its input as (C, W, H, N) with channels contiguous.  A tensor that
     // already is channels-last (the output of a previous tensor-core convolution) is used in place.
     PlanTensor channels_last(const PlanTensor& x, int value) {
@@ -2022,9 +2042,9 @@ class Planner {
         return dst;
     }
 
-    // Filter [K, C, R, S] -> [R*S][K][C_pad] rounded to TF32 (round to nearest, ties away).  Constant
+    // Filter [K, C, R, S] -> [R*S][K][C_pad], rounded to TF32 (round to nearest, ties away) if `round`.  Constant
     // filters are rearranged here on the host, once; computed filters get a strided copy step.
-    PlanTensor tap_major_filter(const PlanTensor& w, int value) {
+    PlanTensor tap_major_filter(const PlanTensor& w, int value, bool round = true) {
         const int64_t K = w.ss.shape[0], C = w.ss.shape[1], R = w.ss.shape[2], S = w.ss.shape[3];
         const int64_t c_pad = (C + 3) / 4 * 4;
         const ValueInfo& wi = g_.values[value];
@@ -2038,7 +2058,7 @@ class Planner {
                         for (int64_t s2 = 0; s2 < S; s2++) {
                             uint32_t bits;
                             memcpy(&bits, (const uint8_t*)src + 4 * (((k * C + c) * R + r) * S + s2), 4);
-                            if ((bits & 0x7F800000u) != 0x7F800000u) bits = (bits + 0x1000u) & 0xFFFFE000u;
+                            if (round && (bits & 0x7F800000u) != 0x7F800000u) bits = (bits + 0x1000u) & 0xFFFFE000u;
                             dst[((r * S + s2) * K + k) * c_pad + c] = bits;
                         }
             PlanTensor t = alloc_const({R, S, K, c_pad}, DType::F32, value, nullptr, data);

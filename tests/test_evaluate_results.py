@@ -1,0 +1,31 @@
+"""Results of `evaluate` belong to the caller: whatever later evaluations do, and beyond the executor's life, for results
+that are handed out as pinned memory (64 KB and more), for small ones and when more are kept than there are sets."""
+import numpy as np
+import pytest
+
+from kyanite_b200.executor import CudaExecutor
+from kyanite_b200.graph import BATCH, Graph, shape
+
+pytestmark = pytest.mark.gpu
+
+
+# columns on either side of the limits of the transfer kernel and of handing results out; enough input for staged uploads
+@pytest.mark.parametrize("columns", [3, 16384, 16388, 300001])
+def test_results_are_the_callers(columns):
+    g = Graph()
+    x = g.input(shape(BATCH, columns))
+    g.output_all([g.add(x, g.scalar(1.0)), g.mul(x, g.scalar(2.0))])
+    rng = np.random.default_rng(columns)
+    inputs = [rng.standard_normal((1, columns)).astype(np.float32) for _ in range(9)]
+    with CudaExecutor(0, g, 1) as ex:
+        kept = [ex.evaluate([a]) for a in inputs]          # more than an executor has sets
+        del kept[3]
+        again = ex.evaluate([inputs[3]])                   # a returned set serves again
+        ex.evaluate_begin([inputs[0]])
+        staged = [a.copy() for a in ex.evaluate_end()]
+    kept.insert(3, again)
+    kept.append(staged)
+    for a, (plus, twice) in zip(inputs + [inputs[0]], kept):
+        np.testing.assert_array_equal(plus, a + np.float32(1))
+        np.testing.assert_array_equal(twice, a * np.float32(2))
+        plus[...] = 0                                      # and they are writable

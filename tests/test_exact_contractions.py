@@ -1,0 +1,56 @@
+"""The exact-f32 contraction kernel (KN_MATH_F32) at the edges of its tiles, K blocks and K slices, against the oracle."""
+import numpy as np
+import pytest
+
+from kyanite_b200.executor import MATH_F32, CudaExecutor
+from kyanite_b200.graph import DType, Graph, shape
+from oracle.cpu_eval import cpu_eval_graph
+
+pytestmark = pytest.mark.gpu
+
+
+def check(g, inputs):
+    with CudaExecutor(0, g, 0, math_mode=MATH_F32) as ex:
+        got = ex.evaluate(inputs)[0].astype(np.float64)
+    expected = cpu_eval_graph(g.to_bytes(), 0, inputs)[0].astype(np.float64)
+    # products and sums are f32 in both, in different orders: n-term sums of O(1) products of size sqrt(n) differ by
+    # a few roundings of the running sum, sqrt(n) * sqrt(n) * 2^-24 at most in practice; 1e-5 of the scale covers n <= 8192.
+    # f16 results are rounded once more: half an ulp, 2^-11.
+    rel = 1e-5 if ex._out_info[0][1] == DType.F32 else 1e-5 + 2.0 ** -11
+    assert np.abs(got - expected).max() <= rel * max(1.0, np.abs(expected).max())
+
+
+# one tile of 64 and its neighbours, K blocks of 32 and their remainders, sliced K, more tiles than two rounds of large ones
+@pytest.mark.parametrize("b,m,n,k", [(1, 9, 9, 1), (1, 63, 65, 31), (2, 64, 64, 32), (1, 65, 63, 33), (3, 127, 129, 36), (1, 64, 256, 2048),
+                                     (1, 70, 40, 1030), (1, 4700, 1153, 40)])
+@pytest.mark.parametrize("layout", ["plain", "transposed", "half"])
+def test_matmul(b, m, n, k, layout):
+    rng = np.random.default_rng(m * 7 + n * 3 + k)
+    dtype = DType.F16 if layout == "half" else DType.F32
+    g = Graph()
+    if layout == "transposed":   # A along its rows, B along K
+        x = g.permute(g.input(shape(b, k, m)), [0, 2, 1])
+        w = g.permute(g.input(shape(b, n, k)), [0, 2, 1])
+        shapes = [(b, k, m), (b, n, k)]
+    else:
+        x, w = g.input(shape(b, m, k), dtype), g.input(shape(b, k, n), dtype)
+        shapes = [(b, m, k), (b, k, n)]
+    g.output(g.batched_mat_mul(x, w))
+    check(g, [(rng.standard_normal(s) * (k ** -0.25)).astype(dtype.np) for s in shapes])
+
+
+# channels that are and are not whole 16-byte chunks or K blocks, strides, taps outside the image, one tile and many
+@pytest.mark.parametrize("n,c,hw,k,r,stride,pad", [(1, 128, 8, 128, 3, 1, 1), (3, 21, 9, 70, 3, 1, 1), (2, 33, 7, 5, 5, 2, 2), (1, 4, 3, 3, 1, 1, 0),
+                                                   (65, 36, 8, 64, 3, 1, 0), (130, 64, 9, 192, 1, 1, 0)])
+@pytest.mark.parametrize("chained", [False, True])
+def test_convolution(n, c, hw, k, r, stride, pad, chained):
+    rng = np.random.default_rng(n + c + k)
+    g = Graph()
+    x = g.input(shape(n, c, hw, hw))
+    weight = lambda o, i, s: g.constant_tensor((rng.standard_normal((o, i, s, s)) * (i * s * s) ** -0.5).astype(np.float32))  # noqa: E731
+    y = g.conv(x, weight(k, c, r), stride, stride, pad, pad)
+    y = g.relu(g.add(y, g.constant_tensor(rng.standard_normal((1, k, 1, 1)).astype(np.float32))))
+    if chained:   # the first result stays channels-last for the second convolution, and is added to it
+        y = g.add(g.conv(y, weight(k, k, 3), 1, 1, 1, 1), y)
+    g.output(y)
+    check(g, [rng.standard_normal((n, c, hw, hw)).astype(np.float32)])
