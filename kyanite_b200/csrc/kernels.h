@@ -141,6 +141,10 @@ struct GemmParams {
     // ([batch][slice][m][n] f32) and are summed by a second kernel; 1 = no split
     int32_t splits;
     float* scratch;
+    // tensor-core path only: > 0: one tile of 128 x `slices_bn` and one of `slices` slices of K per CTA, the slices of a tile
+    // summed inside a cluster (gemm_slices_kernel; `splits` is 1 then)
+    int32_t slices, slices_bn;
+    int32_t a_const, b_const;   // the operand is a constant: it may be read before the kernels in front have finished
     int32_t half;            // 1: A, B, C and the addends hold f16 elements (the pointers are reinterpreted); products
                              // accumulate in f32 and the result is rounded to f16 once.  `scratch` stays f32.
     // Implicit convolution operand (persistent tensor-core kernel only, f32 storage).  0: none.  1 / 2: the A / B

@@ -701,6 +701,7 @@ struct TcLaunch {
     int smem_bytes;
     std::shared_ptr<void> chain;  // ConvChain step: launch data of kernels/conv_chain.cu
     std::shared_ptr<void> gemm_p; // matmul taken by the persistent kernel (kernels/gemm_persistent.cu)
+    std::shared_ptr<void> gemm_s; // matmul of few tiles, K slices summed inside a cluster (kernels/gemm_persistent.cu)
     std::shared_ptr<void> attn;   // matmul with a row softmax (kernels/attn_softmax.cu)
     std::shared_ptr<void> attention;   // scores, softmax and probabilities . V (kernels/attention.cu)
 };
@@ -916,6 +917,12 @@ void tc_prepare_step(Step& step, uint32_t* status_word, int flags, uint32_t* tra
             step.tc = launch;
             return;
         }
+        if (g.slices > 0) {
+            launch->gemm_s = gemm_slices_prepare(g, status_word);
+            KN_CHECK(launch->gemm_s != nullptr, KN_ERR_INTERNAL, "matmul planned for K slices in a cluster does not qualify");
+            step.tc = launch;
+            return;
+        }
         if (g.half || g.conv_operand != 0 || g.a4.enabled || g.b4.enabled) {
             // f16 storage, or an implicit convolution operand: the persistent kernel is the only tensor-core kernel
             // that takes these; the planner marks such a step tensor-core only when that kernel takes it
@@ -1112,6 +1119,7 @@ int tc_launch_step(const Step& step, cudaStream_t stream) {
     if (l.chain) return chain_launch(l.chain.get(), stream);
     if (l.attention) return attention_launch(l.attention.get(), stream);
     if (l.attn) return attn_softmax_launch(l.attn.get(), stream);
+    if (l.gemm_s) return gemm_slices_launch(l.gemm_s.get(), stream);
     if (l.gemm_p) {
         const int err = gemm_persistent_launch(l.gemm_p.get(), stream);
         if (err != 0 || !l.split_k) return err;

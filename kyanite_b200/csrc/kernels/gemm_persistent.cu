@@ -33,6 +33,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 
 #include "../tc.h"
 #include "tc_host.h"
@@ -96,6 +97,74 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t sr
 __device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+
+// Where the operand tiles of consecutive K blocks lie.  Everything about an operand read in place that does not change
+// along K is worked out once per tile, and what does (the filter tap of a K block) is stepped, not divided: the producer's
+// loop runs once per K block in ONE thread, and three integer divisions by run-time values in it cost more than the four
+// MMAs of the block (measured: a 3x3 convolution over 320 channels ran at 800 cycles per K block instead of 320).
+template <bool HALF, bool PAIR>
+struct OperandCursor {
+    static constexpr int kElems = HALF ? 64 : 32;   // elements per 128-byte K block
+    int k, conv_cb = 0, conv_tx = 0, conv_ty = 0, conv_row0 = 0;
+    int a4_c1 = 0, a4_c2 = 0, a4_c3 = 0, b4_c1 = 0, b4_c2 = 0, b4_c3 = 0;
+
+    __device__ __forceinline__ OperandCursor(const GemmPersistentParams& p, int a_row0, int b_row0, int bt, int k_begin) : k(k_begin) {
+        if (p.conv_operand != 0) {
+            const int tap = k_begin / p.conv_cblocks;
+            conv_cb = k_begin - tap * p.conv_cblocks;
+            conv_ty = tap / p.conv_s;
+            conv_tx = tap - conv_ty * p.conv_s;
+            conv_row0 = (p.conv_operand == 1 ? a_row0 : b_row0) / p.conv_ow;
+        }
+        if (p.a4_rd > 0) a4_c1 = a_row0 % p.a4_rd, a4_c2 = bt % p.a4_bi, a4_c3 = a_row0 / p.a4_rd + bt / p.a4_bi;
+        if (p.b4_rd > 0) b4_c1 = b_row0 % p.b4_rd, b4_c2 = bt % p.b4_bi, b4_c3 = b_row0 / p.b4_rd + bt / p.b4_bi;
+    }
+    __device__ __forceinline__ void load3(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) const {
+        if (PAIR) tma_load_3d_pair(dst, map, bar, c0, c1, c2);
+        else tma_load_3d(dst, map, bar, c0, c1, c2);
+    }
+    __device__ __forceinline__ void load4(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) const {
+        if (PAIR) tma_load_4d_pair(dst, map, bar, c0, c1, c2, c3);
+        else tma_load_4d(dst, map, bar, c0, c1, c2, c3);
+    }
+    // K block k = (filter tap, 32-channel block) of an implicit convolution operand; the tile's rows are whole output rows
+    // of image `bt`, so the operand tile is one box of the image tensor (channel, x, y, image) moved by the tap:
+    // positions outside the image are the copy engine's zero fill
+    __device__ __forceinline__ void load_windows(const GemmPersistentParams& p, const CUtensorMap* map, uint32_t dst, uint32_t bar, int bt) const {
+        load4(dst, map, bar, conv_cb * 32, conv_tx - p.conv_pad_x, conv_row0 + conv_ty - p.conv_pad_y, bt);
+    }
+    // (a head split or merge read in place: the tile's coordinates in the 4-D source, see GemmOperand4D; the row part does
+    // not change along K)
+    __device__ __forceinline__ void load_a(const GemmPersistentParams& p, const CUtensorMap* map, uint32_t dst, uint32_t bar, int row0, int bt) const {
+        const int k0 = k * kElems;
+        if (p.conv_operand == 1) {
+            load_windows(p, map, dst, bar, bt);
+        } else if (p.a4_rd > 0) {
+            const int kh = p.a4_kd_shift ? (k0 >> p.a4_kd_shift) : 0;
+            load4(dst, map, bar, k0 - (kh << p.a4_kd_shift), a4_c1, kh + a4_c2, a4_c3);
+        } else {
+            load3(dst, map, bar, k0, row0, bt * p.a_batch);
+        }
+    }
+    __device__ __forceinline__ void load_b(const GemmPersistentParams& p, const CUtensorMap* map, uint32_t dst, uint32_t bar, int row0, int bt) const {
+        const int k0 = k * kElems;
+        if (p.conv_operand == 2) {
+            load_windows(p, map, dst, bar, bt);
+        } else if (p.b4_rd > 0) {
+            const int kh = p.b4_kd_shift ? (k0 >> p.b4_kd_shift) : 0;
+            load4(dst, map, bar, k0 - (kh << p.b4_kd_shift), b4_c1, kh + b4_c2, b4_c3);
+        } else {
+            load3(dst, map, bar, k0, row0, bt * p.b_batch);
+        }
+    }
+    __device__ __forceinline__ void next(const GemmPersistentParams& p) {
+        k++;
+        if (p.conv_operand != 0 && ++conv_cb == p.conv_cblocks) {
+            conv_cb = 0;
+            if (++conv_tx == p.conv_s) { conv_tx = 0; conv_ty++; }
+        }
+    }
+};
 
 // ---- CTA pairs (PAIR): two CTAs of a cluster compute one 256 x BN tile with `cta_group::2` instructions.  Each
 // CTA loads its own 128 rows of A and HALF of the B tile; the tensor cores of both SMs read both halves, so every SM's
@@ -179,21 +248,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             const int k_begin = sp * p.k_iters_slice, k_end = k_begin + slice_blocks(sp);
             const int a_row0 = (PAIR ? 2 * mt + (int)rank : mt) * kGpBlockM;   // this CTA's rows of A
             const int b_row0 = nt * p.bn + (PAIR ? (int)rank * b_rows : 0);      // and of B (a pair: its half)
-            // Everything about an operand read in place that does not change along K is worked out here, and what does
-            // (the filter tap of a K block) is stepped, not divided: this loop runs once per K block in ONE thread,
-            // and three integer divisions by run-time values in it cost more than the four MMAs of the block
-            // (measured: a 3x3 convolution over 320 channels ran at 800 cycles per K block instead of 320).
-            int conv_cb = 0, conv_tx = 0, conv_ty = 0, conv_row0 = 0;
-            if (p.conv_operand != 0) {
-                const int tap = k_begin / p.conv_cblocks;
-                conv_cb = k_begin - tap * p.conv_cblocks;
-                conv_ty = tap / p.conv_s;
-                conv_tx = tap - conv_ty * p.conv_s;
-                conv_row0 = (p.conv_operand == 1 ? a_row0 : b_row0) / p.conv_ow;
-            }
-            int a4_c1 = 0, a4_c2 = 0, a4_c3 = 0, b4_c1 = 0, b4_c2 = 0, b4_c3 = 0;
-            if (p.a4_rd > 0) a4_c1 = a_row0 % p.a4_rd, a4_c2 = bt % p.a4_bi, a4_c3 = a_row0 / p.a4_rd + bt / p.a4_bi;
-            if (p.b4_rd > 0) b4_c1 = b_row0 % p.b4_rd, b4_c2 = bt % p.b4_bi, b4_c3 = b_row0 / p.b4_rd + bt / p.b4_bi;
+            OperandCursor<HALF, PAIR> cursor(p, a_row0, b_row0, bt, k_begin);
             for (int k = k_begin; k < k_end; k++) {
                 if (round > 0 && !mbar_wait(empty_bar + 8u * s, (uint32_t)((round & 1) ^ 1), abandon, p.status, 21)) { ok = false; break; }
                 const uint32_t bar = full_bar + 8u * s;
@@ -201,46 +256,9 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 // pair: both CTAs' tiles complete on the LEADER's barrier, which expects the bytes of both
                 if (!PAIR || rank == 0) mbar_expect_tx(bar, PAIR ? 2u * stage_bytes : stage_bytes);
                 const uint32_t to_bar = PAIR ? map_to_cta(bar, 0) : bar;
-                auto load3 = [&](uint32_t d, const CUtensorMap* map, int c0, int c1, int c2) {
-                    if (PAIR) tma_load_3d_pair(d, map, to_bar, c0, c1, c2);
-                    else tma_load_3d(d, map, to_bar, c0, c1, c2);
-                };
-                auto load4 = [&](uint32_t d, const CUtensorMap* map, int c0, int c1, int c2, int c3) {
-                    if (PAIR) tma_load_4d_pair(d, map, to_bar, c0, c1, c2, c3);
-                    else tma_load_4d(d, map, to_bar, c0, c1, c2, c3);
-                };
-                if (p.conv_operand != 0) {
-                    // K block k = (filter tap, 32-channel block); the tile's rows are whole output rows of image `bt`,
-                    // so the operand tile is one box of the image tensor (channel, x, y, image) moved by the tap:
-                    // positions outside the image are the copy engine's zero fill
-                    if (p.conv_operand == 1) {
-                        load4(dst, &map_a, conv_cb * 32, conv_tx - p.conv_pad_x, conv_row0 + conv_ty - p.conv_pad_y, bt);
-                        load3(dst + kGpATileBytes, &map_b, k * kBlockKElems, b_row0, bt * p.b_batch);
-                    } else {
-                        load3(dst, &map_a, k * kBlockKElems, a_row0, bt * p.a_batch);
-                        load4(dst + kGpATileBytes, &map_b, conv_cb * 32, conv_tx - p.conv_pad_x, conv_row0 + conv_ty - p.conv_pad_y, bt);
-                    }
-                    if (++conv_cb == p.conv_cblocks) {
-                        conv_cb = 0;
-                        if (++conv_tx == p.conv_s) { conv_tx = 0; conv_ty++; }
-                    }
-                } else {
-                    // (a head split or merge read in place: the tile's coordinates in the 4-D source, see GemmOperand4D;
-                    // the row part does not change along K)
-                    const int k0 = k * kBlockKElems;
-                    if (p.a4_rd > 0) {
-                        const int kh = p.a4_kd_shift ? (k0 >> p.a4_kd_shift) : 0;
-                        load4(dst, &map_a, k0 - (kh << p.a4_kd_shift), a4_c1, kh + a4_c2, a4_c3);
-                    } else {
-                        load3(dst, &map_a, k0, a_row0, bt * p.a_batch);
-                    }
-                    if (p.b4_rd > 0) {
-                        const int kh = p.b4_kd_shift ? (k0 >> p.b4_kd_shift) : 0;
-                        load4(dst + kGpATileBytes, &map_b, k0 - (kh << p.b4_kd_shift), b4_c1, kh + b4_c2, b4_c3);
-                    } else {
-                        load3(dst + kGpATileBytes, &map_b, k0, b_row0, bt * p.b_batch);
-                    }
-                }
+                cursor.load_a(p, &map_a, dst, to_bar, a_row0, bt);
+                cursor.load_b(p, &map_b, dst + kGpATileBytes, to_bar, b_row0, bt);
+                cursor.next(p);
                 dbg_mark(p, 1, (uint32_t)(k + 1));
                 if (++s == stages) { s = 0; round++; }
             }
@@ -478,6 +496,248 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
 }
 
+// ---- Few tiles: a matmul of less than one round of 128 x 256 tiles (a short prompt or sentence, a small image, the last
+// layers of a head).  One tile and one slice of K per CTA; the slices of a tile are a CLUSTER, which sums the partial tiles
+// through distributed shared memory, so there is neither a scratch buffer in global memory nor a second kernel.  What
+// bounds these shapes is how soon and how fast the operands reach shared memory, hence:
+//   - narrower tiles and slices of K until the chip has a CTA per SM (gemm_slices_choose weighs the bytes per CTA),
+//   - an operand that is a constant (the weights) is requested BEFORE `griddepcontrol.wait`, under the previous kernel's
+//     tail, as many K blocks of it as there are stages,
+//   - the next kernel is released at once, so that it can do the same.
+// The partial tile goes to shared memory (row pitch bn + 4 floats: conflict-free for 16-byte accesses), CTA r of the
+// cluster sums rows [r * per, (r + 1) * per) in slice order, adds the addends and stores along the rows; any strides, any
+// alignment.  At most 128 registers a thread: two CTAs to an SM, this kernel's and the next one's among them.
+// us a launch, before (persistent kernel, K slices through a scratch buffer and a second kernel) -> now: 120 x 768 x 768
+// 11.6 -> 7.5, 120 x 768 x 3072 16.6 -> 10.3, 333 x 4096 x 4096 f16 33.7 -> 21.3, 333 x 4096 x 11008 f16 58.7 -> 38.6,
+// 333 x 11008 x 4096 f16 52.7 -> 40.8, 3x3 convolution of 32 x 32 positions, 640 -> 640 channels 37.5 -> 26.6.
+constexpr int kGsThreads = 256;
+constexpr int kGsMaxSlices = 8;   // the largest portable cluster
+
+struct GemmSlicesParams {
+    GemmPersistentParams g;
+    void* out;
+    int64_t so[3];
+    int32_t a_const, b_const;                 // the operand is a constant
+    int32_t out_vec, add1_vec, add2_vec;      // rows contiguous, every row start aligned to four elements
+    int32_t tmem_cols;
+};
+
+template <typename T>
+__device__ __forceinline__ void add_four(float (&v)[4], const T* src, int64_t col_stride, bool vec, int valid) {
+    if (vec && valid == 4) {
+        if (sizeof(T) == 4) {
+            const float4 a = *(const float4*)src;
+            v[0] += a.x, v[1] += a.y, v[2] += a.z, v[3] += a.w;
+        } else {
+            const uint2 a = *(const uint2*)src;
+            const float2 lo = __half22float2(*(const __half2*)&a.x), hi = __half22float2(*(const __half2*)&a.y);
+            v[0] += lo.x, v[1] += lo.y, v[2] += hi.x, v[3] += hi.y;
+        }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (j < valid) v[j] += (float)src[j * col_stride];
+}
+
+template <bool HALF>
+__global__ void __launch_bounds__(kGsThreads, 2)
+gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                   const __grid_constant__ GemmSlicesParams q) {
+    extern __shared__ uint8_t smem_raw[];
+    const GemmPersistentParams& p = q.g;
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
+    const int stages = p.stages;
+    const uint32_t stage_bytes = kGpATileBytes + (uint32_t)p.bn * 128u;
+    const uint32_t pitch = (uint32_t)(p.bn + 4) * 4u;
+    const uint32_t bar_base = base + max((uint32_t)stages * stage_bytes, (uint32_t)kGpBlockM * pitch);
+    const uint32_t full_bar = bar_base, empty_bar = bar_base + 8u * stages, acc_full = bar_base + 16u * stages;
+    const uint32_t slot_addr = acc_full + 8u;
+    volatile uint32_t* tmem_slot = (volatile uint32_t*)(gen_base + (slot_addr - base));
+    volatile int* abandon = (volatile int*)(gen_base + (slot_addr + 4u - base));
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; s++) {
+            mbar_init(full_bar + 8u * s, 1);
+            mbar_init(empty_bar + 8u * s, 1);
+        }
+        mbar_init(acc_full, 1);
+        *abandon = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_addr), "r"((uint32_t)q.tmem_cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    // (after the allocation of tensor memory: a CTA of the next kernel that takes its own first would keep this one waiting)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    const int splits = p.splits;
+    const int sp = (int)(blockIdx.x % (unsigned)splits), t = (int)(blockIdx.x / (unsigned)splits);   // sp: rank in the cluster
+    const int mt = t % p.m_tiles, r = t / p.m_tiles, nt = r % p.n_tiles, bt = r / p.n_tiles;
+    const int k_begin = sp * p.k_iters_slice, k_count = min(p.k_iters_slice, p.k_iters - k_begin);
+    const int a_row0 = mt * kGpBlockM, b_row0 = nt * p.bn;
+
+    bool good = true;
+    if (warp == 0 && lane == 0) {
+        // ---------------- producer
+        const int first = min(stages, k_count);
+        OperandCursor<HALF, false> constant(p, a_row0, b_row0, bt, k_begin), other = constant;
+        for (int s = 0; s < first; s++) {
+            const uint32_t dst = base + (uint32_t)s * stage_bytes, bar = full_bar + 8u * s;
+            mbar_expect_tx(bar, stage_bytes);
+            if (q.a_const) constant.load_a(p, &map_a, dst, bar, a_row0, bt);
+            if (q.b_const) constant.load_b(p, &map_b, dst + kGpATileBytes, bar, b_row0, bt);
+            constant.next(p);
+        }
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        for (int s = 0; s < first; s++) {
+            const uint32_t dst = base + (uint32_t)s * stage_bytes, bar = full_bar + 8u * s;
+            if (!q.a_const) other.load_a(p, &map_a, dst, bar, a_row0, bt);
+            if (!q.b_const) other.load_b(p, &map_b, dst + kGpATileBytes, bar, b_row0, bt);
+            other.next(p);
+        }
+        int s = 0, round = 1;
+        for (int k = first; k < k_count; k++) {
+            if (!mbar_wait(empty_bar + 8u * s, (uint32_t)((round & 1) ^ 1), abandon, p.status, 31)) break;
+            const uint32_t dst = base + (uint32_t)s * stage_bytes, bar = full_bar + 8u * s;
+            mbar_expect_tx(bar, stage_bytes);
+            other.load_a(p, &map_a, dst, bar, a_row0, bt);
+            other.load_b(p, &map_b, dst + kGpATileBytes, bar, b_row0, bt);
+            other.next(p);
+            if (++s == stages) { s = 0; round++; }
+        }
+    } else if (warp == 1 && lane == 0) {
+        // ---------------- MMA issuer (the instruction descriptor of gemm_persistent_kernel)
+        const uint32_t fmt = HALF ? 0u : 2u;
+        const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(kGpBlockM >> 4) << 24);
+        int s = 0, round = 0;
+        for (int k = 0; k < k_count && good; k++) {
+            if (!mbar_wait(full_bar + 8u * s, (uint32_t)(round & 1), abandon, p.status, 32)) { good = false; break; }
+            tc_fence_after();
+            const uint32_t a_addr = base + (uint32_t)s * stage_bytes;
+            const uint64_t da = smem_desc_sw128(a_addr), db = smem_desc_sw128(a_addr + kGpATileBytes);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (HALF) mma_f16(tmem_base, da + 2u * j, db + 2u * j, idesc, (k | j) != 0 ? 1u : 0u);
+                else mma_tf32(tmem_base, da + 2u * j, db + 2u * j, idesc, (k | j) != 0 ? 1u : 0u);
+            }
+            mma_commit(empty_bar + 8u * s);
+            if (++s == stages) { s = 0; round++; }
+        }
+        if (good) mma_commit(acc_full);
+    }
+    __syncwarp();
+    // the accumulator is complete, and with it every read of the stages: they become the partial tile
+    if (lane == 0) good = mbar_wait(acc_full, 0, abandon, p.status, 33, kWaitCycles, 2000) && good;
+    good = __syncthreads_and(good ? 1 : 0) != 0;
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // (the addends and the output belong to earlier kernels until here)
+    if (good) {
+        tc_fence_after();
+        const int quarter = warp & 3;
+        const uint32_t row_addr = base + (uint32_t)(quarter * 32 + lane) * pitch;
+        for (int c = warp >> 2; c < (p.bn >> 5); c += kGsThreads / 128) {
+            uint32_t v[32];
+            tmem_load_32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c * 32), v);
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_addr + (uint32_t)(c * 128 + j * 16)), "r"(v[4 * j]),
+                             "r"(v[4 * j + 1]), "r"(v[4 * j + 2]), "r"(v[4 * j + 3])
+                             : "memory");
+        }
+        tc_fence_before();
+    }
+    __syncthreads();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)q.tmem_cols) : "memory");
+    if (splits > 1) cluster_sync_all();   // every slice's partial tile lies in its CTA's shared memory
+
+    {
+        const int rows = (int)min((int64_t)kGpBlockM, p.m - (int64_t)mt * kGpBlockM), per = (rows + splits - 1) / splits;
+        const int row_end = good ? min(rows, (sp + 1) * per) : 0;
+        const int64_t col_tile = (int64_t)nt * p.bn;
+        const int cols = (int)min((int64_t)p.bn, p.n - col_tile);
+        // lanes of a warp: 8, 16 or 32 groups of four columns, the rest of the warp further rows
+        const int group_bits = p.bn <= 32 ? 3 : (p.bn <= 64 ? 4 : 5), warp_rows = 32 >> group_bits;
+        const int my_group = lane & ((1 << group_bits) - 1), my_row = lane >> group_bits;
+        using T = typename std::conditional<HALF, __half, float>::type;
+        const T* add1 = (const T*)p.add1;
+        const T* add2 = (const T*)p.add2;
+        T* out = (T*)q.out;
+        // items of a warp: (rows, column group); two at a time, so that the reads of both are in flight together (one at a
+        // time the sum of three slices of 128 x 256 took 6 us, of which the reads are 1)
+        const int col_groups = (cols + (4 << group_bits) - 1) / (4 << group_bits);
+        const int step_rows = (kGsThreads / 32) * warp_rows;
+        const int row_steps = max(0, (row_end - sp * per - warp * warp_rows + step_rows - 1) / step_rows);
+        auto fetch = [&](int row, int c, float (&part)[kGsMaxSlices][4]) {
+            if (row >= row_end || c >= cols) return;
+            const uint32_t local = base + (uint32_t)row * pitch + (uint32_t)c * 4u;
+#pragma unroll
+            for (int s = 0; s < kGsMaxSlices; s++)
+                if (s < splits)
+                    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                 : "=f"(part[s][0]), "=f"(part[s][1]), "=f"(part[s][2]), "=f"(part[s][3])
+                                 : "r"(map_to_cta(local, (uint32_t)s)));
+        };
+        auto finish = [&](int row, int c, const float (&part)[kGsMaxSlices][4]) {
+            if (row >= row_end || c >= cols) return;
+            const int64_t m = (int64_t)mt * kGpBlockM + row, n = col_tile + c;
+            const int valid = min(4, cols - c);
+            float v[4] = {part[0][0], part[0][1], part[0][2], part[0][3]};
+#pragma unroll
+            for (int s = 1; s < kGsMaxSlices; s++)
+                if (s < splits) v[0] += part[s][0], v[1] += part[s][1], v[2] += part[s][2], v[3] += part[s][3];
+            if (add1) add_four(v, add1 + bt * p.s1[0] + m * p.s1[1] + n * p.s1[2], p.s1[2], q.add1_vec != 0, valid);
+            if (add2) add_four(v, add2 + bt * p.s2[0] + m * p.s2[1] + n * p.s2[2], p.s2[2], q.add2_vec != 0, valid);
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = apply_activation(v[j], p.act);
+            T* dst = out + bt * q.so[0] + m * q.so[1] + n * q.so[2];
+            if (q.out_vec != 0 && valid == 4) {
+                if (HALF) {
+                    const __half2 lo = __floats2half2_rn(v[0], v[1]), hi = __floats2half2_rn(v[2], v[3]);
+                    *(uint2*)dst = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
+                } else {
+                    *(float4*)dst = make_float4(v[0], v[1], v[2], v[3]);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (j < valid) dst[j * q.so[2]] = (T)v[j];
+            }
+        };
+        int row = sp * per + warp * warp_rows + my_row, group = 0;
+        auto advance = [&]() {
+            if (++group == col_groups) group = 0, row += step_rows;
+        };
+        for (int left = row_steps * col_groups; left > 0; left -= 2) {
+            float first[kGsMaxSlices][4], second[kGsMaxSlices][4];
+            const int row1 = row, c1 = ((group << group_bits) + my_group) * 4;
+            advance();
+            const int row2 = left > 1 ? row : row_end, c2 = ((group << group_bits) + my_group) * 4;
+            advance();
+            fetch(row1, c1, first);
+            fetch(row2, c2, second);
+            finish(row1, c1, first);
+            finish(row2, c2, second);
+        }
+    }
+    __syncthreads();
+    if (splits > 1) cluster_sync_all();   // nobody leaves while its partial tile may still be read
+}
+
+struct GemmSlicesLaunch {
+    CUtensorMap map_a, map_b;
+    GemmSlicesParams p;
+    unsigned grid;
+    int smem_bytes;
+    bool half;
+};
+
 struct GemmPersistentLaunch {
     CUtensorMap map_a, map_b, map_c;
     GemmPersistentParams p;
@@ -510,6 +770,73 @@ int gemm_persistent_bn(int64_t n) {
     // next block's columns; a single block is clipped by the store's tensor bounds)
     const int64_t unit = blocks > 1 ? 32 : 16;
     return (int)std::min<int64_t>(((n + blocks - 1) / blocks + unit - 1) / unit * unit, 256);
+}
+
+// Tensor maps of the two operands, tiles of 128 rows of A and `b_rows` rows of B, and the parameters that locate a tile
+// in them.  False if an operand cannot be read that way.
+static bool operand_maps(const GemmParams& g, int b_rows, GemmPersistentParams& p, CUtensorMap* map_a, CUtensorMap* map_b) {
+    const bool half = g.half != 0;
+    const int64_t align = half ? 8 : 4;            // elements per 16 bytes
+    const int block_k = half ? 64 : 32;
+    p.a_batch = (g.batch > 1 && g.sa[0] == 0) ? 0 : 1;
+    int64_t adims[3] = {g.k, g.m, p.a_batch ? g.batch : 1}, astr[3] = {1, g.sa[1], p.a_batch ? g.sa[0] : align};
+    int abox[3] = {block_k, kGpBlockM, 1};
+    p.b_batch = (g.batch > 1 && g.sb[0] == 0) ? 0 : 1;
+    int64_t bdims[3] = {g.k, g.n, p.b_batch ? g.batch : 1}, bstr[3] = {1, g.sb[2], p.b_batch ? g.sb[0] : align};
+    int bbox[3] = {block_k, b_rows, 1};
+    // the implicit convolution operand: a 4-D map of the image tensor (channel, x, y, image) whose box is one K
+    // block of channels by whole output rows
+    int64_t idims[4] = {g.conv_c, g.conv_w, g.conv_h, g.batch}, istr[4] = {1, g.conv_strides[2], g.conv_strides[1], g.conv_strides[0]};
+    int ibox[4] = {32, 1, 1, 1};
+    if (g.conv_operand != 0) {
+        const int rows = g.conv_operand == 1 ? kGpBlockM : b_rows;
+        if (half || g.conv_c % 32 != 0 || g.conv_ow < 1 || g.conv_ow > 256 || rows % g.conv_ow != 0 || g.conv_r < 1 || g.conv_s < 1 ||
+            g.k != (int64_t)g.conv_r * g.conv_s * g.conv_c)
+            return false;
+        ibox[1] = g.conv_ow;
+        ibox[2] = rows / g.conv_ow;
+        p.conv_operand = g.conv_operand;
+        p.conv_cblocks = g.conv_c / 32;
+        p.conv_s = g.conv_s;
+        p.conv_pad_y = g.conv_pad_y;
+        p.conv_pad_x = g.conv_pad_x;
+        p.conv_ow = g.conv_ow;
+    }
+    // 4-D operands: the box is one K block by the tile's rows inside one (x, y) entry
+    auto operand_4d = [&](const GemmOperand4D& o, const void* base, int rows, int64_t matrix_rows, int32_t* kd_shift, int32_t* rd, int32_t* bi,
+                          CUtensorMap* map) {
+        if (!o.enabled) return true;
+        if (o.kd < 1 || o.rd < 1 || o.bi < 1 || o.strides[0] != 1 || g.conv_operand != 0) return false;
+        int shift = 0;
+        if (o.kd != g.k) {   // the K offset is split: whole K blocks inside one entry, by a shift
+            if (o.kd % block_k != 0 || (o.kd & (o.kd - 1)) != 0) return false;
+            while ((1 << shift) < o.kd) shift++;
+        }
+        // a tile's rows lie inside one entry: an entry's rows are a multiple of the tile's, or the matrix is one entry
+        // tall (then rows past its end are past the tensor's extent: zero fill)
+        if (o.rd % rows != 0 && o.rd < matrix_rows) return false;
+        int box[4] = {block_k, rows, 1, 1};
+        *map = half ? tc_make_map_f16(base, 4, o.dims, o.strides, box, true) : tc_make_map(base, 4, o.dims, o.strides, box, true);
+        *kd_shift = shift;
+        *rd = o.rd;
+        *bi = o.bi;
+        return true;
+    };
+    if (!operand_4d(g.a4, g.a, kGpBlockM, g.m, &p.a4_kd_shift, &p.a4_rd, &p.a4_bi, map_a)) return false;
+    if (!operand_4d(g.b4, g.b, b_rows, g.n, &p.b4_kd_shift, &p.b4_rd, &p.b4_bi, map_b)) return false;
+    if (g.a4.enabled && g.b4.enabled) {
+    } else if (g.a4.enabled) {
+        *map_b = half ? tc_make_map_f16(g.b, 3, bdims, bstr, bbox, true) : tc_make_map(g.b, 3, bdims, bstr, bbox, true);
+    } else if (g.b4.enabled) {
+        *map_a = half ? tc_make_map_f16(g.a, 3, adims, astr, abox, true) : tc_make_map(g.a, 3, adims, astr, abox, true);
+    } else if (half) {
+        *map_a = tc_make_map_f16(g.a, 3, adims, astr, abox, true);
+        *map_b = tc_make_map_f16(g.b, 3, bdims, bstr, bbox, true);
+    } else {
+        *map_a = g.conv_operand == 1 ? tc_make_map(g.a, 4, idims, istr, ibox, true) : tc_make_map(g.a, 3, adims, astr, abox, true);
+        *map_b = g.conv_operand == 2 ? tc_make_map(g.b, 4, idims, istr, ibox, true) : tc_make_map(g.b, 3, bdims, bstr, bbox, true);
+    }
+    return true;
 }
 
 std::shared_ptr<void> gemm_persistent_prepare(const GemmParams& g, uint32_t* status_word, int splits, int k_iters_slice,
@@ -592,64 +919,7 @@ std::shared_ptr<void> gemm_persistent_prepare(const GemmParams& g, uint32_t* sta
     const int fixed = 1024 + 2 * kGpStageTileBytes + 16 * 8 + 64 + 64;
     p.stages = std::max(2, std::min(6, (227 * 1024 - fixed) / stage_bytes));
     l->smem_bytes = fixed + p.stages * stage_bytes;
-    p.a_batch = (g.batch > 1 && g.sa[0] == 0) ? 0 : 1;
-    int64_t adims[3] = {g.k, g.m, p.a_batch ? g.batch : 1}, astr[3] = {1, g.sa[1], p.a_batch ? g.sa[0] : align};
-    int abox[3] = {block_k, kGpBlockM, 1};
-    p.b_batch = (g.batch > 1 && g.sb[0] == 0) ? 0 : 1;
-    int64_t bdims[3] = {g.k, g.n, p.b_batch ? g.batch : 1}, bstr[3] = {1, g.sb[2], p.b_batch ? g.sb[0] : align};
-    int bbox[3] = {block_k, pair ? p.bn / 2 : p.bn, 1};
-    // the implicit convolution operand: a 4-D map of the image tensor (channel, x, y, image) whose box is one K
-    // block of channels by whole output rows
-    int64_t idims[4] = {g.conv_c, g.conv_w, g.conv_h, g.batch}, istr[4] = {1, g.conv_strides[2], g.conv_strides[1], g.conv_strides[0]};
-    int ibox[4] = {32, 1, 1, 1};
-    if (g.conv_operand != 0) {
-        const int rows = g.conv_operand == 1 ? kGpBlockM : p.bn;
-        if (half || g.conv_c % 32 != 0 || g.conv_ow < 1 || g.conv_ow > 256 || rows % g.conv_ow != 0 || g.conv_r < 1 || g.conv_s < 1 ||
-            g.k != (int64_t)g.conv_r * g.conv_s * g.conv_c)
-            return nullptr;
-        ibox[1] = g.conv_ow;
-        ibox[2] = rows / g.conv_ow;
-        p.conv_operand = g.conv_operand;
-        p.conv_cblocks = g.conv_c / 32;
-        p.conv_s = g.conv_s;
-        p.conv_pad_y = g.conv_pad_y;
-        p.conv_pad_x = g.conv_pad_x;
-        p.conv_ow = g.conv_ow;
-    }
-    // 4-D operands: the box is one K block by the tile's rows inside one (x, y) entry
-    auto operand_4d = [&](const GemmOperand4D& o, const void* base, int rows, int64_t matrix_rows, int32_t* kd_shift, int32_t* rd, int32_t* bi,
-                          CUtensorMap* map) {
-        if (!o.enabled) return true;
-        if (o.kd < 1 || o.rd < 1 || o.bi < 1 || o.strides[0] != 1 || g.conv_operand != 0) return false;
-        int shift = 0;
-        if (o.kd != g.k) {   // the K offset is split: whole K blocks inside one entry, by a shift
-            if (o.kd % block_k != 0 || (o.kd & (o.kd - 1)) != 0) return false;
-            while ((1 << shift) < o.kd) shift++;
-        }
-        // a tile's rows lie inside one entry: an entry's rows are a multiple of the tile's, or the matrix is one entry
-        // tall (then rows past its end are past the tensor's extent: zero fill)
-        if (o.rd % rows != 0 && o.rd < matrix_rows) return false;
-        int box[4] = {block_k, rows, 1, 1};
-        *map = half ? tc_make_map_f16(base, 4, o.dims, o.strides, box, true) : tc_make_map(base, 4, o.dims, o.strides, box, true);
-        *kd_shift = shift;
-        *rd = o.rd;
-        *bi = o.bi;
-        return true;
-    };
-    if (!operand_4d(g.a4, g.a, kGpBlockM, g.m, &p.a4_kd_shift, &p.a4_rd, &p.a4_bi, &l->map_a)) return nullptr;
-    if (!operand_4d(g.b4, g.b, p.bn, g.n, &p.b4_kd_shift, &p.b4_rd, &p.b4_bi, &l->map_b)) return nullptr;
-    if (g.a4.enabled && g.b4.enabled) {
-    } else if (g.a4.enabled) {
-        l->map_b = half ? tc_make_map_f16(g.b, 3, bdims, bstr, bbox, true) : tc_make_map(g.b, 3, bdims, bstr, bbox, true);
-    } else if (g.b4.enabled) {
-        l->map_a = half ? tc_make_map_f16(g.a, 3, adims, astr, abox, true) : tc_make_map(g.a, 3, adims, astr, abox, true);
-    } else if (half) {
-        l->map_a = tc_make_map_f16(g.a, 3, adims, astr, abox, true);
-        l->map_b = tc_make_map_f16(g.b, 3, bdims, bstr, bbox, true);
-    } else {
-        l->map_a = g.conv_operand == 1 ? tc_make_map(g.a, 4, idims, istr, ibox, true) : tc_make_map(g.a, 3, adims, astr, abox, true);
-        l->map_b = g.conv_operand == 2 ? tc_make_map(g.b, 4, idims, istr, ibox, true) : tc_make_map(g.b, 3, bdims, bstr, bbox, true);
-    }
+    if (!operand_maps(g, pair ? p.bn / 2 : p.bn, p, &l->map_a, &l->map_b)) return nullptr;
     int64_t cdims[3] = {g.n, g.m, g.batch * splits}, cstr[3] = {1, split ? g.n : g.sc[1], split ? g.m * g.n : g.sc[0]};
     int cbox[3] = {32, kGpBlockM, 1};
     if (p.out_half) l->map_c = tc_make_map_f16(g.c, 3, cdims, cstr, cbox, false);
@@ -698,6 +968,133 @@ int gemm_persistent_launch(const void* launch, cudaStream_t stream) {
     if (l.half) launch_pdl(gemm_persistent_kernel<true, false>, dim3(l.grid), dim3(kGpThreads), (size_t)(l.smem_bytes), stream, l.map_a, l.map_b, l.map_c, l.p);
     else launch_pdl(gemm_persistent_kernel<false, false>, dim3(l.grid), dim3(kGpThreads), (size_t)(l.smem_bytes), stream, l.map_a, l.map_b, l.map_c, l.p);
     return (int)cudaGetLastError();
+}
+
+// Tile width and K slices for gemm_slices_kernel; slices = 0: the matmul is for the persistent kernel.
+//
+// The line: less than one round of the chip in the persistent kernel's tiles (at most 148 of 128 rows x its block width), or
+// an f16 result whose rows do not start on 16-byte boundaries, which that kernel's stores cannot write.  Within it the
+// narrowest total wins, in SM cycles: a K block costs its MMAs (bn / 2 cycles each, four of them) or its bytes at the 60 per
+// cycle that an SM was measured to take from L2, whichever is longer; storing and summing a partial tile costs by its width,
+// a cluster some 1 200 cycles more, a CTA 2 500 before its first MMA.  A round holds fewer CTAs than there are SMs when
+// they come in clusters, which lie inside a GPC (kClusterCtas).
+GemmSlices gemm_slices_choose(const GemmParams& g) {
+    // CTAs of one per SM that fit the chip at once, by the size of their clusters (cudaOccupancyMaxActiveClusters)
+    static const int kClusterCtas[kGsMaxSlices + 1] = {0, 148, 148, 135, 132, 130, 132, 105, 120};
+    GemmSlices none{};
+    if (g.batch < 1 || g.m < 1 || g.n < 8 || g.k < 1 || g.row_softmax != 0) return none;
+    const int64_t m_tiles = (g.m + kGpBlockM - 1) / kGpBlockM;
+    const int64_t wide = gemm_persistent_bn(g.n);
+    const int64_t persistent_tiles = m_tiles * ((g.n + wide - 1) / wide) * g.batch;
+    const bool unaligned_half = g.half != 0 && (g.sc[2] != 1 || g.sc[1] % 8 != 0 || (g.batch > 1 && g.sc[0] % 8 != 0));
+    if (persistent_tiles > 148 && !unaligned_half) return none;
+    const int64_t k_blocks = (g.k + (g.half ? 63 : 31)) / (g.half ? 64 : 32);
+    GemmSlices best{};
+    double best_cost = 0;
+    for (int bn = 32; bn <= 256; bn += 32) {
+        if (bn > 32 && bn - 32 >= g.n) break;
+        if (g.conv_operand == 2 && bn % g.conv_ow != 0) continue;
+        if (g.b4.enabled && g.b4.rd % bn != 0 && g.b4.rd < g.n) continue;
+        const int64_t tiles = m_tiles * ((g.n + bn - 1) / bn) * g.batch;
+        if (tiles > (1 << 24)) continue;
+        const double block = std::max(2.0 * bn, (kGpATileBytes + 128.0 * bn) / 60.0);
+        for (int64_t want = 1; want <= kGsMaxSlices && want <= k_blocks; want++) {
+            const int64_t per = (k_blocks + want - 1) / want, slices = (k_blocks + per - 1) / per;
+            if (slices != want) continue;
+            const double rounds = std::ceil((double)(tiles * slices) / kClusterCtas[slices]);
+            const double cost = rounds * (2500.0 + per * block + (slices > 1 ? 24.0 * bn + 1200.0 : 16.0 * bn));
+            if (best.slices == 0 || cost < best_cost) {
+                best_cost = cost;
+                best.slices = (int)slices;
+                best.bn = bn;
+            }
+        }
+    }
+    return best;
+}
+
+std::shared_ptr<void> gemm_slices_prepare(const GemmParams& g, uint32_t* status_word) {
+    if (g.slices < 1 || g.slices > kGsMaxSlices || g.slices_bn < 32 || g.slices_bn > 256 || g.slices_bn % 32 != 0) return nullptr;
+    auto l = std::make_shared<GemmSlicesLaunch>();
+    memset(&l->p, 0, sizeof(l->p));
+    GemmPersistentParams& p = l->p.g;
+    l->half = g.half != 0;
+    p.bn = g.slices_bn;
+    p.k_iters = (int)((g.k + (l->half ? 63 : 31)) / (l->half ? 64 : 32));
+    p.k_iters_slice = (p.k_iters + g.slices - 1) / g.slices;
+    p.splits = g.slices;
+    if ((int64_t)(p.splits - 1) * p.k_iters_slice >= p.k_iters) return nullptr;   // an empty slice
+    p.m_tiles = (int)((g.m + kGpBlockM - 1) / kGpBlockM);
+    p.n_tiles = (int)((g.n + p.bn - 1) / p.bn);
+    p.batch = (int)g.batch;
+    const int64_t ctas = (int64_t)p.m_tiles * p.n_tiles * g.batch * p.splits;
+    if (ctas > (1 << 30)) return nullptr;
+    p.m = g.m;
+    p.n = g.n;
+    p.add1 = g.add1;
+    p.add2 = g.add2;
+    for (int i = 0; i < 3; i++) {
+        p.s1[i] = g.s1[i];
+        p.s2[i] = g.s2[i];
+        l->p.so[i] = g.sc[i];
+    }
+    p.act = g.act;
+    p.status = status_word;
+    l->p.out = g.c;
+    l->p.a_const = g.a_const;
+    l->p.b_const = g.b_const;
+    const uintptr_t align = l->half ? 7 : 15;
+    auto vec = [&](const void* ptr, const int64_t* st) {
+        return ((uintptr_t)ptr & align) == 0 && st[2] == 1 && st[1] % 4 == 0 && st[0] % 4 == 0 ? 1 : 0;
+    };
+    l->p.out_vec = vec(g.c, g.sc);
+    l->p.add1_vec = vec(g.add1, g.s1);
+    l->p.add2_vec = vec(g.add2, g.s2);
+    l->p.tmem_cols = 32;
+    while (l->p.tmem_cols < p.bn) l->p.tmem_cols *= 2;
+    const int stage_bytes = kGpATileBytes + p.bn * 128, tile_bytes = kGpBlockM * (p.bn + 4) * 4;
+    // (a short slice: no more than half of an SM's shared memory, so that the next kernel's CTA finds room beside it)
+    const bool shared_sm = tile_bytes <= 100 * 1024 && (ctas > 148 || p.k_iters_slice * stage_bytes <= 200 * 1024);
+    const int room = (shared_sm ? 108 : 224) * 1024;
+    p.stages = std::max(1, std::min(std::min(p.k_iters_slice, 8), room / stage_bytes));
+    l->smem_bytes = 1024 + std::max(p.stages * stage_bytes, tile_bytes) + 16 * p.stages + 32;
+    if (!operand_maps(g, p.bn, p, &l->map_a, &l->map_b)) return nullptr;
+    l->grid = (unsigned)ctas;
+    return l;
+}
+
+int gemm_slices_launch(const void* launch, cudaStream_t stream) {
+    const GemmSlicesLaunch& l = *(const GemmSlicesLaunch*)launch;
+    static std::mutex mu;
+    static bool done[64] = {false};
+    int device = 0;
+    cudaGetDevice(&device);
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (device >= 0 && device < 64 && !done[device]) {
+            for (const void* v : {(const void*)gemm_slices_kernel<false>, (const void*)gemm_slices_kernel<true>}) {
+                cudaError_t e = cudaFuncSetAttribute(v, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+                if (e != cudaSuccess) return (int)e;
+            }
+            done[device] = true;
+        }
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(l.grid);
+    cfg.blockDim = dim3(kGsThreads);
+    cfg.dynamicSmemBytes = (size_t)l.smem_bytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)l.p.g.splits;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = l.p.g.splits > 1 ? 2 : 1;
+    if (l.half) return (int)cudaLaunchKernelEx(&cfg, gemm_slices_kernel<true>, l.map_a, l.map_b, l.p);
+    return (int)cudaLaunchKernelEx(&cfg, gemm_slices_kernel<false>, l.map_a, l.map_b, l.p);
 }
 
 }  // namespace kn

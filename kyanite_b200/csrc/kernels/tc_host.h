@@ -32,6 +32,10 @@ CUtensorMap tc_make_map_f16(const void* base, int rank, const int64_t* dims, con
 std::shared_ptr<void> gemm_persistent_prepare(const GemmParams& g, uint32_t* status_word, int splits, int k_iters_slice,
                                               uint32_t* trace_words = nullptr);
 int gemm_persistent_launch(const void* launch, cudaStream_t stream);
+// One tile and one K slice per CTA, slices summed inside a cluster (kernels/gemm_persistent.cu): null if the step does not
+// qualify.
+std::shared_ptr<void> gemm_slices_prepare(const GemmParams& g, uint32_t* status_word);
+int gemm_slices_launch(const void* launch, cudaStream_t stream);
 
 // Matmul with a row softmax (attention scores, kernels/attn_softmax.cu): null if the step does not qualify.
 bool attn_softmax_fits(int64_t batch, int64_t m, int64_t n, int64_t k);

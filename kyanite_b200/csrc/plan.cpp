@@ -228,6 +228,10 @@ class Planner {
             for (size_t j = 0; j < i; j++) dup = dup || s.operands[j].same_storage(s.operands[i]);
             if (!dup) s.alg_bytes += touched_bytes(s.operands[i]);
         }
+        if (s.kind == StepKind::Gemm) {
+            s.gemm.a_const = plan_.buffers[s.operands[0].buf].kind == BufKind::Const ? 1 : 0;
+            s.gemm.b_const = plan_.buffers[s.operands[1].buf].kind == BufKind::Const ? 1 : 0;
+        }
         plan_.steps.push_back(std::move(s));
     }
 
@@ -1120,6 +1124,14 @@ class Planner {
             if (g_.values[u].op == OpKind::MatMul) matmuls_of_[g_.values[u].inputs[0]].push_back(u);
         }
     }
+    bool is_output_view(int v) {   // `v` or a view of it is an output of the graph
+        ensure_readers();
+        for (int o : g_.outputs)
+            if (o == v) return true;
+        for (int u : readers_[v])
+            if (g_.values[u].op == OpKind::View && is_output_view(u)) return true;
+        return false;
+    }
     bool only_contraction_readers(int v) {
         ensure_readers();
         for (int u : readers_[v]) {
@@ -1186,7 +1198,7 @@ class Planner {
         if (!first) return std::nullopt;
         const std::vector<int64_t> xs = shape_of(x);
         const int64_t m = xs[1], k = xs[2];
-        if (m < 256 || k % 4 != 0) return std::nullopt;
+        if (m < 64 || k % 4 != 0) return std::nullopt;
         // the other projections of x: an Add over a MatMul of x that nothing else reads
         std::vector<Projection> all{*first};
         ensure_readers();
@@ -1212,13 +1224,19 @@ class Planner {
         if (all.size() < 2) return std::nullopt;
         int64_t n_total = 0;
         for (auto& p : all) n_total += p.n;
-        // only where the separate matmuls leave CTA pairs idle in their last round of 256 x 256 tiles
+        if (n_total > (1 << 20)) return std::nullopt;
+        // One round of the chip or less: one launch instead of several (120 x 768 x 768 three times: every one of them is
+        // a launch and the latency of its first loads).  Beyond that only where the separate matmuls leave CTA pairs idle
+        // in their last round of 256 x 256 tiles.
+        // (few rows: not where a result is an output of the graph, for which the column slice would have to be copied)
+        const bool one_round = ((m + 127) / 128) * ((n_total + 255) / 256) <= 148;
+        if (m < 256)
+            for (auto& p : all)
+                if (is_output_view(p.root)) return std::nullopt;
         auto rounds = [&](int64_t n) { return (double)(((m + 255) / 256) * ((n + 255) / 256)) / 74.0; };
         double separate = 0;
         for (auto& p : all) separate += std::ceil(rounds(p.n));
-        if (std::ceil(rounds(n_total)) >= separate || n_total > (1 << 20)) return std::nullopt;
-        // (a result of few tiles under a long reduction is cut along K by the planner: not here)
-        if (((m + 127) / 128) * ((n_total + 255) / 256) < 74 && k >= 512) return std::nullopt;
+        if (!one_round && (m < 256 || std::ceil(rounds(n_total)) >= separate)) return std::nullopt;
         bool any_bias = false;
         for (auto& p : all) any_bias = any_bias || p.has_bias;
         PlanTensor xt = visit(x);
@@ -1271,9 +1289,10 @@ class Planner {
             if (any_bias) p.s1[i] = bias.ss.strides[i];
         }
         p.splits = 1;
+        take_slices(p);
         s.flops = 2.0 * (double)m * (double)n_total * (double)k;
         s.desc = "matmul b=1 m=" + std::to_string(m) + " n=" + std::to_string(n_total) + " k=" + std::to_string(k) + (any_bias ? " +1" : " +0") + " tf32 (" +
-                 std::to_string(all.size()) + " projections of one tensor)";
+                 std::to_string(all.size()) + " projections of one tensor)" + slices_desc(p);
         push_step(std::move(s));
         // every projection is a column slice of the result, seen in the shape of its sum
         col = 0;
@@ -1465,7 +1484,7 @@ class Planner {
                 const int64_t bn = std::min<int64_t>(((p.n + n_blocks - 1) / n_blocks + 31) / 32 * 32, 256);
                 const int64_t tiles = ((p.m + 127) / 128) * ((p.n + bn - 1) / bn) * p.batch;
                 const int64_t k_blocks = (p.k + 31) / 32;
-                if (tiles < 74 && k_blocks >= 16) {
+                if (!take_slices(p) && tiles < 74 && k_blocks >= 16) {
                     // aim at one CTA per SM
                     int64_t splits = std::min<int64_t>(std::min<int64_t>(k_blocks / 4, (148 + tiles - 1) / tiles), 32);
                     if (splits > 1) {
@@ -1519,6 +1538,7 @@ class Planner {
                   (m->act == Activation::Relu ? " relu" : (m->act == Activation::Gelu ? " gelu" : ""));
         if (tensor_core) s.desc += " tf32";
         if (s.kind == StepKind::Gemm && s.gemm.splits > 1) s.desc += " splitk=" + std::to_string(s.gemm.splits);
+        if (s.kind == StepKind::Gemm) s.desc += slices_desc(s.gemm);
         int64_t total = 1;
         for (int64_t d : native) total *= d;
         if (a4.enabled || b4.enabled)
@@ -1743,7 +1763,7 @@ class Planner {
             const int64_t bn = std::min<int64_t>(((p.n + n_blocks - 1) / n_blocks + 31) / 32 * 32, 256);
             const int64_t tiles = ((p.m + 127) / 128) * ((p.n + bn - 1) / bn) * p.batch;
             const int64_t k_blocks = (p.k + 63) / 64;
-            if (tiles < 74 && k_blocks >= 16 && p.n % 4 == 0) {
+            if (!take_slices(p) && tiles < 74 && k_blocks >= 16 && p.n % 4 == 0) {
                 int64_t splits = std::min<int64_t>(std::min<int64_t>(k_blocks / 4, (148 + tiles - 1) / tiles), 32);
                 if (splits > 1) {
                     const int64_t per = (k_blocks + splits - 1) / splits;
@@ -1758,9 +1778,23 @@ class Planner {
         }
         s.flops = 2.0 * (double)p.batch * (double)p.m * (double)p.n * (double)p.k;
         s.desc = "matmul b=" + std::to_string(p.batch) + " m=" + std::to_string(p.m) + " n=" + std::to_string(p.n) + " k=" +
-                 std::to_string(p.k) + " +0 f16" + (p.splits > 1 ? " splitk=" + std::to_string(p.splits) : "");
+                 std::to_string(p.k) + " +0 f16" + (p.splits > 1 ? " splitk=" + std::to_string(p.splits) : "") +
+                 slices_desc(p);
         if (out.ss.size() != 0) push_step(std::move(s));
         return out;
+    }
+
+    // a tensor-core matmul of few tiles: its K slices are summed inside a cluster
+    bool take_slices(GemmParams& p) const {
+        if (opts_.flags & KN_FLAG_NO_PERSISTENT_GEMM) return false;
+        const GemmSlices c = gemm_slices_choose(p);
+        p.slices = c.slices;
+        p.slices_bn = c.bn;
+        return c.slices > 0;
+    }
+    static std::string slices_desc(const GemmParams& p) {
+        if (p.slices < 1) return "";
+        return (p.slices > 1 ? " splitk=" + std::to_string(p.slices) + " in a cluster" : std::string()) + " tile=" + std::to_string(p.slices_bn);
     }
 
     // ---------------------------------------------------------------- tensor-core eligibility

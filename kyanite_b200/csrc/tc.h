@@ -18,6 +18,13 @@ void set_last_error(const std::string& message);
 
 // Column-block width the persistent matmul kernel picks for a matrix with n columns (kernels/gemm_persistent.cu).
 int gemm_persistent_bn(int64_t n);
+// Tile width and number of K slices for a tensor-core matmul of few tiles, whose slices are summed inside a cluster
+// (GemmParams::slices); slices = 0 where the persistent kernel is the better one.
+struct GemmParams;
+struct GemmSlices {
+    int slices = 0, bn = 0;
+};
+GemmSlices gemm_slices_choose(const GemmParams& g);
 
 // Shapes the fused attention-scores kernel takes (kernels/attn_softmax.cu): pure host arithmetic.
 bool attn_softmax_fits(int64_t batch, int64_t m, int64_t n, int64_t k);

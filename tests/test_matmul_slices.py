@@ -1,0 +1,83 @@
+"""Matmuls of less than one round of the chip: one tile and one K slice per CTA, the slices of a tile summed inside a cluster
+(gemm_slices_kernel).  The reference calls cublasSgemmStridedBatched and a kernel for what follows:
+kn-cuda-sys/src/wrapper/group.rs:120-171."""
+import re
+
+import numpy as np
+import pytest
+
+from kyanite_b200.executor import FLAG_NO_PERSISTENT_GEMM, MATH_F32, MATH_TF32, plan_describe
+from kyanite_b200.graph import DType, Graph, shape
+from oracle.cpu_eval import assert_tensors_match, cpu_eval_graph
+
+SHAPES = [
+    # (b, m, n, k)
+    (1, 64, 16, 512),        # one tile, narrower than its 32 columns
+    (1, 120, 768, 768),
+    (1, 129, 100, 1000),     # a row past a tile, a ragged last column block, a K tail
+    (1, 333, 200, 96),       # fewer K blocks than a cluster has CTAs
+    (3, 100, 72, 260),
+    (1, 256, 1024, 4096),
+    (2, 128, 33 * 4, 2048),
+]
+
+
+def build(b, m, n, k, half=False, bias=False, residual=False, relu=False, constant=True, seed=0):
+    r = np.random.Generator(np.random.PCG64(seed))
+    dtype, np_dtype = (DType.F16, np.float16) if half else (DType.F32, np.float32)
+    g = Graph()
+    x = g.input(shape(b, m, k), dtype)
+    inputs = [r.standard_normal((b, m, k)).astype(np_dtype)]
+    weights = (r.standard_normal((b, n, k)) / np.sqrt(k)).astype(np_dtype)
+    if constant:
+        w = g.constant_tensor(weights)
+    else:
+        w = g.input(shape(b, n, k), dtype)
+        inputs.append(weights)
+    y = g.batched_mat_mul(x, g.permute(w, [0, 2, 1]))
+    if bias:
+        y = g.add(y, g.constant_tensor(r.standard_normal((1, 1, n)).astype(np_dtype)))
+    if residual:
+        y = g.add(y, g.input(shape(b, m, n), dtype))
+        inputs.append(r.standard_normal((b, m, n)).astype(np_dtype))
+    if relu:
+        y = g.relu(y)
+    g.output(y)
+    return g, inputs
+
+
+def tile(g, mode=MATH_TF32, flags=0):
+    lines = [l for l in plan_describe(g, 0, mode, flags=flags).splitlines() if " tile=" in l]
+    return lines[0] if lines else ""
+
+
+def test_rule():
+    for b, m, n, k in SHAPES:
+        line = tile(build(b, m, n, k)[0])
+        assert line, (b, m, n, k)
+        slices = re.search(r"splitk=(\d+) in a cluster", line)
+        width = int(re.search(r"tile=(\d+)", line).group(1))
+        assert width % 32 == 0 and 32 <= width <= 256 and width - 32 < n
+        assert slices is None or 2 <= int(slices.group(1)) <= min(8, -(-k // 32)), line
+        assert not tile(build(b, m, n, k)[0], MATH_F32) and not tile(build(b, m, n, k)[0], flags=FLAG_NO_PERSISTENT_GEMM)
+    assert not tile(build(1, 4096, 4096, 512)[0])     # rounds of wide tiles: the persistent kernel
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", ["plain", "bias_relu", "bias_residual", "both_inputs", "f16"])
+@pytest.mark.parametrize("b,m,n,k", SHAPES)
+def test_matches_oracle(b, m, n, k, what):
+    from kyanite_b200.executor import CudaExecutor
+    half = what == "f16"
+    if half and (k % 8 != 0 or n % 8 != 0):
+        pytest.skip("rows of f16 that are no multiple of 16 bytes are copied or computed elsewhere")
+    g, inputs = build(b, m, n, k, half, bias="bias" in what, residual="residual" in what, relu="relu" in what,
+                      constant=what != "both_inputs", seed=3)
+    assert tile(g)
+    expected = cpu_eval_graph(g.to_bytes(), 0, inputs)
+    with CudaExecutor(0, g, 0, math_mode=MATH_TF32) as ex:
+        got = ex.evaluate(inputs)
+        again = ex.evaluate(inputs)
+    # products of operands of 11 bits (TF32, f16), f32 sums; results of size 1: 2e-3 of the largest
+    assert_tensors_match(expected, got, 2e-3, 2e-3, abs_scaled=True)
+    assert np.array_equal(got[0], again[0])
