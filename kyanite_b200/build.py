@@ -37,6 +37,7 @@ SOURCES = [
     "kernels/gemm_persistent.cu",
     "kernels/attn_softmax.cu",
     "kernels/attention.cu",
+    "kernels/flash.cu",
 ]
 
 NVCC_FLAGS = [

@@ -179,6 +179,11 @@ struct Executor {
                     if (s.gemm.row_softmax == 2) {   // fused attention: the fourth operand is V^T, there are no addends
                         s.gemm.values = s.gemm.add1;
                         s.gemm.add1 = nullptr;
+                    } else if (s.gemm.row_softmax == 3) {   // V, then the additive term and its table, if there are any
+                        s.gemm.values = s.gemm.add1;
+                        s.gemm.add1 = s.gemm.add2;
+                        s.gemm.add2 = nullptr;
+                        s.gemm.term_blocks = ptr.size() > 5 ? ptr[5] : nullptr;
                     }
                     break;
                 case StepKind::Conv:

@@ -157,8 +157,14 @@ struct GemmParams {
     // at most 512 columns, no addends, no activation (kernels/attn_softmax.cu; tensor cores only).
     // 2: the step goes on to C = softmax(...) . V without writing the probabilities: `values` is V^T, [batch][values_cols][n]
     // with element strides `values_strides` (the last is 1), C is [batch][m][values_cols] (kernels/attention.cu).
+    // 3: attention over any number of keys (kernels/flash.cu): as 2 with `values_mn`, f32 or f16; the additive term of
+    // softmax(softmax_scale * A.B + term), if there is one, is `add1` with strides `s1`, of which `term_cols` columns of a row
+    // may be read (past n: padding); batch entry bt of C lies at (bt / out_heads) * sc[0] + (bt % out_heads) * sc[1], its
+    // rows sc[2] apart, columns contiguous.
     int32_t row_softmax;
     float softmax_scale;
+    int32_t out_heads, term_cols;
+    const void* term_blocks;   // I16 table of a constant term, or null (FlashParams::term_blocks)
     // `values_mn`: `values` is V itself, [batch][n][values_cols] with the columns contiguous (strides as above), or, with
     // `v4`, a head split read in place (rows = keys, K = columns).
     const float* values;

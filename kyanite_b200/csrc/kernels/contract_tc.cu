@@ -703,6 +703,7 @@ struct TcLaunch {
     std::shared_ptr<void> gemm_p; // matmul taken by the persistent kernel (kernels/gemm_persistent.cu)
     std::shared_ptr<void> gemm_s; // matmul of few tiles, K slices summed inside a cluster (kernels/gemm_persistent.cu)
     std::shared_ptr<void> attn;   // matmul with a row softmax (kernels/attn_softmax.cu)
+    std::shared_ptr<void> flash;  // attention over any number of keys (kernels/flash.cu)
     std::shared_ptr<void> attention;   // scores, softmax and probabilities . V (kernels/attention.cu)
 };
 
@@ -905,6 +906,12 @@ void tc_prepare_step(Step& step, uint32_t* status_word, int flags, uint32_t* tra
     int64_t n_cols;
     if (step.kind == StepKind::Gemm) {
         const GemmParams& g = step.gemm;
+        if (g.row_softmax == 3) {
+            launch->flash = flash_attention_prepare(g, status_word);
+            KN_CHECK(launch->flash != nullptr, KN_ERR_INTERNAL, "attention step does not qualify");
+            step.tc = launch;
+            return;
+        }
         if (g.row_softmax == 2) {
             launch->attention = attention_prepare(g, status_word);
             KN_CHECK(launch->attention != nullptr, KN_ERR_INTERNAL, "fused attention step does not qualify");
@@ -1117,6 +1124,7 @@ static int launch_splitk_reduce(const SplitKReduceParams& r, cudaStream_t stream
 int tc_launch_step(const Step& step, cudaStream_t stream) {
     const TcLaunch& l = *step.tc;
     if (l.chain) return chain_launch(l.chain.get(), stream);
+    if (l.flash) return flash_attention_launch(l.flash.get(), stream);
     if (l.attention) return attention_launch(l.attention.get(), stream);
     if (l.attn) return attn_softmax_launch(l.attn.get(), stream);
     if (l.gemm_s) return gemm_slices_launch(l.gemm_s.get(), stream);

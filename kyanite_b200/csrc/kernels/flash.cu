@@ -1,0 +1,474 @@
+// Attention over any number of keys for sm_100a: out = softmax(scale * Q . K^T + term) . V without the scores or the
+// probabilities ever leaving the SM, one CTA per (batch entry, 128 query rows).  Operands in f32 storage (TF32 on load,
+// kind::tf32) or f16 storage (kind::f16); statistics, sums and both accumulators are f32 in either.
+//
+// The keys are taken 128 at a time.  A block's scores are one accumulator of 128 columns in tensor memory; its
+// probabilities take the place of the scores (f16: packed, half the columns) and are the A operand of the second MMA, whose
+// accumulator of up to 128 columns is kept over all blocks.  Exponentials are taken against a reference that follows the
+// row's running maximum only when that has risen by more than 8 (in powers of two): then the row's accumulator and sum are
+// rescaled, which after the first few blocks hardly ever happens; the quotient does not depend on the reference.
+//
+//   warps 0..7      softmax: a row per lane quarter and lane, its 128 columns on two warps of 64 (the maximum and, at the
+//                   end, the sum are exchanged through shared memory)
+//   warp 8 lane 0   producer: Q once, keys and values of a block through one buffer each; the next block's keys are
+//                   requested when the score MMAs have read this block's, under the exponentials
+//   warp 9 lane 0   MMA issuer
+//
+// Inside a CTA the phases of a block follow one another (scores, exponentials, context); what fills the tensor cores and
+// the special-function unit meanwhile is the SM's second CTA: 256 columns of tensor memory, some 100 KB of shared memory
+// (head dimensions up to 64 in f32 or 128 in f16; larger ones run one CTA per SM).
+//
+// Measured, scores matmul + softmax + copies + context matmul planned node by node -> this step: 32 heads of 2048 causal
+// rows, f16, d = 128: 122 + 155 + 15 + 57 -> 84 us; 8 heads of 4096 rows, f32,
+// d = 40: 117 + 198 + 99 -> 137 us; 12 heads of 120 rows: 5 + 3 + 14 + 4 -> 9 us; 32 heads of 333 rows, f16: 215 -> 18 us.
+// What bounds it: a block is some 6 000 cycles of a CTA (scores seen 1 200 after the issuer starts them, read 1 000, maximum
+// 300, exponentials 1 800, context MMAs 1 300 at 80 cycles an instruction with A from tensor memory), two CTAs in turn.
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
+#include <memory>
+#include <mutex>
+#include <type_traits>
+
+#include "../tc.h"
+#include "tc_host.h"
+#include "tc_ptx.cuh"
+#include "launch.cuh"
+
+namespace kn {
+
+namespace {
+
+using namespace tcp;
+
+constexpr int kFlThreads = 320;
+constexpr int kFlRows = 128, kFlKeys = 128;
+constexpr int kFlBlockBytes = 128 * 128;   // 128 rows of 128 bytes
+constexpr int kFlTmemCols = 256, kFlOutCol = 128;
+constexpr float kLog2e = 1.44269504088896340736f;
+constexpr float kRiseLimit = 8.0f;
+constexpr uint32_t kFlSleepNs = 1000;
+
+struct FlashParams {
+    int32_t m, n, batch, m_tiles, key_blocks;
+    int32_t qk_blocks, qk_steps;     // 128-byte blocks of a row of Q; instructions of 32 bytes along it
+    int32_t dv, v_panels, out_cols;  // columns of V, 128-byte panels of them, N of the context MMAs
+    int32_t a_bi, b_bi, v_bi;        // batch entry bt -> map coordinates (bt % bi, bt / bi)
+    float scale;
+    void* out;
+    int32_t out_heads;               // out[bt / out_heads][bt % out_heads][row][column] with strides out_s (the last 1)
+    int64_t out_s[3];
+    const void* term;                // additive term [batch][m][n], or null
+    int64_t term_s[3];
+    int32_t term_cols;               // columns of a row that may be read: n, or more with padding
+    // of a constant term that all batch entries share: per row block the number of key blocks to visit (what follows is
+    // -infinity), then per key block whether the term has to be read (0: it is zero); else null
+    const int16_t* term_blocks;
+    uint32_t* status;
+};
+
+__device__ __forceinline__ void mma_f16_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void arrive_one(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tmem_loads_done() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_stores_done() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+template <bool HALF, bool TERM>
+__global__ void __launch_bounds__(kFlThreads, 2)
+flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ FlashParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    constexpr int kElems = HALF ? 64 : 32;   // elements per 128 bytes
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t k_base = base + (uint32_t)(p.qk_blocks * kFlBlockBytes);
+    const uint32_t v_base = k_base + (uint32_t)(p.qk_blocks * kFlBlockBytes);
+    const uint32_t exch = v_base + (uint32_t)(p.v_panels * kFlBlockBytes);
+    float* exchange = (float*)(gen_base + (exch - base));   // [2 column halves][128 rows]
+    const uint32_t q_full = exch + 1024u, k_full = q_full + 8u, s_full = q_full + 16u, v_full = q_full + 24u, p_ready = q_full + 32u,
+                   pv_done = q_full + 40u, slot_addr = q_full + 48u;
+    volatile uint32_t* tmem_slot = (volatile uint32_t*)(gen_base + (slot_addr - base));
+    volatile int* abandon = (volatile int*)(gen_base + (slot_addr + 4u - base));
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        mbar_init(q_full, 1);
+        mbar_init(k_full, 1);
+        mbar_init(s_full, 1);
+        mbar_init(v_full, 1);
+        mbar_init(p_ready, 8);
+        mbar_init(pv_done, 1);
+        *abandon = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 8) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_addr), "r"((uint32_t)kFlTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_s = *tmem_slot, tmem_o = tmem_s + (uint32_t)kFlOutCol;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    // the last row blocks first: under a causal mask they have the most keys
+    const int bt = (int)(blockIdx.x % (unsigned)p.batch), mt = p.m_tiles - 1 - (int)(blockIdx.x / (unsigned)p.batch);
+    const int16_t* blocks_of = TERM && p.term_blocks ? p.term_blocks + (int64_t)mt * (p.key_blocks + 1) : nullptr;   // (a constant)
+    const int n_blocks = blocks_of ? (int)blocks_of[0] : p.key_blocks;
+    auto block_cols = [&](int j) { return min(kFlKeys, (p.n - j * kFlKeys + 31) & ~31); };   // (past n: zero fill, masked below)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    if (warp == 8) {
+        if (lane == 0) {
+            // ---------------- producer
+            const uint32_t qk_bytes = (uint32_t)(p.qk_blocks * kFlBlockBytes), v_bytes = (uint32_t)(p.v_panels * kFlBlockBytes);
+            mbar_expect_tx(q_full, qk_bytes);
+            for (int b = 0; b < p.qk_blocks; b++)
+                tma_load_4d(base + (uint32_t)(b * kFlBlockBytes), &map_q, q_full, b * kElems, mt * kFlRows, bt % p.a_bi, bt / p.a_bi);
+            const int k2 = bt % p.b_bi, k3 = bt / p.b_bi, v2 = bt % p.v_bi, v3 = bt / p.v_bi;
+            for (int j = 0; j < n_blocks; j++) {
+                if (j > 0 && !mbar_wait(s_full, (uint32_t)((j - 1) & 1), abandon, p.status, 51, kWaitCycles, kFlSleepNs)) break;
+                mbar_expect_tx(k_full, qk_bytes);
+                for (int b = 0; b < p.qk_blocks; b++)
+                    tma_load_4d(k_base + (uint32_t)(b * kFlBlockBytes), &map_k, k_full, b * kElems, j * kFlKeys, k2, k3);
+                if (j > 0 && !mbar_wait(pv_done, (uint32_t)((j - 1) & 1), abandon, p.status, 52, kWaitCycles, kFlSleepNs)) break;
+                mbar_expect_tx(v_full, v_bytes);
+                for (int b = 0; b < p.v_panels; b++)
+                    tma_load_4d(v_base + (uint32_t)(b * kFlBlockBytes), &map_v, v_full, b * kElems, j * kFlKeys, v2, v3);
+            }
+        }
+    } else if (warp == 9) {
+        if (lane == 0) {
+            // ---------------- MMA issuer: f32 accumulate, M = 128; Q and the keys K-major, V with its columns contiguous
+            // (bit 16: the MN-major B operand)
+            const uint32_t fmt = HALF ? 0u : 2u;
+            const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(kFlRows >> 4) << 24);
+            const uint32_t idesc_o = idesc | (1u << 16) | ((uint32_t)(p.out_cols >> 3) << 17);
+            // MN-major B: panels of 128 bytes of columns lie `leading byte offset` apart, groups of keys `stride byte
+            // offset`: eight keys and the 128-byte swizzle for 16-bit elements, four and the swizzle in 32-byte pieces for
+            // 32-bit ones (see attention.cu)
+            const uint64_t v_desc = ((uint64_t)(kFlBlockBytes >> 4) << 16) | ((uint64_t)((HALF ? 1024 : 512) >> 4) << 32) | ((uint64_t)1 << 46) |
+                                    ((uint64_t)(HALF ? 2 : 1) << 61);
+            constexpr int kStepKeys = HALF ? 16 : 8, kStepCols = 8;   // keys of an instruction; their columns in tensor memory
+            const bool ok = mbar_wait(q_full, 0, abandon, p.status, 53, kWaitCycles, kFlSleepNs);
+            for (int j = 0; j < n_blocks && ok; j++) {
+                const uint32_t parity = (uint32_t)(j & 1);
+                const int cols = block_cols(j);
+                if (!mbar_wait(k_full, parity, abandon, p.status, 54, kWaitCycles, kFlSleepNs)) break;
+                // (the probabilities of the block before lie where the scores go)
+                if (j > 0 && !mbar_wait(pv_done, parity ^ 1u, abandon, p.status, 55, kWaitCycles, kFlSleepNs)) break;
+                tc_fence_after();
+                const uint32_t idesc_s = idesc | ((uint32_t)(cols >> 3) << 17);
+                for (int s = 0; s < p.qk_steps; s++) {
+                    const uint32_t at = (uint32_t)((s >> 2) * kFlBlockBytes);
+                    const uint64_t da = smem_desc_sw128(base + at) + 2u * (s & 3), db = smem_desc_sw128(k_base + at) + 2u * (s & 3);
+                    if (HALF) mma_f16(tmem_s, da, db, idesc_s, s != 0 ? 1u : 0u);
+                    else mma_tf32(tmem_s, da, db, idesc_s, s != 0 ? 1u : 0u);
+                }
+                mma_commit(s_full);
+                if (!mbar_wait(v_full, parity, abandon, p.status, 56, kWaitCycles, kFlSleepNs)) break;
+                if (!mbar_wait(p_ready, parity, abandon, p.status, 57, kWaitCycles, kFlSleepNs)) break;
+                tc_fence_after();
+                for (int s = 0; s < cols / kStepKeys; s++) {
+                    const uint64_t db = v_desc | (uint64_t)(((v_base + (uint32_t)(s * kStepKeys * 128)) & 0x3FFFFu) >> 4);
+                    if (HALF) mma_f16_a_tmem(tmem_o, tmem_s + (uint32_t)(s * kStepCols), db, idesc_o, (j | s) != 0 ? 1u : 0u);
+                    else mma_tf32_a_tmem(tmem_o, tmem_s + (uint32_t)(s * kStepCols), db, idesc_o, (j | s) != 0 ? 1u : 0u);
+                }
+                mma_commit(pv_done);
+            }
+        }
+    } else {
+        // ---------------- softmax
+        const int quarter = warp & 3, half = warp >> 2;
+        const int row_in_tile = quarter * 32 + lane, row = mt * kFlRows + row_in_tile;
+        const uint32_t lane_bits = (uint32_t)(quarter * 32) << 16;
+        const uint32_t my_s = tmem_s + lane_bits + (uint32_t)(half * 64), my_o = tmem_o + lane_bits;
+        using T = typename std::conditional<HALF, __half, float>::type;
+        const T* term_row = TERM ? (const T*)p.term + bt * p.term_s[0] + (int64_t)min(row, p.m - 1) * p.term_s[1] : nullptr;
+        // (the warps meet at barriers, so they must agree on going on: one lane waits, then all vote)
+        auto wait_agreed = [&](uint32_t bar, uint32_t parity, uint32_t code) -> bool {
+            uint32_t good = 1;
+            if (lane == 0) good = mbar_wait(bar, parity, abandon, p.status, code, kWaitCycles, kFlSleepNs) ? 1u : 0u;
+            good = __shfl_sync(0xffffffffu, good, 0);
+            uint32_t all_good;
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\t"
+                "setp.ne.u32 p, %1, 0;\n\t"
+                "bar.red.and.pred q, 1, 256, p;\n\t"
+                "selp.u32 %0, 1, 0, q;\n\t}"
+                : "=r"(all_good)
+                : "r"(good)
+                : "memory");
+            tc_fence_after();
+            return all_good != 0;
+        };
+        // x in units of its exponent: with a term  x = scale * s + term, exponent (x - ref) * log2(e); without one x = s
+        const float unit = TERM ? kLog2e : p.scale * kLog2e;
+        float seen = -INFINITY, ref = 0.f, sum = 0.f;
+        bool ok = true;
+        for (int j = 0; j < n_blocks; j++) {
+            if (!wait_agreed(s_full, (uint32_t)(j & 1), 58)) { ok = false; break; }
+            uint32_t v[2][32];
+            tmem_load_32_nowait(my_s, v[0]);
+            tmem_load_32_nowait(my_s + 32u, v[1]);
+            tmem_loads_done();
+            const int col0 = j * kFlKeys + half * 64;
+            if (TERM) {
+                const bool add = blocks_of == nullptr || blocks_of[1 + j] != 0;
+                if (!add) {
+#pragma unroll
+                    for (int i = 0; i < 64; i++) v[i >> 5][i & 31] = __float_as_uint(p.scale * __uint_as_float(v[i >> 5][i & 31]));
+                } else {
+                    const T* t = term_row + (int64_t)col0 * p.term_s[2];
+                    const bool vec = p.term_s[2] == 1 && col0 + 64 <= p.term_cols && ((uintptr_t)t & 15) == 0;
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+#pragma unroll
+                        for (int i = 0; i < 32; i += 8) {
+                            float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                            if (vec) {
+                                if (HALF) {
+                                    const uint4 u = __ldg((const uint4*)(t + c * 32 + i));
+                                    const __half2* h = (const __half2*)&u;
+#pragma unroll
+                                    for (int q = 0; q < 4; q++) {
+                                        const float2 f = __half22float2(h[q]);
+                                        a[2 * q] = f.x, a[2 * q + 1] = f.y;
+                                    }
+                                } else {
+#pragma unroll
+                                    for (int q = 0; q < 2; q++) {
+                                        const float4 f = __ldg((const float4*)(t + c * 32 + i) + q);
+                                        a[4 * q] = f.x, a[4 * q + 1] = f.y, a[4 * q + 2] = f.z, a[4 * q + 3] = f.w;
+                                    }
+                                }
+                            } else {
+#pragma unroll
+                                for (int q = 0; q < 8; q++)
+                                    if (col0 + c * 32 + i + q < p.n) a[q] = (float)t[(int64_t)(c * 32 + i + q) * p.term_s[2]];
+                            }
+#pragma unroll
+                            for (int q = 0; q < 8; q++) v[c][i + q] = __float_as_uint(fmaf(p.scale, __uint_as_float(v[c][i + q]), a[q]));
+                        }
+                    }
+                }
+            }
+            if (col0 + 64 > p.n) {   // columns past the last key
+#pragma unroll
+                for (int i = 0; i < 64; i++)
+                    if (col0 + i >= p.n) v[i >> 5][i & 31] = 0xFF800000u;
+            }
+            float top = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < 64; i++) top = fmaxf(top, __uint_as_float(v[i >> 5][i & 31]));
+            exchange[half * 128 + row_in_tile] = top;
+            asm volatile("bar.sync 2, 256;" ::: "memory");   // (also: every score of the block has been read)
+            top = fmaxf(top, exchange[(half ^ 1) * 128 + row_in_tile]);
+            // a row whose scores were all -infinity so far has no reference yet (and zeros in its sum and output)
+            const bool first = seen == -INFINITY;
+            seen = fmaxf(seen, top);
+            const bool rise = first || (top - ref) * unit > kRiseLimit;
+            if (__any_sync(0xffffffffu, rise)) {
+                const float next = rise && seen > -INFINITY ? seen : ref;
+                const float factor = rise && !first ? exp2_approx((ref - next) * unit) : 1.f;
+                ref = next;
+                sum *= factor;
+                if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
+                    for (int c = half; c < (p.out_cols + 31) >> 5; c += 2) {
+                        uint32_t o[32];
+                        tmem_load_32(my_o + (uint32_t)(c * 32), o);
+#pragma unroll
+                        for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+                        tmem_store_32(my_o + (uint32_t)(c * 32), o);
+                    }
+                }
+            }
+            const float shift = -ref * unit;
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                    const float x0 = __uint_as_float(v[c][i]), x1 = __uint_as_float(v[c][i + 1]);
+                    // (with a term the difference first: the lowest finite value times log2(e) would overflow)
+                    const float e0 = exp2_approx(TERM ? (x0 - ref) * unit : fmaf(x0, unit, shift));
+                    const float e1 = exp2_approx(TERM ? (x1 - ref) * unit : fmaf(x1, unit, shift));
+                    if (HALF) {
+                        sum += e0 + e1;
+                        const __half2 h = __floats2half2_rn(e0, e1);
+                        v[0][c * 16 + (i >> 1)] = *(const uint32_t*)&h;
+                    } else {
+                        // rounded to the operand's eleven bits here, so that the sum is of what the MMAs see
+                        uint32_t r0, r1;
+                        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r0) : "f"(e0));
+                        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r1) : "f"(e1));
+                        sum += __uint_as_float(r0) + __uint_as_float(r1);
+                        v[c][i] = r0, v[c][i + 1] = r1;
+                    }
+                }
+            }
+            if (HALF) {
+                tmem_store_32(tmem_s + lane_bits + (uint32_t)(half * 32), v[0]);
+            } else {
+                tmem_store_32(my_s, v[0]);
+                tmem_store_32(my_s + 32u, v[1]);
+            }
+            tmem_stores_done();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive_one(p_ready);
+        }
+        if (ok && wait_agreed(pv_done, (uint32_t)((n_blocks - 1) & 1), 59)) {
+            exchange[half * 128 + row_in_tile] = sum;
+            asm volatile("bar.sync 2, 256;" ::: "memory");
+            const float inv = 1.f / (sum + exchange[(half ^ 1) * 128 + row_in_tile]);
+            T* dst = (T*)p.out + (bt / p.out_heads) * p.out_s[0] + (bt % p.out_heads) * p.out_s[1] + (int64_t)row * p.out_s[2];
+            for (int c = half; c < (p.dv + 31) >> 5; c += 2) {
+                uint32_t o[32];
+                tmem_load_32(my_o + (uint32_t)(c * 32), o);
+#pragma unroll
+                for (int i = 0; i < 32; i += 8) {
+                    if (row >= p.m || c * 32 + i >= p.dv) continue;
+                    float f[8];
+#pragma unroll
+                    for (int q = 0; q < 8; q++) f[q] = __uint_as_float(o[i + q]) * inv;
+                    if (HALF) {
+                        uint32_t h[4];
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const __half2 pair = __floats2half2_rn(f[2 * q], f[2 * q + 1]);
+                            h[q] = *(const uint32_t*)&pair;
+                        }
+                        *(uint4*)(dst + c * 32 + i) = make_uint4(h[0], h[1], h[2], h[3]);
+                    } else {
+                        *(float4*)(dst + c * 32 + i) = make_float4(f[0], f[1], f[2], f[3]);
+                        *(float4*)(dst + c * 32 + i + 4) = make_float4(f[4], f[5], f[6], f[7]);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        tc_fence_before();
+    }
+    __syncthreads();
+    if (warp == 8) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_s), "r"((uint32_t)kFlTmemCols) : "memory");
+    }
+}
+
+struct FlashLaunch {
+    CUtensorMap map_q, map_k, map_v;
+    FlashParams p;
+    unsigned grid;
+    int smem_bytes;
+    bool half;
+};
+
+int flash_smem_bytes(int64_t k, int64_t dv, bool half) {
+    const int64_t elems = half ? 64 : 32;
+    return (int)(1024 + (2 * ((k + elems - 1) / elems) + (dv + elems - 1) / elems) * kFlBlockBytes + 1024 + 64);
+}
+
+}  // namespace
+
+bool flash_attention_fits(int64_t batch, int64_t m, int64_t n, int64_t k, int64_t dv, bool half) {
+    if (batch < 1 || m < 1 || n < 1 || k < 8 || dv < 8) return false;
+    if (k > 128 || dv > 128 || k % 8 != 0 || dv % 8 != 0 || n > (1 << 21) || m > (1 << 24)) return false;
+    return batch * ((m + kFlRows - 1) / kFlRows) < (1ll << 30) && flash_smem_bytes(k, dv, half) <= 227 * 1024;
+}
+
+std::shared_ptr<void> flash_attention_prepare(const GemmParams& g, uint32_t* status_word) {
+    const bool half = g.half != 0;
+    const int64_t align = half ? 8 : 4, elems = half ? 64 : 32;
+    if (g.conv_operand != 0 || g.splits > 1 || g.add2 || g.act != 0 || g.row_softmax != 3 || !g.values || !g.values_mn) return nullptr;
+    if (!flash_attention_fits(g.batch, g.m, g.n, g.k, g.values_cols, half)) return nullptr;
+    if (g.out_heads < 1 || g.sc[0] % align != 0 || g.sc[1] % align != 0 || g.sc[2] % align != 0 || ((uintptr_t)g.c & 15) != 0) return nullptr;
+    auto l = std::make_shared<FlashLaunch>();
+    FlashParams& p = l->p;
+    memset(&p, 0, sizeof(p));
+    l->half = half;
+    p.m = (int)g.m;
+    p.n = (int)g.n;
+    p.batch = (int)g.batch;
+    p.m_tiles = (int)((g.m + kFlRows - 1) / kFlRows);
+    p.key_blocks = (int)((g.n + kFlKeys - 1) / kFlKeys);
+    p.qk_blocks = (int)((g.k + elems - 1) / elems);
+    p.qk_steps = (int)((g.k + elems / 4 - 1) / (elems / 4));
+    p.dv = (int)g.values_cols;
+    p.v_panels = (int)((g.values_cols + elems - 1) / elems);
+    p.out_cols = (p.dv + 15) / 16 * 16;
+    p.scale = g.softmax_scale;
+    p.out = g.c;
+    p.out_heads = g.out_heads;
+    for (int i = 0; i < 3; i++) p.out_s[i] = g.sc[i];
+    p.term = g.add1;
+    for (int i = 0; i < 3; i++) p.term_s[i] = g.s1[i];
+    p.term_cols = g.term_cols;
+    p.term_blocks = (const int16_t*)g.term_blocks;
+    p.status = status_word;
+    // an operand [batch, rows, k] as a 4-D map (K offset, row, x, y): a head split read in place as it is, a plain one with
+    // x = the batch entry (bi = batch + 1: coordinates (bt, 0))
+    auto operand = [&](const GemmOperand4D& o, const void* base, int64_t rows, int64_t cols, int64_t s_batch, int64_t s_row, int64_t s_col,
+                       bool mn_major, CUtensorMap* map, int32_t* bi) {
+        int box[4] = {(int)elems, kFlRows, 1, 1};
+        int64_t dims[4] = {cols, rows, g.batch, 1}, strides[4] = {1, s_row, s_batch, align};
+        if (o.enabled) {
+            if (o.kd != cols || o.rd < rows || o.strides[0] != 1) return false;
+            for (int i = 0; i < 4; i++) dims[i] = o.dims[i], strides[i] = o.strides[i];
+            *bi = o.bi;
+        } else {
+            if (s_col != 1 || (rows > 1 && (s_row <= 0 || s_row % align != 0)) || (g.batch > 1 && (s_batch <= 0 || s_batch % align != 0))) return false;
+            *bi = (int)g.batch + 1;
+        }
+        if (((uintptr_t)base & 15) != 0) return false;
+        if (half) *map = tc_make_map_f16(base, 4, dims, strides, box, true);
+        else if (mn_major) *map = tc_make_map_mn_major(base, 4, dims, strides, box);
+        else *map = tc_make_map(base, 4, dims, strides, box, true);
+        return true;
+    };
+    if (!operand(g.a4, g.a, g.m, g.k, g.sa[0], g.sa[1], g.sa[2], false, &l->map_q, &p.a_bi)) return nullptr;
+    if (!operand(g.b4, g.b, g.n, g.k, g.sb[0], g.sb[2], g.sb[1], false, &l->map_k, &p.b_bi)) return nullptr;
+    if (!operand(g.v4, g.values, g.n, g.values_cols, g.values_strides[0], g.values_strides[1], g.values_strides[2], true, &l->map_v, &p.v_bi)) return nullptr;
+    l->smem_bytes = flash_smem_bytes(g.k, g.values_cols, half);
+    l->grid = (unsigned)(g.batch * p.m_tiles);
+    return l;
+}
+
+int flash_attention_launch(const void* launch, cudaStream_t stream) {
+    const FlashLaunch& l = *(const FlashLaunch*)launch;
+    static std::mutex mu;
+    static bool done[64] = {false};
+    int device = 0;
+    cudaGetDevice(&device);
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (device >= 0 && device < 64 && !done[device]) {
+            for (const void* v : {(const void*)flash_attention_kernel<false, false>, (const void*)flash_attention_kernel<false, true>,
+                                  (const void*)flash_attention_kernel<true, false>, (const void*)flash_attention_kernel<true, true>}) {
+                cudaError_t e = cudaFuncSetAttribute(v, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+                if (e != cudaSuccess) return (int)e;
+            }
+            done[device] = true;
+        }
+    }
+    const dim3 grid(l.grid), block(kFlThreads);
+    const size_t smem = (size_t)l.smem_bytes;
+    if (l.half && l.p.term) launch_pdl(flash_attention_kernel<true, true>, grid, block, smem, stream, l.map_q, l.map_k, l.map_v, l.p);
+    else if (l.half) launch_pdl(flash_attention_kernel<true, false>, grid, block, smem, stream, l.map_q, l.map_k, l.map_v, l.p);
+    else if (l.p.term) launch_pdl(flash_attention_kernel<false, true>, grid, block, smem, stream, l.map_q, l.map_k, l.map_v, l.p);
+    else launch_pdl(flash_attention_kernel<false, false>, grid, block, smem, stream, l.map_q, l.map_k, l.map_v, l.p);
+    return (int)cudaGetLastError();
+}
+
+}  // namespace kn

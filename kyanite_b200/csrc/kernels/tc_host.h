@@ -45,6 +45,10 @@ int attn_softmax_launch(const void* launch, cudaStream_t stream);
 bool attention_fits(int64_t batch, int64_t m, int64_t n, int64_t k, int64_t dv);
 std::shared_ptr<void> attention_prepare(const GemmParams& g, uint32_t* status_word);
 int attention_launch(const void* launch, cudaStream_t stream);
+// The same over any number of keys, with an additive term, in f32 or f16 (kernels/flash.cu).
+bool flash_attention_fits(int64_t batch, int64_t m, int64_t n, int64_t k, int64_t dv, bool half);
+std::shared_ptr<void> flash_attention_prepare(const GemmParams& g, uint32_t* status_word);
+int flash_attention_launch(const void* launch, cudaStream_t stream);
 
 // Convolution chain (kernels/conv_chain.cu): launch data built once the device pointers are known.
 std::shared_ptr<void> chain_prepare(const ConvChainParams& c, uint32_t* status_word);

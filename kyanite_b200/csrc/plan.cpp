@@ -528,6 +528,8 @@ class Planner {
 
     PlanTensor visit_new(int v) {
         if (auto fused = try_fused_attention_context(v)) return *fused;
+        if (auto fused = try_flash_attention(v, 0)) return *fused;
+        if (auto fused = try_merged_attention(v)) return *fused;
         if (auto fused = try_fused_contraction(v)) return *fused;
         if (auto fused = try_fused_rmsnorm(v)) return *fused;
         const ValueInfo& info = g_.values[v];
@@ -872,7 +874,7 @@ class Planner {
     // operand is B, given in the graph as [batch, K, rows], so the chain sits under a permute [0, 2, 1].
     // Sets `source` to the planned source tensor (visited here) on success.
     bool head_chain_operand(int value, bool as_b, DType dtype, GemmOperand4D* out, PlanTensor* source, int64_t* batch, int64_t* rows,
-                            int64_t* k) {
+                            int64_t* k, int64_t min_rows = 64) {
         if (opts_.flags & KN_FLAG_NO_PERSISTENT_GEMM) return false;
         if (as_b) {
             const ValueInfo& vi = g_.values[value];
@@ -893,7 +895,7 @@ class Planner {
             o.strides[1] = c->H * c->D; o.strides[2] = c->D; o.strides[3] = c->S * c->H * c->D;
             o.kd = (int32_t)c->D; o.rd = (int32_t)c->S; o.bi = (int32_t)c->H;
             *batch = c->B * c->H; *rows = c->S; *k = c->D;
-            if (c->S < 64) return false;
+            if (c->S < min_rows) return false;
         } else {
             // [B*H, S, D] read as [B*S, H*D]: the K offset is split into (head, offset), whole K blocks per head, and a
             // tile's rows must lie inside one batch entry
@@ -1099,6 +1101,205 @@ class Planner {
             s.desc += std::string(" (head split read in place: operand") + (a4.enabled && b4.enabled ? "s a, b" : (a4.enabled ? " a" : " b")) + ")";
         push_step(std::move(s));
         return out;
+    }
+
+    // ---------------------------------------------------------------- attention over any number of keys
+    // matmul(softmax([c *] matmul(Q, K^T) [+ term]), V), every node in between read by this expression only, in f32 (TF32
+    // mode) or f16: ONE step (kernels/flash.cu) where the steps above do not apply: any number of keys and rows, an
+    // additive term (a mask), f16 storage, head dimensions up to 128.  `heads` > 0: the caller wants the result as
+    // [batch / heads, m, heads, dv] (the head merge that follows), else [batch, m, dv].
+    std::optional<PlanTensor> try_flash_attention(int v, int64_t heads) {
+        const ValueInfo& mi = g_.values[v];
+        const DType type = mi.dtype;
+        if (mi.op != OpKind::MatMul || (type != DType::F32 && type != DType::F16) || shape_of(v).size() != 3) return std::nullopt;
+        if (opts_.math_mode != KN_MATH_TF32 || (opts_.flags & KN_FLAG_NO_PERSISTENT_GEMM)) return std::nullopt;
+        const int sv = mi.inputs[0], vin = mi.inputs[1];
+        const ValueInfo& si = g_.values[sv];
+        if (si.op != OpKind::Softmax || si.dtype != type || si.axis != 2 || !fusable(sv) || map_[sv] || vin == sv) return std::nullopt;
+        const std::vector<int64_t> ss = shape_of(sv), vs = shape_of(vin);
+        if (ss.size() != 3 || vs.size() != 3 || vs[0] != ss[0]) return std::nullopt;
+        const int64_t batch = ss[0], m = ss[1], n = ss[2], dv = vs[2];
+        // softmax's input: the scores matmul, scaled by a constant, plus a term
+        auto scores_of = [&](int y, double* scale) {
+            *scale = 1.0;
+            if (!fusable(y) || map_[y]) return -1;
+            const ValueInfo* yi = &g_.values[y];
+            if (yi->op == OpKind::Binary && (yi->binary_op == BinaryOp::Mul || yi->binary_op == BinaryOp::Div)) {
+                auto c0 = g_.as_single_const(yi->inputs[0]), c1 = g_.as_single_const(yi->inputs[1]);
+                int other;
+                if (c1) *scale = c1->as_f64_value(), other = yi->inputs[0];
+                else if (c0 && yi->binary_op == BinaryOp::Mul) *scale = c0->as_f64_value(), other = yi->inputs[1];
+                else return -1;
+                if (yi->binary_op == BinaryOp::Div) *scale = 1.0 / *scale;
+                if (!std::isfinite(*scale)) return -1;
+                y = other;
+                if (!fusable(y) || map_[y]) return -1;
+                yi = &g_.values[y];
+            }
+            return yi->op == OpKind::MatMul && yi->dtype == type && shape_of(y) == ss ? y : -1;
+        };
+        double scale = 1.0;
+        int scores = scores_of(si.inputs[0], &scale), term = -1;
+        if (scores < 0) {
+            const int sum = si.inputs[0];
+            const ValueInfo& ai = g_.values[sum];
+            if (ai.op != OpKind::Binary || ai.binary_op != BinaryOp::Add || ai.dtype != type || !fusable(sum) || map_[sum]) return std::nullopt;
+            for (int side = 0; side < 2 && scores < 0; side++) {
+                scores = scores_of(ai.inputs[side], &scale);
+                term = ai.inputs[1 - side];
+            }
+            if (scores < 0 || g_.values[term].dtype != type || shape_of(term) != ss) return std::nullopt;
+        }
+        // (without a term the maximum is taken before scaling)
+        if (term < 0 && !(scale > 0.0)) return std::nullopt;
+        const ValueInfo& ci = g_.values[scores];
+        const int64_t k = shape_of(ci.inputs[0])[2];
+        const bool half = type == DType::F16;
+        // (a handful of rows or keys: launches of the small kernels are as short, and exact)
+        if (m < 16 || n < 16 || !flash_attention_fits(batch, m, n, k, dv, half)) return std::nullopt;
+        if (!half && term < 0 && attn_softmax_fits(batch, m, n, k)) return std::nullopt;   // the steps above
+        // operands [batch, rows, cols] with the columns contiguous: head splits read in place, tensors as they are, or copies
+        const int64_t align = half ? 8 : 4;
+        auto operand = [&](int value, bool transposed, int64_t rows, int64_t cols, GemmOperand4D* o) {
+            PlanTensor t;
+            int64_t ob = 0, orows = 0, ocols = 0;
+            if (head_chain_operand(value, transposed, type, o, &t, &ob, &orows, &ocols, 1) && o->kd == cols && ob == batch && orows == rows) return t;
+            *o = GemmOperand4D{};
+            t = visit(value);
+            if (transposed) t = t.with(t.ss.permute({0, 2, 1}));
+            const auto& st = t.ss.strides;
+            auto ok = [&](int64_t dim, int64_t stride) { return dim <= 1 || (stride > 0 && stride % align == 0); };
+            if ((cols > 1 && st[2] != 1) || !ok(rows, st[1]) || !ok(batch, st[0]) || t.offset % align != 0) t = ensure_simple_copy(t, value);
+            return t;
+        };
+        GemmOperand4D a4{}, b4{}, v4{};
+        PlanTensor q = operand(ci.inputs[0], false, m, k, &a4), keys = operand(ci.inputs[1], true, n, k, &b4);
+        PlanTensor values = operand(vin, false, n, dv, &v4);
+        std::optional<PlanTensor> added, table;
+        int64_t term_cols = n;
+        if (term >= 0) {
+            added = visit(term);
+            table = flash_term_blocks(*added, batch, m, n);
+            if (table) added = flash_padded_term(*added, batch, m, n, &term_cols);
+        }
+        const int64_t out_heads = heads > 0 ? heads : batch;
+        PlanTensor out = heads > 0 ? alloc_shared({batch / heads, m, heads, dv}, type, v) : alloc_shared({batch, m, dv}, type, v);
+        Step s;
+        s.kind = StepKind::Gemm;
+        s.value = v;
+        s.tensor_core = true;
+        s.operands = {q, keys, out, values};
+        s.writes = {0, 0, 1, 0};
+        GemmParams& p = s.gemm;
+        if (added) {
+            s.operands.push_back(*added);
+            s.writes.push_back(0);
+            for (int i = 0; i < 3; i++) p.s1[i] = added->ss.strides[i];
+            if (table) {
+                s.operands.push_back(*table);
+                s.writes.push_back(0);
+            }
+        }
+        p.batch = batch;
+        p.m = m;
+        p.n = n;
+        p.k = k;
+        p.half = half ? 1 : 0;
+        p.a4 = a4;
+        p.b4 = b4;
+        p.v4 = v4;
+        if (!a4.enabled)
+            for (int i = 0; i < 3; i++) p.sa[i] = q.ss.strides[i];
+        if (!b4.enabled) p.sb[0] = keys.ss.strides[0], p.sb[1] = keys.ss.strides[2], p.sb[2] = keys.ss.strides[1];
+        if (!v4.enabled)
+            for (int i = 0; i < 3; i++) p.values_strides[i] = values.ss.strides[i];
+        p.out_heads = (int32_t)out_heads;
+        p.term_cols = (int32_t)term_cols;
+        p.sc[0] = m * out_heads * dv;
+        p.sc[1] = heads > 0 ? dv : m * dv;
+        p.sc[2] = heads > 0 ? out_heads * dv : dv;
+        p.values_mn = 1;
+        p.values_cols = dv;
+        p.splits = 1;
+        p.row_softmax = 3;
+        p.softmax_scale = (float)scale;
+        s.flops = 2.0 * (double)batch * (double)m * (double)n * (double)(k + dv);
+        s.desc = "blockwise-attention b=" + std::to_string(batch) + " m=" + std::to_string(m) + " keys=" + std::to_string(n) + " k=" + std::to_string(k) +
+                 " dv=" + std::to_string(dv) + (half ? " f16" : " tf32") + (term >= 0 ? " +term" : "") + (table ? " (by blocks)" : "") +
+                 (heads > 0 ? ", heads merged" : "");
+        if (a4.enabled || b4.enabled || v4.enabled) {
+            std::string which;
+            for (const char* name : {a4.enabled ? "a" : "", b4.enabled ? "b" : "", v4.enabled ? "v" : ""})
+                if (*name) which += (which.empty() ? "" : ", ") + std::string(name);
+            s.desc += std::string(" (head split read in place: operand") + (which.size() > 1 ? "s " : " ") + which + ")";
+        }
+        if (out.ss.size() != 0) push_step(std::move(s));
+        return out;
+    }
+
+    // Of a constant term that every batch entry shares (a causal mask): per 128 rows the number of 128-key blocks up to the
+    // last one that is not -infinity throughout (at least one), then per block whether it holds anything but zeros.
+    std::optional<PlanTensor> flash_term_blocks(const PlanTensor& t, int64_t batch, int64_t m, int64_t n) {
+        const BufferInfo& b = plan_.buffers[t.buf];
+        if (b.kind != BufKind::Const || b.host_data == nullptr || (batch > 1 && t.ss.strides[0] != 0)) return std::nullopt;
+        const int64_t tiles = (m + 127) / 128, blocks = (n + 127) / 128;
+        if (blocks > 32000) return std::nullopt;
+        auto data = std::make_shared<std::vector<uint8_t>>((size_t)(tiles * (blocks + 1)) * 2);
+        int16_t* out = (int16_t*)data->data();
+        const bool half = t.dtype == DType::F16;
+        for (int64_t i = 0; i < tiles; i++) {
+            int16_t* row = out + i * (blocks + 1);
+            row[0] = 1;
+            for (int64_t j = 0; j < blocks; j++) {
+                bool zero = true, minus_infinity = true;
+                for (int64_t r = i * 128; r < std::min(m, i * 128 + 128); r++)
+                    for (int64_t c = j * 128; c < std::min(n, j * 128 + 128); c++) {
+                        const int64_t at = t.offset + r * t.ss.strides[1] + c * t.ss.strides[2];
+                        uint32_t bits;
+                        if (half) {
+                            uint16_t h;
+                            memcpy(&h, b.host_data + 2 * at, 2);
+                            bits = (uint32_t)h << 16;
+                            minus_infinity = minus_infinity && h == 0xFC00u;
+                        } else {
+                            memcpy(&bits, b.host_data + 4 * at, 4);
+                            minus_infinity = minus_infinity && bits == 0xFF800000u;
+                        }
+                        zero = zero && (bits << 1) == 0;
+                    }
+                row[1 + j] = zero ? 0 : 1;
+                if (!minus_infinity) row[0] = (int16_t)(j + 1);
+            }
+        }
+        return alloc_const({tiles, blocks + 1}, DType::I16, t.buf < 0 ? -1 : b.value, nullptr, data);
+    }
+
+    // Such a term with its columns contiguous, its rows aligned and padded to whole blocks (what is past n is masked by the
+    // kernel), so that all of it can be read 16 bytes at a time: 333 keys of f16 lie 666 bytes apart otherwise.
+    PlanTensor flash_padded_term(const PlanTensor& t, int64_t batch, int64_t m, int64_t n, int64_t* term_cols) {
+        const int64_t padded = (n + 127) / 128 * 128, size = dtype_size(t.dtype);
+        if (t.ss.strides[2] == 1 && n == padded && t.offset % 8 == 0 && (m <= 1 || t.ss.strides[1] % 8 == 0)) return t;
+        const BufferInfo b = plan_.buffers[t.buf];
+        auto data = std::make_shared<std::vector<uint8_t>>((size_t)(m * padded * size), 0);
+        for (int64_t r = 0; r < m; r++)
+            for (int64_t c = 0; c < n; c++)
+                memcpy(data->data() + (r * padded + c) * size, b.host_data + (t.offset + r * t.ss.strides[1] + c * t.ss.strides[2]) * size, (size_t)size);
+        PlanTensor out = alloc_const({m, padded}, t.dtype, b.value, nullptr, data);
+        *term_cols = padded;
+        return out.with(StridedShape({batch, m, n}, {0, padded, 1}));
+    }
+
+    // permute [0, 2, 1, 3] of a view [B, heads, m, dv] of an attention step's result: written in that order to begin with
+    std::optional<PlanTensor> try_merged_attention(int v) {
+        const ValueInfo& pi = g_.values[v];
+        if (pi.op != OpKind::Permute || pi.permutation != std::vector<int>{0, 2, 1, 3}) return std::nullopt;
+        const int w = pi.inputs[0];
+        if (g_.values[w].op != OpKind::View || !fusable(w) || map_[w]) return std::nullopt;
+        const int c = g_.values[w].inputs[0];
+        if (g_.values[c].op != OpKind::MatMul || !fusable(c) || map_[c]) return std::nullopt;
+        const std::vector<int64_t> split = shape_of(w), whole = shape_of(c);
+        if (split.size() != 4 || whole.size() != 3 || split[0] * split[1] != whole[0] || split[2] != whole[1] || split[3] != whole[2]) return std::nullopt;
+        return try_flash_attention(c, split[1]);
     }
 
     // ---------------------------------------------------------------- projections of one tensor as one matmul

@@ -1,0 +1,110 @@
+"""Attention in one step over any number of keys (kernels/flash.cu): ragged rows and keys, an additive term, f16 storage, head
+dimensions up to 128.  The reference runs the scores matmul, the scaling, the sum, the softmax and the second matmul as
+operations of their own: kn-cuda-eval/src/planner.rs:300-330 and 560-600."""
+import numpy as np
+import pytest
+
+from kyanite_b200.configs import _attention
+from kyanite_b200.executor import FLAG_NO_PERSISTENT_GEMM, MATH_F32, MATH_TF32, plan_describe
+from kyanite_b200.graph import BATCH, DType, Graph, shape
+from oracle.cpu_eval import assert_tensors_match, cpu_eval_graph
+
+SHAPES = {
+    # name: (b, m, n, k, dv)
+    "one_short_block": (12, 120, 120, 64, 64),
+    "smallest": (2, 16, 16, 8, 8),
+    "one_column_past_a_block": (3, 129, 129, 40, 40),
+    "cross_attention": (4, 200, 77, 80, 80),
+    "many_blocks": (2, 130, 1000, 64, 64),
+    "widest_head": (2, 333, 333, 128, 128),
+    "values_wider_than_head": (2, 77, 260, 32, 128),
+    "more_items_than_the_chip_holds": (320, 100, 150, 64, 64),
+}
+TERMS = ["none", "input", "per_head", "causal", "lowest", "blocks_of_infinity"]
+CONSTANT = ("causal", "lowest", "blocks_of_infinity")
+
+
+def constant_term(kind, m, n, dtype, r):
+    if kind == "causal":
+        return np.triu(np.full((1, m, n), -np.inf, dtype), 1)
+    if kind == "lowest":        # the lowest finite value; in f32, which absorbs the scores, one row has nothing else
+        t = np.where(r.random((1, m, n)) < 0.5, np.finfo(dtype).min, 0).astype(dtype)
+        if dtype == np.float32:
+            t[0, 3] = np.finfo(dtype).min
+        return t
+    t = np.zeros((1, m, n), dtype)   # a row whose first keys are all masked, one that sees the last key only, a dead one
+    t[0, 1, : max(n - 3, 1)] = -np.inf
+    t[0, 2, : n - 1] = -np.inf
+    t[0, 5] = -np.inf
+    return t
+
+
+def build(name, half, kind, seed=0):
+    b, m, n, k, dv = SHAPES[name]
+    dtype, np_dtype = (DType.F16, np.float16) if half else (DType.F32, np.float32)
+    r = np.random.Generator(np.random.PCG64(seed))
+    g = Graph()
+    q, keys, v = (g.input(shape(*s), dtype) for s in ((b, m, k), (b, n, k), (b, n, dv)))
+    inputs = [r.standard_normal(s).astype(np_dtype) for s in ((b, m, k), (b, n, k), (b, n, dv))]
+    scores = g.mul(g.batched_mat_mul(q, g.permute(keys, [0, 2, 1])), g.scalar(1.0 / np.sqrt(k), dtype))
+    if kind in ("input", "per_head"):
+        s = (b if kind == "per_head" else 1, m, n)
+        scores = g.add(scores, g.input(shape(*s), dtype))
+        inputs.append(r.standard_normal(s).astype(np_dtype))
+    elif kind != "none":
+        scores = g.add(scores, g.constant_tensor(constant_term(kind, m, n, np_dtype, r)))
+    g.output(g.batched_mat_mul(g.softmax(scores, 2), v))
+    return g, inputs
+
+
+def one_step(g, mode=MATH_TF32, flags=0):
+    return [l for l in plan_describe(g, 0, mode, flags=flags).splitlines() if "blockwise-attention" in l]
+
+
+@pytest.mark.parametrize("half", [False, True], ids=["f32", "f16"])
+def test_route(half):
+    for kind in TERMS:
+        g, _ = build("widest_head", half, kind)
+        lines = one_step(g)
+        assert len(lines) == 1 and ("+term" in lines[0]) == (kind != "none"), lines
+        assert ("by blocks" in lines[0]) == (kind in CONSTANT), lines
+        assert not one_step(g, MATH_F32) and not one_step(g, flags=FLAG_NO_PERSISTENT_GEMM)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("half", [False, True], ids=["f32", "f16"])
+@pytest.mark.parametrize("kind", TERMS)
+@pytest.mark.parametrize("name", sorted(SHAPES))
+def test_matches_oracle(name, kind, half):
+    from kyanite_b200.executor import CudaExecutor
+    if name == "more_items_than_the_chip_holds" and kind not in ("none", "causal"):
+        pytest.skip("the oracle takes long over it, and the smaller shapes have this term")
+    g, inputs = build(name, half, kind, seed=7)
+    assert len(one_step(g)) == 1
+    expected = cpu_eval_graph(g.to_bytes(), 0, inputs)
+    with CudaExecutor(0, g, 0, math_mode=MATH_TF32) as ex:
+        got = ex.evaluate(inputs)
+        again = ex.evaluate(inputs)
+    # two chained contractions over operands of 11 bits, and in f16 the oracle's own rounding of scores up to 16 in size
+    # (2^-8 apart at most, half of that in the exponent): 4e-3 of the largest magnitude
+    assert_tensors_match(expected, got, 4e-3, 4e-3, abs_scaled=True)
+    assert np.array_equal(got[0], again[0], equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("half", [False, True], ids=["f32", "f16"])
+@pytest.mark.parametrize("b,s,h,d", [(1, 100, 3, 64), (3, 100, 3, 64), (2, 33, 4, 32)])
+def test_heads_split_and_merged(b, s, h, d, half):
+    """The head split is read in place and the heads are merged by the step's own stores."""
+    from kyanite_b200.executor import CudaExecutor
+    dtype = DType.F16 if half else DType.F32
+    g = Graph()
+    q, k, v = (g.input(shape(BATCH * s, h * d), dtype) for _ in range(3))
+    g.output(_attention(g, q, k, v, s, s, h, d, BATCH, dtype=dtype))
+    lines = [l for l in plan_describe(g, b, MATH_TF32).splitlines() if l.startswith("step")]
+    assert len(lines) == 1 and "heads merged" in lines[0], lines
+    r = np.random.Generator(np.random.PCG64(4))
+    inputs = [r.standard_normal((b * s, h * d)).astype(dtype.np) for _ in range(3)]
+    expected = cpu_eval_graph(g.to_bytes(), b, inputs)
+    with CudaExecutor(0, g, b, math_mode=MATH_TF32) as ex:
+        assert_tensors_match(expected, ex.evaluate(inputs), 4e-3, 4e-3, abs_scaled=True)
