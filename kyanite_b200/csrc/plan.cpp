@@ -640,6 +640,7 @@ class Planner {
                 }
             }
         }
+        if (auto t = visit_scalar_by_parts(root, tree_uses)) return *t;
         // Inline as deep as the kernel's program and operand limits allow; on overflow retry with a
         // shallower cut (operands materialised by a failed attempt stay planned and are reused).
         static const int kDepths[] = {1 << 20, 12, 6, 3, 1, 0};
@@ -654,22 +655,103 @@ class Planner {
         fail(KN_ERR_INTERNAL, "elementwise operation does not fit one kernel");
     }
 
+    // An elementwise expression over a concatenation that nothing else reads (the rotated halves of a rotary embedding:
+    // t * cos + concat(-hi, lo) * sin) is computed part by part straight into the result, a step per part, instead of
+    // materialising the parts' own expressions (a step each), copying every part into the concatenation and reading that
+    // back: 2048 x 32 heads x 128 in f16 took 6.3 + 2 x 6.0 + 20.9 us in four steps, now 14.4 + 14.0 in two.
+    struct Window {
+        int axis, concat, part;
+        int64_t start, end;
+    };
+    const Window* window_ = nullptr;
+    PlanTensor windowed(const PlanTensor& t) const { return window_ ? t.slice(window_->axis, window_->start, window_->end, 1) : t; }
+
+    std::optional<PlanTensor> visit_scalar_by_parts(int root, const std::map<int, int>& tree_uses) {
+        int concat = -1;
+        std::vector<int> stack{root};
+        std::map<int, bool> seen;
+        while (!stack.empty()) {
+            const int x = stack.back();
+            stack.pop_back();
+            if (seen[x] || (x != root && map_[x])) continue;
+            seen[x] = true;
+            const ValueInfo& xi = g_.values[x];
+            if (xi.op == OpKind::Concat && concat < 0 && fusable(x)) concat = x;
+            if ((xi.op == OpKind::Unary || xi.op == OpKind::Binary) && (x == root || can_inline(x, tree_uses)))
+                for (int in : xi.inputs) stack.push_back(in);
+        }
+        if (concat < 0) return std::nullopt;
+        const ValueInfo& ci = g_.values[concat];
+        const int64_t parts = (int64_t)ci.inputs.size();
+        if (parts < 2 || parts > 4 || shape_of(concat) != shape_of(root)) return std::nullopt;
+        for (int in : ci.inputs)
+            if (shape_of(in)[ci.axis] < 1) return std::nullopt;
+        std::vector<std::pair<ScalarBlock, Ref>> programs;
+        Window w{ci.axis, concat, 0, 0, 0};
+        std::vector<Window> windows;
+        for (int i = 0; i < (int)parts; i++) {
+            w.part = ci.inputs[i];
+            w.start = w.end;
+            w.end = w.start + shape_of(w.part)[ci.axis];
+            ScalarBlock block;
+            window_ = &w;
+            const Ref r = build_scalar(root, 0, 1 << 20, block, tree_uses);
+            window_ = nullptr;
+            if ((int)block.loads.size() + 1 > SCALAR_MAX_OPERANDS || (int)block.instrs.size() > SCALAR_MAX_INSTR) return std::nullopt;
+            programs.emplace_back(std::move(block), r);
+            windows.push_back(w);
+        }
+        PlanTensor out = alloc_shared(shape_of(root), g_.values[root].dtype, root);
+        for (size_t i = 0; i < programs.size(); i++)
+            emit_scalar(programs[i].first, {{out.slice(ci.axis, windows[i].start, windows[i].end, 1), programs[i].second}}, root, "fused part");
+        return out;
+    }
+
+    // `visit` with no window in force: what it plans is planned whole
+    PlanTensor visit_whole(int v) {
+        const Window* w = window_;
+        window_ = nullptr;
+        PlanTensor t = visit(v);
+        window_ = w;
+        return t;
+    }
+
     Ref build_scalar(int v, int depth, int max_depth, ScalarBlock& block, const std::map<int, int>& tree_uses) {
         const bool is_root = depth == 0;
         if (!is_root) {
             auto cached = block.value_ref.find(v);
             if (cached != block.value_ref.end()) return cached->second;
-            if (map_[v]) return block.load(*map_[v]);
+            if (map_[v]) return block.load(windowed(*map_[v]));
+            if (window_ && v == window_->concat) {
+                // the part itself, of its own shape (shorter along the axis than anything with a window): its expression if
+                // only the concatenation reads it, else a load
+                const Window* w = window_;
+                window_ = nullptr;
+                const ValueInfo& pi = g_.values[w->part];
+                Ref r;
+                if (!map_[w->part] && (pi.op == OpKind::Unary || pi.op == OpKind::Binary) && fusable(w->part) && !match_epilogue(w->part)) {
+                    const Ref a = build_scalar(pi.inputs[0], depth + 1, max_depth, block, tree_uses);
+                    if (pi.op == OpKind::Unary) r = block.unary(pi.unary_op, pi.cast_from, pi.dtype, a);
+                    else r = block.binary(pi.binary_op, pi.dtype, a, build_scalar(pi.inputs[1], depth + 1, max_depth, block, tree_uses));
+                } else if (auto c = g_.as_single_const(w->part)) {
+                    r = block.constant(*c);
+                } else {
+                    r = block.load(visit(w->part));
+                }
+                window_ = w;
+                block.value_ref[v] = r;
+                return r;
+            }
         }
         const ValueInfo& info = g_.values[v];
         bool is_scalar_op = info.op == OpKind::Unary || info.op == OpKind::Binary;
         Ref result;
         if (!is_root && !is_scalar_op) {
             if (auto c = g_.as_single_const(v)) result = block.constant(*c);
-            else result = block.load(visit(v));
+            else result = block.load(windowed(visit_whole(v)));
         } else if (!is_root && (depth > max_depth || !can_inline(v, tree_uses))) {
             if (auto c = g_.as_single_const(v)) result = block.constant(*c);
-            else result = block.load(visit(v));
+            else result = block.load(windowed(visit_whole(v)));
         } else if (info.op == OpKind::Unary) {
             Ref a = build_scalar(info.inputs[0], depth + 1, max_depth, block, tree_uses);
             result = block.unary(info.unary_op, info.cast_from, info.dtype, a);
@@ -858,7 +940,8 @@ class Planner {
             if (d < 1) return std::nullopt;
         HeadChain c;
         c.src = src;
-        if (from == std::vector<int64_t>{a[0] * a[1], a[2] * a[3]} && target == std::vector<int64_t>{a[0] * a[2], a[1], a[3]}) {
+        // (the source may have the four axes already: the rotary embedding works on them)
+        if ((from == std::vector<int64_t>{a[0] * a[1], a[2] * a[3]} || (a[0] > 1 && from == a)) && target == std::vector<int64_t>{a[0] * a[2], a[1], a[3]}) {
             c.B = a[0]; c.S = a[1]; c.H = a[2]; c.D = a[3];
             c.merge = false;
             return c;
