@@ -2307,18 +2307,14 @@ class Planner {
         return g;
     }
 
-    // A tile of the tensor-core kernels is 128 output positions.  With fewer than that a part of it is idle, which still
-    // beats the exact-f32 kernel (one board of 8 x 8 positions, 128 -> 128 channels: 9 us a layer in a chain against 320)
-    // unless the whole convolution is a few hundred thousand multiply-adds, where either is a launch and little more.
-    static bool conv_worth_tensor_core(const std::vector<int64_t>& out, const std::vector<int64_t>& filter) {
-        const int64_t positions = out[0] * out[2] * out[3];
-        return positions >= 128 || (positions >= 32 && positions * out[1] * filter[1] * filter[2] * filter[3] >= 200000);
-    }
+    // A tile of the tensor-core convolution kernels is this many output positions.  A convolution over fewer (one board of
+    // 8 x 8) keeps f32 operands and runs on the exact kernel: TF32 operands would move its results by 3e-4 of their scale.
+    static constexpr int64_t kConvTilePositions = 128;
 
     bool conv_fits_tensor_core(const ValueInfo& ci, const PlanTensor& x, const PlanTensor& w, const std::vector<int64_t>& out) const {
         if (ci.stride_y != 1 || ci.stride_x != 1) return false;
         if (x.ss.rank() != 4 || w.ss.rank() != 4) return false;
-        if (!conv_worth_tensor_core(out, w.ss.shape) || out[1] < 4 || x.ss.shape[1] < 1) return false;
+        if (out[0] * out[2] * out[3] < kConvTilePositions || out[1] < 4 || x.ss.shape[1] < 1) return false;
         if (out[2] > 32768 || out[3] > 32768 || out[0] > (1 << 24) || w.ss.shape[2] * w.ss.shape[3] > 1024) return false;
         return true;
     }
@@ -2328,7 +2324,7 @@ class Planner {
         if (ci.op != OpKind::Conv || ci.inputs[0] != input || ci.dtype != DType::F32) return false;
         if (ci.stride_y != 1 || ci.stride_x != 1) return false;
         std::vector<int64_t> o = shape_of(conv);
-        return conv_worth_tensor_core(o, shape_of(ci.inputs[1])) && o[1] >= 4;
+        return o[0] * o[2] * o[3] >= kConvTilePositions && o[1] >= 4;
     }
     bool feeds_tensor_core_conv(int v) {
         for (int u : users_[v])
@@ -2336,12 +2332,16 @@ class Planner {
         return false;
     }
 
-    // multiply-adds of a convolution that the exact-f32 kernel computes under KN_MATH_F32, 0 for any other value
+    // multiply-adds of a convolution that the exact-f32 kernel computes: any under KN_MATH_F32, else those of less than a
+    // tensor-core tile (and too small for conv_as_gemm); 0 for any other value
     double exact_conv_products(int conv) {
         const ValueInfo& ci = g_.values[conv];
-        if (opts_.math_mode != KN_MATH_F32 || ci.dtype != DType::F32 || g_.values[ci.inputs[1]].op != OpKind::Constant) return 0;
+        if (ci.dtype != DType::F32 || g_.values[ci.inputs[1]].op != OpKind::Constant) return 0;
         const std::vector<int64_t> o = shape_of(conv), f = shape_of(ci.inputs[1]);
-        return (double)o[0] * o[2] * o[3] * o[1] * f[1] * f[2] * f[3];
+        const int64_t positions = o[0] * o[2] * o[3];
+        const double products = (double)positions * o[1] * f[1] * f[2] * f[3];
+        if (opts_.math_mode != KN_MATH_F32 && (positions >= kConvTilePositions || products >= 1e8)) return 0;
+        return products;
     }
 
     // The convolution kernel reads its input as (C, W, H, N) with channels contiguous.  A tensor that

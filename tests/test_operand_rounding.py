@@ -1,0 +1,57 @@
+"""Which calls of the default mode (KN_MATH_TF32) round f32 operands to TF32's 11 bits, and which keep them: convolutions over
+less than a tile of positions.  The reference computes its matmuls in f32 throughout
+(kn-cuda-sys/src/wrapper/group.rs:120-171)."""
+import numpy as np
+import pytest
+
+from kyanite_b200.executor import MATH_TF32, plan_describe
+from kyanite_b200.graph import Graph, shape
+from oracle.cpu_eval import cpu_eval_graph
+
+
+def rng(seed, *s):
+    return np.random.Generator(np.random.PCG64(seed)).standard_normal(s).astype(np.float32)
+
+
+def contractions(g):
+    """(on the tensor cores, on the exact kernel)"""
+    kinds = [line.split()[2] for line in plan_describe(g, 0, MATH_TF32).splitlines() if line.startswith("step")]
+    kinds = [k for k in kinds if k.startswith(("Conv", "Gemm"))]
+    return sum(not k in ("Conv", "Gemm") for k in kinds), sum(k in ("Conv", "Gemm") for k in kinds)
+
+
+def check_exact(g):
+    from kyanite_b200.executor import CudaExecutor
+    inputs = [rng(7 + i, *[d.eval(0) for d in g[v].shape]) for i, v in enumerate(g.inputs)]
+    with CudaExecutor(0, g, 0, math_mode=MATH_TF32) as ex:
+        got = ex.evaluate(inputs)
+    for e, o in zip(cpu_eval_graph(g.to_bytes(), 0, inputs), got):
+        # f32 products and sums in another order: 1e-5 of the scale for reductions of up to 8192 terms, a thirtieth of what
+        # rounding the operands to 11 bits moves them by
+        assert np.abs(o.astype(np.float64) - e).max() <= 1e-5 * np.abs(e).max()
+
+
+def tower(images, side, channels, layers=3):
+    g = Graph()
+    y = g.input(shape(images, channels, side, side))
+    for i in range(layers):
+        w = g.constant_tensor(rng(i, channels, channels, 3, 3) / np.float32(3 * channels ** 0.5))
+        y = g.relu(g.add(g.conv(y, w, 1, 1, 1, 1), g.constant_tensor(rng(10 + i, 1, channels, 1, 1))))
+    g.output(y)
+    return g
+
+
+# positions: 64, 81, 127; 128 and more go to the tensor cores as ever
+SMALL = [(1, 8, 128), (1, 9, 64), (127, 1, 64), (2, 7, 33)]
+
+
+def test_convolution_route():
+    for case in SMALL:
+        assert contractions(tower(*case)) == (0, 3), case
+    assert contractions(tower(2, 8, 128))[1] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", SMALL)
+def test_small_convolutions_keep_f32(case):
+    check_exact(tower(*case))
