@@ -1249,15 +1249,36 @@ class Planner {
             if (head_chain_operand(value, transposed, type, o, &t, &ob, &orows, &ocols, 1) && o->kd == cols && ob == batch && orows == rows) return t;
             *o = GemmOperand4D{};
             t = visit(value);
-            if (transposed) t = t.with(t.ss.permute({0, 2, 1}));
-            const auto& st = t.ss.strides;
-            auto ok = [&](int64_t dim, int64_t stride) { return dim <= 1 || (stride > 0 && stride % align == 0); };
-            if ((cols > 1 && st[2] != 1) || !ok(rows, st[1]) || !ok(batch, st[0]) || t.offset % align != 0) t = ensure_simple_copy(t, value);
-            return t;
+            return transposed ? t.with(t.ss.permute({0, 2, 1})) : t;
         };
         GemmOperand4D a4{}, b4{}, v4{};
         PlanTensor q = operand(ci.inputs[0], false, m, k, &a4), keys = operand(ci.inputs[1], true, n, k, &b4);
         PlanTensor values = operand(vin, false, n, dv, &v4);
+        if (!half) {
+            // Of f32 values the MMAs see 11 bits: only where the two matmuls as steps of their own would round both
+            // operands to that too.  Few rows, and less than gemm_worth_a_copy asks for with V along its columns, stay with
+            // the exact kernel.
+            auto matrix = [&](const PlanTensor& t, const GemmOperand4D& o, int64_t rows, int64_t cols) {
+                PlanTensor r = t;
+                if (o.enabled) r.ss = StridedShape({batch, rows, cols}, {rows * cols, cols, 1}), r.offset = 0;
+                return r;
+            };
+            auto rounded = [&](const PlanTensor& a, const PlanTensor& b) { return gemm_fits_tensor_core(a, b) || gemm_worth_a_copy(a, b); };
+            const PlanTensor km = matrix(keys, b4, n, k);
+            PlanTensor probabilities = values;
+            probabilities.ss = StridedShape({batch, m, n}, {m * n, n, 1}), probabilities.offset = 0;
+            if (!rounded(matrix(q, a4, m, k), km.with(km.ss.permute({0, 2, 1}))) || !rounded(probabilities, matrix(values, v4, n, dv)))
+                return std::nullopt;   // (the operands are planned either way)
+        }
+        auto contiguous = [&](const PlanTensor& t, const GemmOperand4D& o, int64_t rows, int64_t cols, int value) {
+            const auto& st = t.ss.strides;
+            auto ok = [&](int64_t dim, int64_t stride) { return dim <= 1 || (stride > 0 && stride % align == 0); };
+            if (o.enabled || ((cols <= 1 || st[2] == 1) && ok(rows, st[1]) && ok(batch, st[0]) && t.offset % align == 0)) return t;
+            return ensure_simple_copy(t, value);
+        };
+        q = contiguous(q, a4, m, k, ci.inputs[0]);
+        keys = contiguous(keys, b4, n, k, ci.inputs[1]);
+        values = contiguous(values, v4, n, dv, vin);
         std::optional<PlanTensor> added, table;
         int64_t term_cols = n;
         if (term >= 0) {

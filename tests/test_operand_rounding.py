@@ -1,5 +1,5 @@
 """Which calls of the default mode (KN_MATH_TF32) round f32 operands to TF32's 11 bits, and which keep them: convolutions over
-less than a tile of positions.  The reference computes its matmuls in f32 throughout
+less than a tile of positions, and attention whose two matmuls by themselves would keep them.  The reference computes its matmuls in f32 throughout
 (kn-cuda-sys/src/wrapper/group.rs:120-171)."""
 import numpy as np
 import pytest
@@ -55,3 +55,35 @@ def test_convolution_route():
 @pytest.mark.parametrize("case", SMALL)
 def test_small_convolutions_keep_f32(case):
     check_exact(tower(*case))
+
+
+def attention(b, m, n, k, dv, masked=False, along_keys=False):
+    g = Graph()
+    q, keys = g.input(shape(b, m, k)), g.input(shape(b, n, k))
+    v = g.permute(g.input(shape(b, dv, n)), [0, 2, 1]) if along_keys else g.input(shape(b, n, dv))
+    scores = g.mul(g.batched_mat_mul(q, g.permute(keys, [0, 2, 1])), g.scalar(0.3))
+    if masked:
+        scores = g.add(scores, g.constant_tensor(np.triu(np.full((1, m, n), -np.inf, np.float32), 1)))
+    g.output(g.batched_mat_mul(g.softmax(scores, 2), v))
+    return g
+
+
+# fewer rows than the tensor-core matmul takes, masked and not, ragged and whole 16-byte rows
+FEW_ROWS = [(3, 63, 77, 40, 40), (2, 20, 300, 64, 64), (1, 16, 16, 8, 8), (12, 48, 48, 64, 64)]
+
+
+def test_attention_route():
+    for case in FEW_ROWS:
+        for masked in (False, True):
+            assert contractions(attention(*case, masked)) == (0, 2), case
+    # 64 rows and more: the scores on the tensor cores, the small second matmul with f32 probabilities and values as ever
+    assert contractions(attention(12, 120, 120, 64, 64)) == (1, 1)
+    assert contractions(attention(12, 120, 120, 64, 64, along_keys=True)) == (1, 0)
+    assert contractions(attention(120, 120, 120, 64, 64)) == (1, 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("case", FEW_ROWS)
+def test_attention_of_few_rows_keeps_f32(case, masked):
+    check_exact(attention(*case, masked))
