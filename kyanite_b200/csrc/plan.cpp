@@ -1541,11 +1541,17 @@ class Planner {
         auto rounds = [&](int64_t n) { return (double)(((m + 255) / 256) * ((n + 255) / 256)) / 74.0; };
         double separate = 0;
         for (auto& p : all) separate += std::ceil(rounds(p.n));
-        if (!one_round && (m < 256 || std::ceil(rounds(n_total)) >= separate)) return std::nullopt;
+        const bool fewer_rounds = m >= 256 && std::ceil(rounds(n_total)) < separate;
+        if (!one_round && !fewer_rounds) return std::nullopt;
         bool any_bias = false;
         for (auto& p : all) any_bias = any_bias || p.has_bias;
         PlanTensor xt = visit(x);
         if (xt.ss.rank() != 3 || xt.ss.strides[2] != 1 || !tma_stride_ok(m, xt.ss.strides[1]) || xt.offset % 4 != 0) return std::nullopt;
+        // (joined for the launches they save: only matmuls whose operands the tensor cores would round by themselves too,
+        // not small ones that the exact kernel computes)
+        if (!fewer_rounds || (((m + 127) / 128) * ((n_total + 255) / 256) < 74 && k >= 512))
+            for (auto& p : all)
+                if (!gemm_fits_tensor_core(xt, p.weight) && !gemm_worth_a_copy(xt, p.weight)) return std::nullopt;
         // [n_total][k] with k contiguous, and the biases side by side
         auto wdata = std::make_shared<std::vector<uint8_t>>((size_t)(n_total * k) * 4);
         auto bdata = std::make_shared<std::vector<uint8_t>>((size_t)n_total * 4);

@@ -1,5 +1,5 @@
 """Which calls of the default mode (KN_MATH_TF32) round f32 operands to TF32's 11 bits, and which keep them: convolutions over
-less than a tile of positions, and attention whose two matmuls by themselves would keep them.  The reference computes its matmuls in f32 throughout
+less than a tile of positions, attention and joined projections whose matmuls by themselves would keep them.  The reference computes its matmuls in f32 throughout
 (kn-cuda-sys/src/wrapper/group.rs:120-171)."""
 import numpy as np
 import pytest
@@ -87,3 +87,33 @@ def test_attention_route():
 @pytest.mark.parametrize("case", FEW_ROWS)
 def test_attention_of_few_rows_keeps_f32(case, masked):
     check_exact(attention(*case, masked))
+
+
+def projections(m, k, widths, n_major):
+    """x . W_i for constant W_i [k, n_i] (n_major: [n_i, k], transposed), each read by a small matmul of its own"""
+    g = Graph()
+    x = g.input(shape(1, m, k))
+    for i, n in enumerate(widths):
+        if n_major:
+            w = g.permute(g.constant_tensor(rng(i, 1, n, k)), [0, 2, 1])
+        else:
+            w = g.constant_tensor(rng(i, 1, k, n))
+        y = g.batched_mat_mul(x, w)
+        g.output(g.batched_mat_mul(g.permute(y, [0, 2, 1]), g.input(shape(1, m, 4))))
+    return g
+
+
+# weights along their columns and too little work for a copy; a width below what the tensor cores take; few rows
+SEPARATE = [(87, 336, [84, 96], False), (122, 104, [36, 28, 4], True), (40, 64, [64, 64], True)]
+
+
+def test_projection_route():
+    for case in SEPARATE[:2]:
+        assert "projections of one tensor" not in plan_describe(projections(*case), 0, MATH_TF32), case
+    assert "2 projections of one tensor" in plan_describe(projections(120, 768, [768, 768], True), 0, MATH_TF32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", [SEPARATE[0], SEPARATE[2]])
+def test_small_projections_keep_f32(case):
+    check_exact(projections(*case))
