@@ -49,6 +49,7 @@ struct GemmProblem {
     __device__ int64_t cols() const { return p.n; }
     struct Row { const float* at; };
     __device__ Row row(int64_t b, int64_t m) const { return Row{p.a + b * p.sa[0] + m * p.sa[1]}; }
+    __device__ const float* a_base() const { return p.a; }
     __device__ const float* a_at(const Row& r, const Tap&) const { return r.at; }
     __device__ int64_t a_stride() const { return p.sa[2]; }
     __device__ const float* col(int64_t b, int64_t n) const { return p.b + b * p.sb[0] + n * p.sb[2]; }
@@ -77,6 +78,7 @@ struct GemmProblemHalf {
     __device__ int64_t cols() const { return p.n; }
     struct Row { const __half* at; };
     __device__ Row row(int64_t b, int64_t m) const { return Row{(const __half*)p.a + b * p.sa[0] + m * p.sa[1]}; }
+    __device__ const __half* a_base() const { return (const __half*)p.a; }
     __device__ const __half* a_at(const Row& r, const Tap&) const { return r.at; }
     __device__ int64_t a_stride() const { return p.sa[2]; }
     __device__ const __half* col(int64_t b, int64_t n) const { return (const __half*)p.b + b * p.sb[0] + n * p.sb[2]; }
@@ -113,6 +115,7 @@ struct ConvProblem {
         const int iy = (int)(t - img * p.oh) * p.stride_y - p.pad_y, ix = (int)(m - t * p.ow) * p.stride_x - p.pad_x;
         return Row{p.in + img * p.s_in[0] + iy * p.s_in[2] + ix * p.s_in[3], iy, ix};
     }
+    __device__ const float* a_base() const { return p.in; }
     __device__ const float* a_at(const Row& r, const Tap& t) const {   // null outside the image
         return (unsigned)(r.iy + t.fy) < (unsigned)p.h && (unsigned)(r.ix + t.fx) < (unsigned)p.w ? r.at + t.a : nullptr;
     }
@@ -229,7 +232,10 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
             a_rows[i] = prob.row(batch, in ? m0 + mm : 0);
         }
     }
-    const E* any = prob.col(0, 0);   // an address to name where nothing is read
+    // An address to name where nothing is read.  cp.async wants its source aligned to the copy's size even then, so each
+    // operand names its own base: the other one may start at any element.
+    const E* const no_a = prob.a_base();
+    const E* const no_b = prob.col(0, 0);
     int load_tap = kb_first / per_tap, load_block = kb_first - load_tap * per_tap;
     typename Problem::Tap tap = prob.tap(load_tap);
     const E* a_at[A_ROWS];
@@ -240,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
     for (int i = 0; i < B_ROWS; i++) {
         const int nn = chunk_row + i * kRowStep;
         const bool in = args.load_b == Load::Wide && nn < BN && n0 + nn < N;
-        b_col[i] = in ? prob.col(batch, n0 + nn) : any;
+        b_col[i] = in ? prob.col(batch, n0 + nn) : no_b;
         b_read |= (uint32_t)in << i;
     }
     auto enter_tap = [&] {
@@ -251,11 +257,11 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
             for (int i = 0; i < A_ROWS; i++) {
                 const E* at = ((a_valid >> i) & 1) ? prob.a_at(a_rows[i], tap) : nullptr;
                 a_read |= (uint32_t)(at != nullptr) << i;
-                a_at[i] = at ? at + k0 : any;
+                a_at[i] = at ? at + k0 : no_a;
             }
         }
 #pragma unroll
-        for (int i = 0; i < B_ROWS; i++) b_at[i] = ((b_read >> i) & 1) ? prob.b_at(b_col[i], tap) + k0 : any;
+        for (int i = 0; i < B_ROWS; i++) b_at[i] = ((b_read >> i) & 1) ? prob.b_at(b_col[i], tap) + k0 : no_b;
     };
     enter_tap();
     const uint32_t fetch_to = smem_addr(smem) + (uint32_t)(chunk_row * LR + chunk * kWide) * (uint32_t)sizeof(E);
@@ -268,7 +274,7 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
 #pragma unroll
             for (int i = 0; i < A_ROWS; i++) {
                 if (BM % kRowStep == 0 || chunk_row + i * kRowStep < BM)
-                    fetch16(to + i * kRowStep * LR * (int)sizeof(E), left > 0 ? a_at[i] : any, ((a_read >> i) & 1) ? bytes : 0);
+                    fetch16(to + i * kRowStep * LR * (int)sizeof(E), left > 0 ? a_at[i] : no_a, ((a_read >> i) & 1) ? bytes : 0);
                 a_at[i] += ((a_read >> i) & 1) ? BK : 0;
             }
         } else {
@@ -279,14 +285,14 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
                 const int mm = along_k ? e / BK : e % BM, kk = along_k ? e % BK : e / BM;
                 const E* src = nullptr;
                 if (m0 + mm < M && k0 + kk < inner) src = prob.a_at(prob.row(batch, m0 + mm), tap);
-                fetch1(As + mm * LR + kk, src ? src + (k0 + kk) * prob.a_stride() : any, src != nullptr);
+                fetch1(As + mm * LR + kk, src ? src + (k0 + kk) * prob.a_stride() : no_a, src != nullptr);
             }
         }
         if (args.load_b == Load::Wide) {
 #pragma unroll
             for (int i = 0; i < B_ROWS; i++) {
                 if (BN % kRowStep == 0 || chunk_row + i * kRowStep < BN)
-                    fetch16(to + (BM + i * kRowStep) * LR * (int)sizeof(E), left > 0 ? b_at[i] : any, ((b_read >> i) & 1) ? bytes : 0);
+                    fetch16(to + (BM + i * kRowStep) * LR * (int)sizeof(E), left > 0 ? b_at[i] : no_b, ((b_read >> i) & 1) ? bytes : 0);
                 b_at[i] += ((b_read >> i) & 1) ? BK : 0;
             }
         } else {
@@ -296,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
             for (int e = tid; e < BN * BK; e += kThreads) {
                 const int nn = along_k ? e / BK : e % BN, kk = along_k ? e % BK : e / BN;
                 const bool in = n0 + nn < N && k0 + kk < inner;
-                fetch1(Bs + nn * LR + kk, in ? prob.b_at(prob.col(batch, n0 + nn), tap) + (k0 + kk) * prob.b_stride() : any, in);
+                fetch1(Bs + nn * LR + kk, in ? prob.b_at(prob.col(batch, n0 + nn), tap) + (k0 + kk) * prob.b_stride() : no_b, in);
             }
         }
         if (++load_block == per_tap) {

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from kyanite_b200.executor import MATH_F32, CudaExecutor
-from kyanite_b200.graph import DType, Graph, shape
+from kyanite_b200.graph import DType, Graph, SliceRange, shape
 from oracle.cpu_eval import cpu_eval_graph
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +54,54 @@ def test_convolution(n, c, hw, k, r, stride, pad, chained):
         y = g.add(g.conv(y, weight(k, k, 3), 1, 1, 1, 1), y)
     g.output(y)
     check(g, [rng.standard_normal((n, c, hw, hw)).astype(np.float32)])
+
+
+def sliced(g, base, dims, axis, start):
+    """`dims` of `base`, which has `start` + 3 more entries along `axis`, from entry `start` on"""
+    return g.slice(base, axis, SliceRange(start, start + dims[axis]))
+
+
+# One operand in whole 16-byte pieces, the other starting at an odd element: each is fetched in its own way, also where
+# nothing is read (rows past the last, taps outside the image, chunks past the end of K).
+@pytest.mark.parametrize("dtype", [DType.F32, DType.F16], ids=["f32", "f16"])
+@pytest.mark.parametrize("offset", ["a", "b"])
+@pytest.mark.parametrize("m,n,k", [(70, 33, 64), (9, 40, 72), (130, 70, 40)])
+def test_matmul_with_one_operand_off_16_bytes(m, n, k, offset, dtype):
+    rng = np.random.default_rng(m + n + k)
+    g = Graph()
+    grown = lambda *s: (*s[:-1], s[-1] + 4)  # noqa: E731
+    a, b = (1, m, k), (1, n, k)
+    shapes = [grown(*a) if offset == "a" else a, grown(*b) if offset == "b" else b]
+    x, w = (g.input(shape(*s), dtype) for s in shapes)
+    if offset == "a":
+        x = sliced(g, x, a, 2, 1)
+    else:
+        w = sliced(g, w, b, 2, 1)
+    g.output(g.batched_mat_mul(x, g.permute(w, [0, 2, 1])))
+    check(g, [(rng.standard_normal(s) * k ** -0.25).astype(dtype.np) for s in shapes])
+
+
+def test_matmul_of_a_column_slice():
+    """x[70, 64] . w[:, 1:33]: B along its rows, its first element 4 bytes past an aligned address"""
+    rng = np.random.default_rng(5)
+    g = Graph()
+    x, w = g.input(shape(1, 70, 64)), g.input(shape(1, 64, 41))
+    g.output(g.batched_mat_mul(x, sliced(g, w, (1, 64, 32), 2, 1)))
+    check(g, [rng.standard_normal((1, 70, 64)).astype(np.float32), rng.standard_normal((1, 64, 41)).astype(np.float32)])
+
+
+@pytest.mark.parametrize("offset", ["image", "filter", "flipped"])
+def test_convolution_with_one_operand_off_16_bytes(offset):
+    rng = np.random.default_rng(6)
+    g = Graph()
+    image, weight = (1, 8, 9, 9), (20, 8, 3, 3)
+    x = g.input(shape(1, 8, 9, 13) if offset == "image" else shape(*image))
+    w = g.input(shape(20, 12, 3, 3) if offset != "image" else shape(*weight))
+    inputs = [rng.standard_normal([d.eval(0) for d in g[v].shape]).astype(np.float32) for v in (x, w)]
+    if offset == "image":
+        x = sliced(g, x, image, 3, 1)
+    else:
+        w = sliced(g, w, weight, 1, 1)
+        x = g.flip(x, 2) if offset == "flipped" else x
+    g.output(g.conv(x, w, 1, 1, 1, 1))
+    check(g, inputs)
