@@ -213,8 +213,9 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
     const int ty = ((lane >> 1) & 7) + 8 * (warp % (TY / 8)), tx = ((lane & 1) | ((lane >> 4) << 1)) + 4 * (warp / (TY / 8));
 
     // K blocks of this slice: block kb is elements (kb % per_tap) * BK .. of tap kb / per_tap
-    const int per_tap = (inner + BK - 1) / BK;
-    const int total = taps * per_tap, per_slice = (total + slices - 1) / slices;
+    // (an empty reduction has none: the result is the addends)
+    const int per_tap = max(1, (inner + BK - 1) / BK);
+    const int total = inner > 0 ? taps * per_tap : 0, per_slice = (total + slices - 1) / slices;
     const int kb_first = min(slice * per_slice, total), blocks = min(kb_first + per_slice, total) - kb_first;
 
     // 16-byte fetches: chunk tid % (BK / kWide) of rows tid / (BK / kWide) + i * kRowStep

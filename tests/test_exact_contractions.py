@@ -105,3 +105,26 @@ def test_convolution_with_one_operand_off_16_bytes(offset):
         x = g.flip(x, 2) if offset == "flipped" else x
     g.output(g.conv(x, w, 1, 1, 1, 1))
     check(g, inputs)
+
+
+# nothing to sum: zeros, and what the epilogue adds to them
+@pytest.mark.parametrize("dtype", [DType.F32, DType.F16], ids=["f32", "f16"])
+def test_empty_matmul(dtype):
+    g = Graph()
+    y = g.batched_mat_mul(g.input(shape(2, 70, 0), dtype), g.input(shape(2, 0, 9), dtype))
+    bias = np.arange(9).astype(dtype.np).reshape(1, 1, 9)
+    g.output_all([y, g.add(y, g.constant_tensor(bias))])
+    with CudaExecutor(0, g, 0, math_mode=MATH_F32) as ex:
+        zeros, biased = ex.evaluate([np.zeros((2, 70, 0), dtype.np), np.zeros((2, 0, 9), dtype.np)])
+    np.testing.assert_array_equal(zeros, np.zeros((2, 70, 9)))
+    np.testing.assert_array_equal(biased, np.broadcast_to(bias, (2, 70, 9)))
+
+
+def test_empty_convolution():
+    g = Graph()
+    y = g.conv(g.input(shape(2, 0, 5, 5)), g.input(shape(70, 0, 3, 3)), 1, 1, 1, 1)
+    bias = np.arange(70).astype(np.float32).reshape(1, 70, 1, 1)
+    g.output(g.add(y, g.constant_tensor(bias)))
+    with CudaExecutor(0, g, 0, math_mode=MATH_F32) as ex:
+        got, = ex.evaluate([np.zeros((2, 0, 5, 5), np.float32), np.zeros((70, 0, 3, 3), np.float32)])
+    np.testing.assert_array_equal(got, np.broadcast_to(bias, (2, 70, 5, 5)))
