@@ -189,7 +189,8 @@ struct TileArgs {
 // Plain multiply-adds: the packed form (fma.rn.f32x2) issues at half the rate and measured 5 % slower, K blocks of 64
 // spilled registers.  4096 positions x 128 channels x 1152: 48 us; 19200 x 256 x 2304: 800 us (two tiles a SM, three
 // rounds of 148 for 300 tiles).
-template <class Problem, int BM, int BN, int TN, int KG>
+// `Index` counts along K: 64 bits for reductions that 32 do not hold.
+template <class Problem, int BM, int BN, int TN, int KG, class Index>
 __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __grid_constant__ Problem prob, const __grid_constant__ TileArgs args) {
     constexpr int TX = BN / TN, TY = BM / TM;
     static_assert(TX * TY * KG == kThreads, "one output tile per CTA");
@@ -199,7 +200,8 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
     pdl_enter();
     const int slices = args.slices;
     const int64_t M = prob.rows(), N = prob.cols();
-    const int inner = (int)prob.inner(), taps = prob.taps();
+    const Index inner = (Index)prob.inner();
+    const int taps = prob.taps();
     const int slice = (int)(blockIdx.z % (unsigned)slices);
     const int64_t batch = blockIdx.z / (unsigned)slices;
     const int64_t m0 = (int64_t)blockIdx.x * BM, n0 = (int64_t)blockIdx.y * BN;
@@ -214,9 +216,9 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
 
     // K blocks of this slice: block kb is elements (kb % per_tap) * BK .. of tap kb / per_tap
     // (an empty reduction has none: the result is the addends)
-    const int per_tap = max(1, (inner + BK - 1) / BK);
-    const int total = inner > 0 ? taps * per_tap : 0, per_slice = (total + slices - 1) / slices;
-    const int kb_first = min(slice * per_slice, total), blocks = min(kb_first + per_slice, total) - kb_first;
+    const Index per_tap = max((Index)1, (inner + BK - 1) / BK);
+    const Index total = inner > 0 ? taps * per_tap : 0, per_slice = (total + slices - 1) / slices;
+    const Index kb_first = min(slice * per_slice, total), blocks = min(kb_first + per_slice, total) - kb_first;
 
     // 16-byte fetches: chunk tid % (BK / kWide) of rows tid / (BK / kWide) + i * kRowStep
     constexpr int kChunks = BK / kWide, kRowStep = kThreads / kChunks;
@@ -237,7 +239,8 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
     // operand names its own base: the other one may start at any element.
     const E* const no_a = prob.a_base();
     const E* const no_b = prob.col(0, 0);
-    int load_tap = kb_first / per_tap, load_block = kb_first - load_tap * per_tap;
+    int load_tap = (int)(kb_first / per_tap);
+    Index load_block = kb_first - load_tap * per_tap;
     typename Problem::Tap tap = prob.tap(load_tap);
     const E* a_at[A_ROWS];
     const E* b_at[B_ROWS];
@@ -252,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
     }
     auto enter_tap = [&] {
         a_read = 0;
-        const int k0 = load_block * BK + chunk * kWide;
+        const Index k0 = load_block * BK + chunk * kWide;
         if (args.load_a == Load::Wide) {
 #pragma unroll
             for (int i = 0; i < A_ROWS; i++) {
@@ -268,9 +271,9 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
     const uint32_t fetch_to = smem_addr(smem) + (uint32_t)(chunk_row * LR + chunk * kWide) * (uint32_t)sizeof(E);
     auto load_stage = [&](int stage) {
         const uint32_t to = fetch_to + (uint32_t)stage * stage_bytes<E, BM, BN>;
-        const int k0 = load_block * BK;
-        const int left = (inner - k0 - chunk * kWide) * (int)sizeof(E);
-        const int bytes = min(16, max(0, left));
+        const Index k0 = load_block * BK;
+        const Index left = inner - k0 - chunk * kWide;   // elements of the row from this chunk on
+        const int bytes = (int)min((Index)kWide, max((Index)0, left)) * (int)sizeof(E);
         if (args.load_a == Load::Wide) {
 #pragma unroll
             for (int i = 0; i < A_ROWS; i++) {
@@ -328,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
     }
     int stage = 0, next = kStages - 1;
 #pragma unroll 1
-    for (int b = 0; b < blocks; b++) {
+    for (Index b = 0; b < blocks; b++) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
         __syncthreads();   // stage `b` is complete, and everybody has read stage `b - 1`, which is filled next
         if (b + kStages - 1 < blocks) load_stage(next);
@@ -399,9 +402,9 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
     }
 }
 
-template <class Problem, int BM, int BN, int TN, int KG>
+template <class Problem, int BM, int BN, int TN, int KG, class Index = int>
 int launch_tile(const Problem& prob, int64_t gx, int64_t gy, int64_t batch, const TileArgs& args, cudaStream_t stream) {
-    auto kernel = contract_simt_kernel<Problem, BM, BN, TN, KG>;
+    auto kernel = contract_simt_kernel<Problem, BM, BN, TN, KG, Index>;
     constexpr int smem = smem_bytes<typename Problem::Element, BM, BN, KG>;
     // (the opt-in to more than 48 KB is per device)
     static std::mutex mu;
@@ -436,13 +439,13 @@ int launch_tile(const Problem& prob, int64_t gx, int64_t gy, int64_t batch, cons
 template <class Problem>
 int launch(const Problem& prob, int64_t M, int64_t N, int64_t batch, int64_t taps, int64_t inner, TileArgs args, cudaStream_t stream) {
     if (M == 0 || N == 0 || batch == 0) return 0;
-    if (inner > (1ll << 30)) return (int)cudaErrorInvalidValue;
     const int64_t k_blocks = taps * ((inner + BK - 1) / BK);
     const int64_t large = ((M + 127) / 128) * ((N + 127) / 128) * batch, small = ((M + 63) / 64) * ((N + 63) / 64) * batch;
     // Rounds of tiles over the chip, times the time of a round: a 128 x 128 tile alone on its SM runs at 0.56 of the
     // multiply-add rate, two 64 x 64 tiles sharing one at 0.45 (both measured), and the last round may be nearly empty.
     const double rounds_large = (double)((large + 147) / 148) * 4 / 0.56, rounds_small = (double)((small + 295) / 296) * 2 / 0.45;
-    const bool wide = rounds_large < rounds_small;
+    const bool long_k = k_blocks > (1ll << 25);   // (the counters run one K block past the end)
+    const bool wide = !long_k && rounds_large < rounds_small;
     const int64_t gx = (M + (wide ? 127 : 63)) / (wide ? 128 : 64), gy = (N + (wide ? 127 : 63)) / (wide ? 128 : 64);
     if (gy > 65535 || batch > 65535 || gx > 0x7FFFFFFFll) return (int)cudaErrorInvalidValue;
     args.slices = 1;
@@ -452,6 +455,7 @@ int launch(const Problem& prob, int64_t M, int64_t N, int64_t batch, int64_t tap
     // two cluster barriers, some 3 us), eight at most (the portable cluster size)
     while (args.slices < 8 && gx * gy * batch * args.slices * 2 <= 296 && k_blocks >= 4 * 2 * args.slices && batch * args.slices * 2 <= 65535)
         args.slices *= 2;
+    if (long_k) return launch_tile<Problem, 64, 64, 4, 2, int64_t>(prob, gx, gy, batch, args, stream);
     return launch_tile<Problem, 64, 64, 4, 2>(prob, gx, gy, batch, args, stream);
 }
 

@@ -128,3 +128,18 @@ def test_empty_convolution():
     with CudaExecutor(0, g, 0, math_mode=MATH_F32) as ex:
         got, = ex.evaluate([np.zeros((2, 0, 5, 5), np.float32), np.zeros((70, 0, 3, 3), np.float32)])
     np.testing.assert_array_equal(got, np.broadcast_to(bias, (2, 70, 5, 5)))
+
+
+@pytest.mark.parametrize("dtype,k,side", [(DType.F32, 1 << 29, 9), (DType.F16, 1 << 30, 1)], ids=["f32", "f16"])
+def test_long_reduction(dtype, k, side):
+    """Rows of 2 GB: byte counts along K do not fit 32 bits.  One entry in 2^20 is not zero, so every sum is exact."""
+    period = 1 << 20
+    pattern = np.zeros((1, period), dtype.np)
+    pattern[0, 12345] = 1
+    g = Graph()
+    row = g.add(g.broadcast(g.constant_tensor(pattern), shape(k // period, period)), g.broadcast(g.view(g.input(shape(1), dtype), shape(1, 1)), shape(k // period, period)))
+    row = g.broadcast(g.view(row, shape(1, 1, k)), shape(1, side, k))
+    g.output(g.batched_mat_mul(row, g.permute(row, [0, 2, 1])))
+    with CudaExecutor(0, g, 0, math_mode=MATH_F32) as ex:
+        got, = ex.evaluate([np.zeros(1, dtype.np)])
+    np.testing.assert_array_equal(got, np.full((1, side, side), k // period))
