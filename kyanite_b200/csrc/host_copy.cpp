@@ -87,10 +87,15 @@ class Pool : public CopyPool {
             if (ready) ready(done * kChunk, std::min(bytes, upto * kChunk));
             done = upto;
         };
-        while (job->one()) advance();
-        while (done < chunks) {   // what the helpers still have in hand: a few microseconds
-            advance();
-            if (done < chunks) std::this_thread::yield();
+        try {
+            while (job->one()) advance();
+            while (done < chunks) {   // what the helpers still have in hand: a few microseconds
+                advance();
+                if (done < chunks) std::this_thread::yield();
+            }
+        } catch (...) {   // from `ready`; the caller is free to drop both buffers once it leaves here
+            job->abandon();
+            throw;
         }
     }
 
@@ -109,6 +114,12 @@ class Pool : public CopyPool {
             copy_past_caches(dst + from, src + from, std::min(bytes, from + kChunk) - from);
             complete[c].store(1, std::memory_order_release);
             return true;
+        }
+        // no further chunks are handed out, and those that were are complete
+        void abandon() {
+            const size_t taken = std::min(next.exchange(chunks), chunks);
+            for (size_t c = 0; c < taken; c++)
+                while (!complete[c].load(std::memory_order_acquire)) std::this_thread::yield();
         }
     };
 
