@@ -9,6 +9,7 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -73,8 +74,12 @@ class Pool : public CopyPool {
         auto job = std::make_shared<Job>(dst, src, bytes, chunks);
         {
             std::lock_guard<std::mutex> lock(mu_);
-            if (threads_.empty())
-                for (int i = 0; i < kHelpers; i++) threads_.emplace_back([this] { help(); });
+            if (threads_.empty()) {
+                try {
+                    for (int i = 0; i < kHelpers; i++) threads_.emplace_back([this] { help(); });
+                } catch (const std::system_error&) {   // no more threads to be had: fewer helpers, or none
+                }
+            }
             job_ = job;
             generation_++;
         }

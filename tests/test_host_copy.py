@@ -43,6 +43,39 @@ int main() {
 }
 """
 
+# The process may start no more threads: the copy is made all the same.
+NO_THREADS = r"""
+extern "C" int pthread_create(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*) { return EAGAIN; }
+int main() {
+    const size_t n = (5u << 20) + 77;
+    uint8_t *src = pages(n), *dst = pages(n);
+    fill(src, n, 3);
+    size_t next = 0;
+    kn::CopyPool::shared()->copy(dst, src, n, [&](size_t from, size_t to) { REQUIRE(from == next); next = to; });
+    REQUIRE(next == n && memcmp(src, dst, n) == 0);
+}
+"""
+
+# Several threads at once: one has the helpers, the others copy alone; buffers that start at any byte.
+SEVERAL = r"""
+int main() {
+    auto pool = kn::CopyPool::shared();
+    std::vector<std::thread> users;
+    for (int t = 0; t < 4; t++)
+        users.emplace_back([&, t] {
+            const size_t n = (3u << 20) + 1000 * t + 13;
+            uint8_t *src = pages(n + 16), *dst = pages(n + 16);
+            for (int turn = 0; turn < 30; turn++) {
+                fill(src, n, turn + 100 * t);
+                size_t next = 0;
+                pool->copy(dst + t, src, n, [&](size_t from, size_t to) { REQUIRE(from == next && to > from); next = to; });
+                REQUIRE(next == n && memcmp(src, dst + t, n) == 0);
+            }
+        });
+    for (auto& u : users) u.join();
+}
+"""
+
 
 def run(tmp_path, body, *flags):
     compiler = shutil.which("g++")
@@ -57,3 +90,11 @@ def run(tmp_path, body, *flags):
 
 def test_failing_upload(tmp_path):
     run(tmp_path, THROWING)
+
+
+def test_no_threads(tmp_path):
+    run(tmp_path, NO_THREADS)
+
+
+def test_several_users(tmp_path):
+    run(tmp_path, SEVERAL)
