@@ -101,6 +101,7 @@ struct Executor {
     std::vector<std::shared_ptr<OutputSet>> output_sets;
     std::shared_ptr<CopyPool> copy_pool;         // helpers for large host copies, made on first use
     bool staging_busy = false;                   // transfers to or from the pinned buffers may be in flight
+    bool stream_lent = false;                    // ... also the caller's own, on the stream that kn_executor_stream gave out
     cudaStream_t side_stream = nullptr;          // capture-time fork for early output copies
     bool profile = false;
     std::vector<float> step_us;
@@ -315,7 +316,7 @@ struct Executor {
         KN_CUDA(cudaMemcpyAsync(status_host, status_dev, 4, cudaMemcpyDeviceToHost, stream));
     }
     void settle() {   // the pinned buffers are the host's again
-        if (!staging_busy) return;
+        if (!staging_busy && !stream_lent) return;
         KN_CUDA(cudaStreamSynchronize(stream));
         staging_busy = false;
     }
@@ -807,6 +808,7 @@ int kn_executor_stream(kn_executor* exec, void** stream) {
     return guarded([&] {
         KN_CHECK(exec != nullptr && stream != nullptr, KN_ERR_INVALID_ARG, "null argument");
         *stream = (void*)exec->e->stream;
+        exec->e->stream_lent = true;
     });
 }
 

@@ -29,3 +29,22 @@ def test_results_are_the_callers(columns):
         np.testing.assert_array_equal(plus, a + np.float32(1))
         np.testing.assert_array_equal(twice, a * np.float32(2))
         plus[...] = 0                                      # and they are writable
+
+
+def test_waits_for_the_callers_own_transfers():
+    """A caller that has the stream may copy from the staging buffers on it; `evaluate` stages new inputs after that."""
+    import torch
+    g = Graph()
+    g.output(g.add(g.input(shape(1, 1000)), g.scalar(1.0)))
+    with CudaExecutor(0, g, 1) as ex:
+        ex.evaluate([np.zeros((1, 1000), np.float32)])
+        stream = torch.cuda.ExternalStream(ex.stream())
+        ex.host_inputs[0][...] = 7
+        taken = torch.empty(1, 1000, device="cuda")
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(50_000_000)   # some 25 ms
+            taken.copy_(torch.from_numpy(ex.host_inputs[0]), non_blocking=True)
+        ex.evaluate([np.zeros((1, 1000), np.float32)])
+        stream.synchronize()
+        assert (taken == 7).all()
