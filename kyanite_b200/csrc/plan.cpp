@@ -2096,8 +2096,9 @@ class Planner {
     }
 
     // a tensor-core matmul of few tiles: its K slices are summed inside a cluster
+    // (not under KN_FLAG_TRACE_GEMM: the progress markers are the persistent kernel's)
     bool take_slices(GemmParams& p) const {
-        if (opts_.flags & KN_FLAG_NO_PERSISTENT_GEMM) return false;
+        if (opts_.flags & (KN_FLAG_NO_PERSISTENT_GEMM | KN_FLAG_TRACE_GEMM)) return false;
         const GemmSlices c = gemm_slices_choose(p);
         p.slices = c.slices;
         p.slices_bn = c.bn;

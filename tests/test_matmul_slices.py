@@ -6,6 +6,7 @@ import re
 import numpy as np
 import pytest
 
+from kyanite_b200._lib import KN_FLAG_TRACE_GEMM
 from kyanite_b200.executor import FLAG_NO_PERSISTENT_GEMM, MATH_F32, MATH_TF32, plan_describe
 from kyanite_b200.graph import DType, Graph, shape
 from oracle.cpu_eval import assert_tensors_match, cpu_eval_graph
@@ -60,6 +61,7 @@ def test_rule():
         assert width % 32 == 0 and 32 <= width <= 256 and width - 32 < n
         assert slices is None or 2 <= int(slices.group(1)) <= min(8, -(-k // 32)), line
         assert not tile(build(b, m, n, k)[0], MATH_F32) and not tile(build(b, m, n, k)[0], flags=FLAG_NO_PERSISTENT_GEMM)
+        assert not tile(build(b, m, n, k)[0], flags=KN_FLAG_TRACE_GEMM)   # its markers are the persistent kernel's
     assert not tile(build(1, 4096, 4096, 512)[0])     # rounds of wide tiles: the persistent kernel
 
 
