@@ -615,6 +615,8 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
     } else if (warp == 1 && lane == 0) {
         // ---------------- MMA issuer (the instruction descriptor of gemm_persistent_kernel)
+        // (the clock of a bounded wait starts when the kernels in front are done, however long they take)
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         const uint32_t fmt = HALF ? 0u : 2u;
         const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(kGpBlockM >> 4) << 24);
         int s = 0, round = 0;
@@ -634,10 +636,10 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         if (good) mma_commit(acc_full);
     }
     __syncwarp();
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // (the addends and the output belong to earlier kernels until here)
     // the accumulator is complete, and with it every read of the stages: they become the partial tile
     if (lane == 0) good = mbar_wait(acc_full, 0, abandon, p.status, 33, kWaitCycles, 2000) && good;
     good = __syncthreads_and(good ? 1 : 0) != 0;
-    asm volatile("griddepcontrol.wait;" ::: "memory");   // (the addends and the output belong to earlier kernels until here)
     if (good) {
         tc_fence_after();
         const int quarter = warp & 3;
