@@ -974,9 +974,8 @@ int gemm_persistent_launch(const void* launch, cudaStream_t stream) {
 
 // Tile width and K slices for gemm_slices_kernel; slices = 0: the matmul is for the persistent kernel.
 //
-// The line: less than one round of the chip in the persistent kernel's tiles (at most 148 of 128 rows x its block width), or
-// an f16 result whose rows do not start on 16-byte boundaries, which that kernel's stores cannot write.  Within it the
-// narrowest total wins, in SM cycles: a K block costs its MMAs (bn / 2 cycles each, four of them) or its bytes at the 60 per
+// The line: less than one round of the chip in the persistent kernel's tiles (at most 148 of 128 rows x its block width).
+// Within it the cheapest total wins, in SM cycles: a K block costs its MMAs (bn / 2 cycles each, four of them) or its bytes at the 60 per
 // cycle that an SM was measured to take from L2, whichever is longer; storing and summing a partial tile costs by its width,
 // a cluster some 1 200 cycles more, a CTA 2 500 before its first MMA.  A round holds fewer CTAs than there are SMs when
 // they come in clusters, which lie inside a GPC (kClusterCtas).
@@ -988,8 +987,7 @@ GemmSlices gemm_slices_choose(const GemmParams& g) {
     const int64_t m_tiles = (g.m + kGpBlockM - 1) / kGpBlockM;
     const int64_t wide = gemm_persistent_bn(g.n);
     const int64_t persistent_tiles = m_tiles * ((g.n + wide - 1) / wide) * g.batch;
-    const bool unaligned_half = g.half != 0 && (g.sc[2] != 1 || g.sc[1] % 8 != 0 || (g.batch > 1 && g.sc[0] % 8 != 0));
-    if (persistent_tiles > 148 && !unaligned_half) return none;
+    if (persistent_tiles > 148) return none;
     const int64_t k_blocks = (g.k + (g.half ? 63 : 31)) / (g.half ? 64 : 32);
     GemmSlices best{};
     double best_cost = 0;
