@@ -273,7 +273,11 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #pragma unroll
             for (int i = 0; i < 64; i++) top = fmaxf(top, __uint_as_float(v[i >> 5][i & 31]));
             exchange[half * 128 + row_in_tile] = top;
-            asm volatile("bar.sync 2, 256;" ::: "memory");   // (also: every score of the block has been read)
+            // (also: every score of the block has been read.  In f16 the other half's warps store their probabilities over
+            // columns that this half's have just read, so the barrier orders tensor-memory accesses too)
+            tc_fence_before();
+            asm volatile("bar.sync 2, 256;" ::: "memory");
+            tc_fence_after();
             top = fmaxf(top, exchange[(half ^ 1) * 128 + row_in_tile]);
             // a row whose scores were all -infinity so far has no reference yet (and zeros in its sum and output)
             const bool first = seen == -INFINITY;
