@@ -180,11 +180,12 @@ struct Executor {
                     if (s.gemm.row_softmax == 2) {   // fused attention: the fourth operand is V^T, there are no addends
                         s.gemm.values = s.gemm.add1;
                         s.gemm.add1 = nullptr;
-                    } else if (s.gemm.row_softmax == 3) {   // V, then the additive term and its table, if there are any
+                    } else if (s.gemm.row_softmax == 3) {   // V, then the additive term, its table and flags, if there are any
                         s.gemm.values = s.gemm.add1;
                         s.gemm.add1 = s.gemm.add2;
                         s.gemm.add2 = nullptr;
                         s.gemm.term_blocks = ptr.size() > 5 ? ptr[5] : nullptr;
+                        s.gemm.scratch = ptr.size() > 6 ? (float*)ptr[6] : nullptr;
                     }
                     break;
                 case StepKind::Conv:

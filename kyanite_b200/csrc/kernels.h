@@ -159,7 +159,8 @@ struct GemmParams {
     // with element strides `values_strides` (the last is 1), C is [batch][m][values_cols] (kernels/attention.cu).
     // 3: attention over any number of keys (kernels/flash.cu): as 2 with `values_mn`, f32 or f16; the additive term of
     // softmax(softmax_scale * A.B + term), if there is one, is `add1` with strides `s1`, of which `term_cols` columns of a row
-    // may be read (past n: padding); batch entry bt of C lies at (bt / out_heads) * sc[0] + (bt % out_heads) * sc[1], its
+    // may be read (past n: padding); `scratch`, if there is one, takes an I32 flag per batch entry and key block (see
+    // flash_finite_kernel); batch entry bt of C lies at (bt / out_heads) * sc[0] + (bt % out_heads) * sc[1], its
     // rows sc[2] apart, columns contiguous.
     int32_t row_softmax;
     float softmax_scale;

@@ -65,8 +65,9 @@ struct FlashParams {
     int64_t term_s[3];
     int32_t term_cols;               // columns of a row that may be read: n, or more with padding
     // of a constant term that all batch entries share: per row block the number of key blocks to visit (what follows is
-    // -infinity), then per key block whether the term has to be read (0: it is zero); else null
+    // -infinity), then per key block what the term is there: 0 zero, 2 -infinity, 1 anything else (it is read); else null
     const int16_t* term_blocks;
+    const int32_t* not_finite;       // [batch][key blocks] of flash_finite_kernel, or null: no block is left out
     uint32_t* status;
 };
 
@@ -125,9 +126,15 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     // the last row blocks first: under a causal mask they have the most keys
     const int bt = (int)(blockIdx.x % (unsigned)p.batch), mt = p.m_tiles - 1 - (int)(blockIdx.x / (unsigned)p.batch);
     const int16_t* blocks_of = TERM && p.term_blocks ? p.term_blocks + (int64_t)mt * (p.key_blocks + 1) : nullptr;   // (a constant)
-    const int n_blocks = blocks_of ? (int)blocks_of[0] : p.key_blocks;
+    int n_blocks = blocks_of ? (int)blocks_of[0] : p.key_blocks;
     auto block_cols = [&](int j) { return min(kFlKeys, (p.n - j * kFlKeys + 31) & ~31); };   // (past n: zero fill, masked below)
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (TERM && p.not_finite && n_blocks < p.key_blocks) {   // up to the last masked block that does not give exact zeros
+        const int32_t* flags = p.not_finite + (int64_t)bt * p.key_blocks;
+        int last = 0;
+        for (int j = n_blocks + lane; j < p.key_blocks; j += 32) last = flags[j] != 0 ? j + 1 : last;
+        n_blocks = max(n_blocks, __reduce_max_sync(0xffffffffu, last));
+    }
 
     if (warp == 8) {
         if (lane == 0) {
@@ -225,10 +232,11 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             tmem_loads_done();
             const int col0 = j * kFlKeys + half * 64;
             if (TERM) {
-                const bool add = blocks_of == nullptr || blocks_of[1 + j] != 0;
-                if (!add) {
+                const int kind = blocks_of == nullptr ? 1 : (int)blocks_of[1 + j];
+                if (kind != 1) {
+                    const float same = kind == 2 ? -INFINITY : 0.f;
 #pragma unroll
-                    for (int i = 0; i < 64; i++) v[i >> 5][i & 31] = __float_as_uint(p.scale * __uint_as_float(v[i >> 5][i & 31]));
+                    for (int i = 0; i < 64; i++) v[i >> 5][i & 31] = __float_as_uint(fmaf(p.scale, __uint_as_float(v[i >> 5][i & 31]), same));
                 } else {
                     const T* t = term_row + (int64_t)col0 * p.term_s[2];
                     const bool vec = p.term_s[2] == 1 && col0 + 64 <= p.term_cols && ((uintptr_t)t & 15) == 0;
@@ -371,9 +379,48 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
 }
 
+// Per key block of 128: does a key or a value of it hold a NaN or an infinity?  A block that the term masks throughout may
+// be left out only if not: -infinity added to a score of NaN or infinity, and a probability of 0 times a value of either,
+// are NaN.  One pass over K and V: 10 us for 32 heads of 2048 x 128 in f16.
+struct FiniteParams {
+    const void* base[2];   // keys, values: row r of entry bt at (bt % bi) * s_x + (bt / bi) * s_y + r * s_row
+    int64_t s_row[2], s_x[2], s_y[2];
+    int32_t bi[2], cols[2];
+    int32_t n, key_blocks;
+    int32_t* flags;
+};
+
+template <bool HALF>
+__global__ void __launch_bounds__(256) flash_finite_kernel(const __grid_constant__ FiniteParams p) {
+    pdl_enter();
+    constexpr int kSize = HALF ? 2 : 4;
+    const int j = (int)(blockIdx.x % (unsigned)p.key_blocks), bt = (int)(blockIdx.x / (unsigned)p.key_blocks);
+    const int rows = min(kFlKeys, p.n - j * kFlKeys);
+    auto exponent_full = [](uint32_t w) {
+        return HALF ? (w & 0x7C00u) == 0x7C00u || (w & 0x7C000000u) == 0x7C000000u : (w & 0x7F800000u) == 0x7F800000u;
+    };
+    bool found = false;
+#pragma unroll
+    for (int o = 0; o < 2; o++) {
+        const char* base = (const char*)p.base[o] + ((bt % p.bi[o]) * p.s_x[o] + (bt / p.bi[o]) * p.s_y[o] + (int64_t)j * kFlKeys * p.s_row[o]) * kSize;
+        const int chunks = p.cols[o] * kSize / 16, row_step = 256 / chunks, chunk_step = 256 % chunks;
+        int r = threadIdx.x / chunks, c = threadIdx.x % chunks;
+#pragma unroll 8
+        for (int i = threadIdx.x; i < rows * chunks; i += 256) {
+            const uint4 u = *(const uint4*)(base + r * p.s_row[o] * kSize + c * 16);
+            found = found | exponent_full(u.x) | exponent_full(u.y) | exponent_full(u.z) | exponent_full(u.w);
+            r += row_step, c += chunk_step;
+            if (c >= chunks) c -= chunks, r++;
+        }
+    }
+    const int any = __syncthreads_or(found ? 1 : 0);
+    if (threadIdx.x == 0) p.flags[blockIdx.x] = any;
+}
+
 struct FlashLaunch {
     CUtensorMap map_q, map_k, map_v;
     FlashParams p;
+    FiniteParams finite;
     unsigned grid;
     int smem_bytes;
     bool half;
@@ -420,11 +467,17 @@ std::shared_ptr<void> flash_attention_prepare(const GemmParams& g, uint32_t* sta
     for (int i = 0; i < 3; i++) p.term_s[i] = g.s1[i];
     p.term_cols = g.term_cols;
     p.term_blocks = (const int16_t*)g.term_blocks;
+    p.not_finite = (const int32_t*)g.scratch;
     p.status = status_word;
+    FiniteParams& f = l->finite;
+    memset(&f, 0, sizeof(f));
+    f.n = p.n;
+    f.key_blocks = p.key_blocks;
+    f.flags = (int32_t*)g.scratch;
     // an operand [batch, rows, k] as a 4-D map (K offset, row, x, y): a head split read in place as it is, a plain one with
     // x = the batch entry (bi = batch + 1: coordinates (bt, 0))
     auto operand = [&](const GemmOperand4D& o, const void* base, int64_t rows, int64_t cols, int64_t s_batch, int64_t s_row, int64_t s_col,
-                       bool mn_major, CUtensorMap* map, int32_t* bi) {
+                       bool mn_major, CUtensorMap* map, int32_t* bi, int scanned) {
         int box[4] = {(int)elems, kFlRows, 1, 1};
         int64_t dims[4] = {cols, rows, g.batch, 1}, strides[4] = {1, s_row, s_batch, align};
         if (o.enabled) {
@@ -436,14 +489,21 @@ std::shared_ptr<void> flash_attention_prepare(const GemmParams& g, uint32_t* sta
             *bi = (int)g.batch + 1;
         }
         if (((uintptr_t)base & 15) != 0) return false;
+        if (scanned >= 0) {
+            f.base[scanned] = base;
+            f.s_row[scanned] = strides[1], f.s_x[scanned] = strides[2], f.s_y[scanned] = strides[3];
+            f.bi[scanned] = *bi;
+            f.cols[scanned] = (int32_t)cols;
+        }
         if (half) *map = tc_make_map_f16(base, 4, dims, strides, box, true);
         else if (mn_major) *map = tc_make_map_mn_major(base, 4, dims, strides, box);
         else *map = tc_make_map(base, 4, dims, strides, box, true);
         return true;
     };
-    if (!operand(g.a4, g.a, g.m, g.k, g.sa[0], g.sa[1], g.sa[2], false, &l->map_q, &p.a_bi)) return nullptr;
-    if (!operand(g.b4, g.b, g.n, g.k, g.sb[0], g.sb[2], g.sb[1], false, &l->map_k, &p.b_bi)) return nullptr;
-    if (!operand(g.v4, g.values, g.n, g.values_cols, g.values_strides[0], g.values_strides[1], g.values_strides[2], true, &l->map_v, &p.v_bi)) return nullptr;
+    if (!operand(g.a4, g.a, g.m, g.k, g.sa[0], g.sa[1], g.sa[2], false, &l->map_q, &p.a_bi, -1)) return nullptr;
+    if (!operand(g.b4, g.b, g.n, g.k, g.sb[0], g.sb[2], g.sb[1], false, &l->map_k, &p.b_bi, 0)) return nullptr;
+    if (!operand(g.v4, g.values, g.n, g.values_cols, g.values_strides[0], g.values_strides[1], g.values_strides[2], true, &l->map_v, &p.v_bi, 1))
+        return nullptr;
     l->smem_bytes = flash_smem_bytes(g.k, g.values_cols, half);
     l->grid = (unsigned)(g.batch * p.m_tiles);
     return l;
@@ -465,6 +525,10 @@ int flash_attention_launch(const void* launch, cudaStream_t stream) {
             }
             done[device] = true;
         }
+    }
+    if (l.finite.flags) {
+        const dim3 blocks((unsigned)l.p.batch * (unsigned)l.p.key_blocks);
+        launch_pdl(l.half ? flash_finite_kernel<true> : flash_finite_kernel<false>, blocks, dim3(256), (size_t)0, stream, l.finite);
     }
     const dim3 grid(l.grid), block(kFlThreads);
     const size_t smem = (size_t)l.smem_bytes;

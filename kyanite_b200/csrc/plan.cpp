@@ -1281,9 +1281,12 @@ class Planner {
         values = contiguous(values, v4, n, dv, vin);
         std::optional<PlanTensor> added, table;
         int64_t term_cols = n;
+        bool left_out = false;
         if (term >= 0) {
             added = visit(term);
-            table = flash_term_blocks(*added, batch, m, n);
+            // (with a CTA or less per SM the last row block, which sees every key, decides: leaving blocks out gains nothing)
+            left_out = batch * ((m + 127) / 128) > 148;
+            table = flash_term_blocks(*added, batch, m, n, &left_out);
             if (table) added = flash_padded_term(*added, batch, m, n, &term_cols);
         }
         const int64_t out_heads = heads > 0 ? heads : batch;
@@ -1302,6 +1305,11 @@ class Planner {
             if (table) {
                 s.operands.push_back(*table);
                 s.writes.push_back(0);
+            }
+            if (table && left_out) {   // what a first kernel finds in K and V (flash_finite_kernel)
+                s.operands.push_back(alloc_shared({batch, (n + 127) / 128}, DType::I32, v));
+                s.writes.push_back(1);
+                s.launches = 2;
             }
         }
         p.batch = batch;
@@ -1329,7 +1337,7 @@ class Planner {
         p.softmax_scale = (float)scale;
         s.flops = 2.0 * (double)batch * (double)m * (double)n * (double)(k + dv);
         s.desc = "blockwise-attention b=" + std::to_string(batch) + " m=" + std::to_string(m) + " keys=" + std::to_string(n) + " k=" + std::to_string(k) +
-                 " dv=" + std::to_string(dv) + (half ? " f16" : " tf32") + (term >= 0 ? " +term" : "") + (table ? " (by blocks)" : "") +
+                 " dv=" + std::to_string(dv) + (half ? " f16" : " tf32") + (term >= 0 ? " +term" : "") + (table ? (left_out ? " (by blocks, masked ones left out)" : " (by blocks)") : "") +
                  (heads > 0 ? ", heads merged" : "");
         if (a4.enabled || b4.enabled || v4.enabled) {
             std::string which;
@@ -1341,9 +1349,10 @@ class Planner {
         return out;
     }
 
-    // Of a constant term that every batch entry shares (a causal mask): per 128 rows the number of 128-key blocks up to the
-    // last one that is not -infinity throughout (at least one), then per block whether it holds anything but zeros.
-    std::optional<PlanTensor> flash_term_blocks(const PlanTensor& t, int64_t batch, int64_t m, int64_t n) {
+    // Of a constant term that every batch entry shares (a causal mask): per 128 rows the number of 128-key blocks to visit,
+    // then per block 0 if it is zero, 2 if it is -infinity throughout and 1 otherwise.  With `*leave_out` only up to the last
+    // block that is not -infinity throughout (at least one); it is cleared if no row block has fewer to visit for it.
+    std::optional<PlanTensor> flash_term_blocks(const PlanTensor& t, int64_t batch, int64_t m, int64_t n, bool* leave_out) {
         const BufferInfo& b = plan_.buffers[t.buf];
         if (b.kind != BufKind::Const || b.host_data == nullptr || (batch > 1 && t.ss.strides[0] != 0)) return std::nullopt;
         const int64_t tiles = (m + 127) / 128, blocks = (n + 127) / 128;
@@ -1351,9 +1360,10 @@ class Planner {
         auto data = std::make_shared<std::vector<uint8_t>>((size_t)(tiles * (blocks + 1)) * 2);
         int16_t* out = (int16_t*)data->data();
         const bool half = t.dtype == DType::F16;
+        bool fewer = false;
         for (int64_t i = 0; i < tiles; i++) {
             int16_t* row = out + i * (blocks + 1);
-            row[0] = 1;
+            row[0] = *leave_out ? 1 : (int16_t)blocks;
             for (int64_t j = 0; j < blocks; j++) {
                 bool zero = true, minus_infinity = true;
                 for (int64_t r = i * 128; r < std::min(m, i * 128 + 128); r++)
@@ -1371,10 +1381,12 @@ class Planner {
                         }
                         zero = zero && (bits << 1) == 0;
                     }
-                row[1 + j] = zero ? 0 : 1;
-                if (!minus_infinity) row[0] = (int16_t)(j + 1);
+                row[1 + j] = zero ? 0 : (minus_infinity ? 2 : 1);
+                if (*leave_out && !minus_infinity) row[0] = (int16_t)(j + 1);
             }
+            fewer = fewer || row[0] < blocks;
         }
+        *leave_out = fewer;
         return alloc_const({tiles, blocks + 1}, DType::I16, t.buf < 0 ? -1 : b.value, nullptr, data);
     }
 

@@ -116,3 +116,31 @@ def test_heads_split_and_merged(b, s, h, d, half):
     expected = cpu_eval_graph(g.to_bytes(), b, inputs)
     with CudaExecutor(0, g, b, math_mode=MATH_TF32) as ex:
         assert_tensors_match(expected, ex.evaluate(inputs), 4e-3, 4e-3, abs_scaled=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("half", [False, True], ids=["f32", "f16"])
+def test_not_finite_behind_the_mask(half):
+    """Blocks that a causal mask hides are left out only where they would add exact zeros: a NaN or an infinity in a hidden key
+    or value reaches the rows that do not see it, as -infinity + infinity and 0 * infinity are NaN."""
+    from kyanite_b200.executor import CudaExecutor
+    b, s, d = 80, 300, 32
+    dtype = DType.F16 if half else DType.F32
+    r = np.random.Generator(np.random.PCG64(11))
+    g = Graph()
+    q, keys, v = (g.input(shape(b, s, d), dtype) for _ in range(3))
+    scores = g.add(g.mul(g.batched_mat_mul(q, g.permute(keys, [0, 2, 1])), g.scalar(0.2, dtype)), g.constant_tensor(constant_term("causal", s, s, dtype.np, r)))
+    g.output(g.batched_mat_mul(g.softmax(scores, 2), v))
+    assert "masked ones left out" in one_step(g)[0]
+    inputs = [r.standard_normal((b, s, d)).astype(dtype.np) for _ in range(3)]
+    inputs[1][7, 290, 0], inputs[1][20, 150, 3], inputs[1][33, 299, 1] = np.inf, -np.inf, np.nan
+    inputs[2][3, 299, 5], inputs[2][11, 200, 7], inputs[2][12, 130, 31] = np.nan, np.inf, -np.inf
+    with np.errstate(all="ignore"):
+        expected = cpu_eval_graph(g.to_bytes(), 0, inputs)[0]
+    with CudaExecutor(0, g, 0, math_mode=MATH_TF32) as ex:
+        got = ex.evaluate(inputs)[0]
+    assert 1000 < np.isnan(expected).sum() < expected.size / 10
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(expected))
+    infinite, finite = np.isinf(expected), np.isfinite(expected)
+    np.testing.assert_array_equal(got[infinite], expected[infinite])
+    assert_tensors_match([expected[finite]], [got[finite]], 4e-3, 4e-3, abs_scaled=True)
