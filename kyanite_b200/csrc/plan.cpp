@@ -3,6 +3,7 @@
 #include <pthread.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <map>
@@ -1285,9 +1286,12 @@ class Planner {
         if (term >= 0) {
             added = visit(term);
             // (with a CTA or less per SM the last row block, which sees every key, decides: leaving blocks out gains nothing)
-            left_out = batch * ((m + 127) / 128) > 148;
-            table = flash_term_blocks(*added, batch, m, n, &left_out);
-            if (table) added = flash_padded_term(*added, batch, m, n, &term_cols);
+            if (const FlashTerm* t = flash_term(*added, batch, m, n, batch * ((m + 127) / 128) > 148)) {
+                added = t->term.with(t->term.ss.broadcast({batch, m, n}));
+                table = t->table;
+                term_cols = t->cols;
+                left_out = t->left_out;
+            }
         }
         const int64_t out_heads = heads > 0 ? heads : batch;
         PlanTensor out = heads > 0 ? alloc_shared({batch / heads, m, heads, dv}, type, v) : alloc_shared({batch, m, dv}, type, v);
@@ -1349,14 +1353,36 @@ class Planner {
         return out;
     }
 
-    // Of a constant term that every batch entry shares (a causal mask): per 128 rows the number of 128-key blocks to visit,
-    // then per block 0 if it is zero, 2 if it is -infinity throughout and 1 otherwise.  With `*leave_out` only up to the last
-    // block that is not -infinity throughout (at least one); it is cleared if no row block has fewer to visit for it.
-    std::optional<PlanTensor> flash_term_blocks(const PlanTensor& t, int64_t batch, int64_t m, int64_t n, bool* leave_out) {
+    // A constant term that every batch entry shares (a causal mask) as the kernel wants it.  Made once for all the attention
+    // steps that read it: the layers of a decoder share one mask, 8 MB in f16 at 2000 tokens.
+    struct FlashTerm {
+        PlanTensor term;    // [1, m, n], columns contiguous
+        PlanTensor table;   // see flash_term_blocks
+        int64_t cols;       // columns of a row that may be read
+        bool left_out;      // a row block has fewer blocks to visit than there are
+    };
+    std::map<std::array<int64_t, 7>, FlashTerm> flash_terms_;
+
+    const FlashTerm* flash_term(const PlanTensor& t, int64_t batch, int64_t m, int64_t n, bool leave_out) {
         const BufferInfo& b = plan_.buffers[t.buf];
-        if (b.kind != BufKind::Const || b.host_data == nullptr || (batch > 1 && t.ss.strides[0] != 0)) return std::nullopt;
+        if (b.kind != BufKind::Const || b.host_data == nullptr || (batch > 1 && t.ss.strides[0] != 0) || (n + 127) / 128 > 32000) return nullptr;
+        // (the buffer is the planner's only one for this constant; its type goes with it)
+        const std::array<int64_t, 7> key{t.buf, t.offset, t.ss.strides[1], t.ss.strides[2], m, n, leave_out ? 1 : 0};
+        auto have = flash_terms_.find(key);
+        if (have != flash_terms_.end()) return &have->second;
+        FlashTerm f;
+        f.left_out = leave_out;
+        f.table = flash_term_blocks(t, m, n, &f.left_out);
+        f.term = flash_padded_term(t.with(StridedShape({1, m, n}, {0, t.ss.strides[1], t.ss.strides[2]})), m, n, &f.cols);
+        return &flash_terms_.emplace(key, f).first->second;
+    }
+
+    // Per 128 rows the number of 128-key blocks to visit, then per block 0 if it is zero, 2 if it is -infinity throughout
+    // and 1 otherwise.  With `*leave_out` only up to the last block that is not -infinity throughout (at least one); it is
+    // cleared if no row block has fewer to visit for it.
+    PlanTensor flash_term_blocks(const PlanTensor& t, int64_t m, int64_t n, bool* leave_out) {
+        const BufferInfo& b = plan_.buffers[t.buf];
         const int64_t tiles = (m + 127) / 128, blocks = (n + 127) / 128;
-        if (blocks > 32000) return std::nullopt;
         auto data = std::make_shared<std::vector<uint8_t>>((size_t)(tiles * (blocks + 1)) * 2);
         int16_t* out = (int16_t*)data->data();
         const bool half = t.dtype == DType::F16;
@@ -1387,13 +1413,14 @@ class Planner {
             fewer = fewer || row[0] < blocks;
         }
         *leave_out = fewer;
-        return alloc_const({tiles, blocks + 1}, DType::I16, t.buf < 0 ? -1 : b.value, nullptr, data);
+        return alloc_const({tiles, blocks + 1}, DType::I16, b.value, nullptr, data);
     }
 
-    // Such a term with its columns contiguous, its rows aligned and padded to whole blocks (what is past n is masked by the
-    // kernel), so that all of it can be read 16 bytes at a time: 333 keys of f16 lie 666 bytes apart otherwise.
-    PlanTensor flash_padded_term(const PlanTensor& t, int64_t batch, int64_t m, int64_t n, int64_t* term_cols) {
+    // The term [1, m, n] with its columns contiguous, its rows aligned and padded to whole blocks (what is past n is masked
+    // by the kernel), so that all of it can be read 16 bytes at a time: 333 keys of f16 lie 666 bytes apart otherwise.
+    PlanTensor flash_padded_term(const PlanTensor& t, int64_t m, int64_t n, int64_t* term_cols) {
         const int64_t padded = (n + 127) / 128 * 128, size = dtype_size(t.dtype);
+        *term_cols = padded;
         if (t.ss.strides[2] == 1 && n == padded && t.offset % 8 == 0 && (m <= 1 || t.ss.strides[1] % 8 == 0)) return t;
         const BufferInfo b = plan_.buffers[t.buf];
         auto data = std::make_shared<std::vector<uint8_t>>((size_t)(m * padded * size), 0);
@@ -1401,8 +1428,7 @@ class Planner {
             for (int64_t c = 0; c < n; c++)
                 memcpy(data->data() + (r * padded + c) * size, b.host_data + (t.offset + r * t.ss.strides[1] + c * t.ss.strides[2]) * size, (size_t)size);
         PlanTensor out = alloc_const({m, padded}, t.dtype, b.value, nullptr, data);
-        *term_cols = padded;
-        return out.with(StridedShape({batch, m, n}, {0, padded, 1}));
+        return out.with(StridedShape({1, m, n}, {0, padded, 1}));
     }
 
     // permute [0, 2, 1, 3] of a view [B, heads, m, dv] of an attention step's result: written in that order to begin with

@@ -1,6 +1,8 @@
 """Attention in one step over any number of keys (kernels/flash.cu): ragged rows and keys, an additive term, f16 storage, head
 dimensions up to 128.  The reference runs the scores matmul, the scaling, the sum, the softmax and the second matmul as
 operations of their own: kn-cuda-eval/src/planner.rs:300-330 and 560-600."""
+import re
+
 import numpy as np
 import pytest
 
@@ -144,3 +146,19 @@ def test_not_finite_behind_the_mask(half):
     infinite, finite = np.isinf(expected), np.isfinite(expected)
     np.testing.assert_array_equal(got[infinite], expected[infinite])
     assert_tensors_match([expected[finite]], [got[finite]], 4e-3, 4e-3, abs_scaled=True)
+
+
+def test_a_mask_is_prepared_once():
+    """The layers of a decoder share one mask: its padded form and its table by blocks are made once and read by all."""
+    s, d = 333, 32
+    r = np.random.Generator(np.random.PCG64(1))
+    g = Graph()
+    mask = g.constant_tensor(constant_term("causal", s, s, np.float16, r))
+    for heads in (2, 2, 5):
+        q, keys, v = (g.input(shape(heads, s, d), DType.F16) for _ in range(3))
+        g.output(g.batched_mat_mul(g.softmax(g.add(g.batched_mat_mul(q, g.permute(keys, [0, 2, 1])), mask), 2), v))
+    lines = one_step(g)
+    prepared = {tuple(re.findall(r"r:\w+@(b\d+)", line)[-2:]) for line in lines}
+    assert len(lines) == 3 and len(prepared) == 1, lines
+    const_bytes = int(re.search(r"const_bytes=(\d+)", plan_describe(g, 0, MATH_TF32)).group(1))
+    assert const_bytes < 2 * s * (s + 384) + 4096     # the mask, its rows padded to 384, the table
