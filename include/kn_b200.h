@@ -144,7 +144,8 @@ KN_API int kn_executor_evaluate(kn_executor* exec, const void* const* inputs, vo
  * a handle that keeps them, also beyond the executor's life.  An evaluation that is given exactly these pointers
  * downloads straight into them (no second host copy).  They stay the caller's until `kn_outputs_release`, which any thread
  * may call; the executor then uses them again.  `*set` is NULL, and nothing is filled in, when the outputs are
- * too small for it to pay or all of the executor's (few) sets are held: evaluate into buffers of your own then.
+ * too small for it to pay (below 64 KB) or too large to pin (above 128 MB), or all of the executor's sets (four, fewer
+ * from 64 MB on) are held: evaluate into buffers of your own then.
  * The reference hands out borrowed tensors instead (kn-cuda-eval/src/executor.rs:194). */
 typedef struct kn_outputs kn_outputs;
 KN_API int kn_executor_outputs_acquire(kn_executor* exec, void** outputs, kn_outputs** set);

@@ -75,10 +75,12 @@ struct OutputSet {
         for (void* p : ptr) if (p) cudaFreeHost(p);
     }
 };
-// An executor owns at most this many sets, and at most this many bytes of them (but two whatever their size); a caller
-// that keeps more results than that gets them copied instead.
+// An executor owns at most this many sets and pins at most this many bytes for them (a caller needs two: one to evaluate into
+// while it still holds the results before).  Its first such evaluation makes them all, and the graphs that download into
+// them, so that no later one pays for it (a set and a graph are 2 to 4 ms).  A caller that keeps more results than that,
+// or whose results do not fit twice, gets them copied instead.
 constexpr size_t kMaxOutputSets = 4;
-constexpr size_t kMaxOutputSetBytes = 512ull << 20;
+constexpr size_t kMaxOutputSetBytes = 256ull << 20;
 // Outputs smaller than this in all are copied: the copy costs less than handing a set over.
 constexpr size_t kMinOutputSetBytes = 64 << 10;
 // Inputs of up to this many bytes in all go up, and outputs of up to as many come down, by a kernel (host_copy.cu).
@@ -425,27 +427,28 @@ struct Executor {
         return exec;
     }
 
-    // A set of result buffers nobody holds, or null: outputs too small for it to pay, or the executor's sets all held.
+    // A set of result buffers nobody holds, or null: outputs too small for it to pay or too large to pin, or all sets held.
     std::shared_ptr<OutputSet> acquire_outputs() {
         const size_t bytes = sum(bytes_out);
-        if (bytes < kMinOutputSetBytes) return nullptr;
+        if (bytes < kMinOutputSetBytes || bytes * 2 > kMaxOutputSetBytes) return nullptr;
+        while (output_sets.size() < std::min(kMaxOutputSets, kMaxOutputSetBytes / bytes)) {
+            auto set = std::make_shared<OutputSet>();
+            for (size_t n : bytes_out) {
+                void* p = nullptr;
+                if (cudaHostAlloc(&p, std::max<size_t>(n, 16), cudaHostAllocDefault) != cudaSuccess) {
+                    cudaGetLastError();
+                    return nullptr;
+                }
+                set->ptr.push_back(p);
+            }
+            output_sets.push_back(set);
+        }
         for (auto& s : output_sets)
             if (s.use_count() == 1) {
                 std::atomic_thread_fence(std::memory_order_acquire);   // the last holder's reads are over
                 return s;
             }
-        if (output_sets.size() >= kMaxOutputSets || (output_sets.size() >= 2 && (output_sets.size() + 1) * bytes > kMaxOutputSetBytes)) return nullptr;
-        auto set = std::make_shared<OutputSet>();
-        for (size_t n : bytes_out) {
-            void* p = nullptr;
-            if (cudaHostAlloc(&p, std::max<size_t>(n, 16), cudaHostAllocDefault) != cudaSuccess) {
-                cudaGetLastError();
-                return nullptr;
-            }
-            set->ptr.push_back(p);
-        }
-        output_sets.push_back(set);
-        return set;
+        return nullptr;
     }
     // The pinned buffers an evaluation with these output pointers downloads into: 0 the staging, 1 + i output set i
     size_t destination_of(void* const* outputs) const {
@@ -498,8 +501,10 @@ struct Executor {
             }
         }
         if (graph) {
-            if (eval_graphs.size() <= to) eval_graphs.resize(to + 1, nullptr);
-            if (!eval_graphs[to]) eval_graphs[to] = capture_evaluate(destination(to));
+            if (eval_graphs.size() < 1 + output_sets.size()) eval_graphs.resize(1 + output_sets.size(), nullptr);
+            if (!eval_graphs[to])
+                for (size_t d = 0; d < eval_graphs.size(); d++)
+                    if (!eval_graphs[d]) eval_graphs[d] = capture_evaluate(destination(d));
             KN_CUDA(cudaGraphLaunch(eval_graphs[to], stream));
         } else {
             run_async();

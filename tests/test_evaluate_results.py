@@ -48,3 +48,33 @@ def test_waits_for_the_callers_own_transfers():
         ex.evaluate([np.zeros((1, 1000), np.float32)])
         stream.synchronize()
         assert (taken == 7).all()
+
+
+def test_results_too_large_to_pin():
+    g = Graph()
+    x = g.input(shape(1, 1))
+    g.output(g.add(g.broadcast(x, shape(1, 33 << 20)), g.scalar(1.0)))     # 132 MB
+    with CudaExecutor(0, g, 0) as ex:
+        got, = ex.evaluate([np.full((1, 1), 4, np.float32)])
+    assert got.flags.owndata and (got == 5).all()
+
+
+def test_no_later_evaluation_prepares_results():
+    """The first evaluation makes all the sets of pinned results and the graphs that download into them: whatever the ones after
+    it hold, no other pinned memory appears."""
+    g = Graph()
+    x = g.input(shape(BATCH, 100000))
+    g.output(g.add(x, g.scalar(1.0)))
+    a = np.arange(100000, dtype=np.float32).reshape(1, -1)
+    with CudaExecutor(0, g, 1) as ex:
+        kept, addresses = [], set()
+        for _ in range(9):
+            del kept[:-3]                       # three held, the fourth set free
+            kept.append(ex.evaluate([a])[0])
+            assert not kept[-1].flags.owndata
+            addresses.update(r.ctypes.data for r in kept)
+        assert len(addresses) == 4
+        more = [ex.evaluate([a])[0], ex.evaluate([a])[0]]   # all sets held: arrays of their own
+        assert all(r.flags.owndata for r in more)
+        for r in kept + more:
+            np.testing.assert_array_equal(r, a + np.float32(1))
