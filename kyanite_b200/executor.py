@@ -32,8 +32,8 @@ FLAG_NO_CONV_CHAIN = _lib.KN_FLAG_NO_CONV_CHAIN
 FLAG_NO_PERSISTENT_GEMM = _lib.KN_FLAG_NO_PERSISTENT_GEMM
 
 
-# results smaller than this in all are copied into ordinary arrays: handing pinned memory out costs more than the copy
-# (the library refuses below 64 KB too)
+# results smaller than this are copied into ordinary arrays: handing pinned memory out costs more than the copy, and a small
+# array that is kept would hold the large ones' memory
 _HAND_OUT_BYTES = 64 << 10
 
 
@@ -211,7 +211,7 @@ class CudaExecutor:
         self._in_ptrs_type = c_void_p * max(1, n_in.value)
         self._out_ptrs_type = c_void_p * max(1, n_out.value)
         self._out_bytes_types = [ctypes.c_uint8 * n for _, _, n in self._out_info]
-        self._hand_out = sum(n for _, _, n in self._out_info) >= _HAND_OUT_BYTES
+        self._hand_out = any(n >= _HAND_OUT_BYTES for _, _, n in self._out_info)
 
     # ---------------------------------------------------------------- info
     def _io_info(self, is_output: int, index: int):
@@ -261,8 +261,10 @@ class CudaExecutor:
 
     # ---------------------------------------------------------------- running
     def evaluate(self, inputs: Sequence[np.ndarray]) -> List[np.ndarray]:
-        """Copies inputs to the device, runs the graph, returns fresh host arrays.  Large results are views of pinned
-        memory that the download went to directly; it is theirs as long as any of them lives."""
+        """Copies inputs to the device, runs the graph, returns fresh host arrays.  Results of 64 KB and more are views of
+        pinned memory that the download went to directly: writable and theirs as long as any of them lives, but not to be
+        resized in place (`flags.owndata` is false).  An executor has up to four such sets of results; a caller that
+        holds them all, or results of more than 128 MB, gets ordinary arrays.  `host_outputs` is not written then."""
         if len(inputs) != len(self._in_spec):
             raise ValueError(f"Wrong input count, expected {len(self._in_spec)} but got {len(inputs)}")
         arrays = []
@@ -290,6 +292,9 @@ class CudaExecutor:
                         outs.append(np.empty(shape, dtype=dtype))
                         continue
                     raw = raw_type.from_address(ptr)
+                    if raw_type._length_ < _HAND_OUT_BYTES:
+                        outs.append(np.frombuffer(raw, dtype=dtype).reshape(shape).copy())
+                        continue
                     raw.held = held         # the array views `raw`, which keeps the set
                     outs.append(np.frombuffer(raw, dtype=dtype).reshape(shape))
                 return outs

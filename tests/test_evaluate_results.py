@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from kyanite_b200.executor import CudaExecutor
-from kyanite_b200.graph import BATCH, Graph, shape
+from kyanite_b200.graph import BATCH, Graph, SliceRange, shape
 
 pytestmark = pytest.mark.gpu
 
@@ -78,3 +78,25 @@ def test_no_later_evaluation_prepares_results():
         assert all(r.flags.owndata for r in more)
         for r in kept + more:
             np.testing.assert_array_equal(r, a + np.float32(1))
+
+
+def test_small_results_do_not_hold_large_ones():
+    """A small result is an array of its own: one that is kept does not keep the memory of the large one beside it, and later
+    evaluations go on being handed out without a copy."""
+    g = Graph()
+    x = g.input(shape(BATCH, 40000))
+    g.output_all([g.mul(x, g.scalar(2.0)), g.add(g.slice(x, 1, SliceRange(0, 5)), g.scalar(1.0))])
+    rng = np.random.default_rng(1)
+    inputs = [rng.standard_normal((1, 40000)).astype(np.float32) for _ in range(6)]
+    with CudaExecutor(0, g, 1) as ex:
+        small, addresses = [], set()
+        for a in inputs:
+            large, few = ex.evaluate([a])
+            np.testing.assert_array_equal(large, a * np.float32(2))
+            assert few.flags.owndata and not large.flags.owndata
+            addresses.add(large.ctypes.data)
+            small.append(few)
+            del large
+    for a, few in zip(inputs, small):
+        np.testing.assert_array_equal(few, a[:, :5] + np.float32(1))
+    assert len(addresses) <= 4
