@@ -467,7 +467,7 @@ struct Executor {
     bool in_flight = false;   // evaluate_begin without its evaluate_end
     size_t target = 0;        // where that evaluation downloads to (destination_of)
 
-    // Host copy `dst` <- `src`, large ones shared out over helper threads
+    // Host copy `dst` <- `src`, large ones shared out over helper threads; with `ready`, what is ready is uploaded from `dst`
     void copy_host(void* dst, const void* src, size_t bytes, const std::function<void(size_t, size_t)>& ready = nullptr) {
         if (bytes < kParallelCopyBytes) {
             memcpy(dst, src, bytes);
@@ -475,7 +475,7 @@ struct Executor {
             return;
         }
         if (!copy_pool) copy_pool = CopyPool::shared();
-        copy_pool->copy(dst, src, bytes, ready);
+        copy_pool->copy(dst, src, bytes, ready != nullptr, ready);
     }
 
     void evaluate_begin(const void* const* inputs, size_t to = 0) {

@@ -60,7 +60,7 @@ class Pool : public CopyPool {
         for (auto& t : threads_) t.join();
     }
 
-    void copy(void* dst, const void* src, size_t bytes, const std::function<void(size_t, size_t)>& ready) override {
+    void copy(void* dst, const void* src, size_t bytes, bool past_caches, const std::function<void(size_t, size_t)>& ready) override {
         const size_t chunks = (bytes + kChunk - 1) / kChunk;
         std::unique_lock<std::mutex> mine(user_, std::try_to_lock);
         if (!mine.owns_lock() || bytes < kParallelCopyBytes) {
@@ -71,7 +71,7 @@ class Pool : public CopyPool {
             }
             return;
         }
-        auto job = std::make_shared<Job>(dst, src, bytes, chunks);
+        auto job = std::make_shared<Job>(dst, src, bytes, chunks, past_caches);
         {
             std::lock_guard<std::mutex> lock(mu_);
             if (threads_.empty()) {
@@ -109,14 +109,18 @@ class Pool : public CopyPool {
         uint8_t* dst;
         const uint8_t* src;
         size_t bytes, chunks;
+        bool past_caches;
         std::atomic<size_t> next{0};
         std::vector<std::atomic<uint8_t>> complete;
-        Job(void* d, const void* s, size_t b, size_t c) : dst((uint8_t*)d), src((const uint8_t*)s), bytes(b), chunks(c), complete(c) {}
+        Job(void* d, const void* s, size_t b, size_t c, bool past)
+            : dst((uint8_t*)d), src((const uint8_t*)s), bytes(b), chunks(c), past_caches(past), complete(c) {}
         bool one() {
             const size_t c = next.fetch_add(1, std::memory_order_relaxed);
             if (c >= chunks) return false;
             const size_t from = c * kChunk;
-            copy_past_caches(dst + from, src + from, std::min(bytes, from + kChunk) - from);
+            const size_t n = std::min(bytes, from + kChunk) - from;
+            if (past_caches) copy_past_caches(dst + from, src + from, n);
+            else memcpy(dst + from, src + from, n);
             complete[c].store(1, std::memory_order_release);
             return true;
         }

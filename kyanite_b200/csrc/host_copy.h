@@ -15,10 +15,11 @@ class CopyPool {
     // The process's pool: started by the first caller, its threads ended when the last holder lets go.
     static std::shared_ptr<CopyPool> shared();
     virtual ~CopyPool() = default;
-    // Copies `bytes` bytes.  `ready(from, to)`, if given, is called on the calling thread for consecutive ranges as they
+    // Copies `bytes` bytes, with stores past the caches for a destination that the GPU reads next (not for one that the
+    // caller does).  `ready(from, to)`, if given, is called on the calling thread for consecutive ranges as they
     // are complete, so that an upload of the first part runs while the rest is still being copied.  Returns when
     // everything is copied.  Safe from several threads: a caller that finds the helpers taken copies alone.
-    virtual void copy(void* dst, const void* src, size_t bytes, const std::function<void(size_t, size_t)>& ready) = 0;
+    virtual void copy(void* dst, const void* src, size_t bytes, bool past_caches, const std::function<void(size_t, size_t)>& ready) = 0;
 };
 
 }  // namespace kn

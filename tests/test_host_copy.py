@@ -32,7 +32,7 @@ int main() {
         fill(src, n, turn);
         bool thrown = false;
         try {
-            pool->copy(dst, src, n, [](size_t, size_t) { throw std::runtime_error("upload"); });
+            pool->copy(dst, src, n, true, [](size_t, size_t) { throw std::runtime_error("upload"); });
         } catch (const std::runtime_error&) {
             thrown = true;
         }
@@ -51,7 +51,7 @@ int main() {
     uint8_t *src = pages(n), *dst = pages(n);
     fill(src, n, 3);
     size_t next = 0;
-    kn::CopyPool::shared()->copy(dst, src, n, [&](size_t from, size_t to) { REQUIRE(from == next); next = to; });
+    kn::CopyPool::shared()->copy(dst, src, n, true, [&](size_t from, size_t to) { REQUIRE(from == next); next = to; });
     REQUIRE(next == n && memcmp(src, dst, n) == 0);
 }
 """
@@ -68,7 +68,7 @@ int main() {
             for (int turn = 0; turn < 30; turn++) {
                 fill(src, n, turn + 100 * t);
                 size_t next = 0;
-                pool->copy(dst + t, src, n, [&](size_t from, size_t to) { REQUIRE(from == next && to > from); next = to; });
+                pool->copy(dst + t, src, n, turn % 2 == 0, [&](size_t from, size_t to) { REQUIRE(from == next && to > from); next = to; });
                 REQUIRE(next == n && memcmp(src, dst + t, n) == 0);
             }
         });
