@@ -725,9 +725,11 @@ class Planner {
             if (map_[v]) return block.load(windowed(*map_[v]));
             if (window_ && v == window_->concat) {
                 // the part itself, of its own shape (shorter along the axis than anything with a window): its expression if
-                // only the concatenation reads it, else a load
+                // only the concatenation reads it, else a load (a root-mean-square norm is a step of its own kind)
                 const Window* w = window_;
                 window_ = nullptr;
+                if (!map_[w->part])
+                    if (auto norm = try_fused_rmsnorm(w->part)) map_[w->part] = *norm;
                 const ValueInfo& pi = g_.values[w->part];
                 Ref r;
                 if (!map_[w->part] && (pi.op == OpKind::Unary || pi.op == OpKind::Binary) && fusable(w->part) && !match_epilogue(w->part)) {
