@@ -6,7 +6,8 @@ over its algorithmic bytes (memory-bound steps) or TFLOP/s over its FLOP (contra
     python -m kyanite_b200.kernel_bench                 # all cases, one JSON line per step
     python -m kyanite_b200.kernel_bench --case softmax  # one case (this is what the ncu captures run)
 
-Working sets are several times the 126 MB L2, so back-to-back launches still stream from HBM.  Peaks come
+Working sets are several times the 126 MB L2, so back-to-back launches still stream from HBM (those of the short calls,
+`*_short*`, and of `conv_exact` lie in it, as the calls' own do).  Peaks come
 from MEASURED_PEAKS.json at the repository root when present (copy bandwidth, bf16 GEMM burst; TF32 is
 taken as half the bf16 figure, f16 operands as the bf16 figure itself), else the fallback 6650 GB/s / 1590 TFLOP/s.
 """
@@ -20,7 +21,7 @@ import sys
 
 import numpy as np
 
-from .executor import MATH_TF32, CudaExecutor
+from .executor import MATH_F32, MATH_TF32, CudaExecutor
 from .graph import BATCH, BinaryOp, DType, Graph, ReduceOp, UnaryOp, shape
 
 
@@ -159,6 +160,21 @@ def case_attention(rng):
     return g, 0, r + [rng.standard_normal((384, 64, 512)).astype(np.float32)]
 
 
+def _blockwise_attention_case(heads, rows, keys, d, half=False, causal=False):
+    def build(rng):
+        dtype = DType.F16 if half else DType.F32
+        g = Graph()
+        q, k, v = (g.input(shape(heads, n, d), dtype) for n in (rows, keys, keys))
+        scores = g.mul(g.batched_mat_mul(q, g.permute(k, [0, 2, 1])), g.scalar(1.0 / math.sqrt(d), dtype))
+        if causal:
+            scores = g.add(scores, g.constant_tensor(np.triu(np.full((1, rows, keys), -np.inf, dtype.np), 1)))
+        g.output(g.batched_mat_mul(g.softmax(scores, 2), v))
+        return g, 0, [rng.standard_normal((heads, n, d)).astype(dtype.np) for n in (rows, keys, keys)]
+    build.__doc__ = (f"Attention by key blocks: {heads} heads of {rows} rows, {keys} keys, d = {d}" + (", f16" if half else "") +
+                     (", causal" if causal else ""))
+    return build
+
+
 def case_conv_trunk(rng):
     """One trunk convolution of the tower on its own: 3x3, 128 -> 128, batch 256, 8x8, + bias + relu."""
     g = Graph()
@@ -285,11 +301,24 @@ CASES = {
     "rmsnorm_f16": case_rmsnorm_f16,
     "swiglu_f16": case_swiglu_f16,
     "residual_add_f16": case_residual_add_f16,
+    "attention_causal_f16": _blockwise_attention_case(32, 2048, 2048, 128, half=True, causal=True),
+    "attention_short_f16": _blockwise_attention_case(32, 333, 333, 128, half=True, causal=True),
+    "attention_latent": _blockwise_attention_case(8, 4096, 4096, 40),
+    "linear_short": _linear_case(120, 768, 768),
+    "linear_short_down": _linear_case(120, 768, 3072),
+    "linear_short_f16": _linear_f16_case(333, 4096, 4096),
+    "linear_short_ffn_f16": _linear_f16_case(333, 11008, 4096),
+    "linear_short_down_f16": _linear_f16_case(333, 4096, 11008),
+    "conv_exact": _conv_case(64, 128, 8, 8, 128, 3, 1, 1, "Residual tower's convolution in exact f32: 4096 positions, 128 -> 128 channels"),
 }
 
 
 def _is_f16(name: str) -> bool:
     return "f16" in name
+
+
+def _is_exact(name: str) -> bool:
+    return "exact" in name
 
 
 def load_peaks():
@@ -305,7 +334,7 @@ def run_case(name: str, launches: int, device: int):
     graph, batch, inputs = CASES[name](np.random.Generator(np.random.PCG64(1)))
     hbm, tf32, source = load_peaks()
     lines = []
-    with CudaExecutor(device, graph, batch, math_mode=MATH_TF32) as ex:
+    with CudaExecutor(device, graph, batch, math_mode=MATH_F32 if _is_exact(name) else MATH_TF32) as ex:
         ex.evaluate(inputs)
         ex.set_profile(True)
         ex.run_async()
@@ -320,8 +349,9 @@ def run_case(name: str, launches: int, device: int):
             rec = {"case": name, "step": idx, "kind": kind, "desc": desc, "us": round(us, 2)}
             if flops > 0:
                 # f16 operands: the dense f16 / bf16 rate (the measured bf16 GEMM figure); f32 storage: TF32, half of it
-                peak = 2.0 * tf32 if _is_f16(name) else tf32
-                rec.update(bound="tensor", achieved=round(flops / us / 1e6, 1), unit="TFLOP/s", peak=peak,
+                # (exact f32: 148 SMs x 128 lanes x 1.965 GHz)
+                peak = 74.4 if _is_exact(name) else (2.0 * tf32 if _is_f16(name) else tf32)
+                rec.update(bound="fma" if _is_exact(name) else "tensor", achieved=round(flops / us / 1e6, 1), unit="TFLOP/s", peak=peak,
                            frac=round(flops / us / 1e6 / peak, 3))
             else:
                 rec.update(bound="hbm", achieved=round(alg_bytes / us / 1e3, 1), unit="GB/s", peak=hbm,

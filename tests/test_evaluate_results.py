@@ -100,3 +100,32 @@ def test_small_results_do_not_hold_large_ones():
     for a, few in zip(inputs, small):
         np.testing.assert_array_equal(few, a[:, :5] + np.float32(1))
     assert len(addresses) <= 4
+
+
+def test_executors_of_several_threads():
+    """Executors of their own, evaluated at once: large inputs and results find the copy helpers taken or free."""
+    import threading
+    g = Graph()
+    g.output(g.add(g.input(shape(BATCH, 300001)), g.scalar(1.0)))
+    failures = []
+
+    def user(seed):
+        rng = np.random.default_rng(seed)
+        kept = []
+        try:
+            with CudaExecutor(0, g, 2) as ex:
+                for _ in range(12):
+                    a = rng.standard_normal((2, 300001)).astype(np.float32)
+                    kept.append((a, ex.evaluate([a])[0]))
+                    kept = kept[-4:]
+                    for a, got in kept:
+                        np.testing.assert_array_equal(got, a + np.float32(1))
+        except BaseException as e:  # noqa: BLE001
+            failures.append(e)
+
+    threads = [threading.Thread(target=user, args=(s,)) for s in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures

@@ -83,3 +83,26 @@ def test_matches_oracle(b, m, n, k, what):
     # products of operands of 11 bits (TF32, f16), f32 sums; results of size 1: 2e-3 of the largest
     assert_tensors_match(expected, got, 2e-3, 2e-3, abs_scaled=True)
     assert np.array_equal(got[0], again[0])
+
+
+@pytest.mark.gpu
+def test_behind_a_long_kernel():
+    """What runs in front of it does not count towards the limit of its waits: a reduction of seconds, then a sliced matmul,
+    which is resident from that kernel's start on."""
+    from kyanite_b200.executor import CudaExecutor
+    alone, inputs = build(1, 120, 96, 512, seed=4)
+    expected = cpu_eval_graph(alone.to_bytes(), 0, inputs)
+    r = np.random.Generator(np.random.PCG64(4))
+    g = Graph()
+    k = 1 << 28
+    row = g.broadcast(g.view(g.input(shape(1), DType.F16), shape(1, 1, 1)), shape(1, 1, k))   # (reads one element k times)
+    g.output(g.batched_mat_mul(row, g.permute(row, [0, 2, 1])))
+    x = g.input(shape(1, 120, 512))
+    r.standard_normal((1, 120, 512))
+    w = g.constant_tensor((r.standard_normal((1, 96, 512)) / np.sqrt(512)).astype(np.float32))
+    g.output(g.batched_mat_mul(x, g.permute(w, [0, 2, 1])))
+    steps = [l for l in plan_describe(g, 0, MATH_TF32).splitlines() if l.startswith("step")]
+    assert len(steps) == 2 and " tile=" in steps[1], steps
+    with CudaExecutor(0, g, 0, math_mode=MATH_TF32) as ex:
+        got = ex.evaluate([np.ones(1, np.float16), inputs[0]])
+    assert_tensors_match(expected, got[1:], 2e-3, 2e-3, abs_scaled=True)
