@@ -16,11 +16,13 @@
 //
 // Inside a CTA the phases of a block follow one another (scores, exponentials, context); what fills the tensor cores and
 // the special-function unit meanwhile is the SM's second CTA: 256 columns of tensor memory, some 100 KB of shared memory
-// (head dimensions up to 64 in f32 or 128 in f16; larger ones run one CTA per SM).
+// (head dimensions up to 64 in f32 or 128 in f16; larger ones run one CTA per SM).  Two CTAs of 320 threads leave a thread 96
+// registers, of which a row's 64 scores take two thirds: every variant spills 240 to 280 bytes.
 //
-// Measured, scores matmul + softmax + copies + context matmul planned node by node -> this step: 32 heads of 2048 causal
-// rows, f16, d = 128: 122 + 155 + 15 + 57 -> 84 us; 8 heads of 4096 rows, f32,
-// d = 40: 117 + 198 + 99 -> 137 us; 12 heads of 120 rows: 5 + 3 + 14 + 4 -> 9 us; 32 heads of 333 rows, f16: 215 -> 18 us.
+// Measured, scores matmul + softmax + copies + context matmul planned node by node -> this step (kernel_bench's
+// attention_causal_f16, attention_latent and attention_short_f16): 32 heads of 2048 causal rows, f16, d = 128:
+// 122 + 155 + 15 + 57 -> 98 us, 10 of them flash_finite_kernel; 8 heads of 4096 rows, f32, d = 40: 117 + 198 + 99 -> 134 us;
+// 32 heads of 333 causal rows, f16, d = 128: 215 -> 20 us.
 // What bounds it: a block is some 6 000 cycles of a CTA (scores seen 1 200 after the issuer starts them, read 1 000, maximum
 // 300, exponentials 1 800, context MMAs 1 300 at 80 cycles an instruction with A from tensor memory), two CTAs in turn.
 #include <cuda.h>

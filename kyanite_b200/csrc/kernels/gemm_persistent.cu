@@ -508,8 +508,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 // cluster sums rows [r * per, (r + 1) * per) in slice order, adds the addends and stores along the rows; any strides, any
 // alignment.  At most 128 registers a thread: two CTAs to an SM, this kernel's and the next one's among them.
 // us a launch, before (persistent kernel, K slices through a scratch buffer and a second kernel) -> now: 120 x 768 x 768
-// 11.6 -> 7.5, 120 x 768 x 3072 16.6 -> 10.3, 333 x 4096 x 4096 f16 33.7 -> 21.3, 333 x 4096 x 11008 f16 58.7 -> 38.6,
-// 333 x 11008 x 4096 f16 52.7 -> 40.8, 3x3 convolution of 32 x 32 positions, 640 -> 640 channels 37.5 -> 26.6.
+// 11.6 -> 7.1, 120 x 768 x 3072 16.6 -> 9.7, 333 x 4096 x 4096 f16 33.7 -> 20.7, 333 x 4096 x 11008 f16 58.7 -> 38.5,
+// 333 x 11008 x 4096 f16 52.7 -> 40.6 (kernel_bench's linear_short*), 3x3 convolution of 32 x 32 positions, 640 -> 640 channels 37.5 -> 26.6.
 constexpr int kGsThreads = 256;
 constexpr int kGsMaxSlices = 8;   // the largest portable cluster
 
