@@ -52,6 +52,7 @@ constexpr int kFlBlockBytes = 128 * 128;   // 128 rows of 128 bytes
 constexpr int kFlTmemCols = 256, kFlOutCol = 128;
 constexpr float kLog2e = 1.44269504088896340736f;
 constexpr float kRiseLimit = 8.0f;
+constexpr float kHalfSumBelow = -1024.f;   // f16 values are one apart here
 constexpr uint32_t kFlSleepNs = 1000;
 
 struct FlashParams {
@@ -269,7 +270,13 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                                     if (col0 + c * 32 + i + q < p.n) a[q] = (float)t[(int64_t)(c * 32 + i + q) * p.term_s[2]];
                             }
 #pragma unroll
-                            for (int q = 0; q < 8; q++) v[c][i + q] = __float_as_uint(fmaf(p.scale, __uint_as_float(v[c][i + q]), a[q]));
+                            for (int q = 0; q < 8; q++) {
+                                float x = fmaf(p.scale, __uint_as_float(v[c][i + q]), a[q]);
+                                // Far below anything a row with an unmasked key looks at, f16 sums are rounded as such: a row
+                                // that is masked by f16's lowest value throughout has the same sum, or -infinity, everywhere.
+                                if (HALF && x < kHalfSumBelow) x = __half2float(__float2half_rn(x));
+                                v[c][i + q] = __float_as_uint(x);
+                            }
                         }
                     }
                 }

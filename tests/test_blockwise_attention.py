@@ -33,10 +33,9 @@ CONSTANT = ("causal", "lowest", "blocks_of_infinity")
 def constant_term(kind, m, n, dtype, r):
     if kind == "causal":
         return np.triu(np.full((1, m, n), -np.inf, dtype), 1)
-    if kind == "lowest":        # the lowest finite value; in f32, which absorbs the scores, one row has nothing else
+    if kind == "lowest":        # the lowest finite value, which absorbs the scores; one row has nothing else
         t = np.where(r.random((1, m, n)) < 0.5, np.finfo(dtype).min, 0).astype(dtype)
-        if dtype == np.float32:
-            t[0, 3] = np.finfo(dtype).min
+        t[0, 3] = np.finfo(dtype).min
         return t
     t = np.zeros((1, m, n), dtype)   # a row whose first keys are all masked, one that sees the last key only, a dead one
     t[0, 1, : max(n - 3, 1)] = -np.inf
