@@ -191,6 +191,7 @@ struct ConvParams {
     int64_t s_in[4], s_f[4], s_out[4], s1[4], s2[4];
     int32_t act;
     int32_t round_tf32;
+    int32_t f_const;     // the filter is a constant: it may be read before the kernels in front have finished
 };
 
 // ---- a run of stride-1 3x3 same-padding convolutions executed by ONE kernel, activations resident

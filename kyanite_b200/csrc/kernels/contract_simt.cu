@@ -7,6 +7,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <initializer_list>
 #include <mutex>
 #include <utility>
@@ -37,6 +38,11 @@ __device__ __forceinline__ float apply_epilogue(float v, int act, int round_tf32
 
 struct OneTap {};
 
+// Where a row of the A operand is, for the table that contract_cols_kernel keeps in shared memory: an element offset and,
+// for a convolution, the window's first tap (kNoRow: the row does not exist).
+struct RowAt { int64_t at; int iy, ix; };
+constexpr int kNoRow = -(1 << 30);
+
 struct GemmProblem {
     GemmParams p;
     using Element = float;
@@ -62,6 +68,19 @@ struct GemmProblem {
         if (p.add2) acc += p.add2[o.b * p.s2[0] + o.m * p.s2[1] + n * p.s2[2]];
         p.c[o.b * p.sc[0] + o.m * p.sc[1] + n * p.sc[2]] = apply_epilogue(acc, p.act, p.round_tf32);
     }
+    __device__ RowAt row_at(int64_t b, int64_t m) const { return RowAt{b * p.sa[0] + m * p.sa[1], 0, 0}; }
+    __device__ bool inside(const RowAt&, const Tap&) const { return true; }
+    __device__ int64_t tap_offset(const Tap&) const { return 0; }
+    __device__ bool b_constant() const { return p.b_const != 0; }
+    // where the result and the addends of a row are; their strides along the columns
+    struct Line { int64_t o, a1, a2; };
+    __device__ Line line(int64_t b, int64_t m) const {
+        return Line{b * p.sc[0] + m * p.sc[1], b * p.s1[0] + m * p.s1[1], b * p.s2[0] + m * p.s2[1]};
+    }
+    __device__ float* result() const { return p.c; }
+    __device__ int64_t result_stride() const { return p.sc[2]; }
+    __device__ int64_t add1_stride() const { return p.s1[2]; }
+    __device__ int64_t add2_stride() const { return p.s2[2]; }
 };
 
 // The same problem with f16 storage: operands and addends are converted on load, products accumulate in f32,
@@ -134,6 +153,19 @@ struct ConvProblem {
         if (p.add2) acc += p.add2[o.a2 + n * p.s2[1]];
         p.out[o.o + n * p.s_out[1]] = apply_epilogue(acc, p.act, p.round_tf32);
     }
+    __device__ RowAt row_at(int64_t b, int64_t m) const {
+        const Row r = row(b, m);
+        return RowAt{r.at - p.in, r.iy, r.ix};
+    }
+    __device__ bool inside(const RowAt& r, const Tap& t) const { return (unsigned)(r.iy + t.fy) < (unsigned)p.h && (unsigned)(r.ix + t.fx) < (unsigned)p.w; }
+    __device__ int64_t tap_offset(const Tap& t) const { return t.a; }
+    __device__ bool b_constant() const { return p.f_const != 0; }
+    using Line = Out;
+    __device__ Line line(int64_t b, int64_t m) const { return out(b, m); }
+    __device__ float* result() const { return p.out; }
+    __device__ int64_t result_stride() const { return p.s_out[1]; }
+    __device__ int64_t add1_stride() const { return p.s1[1]; }
+    __device__ int64_t add2_stride() const { return p.s2[1]; }
 };
 
 // ---------------------------------------------------------------- the kernel
@@ -403,23 +435,378 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
     }
 }
 
+// ---------------------------------------------------------------- B along its columns
+// The kernel for operands B whose columns, not whose reduction, are contiguous: V of an attention step as it comes, and the
+// filters and weights that the planner lays out this way (plan.cpp: `filter_rows`).
+//
+// A tile of B is [K][columns] in shared memory, so two neighbouring columns of a thread are one 64-bit operand of a packed
+// multiply-add (fma.rn.f32x2) whose other factor is one element of A twice: half the instructions of plain multiply-adds and
+// no pair of operands in one register bank.  Tiles along K (contract_simt_kernel above) cannot have that without twice the
+// accumulators.  A matmul of 16384 x 1024 x 2048: 0.73 of 74.4 TFLOP/s (the chip's own limit for either form at the clocks it
+// holds is 70 to 72) against 0.66.
+//    64 x 64, 8 x 8 per thread, two groups, 128 threads, three CTAs per SM: the registers allow no more, and twelve warps an
+//             SM hide the shared reads that eight of a 128 x 128 tile do not (equal where those fill the chip, 0.66 against
+//             0.56 where they do not)
+//    32 x 32, 4 x 4 per thread, four groups: for problems of a few tiles, where it is the number of CTAs that counts
+// What a small problem costs is latency, so: the constant operand is requested ahead of the dependency wait, for as many
+// stages as there are; rows are located once, in a table, and not by divisions in the loop; slices of a tile send their sums to
+// the CTA that stores them (one cluster barrier, no remote reads).
+// One 8 x 8 board, 128 -> 128 channels, 3 x 3: 12.1 us on contract_simt_kernel, 5.5 us here; 64 boards 48 -> 36 us, 256 boards 112 us
+// (0.61 of the rate); 12 heads of 120 x 64 x 120 (probabilities . V) 14.1 -> 4.8 us.
+template <int BM, int BN, int TM, int TN, int KG, int ST>
+struct ColsLayout {
+    static constexpr int kThreads = BM / TM * (BN / TN) * KG;
+    static constexpr int kPitchA = BK + 4, kBytesA = BM * kPitchA * 4, kStage = kBytesA + BK * BN * 4;
+    static constexpr int kPitchC = BN + 4, kTile = KG * BM * kPitchC * 4;
+    static constexpr int kFront = ST * kStage > kTile ? ST * kStage : kTile;   // stages, then (in their place) the partial tiles
+    static constexpr int kUnits = BM * BN / 4;                                  // groups of four columns
+    static constexpr int kReceived = (kUnits + 8) * 16;                         // sums sent by the other slices
+    static constexpr int kBytes = kFront + kReceived + BM * (int)sizeof(RowAt) + BM * 24;
+};
+
+__device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*(uint64_t*)&a), "l"(*(uint64_t*)&b), "l"(*(uint64_t*)&c));
+    return *(float2*)&d;
+}
+
+struct ColsArgs {
+    int slices;
+    Load load_a;
+    bool wide_b;      // 16-byte fetches of B
+    bool rows_fast;   // the result's rows, not its columns, are contiguous
+    bool wide_c;      // four columns of the result are one aligned 16-byte store
+};
+
+template <class Problem, int BM, int BN, int TM, int TN, int KG, int ST, int OCC>
+__global__ void __launch_bounds__(BM / TM * (BN / TN) * KG, OCC)
+contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant__ ColsArgs args) {
+    using L = ColsLayout<BM, BN, TM, TN, KG, ST>;
+    constexpr int TX = BN / TN, TY = BM / TM, NT = L::kThreads;
+    static_assert(TX % 4 == 0 && TY % 8 == 0 && TN % 4 == 0, "lane layout");
+    extern __shared__ __align__(16) uint8_t smem[];
+    float4* const received = (float4*)(smem + L::kFront);
+    RowAt* const rows = (RowAt*)(smem + L::kFront + L::kReceived);
+    typename Problem::Line* const lines = (typename Problem::Line*)(rows + BM);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int slices = args.slices;
+    if (slices > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (waited for before the first remote store)
+    const int64_t M = prob.rows(), N = prob.cols();
+    const int inner = (int)prob.inner(), taps = prob.taps();
+    const int slice = (int)(blockIdx.z % (unsigned)slices);
+    const int64_t batch = blockIdx.z / (unsigned)slices;
+    const int64_t m0 = (int64_t)blockIdx.x * BM, n0 = (int64_t)blockIdx.y * BN;
+    const int tid = threadIdx.x;
+
+    const int per_tap = max(1, (inner + BK - 1) / BK);
+    const int total = inner > 0 ? taps * per_tap : 0, per_slice = (total + slices - 1) / slices;
+    const int kb_first = min(slice * per_slice, total), blocks = min(kb_first + per_slice, total) - kb_first;
+
+    // B: row kk of a K block is row (tap, block * BK + kk) of the operand
+    constexpr int kChunksB = BN / 4, kRowStepB = NT / kChunksB, kRowsB = BK / kRowStepB;
+    static_assert(NT % kChunksB == 0 && BK % kRowStepB == 0 && NT % 8 == 0 && BM % (NT / 8) == 0, "fetch layout");
+    const int64_t b_stride = prob.b_stride();
+    const float* const b_first = prob.col(batch, n0);
+    const int b_chunk = tid % kChunksB, b_row = tid / kChunksB;
+    const int b_bytes = (int)max((int64_t)0, min((int64_t)4, N - n0 - b_chunk * 4)) * 4;
+    auto load_b = [&](int stage, const typename Problem::Tap& tap, int block) {
+        float* Bs = (float*)(smem + stage * L::kStage + L::kBytesA);
+        const int left = inner - block * BK;
+        const float* src = prob.b_at(b_first, tap) + (int64_t)block * BK * b_stride;
+        if (args.wide_b) {
+            const float* at = src + b_row * b_stride + b_chunk * 4;
+            const uint32_t to = smem_addr(Bs + b_row * BN + b_chunk * 4);
+#pragma unroll
+            for (int i = 0; i < kRowsB; i++) {
+                const bool in = b_row + i * kRowStepB < left && b_bytes > 0;
+                fetch16(to + i * kRowStepB * BN * 4, in ? at + (int64_t)i * kRowStepB * b_stride : b_first, in ? b_bytes : 0);
+            }
+        } else {
+#pragma unroll 4
+            for (int e = tid; e < BK * BN; e += NT) {
+                const int kk = e / BN, nn = e % BN;
+                const bool in = kk < left && n0 + nn < N;
+                fetch1(Bs + e, in ? src + kk * b_stride + nn : b_first, in);
+            }
+        }
+    };
+    int load_tap = kb_first / per_tap, load_block = kb_first - load_tap * per_tap;   // what load_a fetches next
+    typename Problem::Tap tap = prob.tap(load_tap);
+    const bool early_b = prob.b_constant();
+    if (early_b) {
+        int t = load_tap, block = load_block;
+        typename Problem::Tap at = tap;
+        for (int s = 0; s < ST - 1 && s < blocks; s++) {
+            load_b(s, at, block);
+            if (++block == per_tap) {
+                block = 0;
+                if (++t < taps) prob.next(at);
+            }
+        }
+    }
+    for (int i = tid; i < BM; i += NT) {
+        const bool in = m0 + i < M;
+        rows[i] = in ? prob.row_at(batch, m0 + i) : RowAt{0, kNoRow, 0};
+        lines[i] = prob.line(batch, in ? m0 + i : 0);
+    }
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    // A, 16-byte fetches: chunk tid % 8 of rows tid / 8 + i * kRowStepA
+    constexpr int kRowStepA = NT / 8, kRowsA = BM / kRowStepA;
+    const float* const a_base = prob.a_base();
+    const int a_chunk = tid % 8, a_row = tid / 8;
+    const float* a_at[kRowsA];
+    uint32_t a_read = 0;
+    auto enter_tap = [&] {
+        a_read = 0;
+        if (args.load_a != Load::Wide) return;
+        const int64_t offset = prob.tap_offset(tap) + load_block * BK + a_chunk * 4;
+#pragma unroll
+        for (int i = 0; i < kRowsA; i++) {
+            const RowAt r = rows[a_row + i * kRowStepA];
+            const bool in = r.iy != kNoRow && prob.inside(r, tap);
+            a_read |= (uint32_t)in << i;
+            a_at[i] = in ? a_base + r.at + offset : a_base;
+        }
+    };
+    enter_tap();
+    auto load_a = [&](int stage) {
+        float* As = (float*)(smem + stage * L::kStage);
+        const int k0 = load_block * BK;
+        if (args.load_a == Load::Wide) {
+            const int left = inner - k0 - a_chunk * 4, bytes = min(4, max(0, left)) * 4;
+            const uint32_t to = smem_addr(As + a_row * L::kPitchA + a_chunk * 4);
+#pragma unroll
+            for (int i = 0; i < kRowsA; i++) {
+                const bool in = (a_read >> i) & 1;
+                fetch16(to + i * kRowStepA * L::kPitchA * 4, left > 0 ? a_at[i] : a_base, in ? bytes : 0);
+                a_at[i] += in ? BK : 0;
+            }
+        } else {
+            const bool along_k = args.load_a == Load::AlongK;
+            const int64_t stride = prob.a_stride(), offset = prob.tap_offset(tap) + k0 * stride;
+#pragma unroll 4
+            for (int e = tid; e < BM * BK; e += NT) {
+                const int mm = along_k ? e / BK : e % BM, kk = along_k ? e % BK : e / BM;
+                const RowAt r = rows[mm];
+                const bool in = r.iy != kNoRow && k0 + kk < inner && prob.inside(r, tap);
+                fetch1(As + mm * L::kPitchA + kk, in ? a_base + r.at + offset + kk * stride : a_base, in);
+            }
+        }
+    };
+    auto advance = [&] {
+        if (++load_block == per_tap) {
+            load_block = 0;
+            if (++load_tap < taps) {
+                prob.next(tap);
+                enter_tap();
+            }
+        }
+    };
+
+    const int group = tid / (TX * TY), rank = tid % (TX * TY), warp = rank >> 5, lane = rank & 31;
+    // (which lanes share rows and columns: see contract_simt_kernel)
+    const int tx = ((lane & 1) | ((lane >> 4) << 1)) + 4 * (warp % (TX / 4)), ty = ((lane >> 1) & 7) + 8 * (warp / (TX / 4));
+    float2 acc[TM][TN / 2];
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN / 2; j++) acc[i][j] = make_float2(0.f, 0.f);
+
+#pragma unroll 1
+    for (int s = 0; s < ST - 1; s++) {
+        if (s < blocks) {
+            if (!early_b) load_b(s, tap, load_block);
+            load_a(s);
+            advance();
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int stage = 0, next = ST - 1;
+#pragma unroll 1
+    for (int b = 0; b < blocks; b++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+        __syncthreads();   // stage `b` is complete, and everybody has read stage `b - 1`, which is filled next
+        if (b + ST - 1 < blocks) {
+            load_b(next, tap, load_block);
+            load_a(next);
+            advance();
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float* As = (const float*)(smem + stage * L::kStage) + ty * L::kPitchA + group * (BK / KG);
+        const float* Bs = (const float*)(smem + stage * L::kStage + L::kBytesA) + group * (BK / KG) * BN + tx * 4;
+#pragma unroll
+        for (int k = 0; k < BK / KG; k += 4) {
+            float4 a[TM];
+#pragma unroll
+            for (int i = 0; i < TM; i++) a[i] = read4(As + i * TY * L::kPitchA + k);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                float4 w[TN / 4];
+#pragma unroll
+                for (int j = 0; j < TN / 4; j++) w[j] = read4(Bs + (k + q) * BN + j * TX * 4);
+#pragma unroll
+                for (int i = 0; i < TM; i++) {
+                    const float x = q == 0 ? a[i].x : q == 1 ? a[i].y : q == 2 ? a[i].z : a[i].w;
+#pragma unroll
+                    for (int j = 0; j < TN / 4; j++) {
+                        acc[i][2 * j] = fma_pair(make_float2(x, x), make_float2(w[j].x, w[j].y), acc[i][2 * j]);
+                        acc[i][2 * j + 1] = fma_pair(make_float2(x, x), make_float2(w[j].z, w[j].w), acc[i][2 * j + 1]);
+                    }
+                }
+            }
+        }
+        if (++stage == ST) stage = 0;
+        if (++next == ST) next = 0;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+
+    // the tile, one per thread group, in shared memory: [KG][BM][BN + 4]
+    float* tile = (float*)smem;
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN / 4; j++)
+            *(float4*)(tile + (group * BM + ty + i * TY) * L::kPitchC + (j * TX + tx) * 4) =
+                make_float4(acc[i][2 * j].x, acc[i][2 * j].y, acc[i][2 * j + 1].x, acc[i][2 * j + 1].y);
+    __syncthreads();
+    if (slices > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // units of four columns, in the order in which the result's contiguous axis comes first; of several slices, each
+    // stores `share` of them
+    const int share = (L::kUnits + slices - 1) / slices;
+    auto place = [&](int u, int& mm, int& nn) {
+        mm = args.rows_fast ? u % BM : u / (BN / 4);
+        nn = (args.rows_fast ? u / BM : u % (BN / 4)) * 4;
+    };
+    float* const result = prob.result();
+    const int64_t c_stride = prob.result_stride(), s1 = prob.add1_stride(), s2 = prob.add2_stride();
+    auto store = [&](int mm, int nn, float4 v) {
+        if (m0 + mm >= M) return;
+        const typename Problem::Line l = lines[mm];
+        float x[4] = {v.x, v.y, v.z, v.w};
+        const int64_t n = n0 + nn;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (n + i >= N) break;
+            if (prob.p.add1) x[i] += prob.p.add1[l.a1 + (n + i) * s1];
+            if (prob.p.add2) x[i] += prob.p.add2[l.a2 + (n + i) * s2];
+            x[i] = apply_epilogue(x[i], prob.p.act, prob.p.round_tf32);
+            if (!args.wide_c) result[l.o + (n + i) * c_stride] = x[i];
+        }
+        if (args.wide_c && n < N) *(float4*)(result + l.o + n) = make_float4(x[0], x[1], x[2], x[3]);
+    };
+    for (int u = tid; u < L::kUnits; u += NT) {
+        int mm, nn;
+        place(u, mm, nn);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int g = 0; g < KG; g++) {
+            const float4 t = *(const float4*)(tile + (g * BM + mm) * L::kPitchC + nn);
+            v.x += t.x, v.y += t.y, v.z += t.z, v.w += t.w;
+        }
+        if (slices == 1) {
+            store(mm, nn, v);
+        } else {
+            const int owner = u / share;
+            uint32_t to;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_addr(received + slice * share + u - owner * share)), "r"(owner));
+            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+        }
+    }
+    if (slices > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        for (int u = tid; u < share && slice * share + u < L::kUnits; u += NT) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+            for (int q = 0; q < slices; q++) {
+                const float4 t = received[q * share + u];
+                v.x += t.x, v.y += t.y, v.z += t.z, v.w += t.w;
+            }
+            int mm, nn;
+            place(slice * share + u, mm, nn);
+            store(mm, nn, v);
+        }
+    }
+}
+
+// Dynamic shared memory above 48 KB is opted in to once per device and kernel.
+template <class Kernel>
+int allow_shared(Kernel kernel, int bytes, bool (&done)[64], std::mutex& mu) {
+    int device = 0;
+    cudaGetDevice(&device);
+    std::lock_guard<std::mutex> lock(mu);
+    if (device >= 0 && device < 64 && !done[device]) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return (int)e;
+        done[device] = true;
+    }
+    return 0;
+}
+
+template <class Problem, int BM, int BN, int TM, int TN, int KG, int ST, int OCC>
+int launch_cols_tile(const Problem& prob, int64_t M, int64_t N, int64_t batch, const ColsArgs& args, int at_least, cudaStream_t stream) {
+    using L = ColsLayout<BM, BN, TM, TN, KG, ST>;
+    auto kernel = contract_cols_kernel<Problem, BM, BN, TM, TN, KG, ST, OCC>;
+    static std::mutex mu;
+    static bool done[64] = {false};
+    const int smem = std::max(L::kBytes, at_least);
+    if (int e = allow_shared(kernel, std::max(L::kBytes, 80 * 1024), done, mu)) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((M + BM - 1) / BM), (unsigned)((N + BN - 1) / BN), (unsigned)(batch * args.slices));
+    cfg.blockDim = dim3(L::kThreads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = (unsigned)args.slices;
+    cfg.attrs = attr;
+    cfg.numAttrs = args.slices > 1 ? 2 : 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, prob, args);
+}
+
+// Can contract_cols_kernel take the problem: as many tiles as the grid holds, K blocks that 32 bits count
+bool cols_fits(int64_t M, int64_t N, int64_t batch, int64_t k_blocks) {
+    return k_blocks < (1 << 25) && (N + 31) / 32 <= 65535 && batch * 8 <= 65535 && (M + 31) / 32 <= 0x7FFFFFFFll;
+}
+
+template <class Problem>
+int launch_cols(const Problem& prob, int64_t M, int64_t N, int64_t batch, int64_t k_blocks, ColsArgs args, cudaStream_t stream) {
+    if (M == 0 || N == 0 || batch == 0) return 0;
+    // The tile and the number of slices whose busiest SM is done first: n CTAs of it, at the cycles that a K block and a CTA
+    // were measured to take when several (or one) share an SM.
+    enum { kLarge, kLargeAlone, kSmall } tile = kSmall;
+    int64_t best = INT64_MAX, per_sm = 1;
+    auto consider = [&](decltype(tile) t, int64_t tiles, int64_t slices) {
+        const int64_t n = (tiles * slices + 147) / 148, blocks = (k_blocks + slices - 1) / slices;
+        const int64_t block = t == kLarge ? (n <= 2 ? 1650 : 1550) : t == kLargeAlone ? 1900 : (n == 1 ? 900 : 650);
+        const int64_t cost = n * (block * blocks + 700) + (slices > 1 ? 1500 : 0);
+        if (cost < best) best = cost, tile = t, args.slices = (int)slices, per_sm = n;
+    };
+    const int64_t large = ((M + 63) / 64) * ((N + 63) / 64) * batch, small = ((M + 31) / 32) * ((N + 31) / 32) * batch;
+    for (int64_t slices = 1; slices <= 8 && (slices == 1 || k_blocks >= 4 * slices); slices++) {
+        consider(kSmall, small, slices);
+        consider(large * slices <= 148 ? kLargeAlone : kLarge, large, slices);
+    }
+    if (tile == kSmall) return launch_cols_tile<Problem, 32, 32, 4, 4, 4, 6, 2>(prob, M, N, batch, args, 0, stream);
+    if (tile == kLargeAlone) return launch_cols_tile<Problem, 64, 64, 8, 8, 4, 3, 1>(prob, M, N, batch, args, 0, stream);
+    // (two CTAs an SM are kept at two by the shared memory they ask for: three on some SMs and one on others took 81 us
+    // instead of 57 for 1024 x 1024 x 1024)
+    return launch_cols_tile<Problem, 64, 64, 8, 8, 2, 3, 3>(prob, M, N, batch, args, per_sm == 2 ? 80 * 1024 : 0, stream);
+}
+
 template <class Problem, int BM, int BN, int TN, int KG, class Index = int>
 int launch_tile(const Problem& prob, int64_t gx, int64_t gy, int64_t batch, const TileArgs& args, cudaStream_t stream) {
     auto kernel = contract_simt_kernel<Problem, BM, BN, TN, KG, Index>;
     constexpr int smem = smem_bytes<typename Problem::Element, BM, BN, KG>;
-    // (the opt-in to more than 48 KB is per device)
     static std::mutex mu;
     static bool done[64] = {false};
-    int device = 0;
-    cudaGetDevice(&device);
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (device >= 0 && device < 64 && !done[device]) {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            if (e != cudaSuccess) return (int)e;
-            done[device] = true;
-        }
-    }
+    if (int e = allow_shared(kernel, smem, done, mu)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)gx, (unsigned)gy, (unsigned)(batch * args.slices));
     cfg.blockDim = dim3(kThreads);
@@ -472,6 +859,12 @@ int launch_gemm(const GemmParams& p, cudaStream_t stream) {
     const int element = p.half ? 2 : 4;
     TileArgs args{1, load_of(p.a, p.sa[2], {p.sa[0], p.sa[1]}, element), load_of(p.b, p.sb[1], {p.sb[0], p.sb[2]}, element), p.sc[1] == 1 && p.sc[2] != 1};
     if (p.half) return launch(GemmProblemHalf{p}, p.m, p.n, p.batch, 1, p.k, args, stream);
+    const int64_t k_blocks = (p.k + BK - 1) / BK;
+    if (p.sb[2] == 1 && cols_fits(p.m, p.n, p.batch, k_blocks)) {
+        const bool wide_c = p.sc[2] == 1 && p.n % 4 == 0 && p.sc[0] % 4 == 0 && p.sc[1] % 4 == 0 && ((uintptr_t)p.c & 15) == 0;
+        const ColsArgs cols{1, args.load_a, load_of(p.b, p.sb[2], {p.sb[0], p.sb[1]}, 4) == Load::Wide, args.rows_fast, wide_c};
+        return launch_cols(GemmProblem{p}, p.m, p.n, p.batch, k_blocks, cols, stream);
+    }
     return launch(GemmProblem{p}, p.m, p.n, p.batch, 1, p.k, args, stream);
 }
 
@@ -565,6 +958,12 @@ int launch_gemm_simt(const GemmParams& p, cudaStream_t stream) {
 int launch_conv_simt(const ConvParams& p, cudaStream_t stream) {
     TileArgs args{1, load_of(p.in, p.s_in[1], {p.s_in[0], p.s_in[2], p.s_in[3]}, 4), load_of(p.filter, p.s_f[1], {p.s_f[0], p.s_f[2], p.s_f[3]}, 4),
                   p.s_out[1] != 1};
+    const int64_t positions = (int64_t)p.n * p.oh * p.ow, k_blocks = (int64_t)p.r * p.s * ((p.c + BK - 1) / BK);
+    if (p.s_f[0] == 1 && cols_fits(positions, p.k, 1, k_blocks)) {
+        const bool wide_c = p.s_out[1] == 1 && p.k % 4 == 0 && p.s_out[0] % 4 == 0 && p.s_out[2] % 4 == 0 && p.s_out[3] % 4 == 0 && ((uintptr_t)p.out & 15) == 0;
+        const ColsArgs cols{1, args.load_a, load_of(p.filter, p.s_f[0], {p.s_f[1], p.s_f[2], p.s_f[3]}, 4) == Load::Wide, args.rows_fast, wide_c};
+        return launch_cols(ConvProblem{p}, positions, p.k, 1, k_blocks, cols, stream);
+    }
     return launch(ConvProblem{p}, (int64_t)p.n * p.oh * p.ow, p.k, 1, (int64_t)p.r * p.s, p.c, args, stream);
 }
 

@@ -233,6 +233,7 @@ class Planner {
             s.gemm.a_const = plan_.buffers[s.operands[0].buf].kind == BufKind::Const ? 1 : 0;
             s.gemm.b_const = plan_.buffers[s.operands[1].buf].kind == BufKind::Const ? 1 : 0;
         }
+        if (s.kind == StepKind::Conv) s.conv.f_const = plan_.buffers[s.operands[1].buf].kind == BufKind::Const ? 1 : 0;
         plan_.steps.push_back(std::move(s));
     }
 
@@ -1757,8 +1758,8 @@ class Planner {
             }
         }
         if (!tensor_core && ci.op == OpKind::Conv && g_.values[ci.inputs[1]].op == OpKind::Constant) {
-            // the exact-f32 kernel, too, reads both operands along the channels when it can
-            w = tap_major_filter(w, ci.inputs[1], false);
+            // the exact-f32 kernel reads the filter along its output channels and, when it can, the image along its channels
+            w = filter_rows(w, ci.inputs[1]);
             if (exact_conv_products(m->contraction) >= 20e6) x = channels_last(x, ci.inputs[0]);   // (a copy is a launch: 3 us)
             bool chained = false;
             for (int u : users_[root])
@@ -2454,6 +2455,23 @@ class Planner {
         PlanTensor dst = dense.with(dense.ss.permute({2, 3, 0, 1})).slice(1, 0, C, 1);
         emit_copy(w, dst, value);
         return dst;
+    }
+
+    // Constant filter [K, C, R, S] -> [R*S][C][K padded to 4], the layout of the exact kernel (a K-major one where it is no
+    // plain constant).
+    PlanTensor filter_rows(const PlanTensor& w, int value) {
+        const int64_t K = w.ss.shape[0], C = w.ss.shape[1], R = w.ss.shape[2], S = w.ss.shape[3];
+        const int64_t k_pad = (K + 3) / 4 * 4;
+        const ValueInfo& wi = g_.values[value];
+        if (wi.op != OpKind::Constant || !w.ss.has_simple_strides() || w.offset != 0) return tap_major_filter(w, value, false);
+        auto data = std::make_shared<std::vector<uint8_t>>((size_t)(R * S * C * k_pad) * 4, 0);
+        const uint8_t* src = (const uint8_t*)wi.const_data;
+        for (int64_t k = 0; k < K; k++)
+            for (int64_t c = 0; c < C; c++)
+                for (int64_t tap = 0; tap < R * S; tap++)
+                    memcpy(data->data() + 4 * ((tap * C + c) * k_pad + k), src + 4 * ((k * C + c) * R * S + tap), 4);
+        PlanTensor t = alloc_const({R, S, C, k_pad}, DType::F32, value, nullptr, data);
+        return t.with(t.ss.permute({3, 2, 0, 1})).slice(0, 0, K, 1);   // logical [K, C, R, S]
     }
 
     // ---------------------------------------------------------------- gather

@@ -143,3 +143,31 @@ def test_long_reduction(dtype, k, side):
     with CudaExecutor(0, g, 0, math_mode=MATH_F32) as ex:
         got, = ex.evaluate([np.zeros(1, dtype.np)])
     np.testing.assert_array_equal(got, np.full((1, side, side), k // period))
+
+
+# B along its columns: tiles of 32 and of 64, with and without slices of K (3, 7 and 8 of them), K blocks that end inside a
+# slice, rows of A and of B that are and are not whole 16-byte pieces, columns past the last tile
+@pytest.mark.parametrize("b,m,n,k", [(1, 64, 128, 1152), (1, 33, 36, 930), (12, 120, 64, 120), (2, 1024, 80, 77), (1, 4096, 128, 420), (1, 2050, 190, 1040),
+                                     (1, 31, 30, 33), (30, 63, 65, 64)])
+@pytest.mark.parametrize("addend", [False, True])
+def test_matmul_along_columns(b, m, n, k, addend):
+    rng = np.random.default_rng(m + n + k)
+    g = Graph()
+    y = g.batched_mat_mul(g.input(shape(b, m, k)), g.input(shape(b, k, n)))
+    if addend:
+        y = g.relu(g.add(g.add(y, g.constant_tensor(rng.standard_normal((1, 1, n)).astype(np.float32))), g.input(shape(b, m, n))))
+    g.output(y)
+    shapes = [(b, m, k), (b, k, n)] + ([(b, m, n)] if addend else [])
+    check(g, [(rng.standard_normal(s) * (k ** -0.25 if i < 2 else 1)).astype(np.float32) for i, s in enumerate(shapes)])
+
+
+# a filter laid out along its output channels at planning time, results along channels and along positions
+@pytest.mark.parametrize("n,c,k,hw", [(1, 128, 128, 8), (1, 21, 70, 9), (64, 40, 128, 8), (2, 64, 34, 7)])
+def test_convolution_chain_of_few_positions(n, c, k, hw):
+    rng = np.random.default_rng(n + c + k)
+    g = Graph()
+    weight = lambda o, i, s: g.constant_tensor((rng.standard_normal((o, i, s, s)) * (i * s * s) ** -0.5).astype(np.float32))  # noqa: E731
+    y = g.relu(g.conv(g.input(shape(n, c, hw, hw)), weight(k, c, 3), 1, 1, 1, 1))
+    y = g.relu(g.add(g.conv(y, weight(k, k, 3), 1, 1, 1, 1), y))
+    g.output(g.conv(y, weight(5, k, 1), 1, 1, 0, 0))
+    check(g, [rng.standard_normal((n, c, hw, hw)).astype(np.float32)])
