@@ -29,6 +29,7 @@ SOURCES = [
     "kernels/elementwise.cu",
     "kernels/rows.cu",
     "kernels/rows_f16.cu",
+    "kernels/softmax_matmul.cu",
     "kernels/gather.cu",
     "kernels/host_copy.cu",
     "kernels/contract_simt.cu",

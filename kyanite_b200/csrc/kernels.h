@@ -162,6 +162,8 @@ struct GemmParams {
     // may be read (past n: padding); `scratch`, if there is one, takes an I32 flag per batch entry and key block (see
     // flash_finite_kernel); batch entry bt of C lies at (bt / out_heads) * sc[0] + (bt % out_heads) * sc[1], its
     // rows sc[2] apart, columns contiguous.
+    // 4: C = softmax(softmax_scale * A + add1) . B in f32 without the tensor cores (kernels/softmax_matmul.cu): A are the scores,
+    // [batch][m][k], C lies as in 3, B's columns are contiguous (or it is a head split read in place, `b4`).
     int32_t row_softmax;
     float softmax_scale;
     int32_t out_heads, term_cols;
@@ -265,6 +267,8 @@ int launch_layernorm_f16(const RowParams& p, cudaStream_t stream);
 int launch_gather(const GatherParams& p, cudaStream_t stream);
 int launch_im2col(const Im2colParams& p, cudaStream_t stream);
 int launch_gemm_simt(const GemmParams& p, cudaStream_t stream);
+constexpr int64_t kSoftmaxMatmulMaxKeys = 1024, kSoftmaxMatmulMaxCols = 128;
+int launch_softmax_matmul(const GemmParams& p, cudaStream_t stream);   // p.row_softmax == 4
 int launch_conv_simt(const ConvParams& p, cudaStream_t stream);
 int launch_host_copy(const HostCopyParams& p, cudaStream_t stream);
 

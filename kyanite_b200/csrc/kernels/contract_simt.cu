@@ -926,6 +926,7 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(const __grid_constant_
 }  // namespace
 
 int launch_gemm_simt(const GemmParams& p, cudaStream_t stream) {
+    if (p.row_softmax == 4) return launch_softmax_matmul(p, stream);
     if (p.half) return launch_gemm(p, stream);
     if (p.n >= 1 && p.n <= kSkinnyMaxN && p.k >= 32 && p.batch * p.m > 0) {
         const int64_t rows = p.batch * p.m;

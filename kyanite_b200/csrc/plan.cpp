@@ -531,6 +531,7 @@ class Planner {
     PlanTensor visit_new(int v) {
         if (auto fused = try_fused_attention_context(v)) return *fused;
         if (auto fused = try_flash_attention(v, 0)) return *fused;
+        if (auto fused = try_softmax_matmul(v, 0)) return *fused;
         if (auto fused = try_merged_attention(v)) return *fused;
         if (auto fused = try_fused_contraction(v)) return *fused;
         if (auto fused = try_fused_rmsnorm(v)) return *fused;
@@ -1444,7 +1445,73 @@ class Planner {
         if (g_.values[c].op != OpKind::MatMul || !fusable(c) || map_[c]) return std::nullopt;
         const std::vector<int64_t> split = shape_of(w), whole = shape_of(c);
         if (split.size() != 4 || whole.size() != 3 || split[0] * split[1] != whole[0] || split[2] != whole[1] || split[3] != whole[2]) return std::nullopt;
-        return try_flash_attention(c, split[1]);
+        if (auto fused = try_flash_attention(c, split[1])) return fused;
+        return try_softmax_matmul(c, split[1]);
+    }
+
+    // matmul(softmax([c *] X [+ term]), V) of f32 values where the matmul keeps f32 operands in the default mode: softmax and product are one step
+    // (kernels/softmax_matmul.cu), with the head merge that follows, if there is one (`heads` > 0, as above).
+    std::optional<PlanTensor> try_softmax_matmul(int v, int64_t heads) {
+        const ValueInfo& mi = g_.values[v];
+        if (mi.op != OpKind::MatMul || mi.dtype != DType::F32 || opts_.math_mode != KN_MATH_TF32 || shape_of(v).size() != 3) return std::nullopt;
+        const int sv = mi.inputs[0], vin = mi.inputs[1];
+        const ValueInfo& si = g_.values[sv];
+        if (si.op != OpKind::Softmax || si.axis != 2 || !fusable(sv) || map_[sv] || vin == sv) return std::nullopt;
+        const std::vector<int64_t> ss = shape_of(sv), vs = shape_of(vin);
+        const int64_t batch = ss[0], m = ss[1], n = ss[2], dv = vs[2];
+        if (batch < 1 || m < 1 || n < 1 || n > kSoftmaxMatmulMaxKeys || dv < 4 || dv > kSoftmaxMatmulMaxCols || dv % 4 != 0) return std::nullopt;
+        // (few rows, any number of heads: larger products are bound by arithmetic, of which contract_cols_kernel does twice as
+        // much per second; fewer than 2^31 CTAs)
+        if (2.0 * (double)batch * (double)m * (double)n * (double)dv >= 4e8 || batch * ((m + 15) / 16) >= (1ll << 31)) return std::nullopt;
+        float unused;
+        const int y = peel_positive_scale(si.inputs[0], &unused);   // scores and softmax are one step already
+        if (y >= 0 && g_.values[y].op == OpKind::MatMul && attn_softmax_fits(batch, m, n, shape_of(g_.values[y].inputs[0])[2])) return std::nullopt;
+        GemmOperand4D v4{};
+        PlanTensor values;
+        int64_t ob = 0, orows = 0, ocols = 0;
+        if (!(head_chain_operand(vin, false, DType::F32, &v4, &values, &ob, &orows, &ocols, 1) && v4.kd == dv && ob == batch && orows == n &&
+              v4.strides[0] == 1 && values.offset % 4 == 0 && v4.strides[1] % 4 == 0 && v4.strides[2] % 4 == 0 && v4.strides[3] % 4 == 0)) {
+            v4 = GemmOperand4D{};
+            values = visit(vin);
+            const auto& st = values.ss.strides;
+            if (st[2] != 1 || st[1] % 4 != 0 || st[0] % 4 != 0 || values.offset % 4 != 0) return std::nullopt;   // (V is planned either way)
+        }
+        PlanTensor probabilities = values, matrix = values;
+        probabilities.ss = StridedShape({batch, m, n}, {m * n, n, 1}), probabilities.offset = 0;
+        if (v4.enabled) matrix.ss = StridedShape({batch, n, dv}, {n * dv, dv, 1}), matrix.offset = 0;
+        if (gemm_fits_tensor_core(probabilities, matrix) || gemm_worth_a_copy(probabilities, matrix)) return std::nullopt;
+        const SoftmaxInput x = softmax_input(sv);
+        const int64_t out_heads = heads > 0 ? heads : batch;
+        PlanTensor out = heads > 0 ? alloc_shared({batch / heads, m, heads, dv}, DType::F32, v) : alloc_shared({batch, m, dv}, DType::F32, v);
+        Step s;
+        s.kind = StepKind::Gemm;
+        s.value = v;
+        s.operands = {x.in, values, out};
+        s.writes = {0, 0, 1};
+        GemmParams& p = s.gemm;
+        p.batch = batch, p.m = m, p.n = dv, p.k = n;
+        for (int i = 0; i < 3; i++) {
+            p.sa[i] = x.in.ss.strides[i];
+            if (!v4.enabled) p.sb[i] = values.ss.strides[i];
+        }
+        p.b4 = v4;
+        if (x.term) {
+            s.operands.push_back(*x.term);
+            s.writes.push_back(0);
+            for (int i = 0; i < 3; i++) p.s1[i] = x.term->ss.strides[i];
+        }
+        p.out_heads = (int32_t)out_heads;
+        p.sc[0] = m * out_heads * dv;
+        p.sc[1] = heads > 0 ? dv : m * dv;
+        p.sc[2] = heads > 0 ? out_heads * dv : dv;
+        p.splits = 1;
+        p.row_softmax = 4;
+        p.softmax_scale = x.scale;
+        s.flops = 2.0 * (double)batch * (double)m * (double)n * (double)dv;
+        s.desc = "softmax(x) . V b=" + std::to_string(batch) + " m=" + std::to_string(m) + " keys=" + std::to_string(n) + " dv=" + std::to_string(dv) +
+                 (x.term ? " +term" : "") + (heads > 0 ? ", heads merged" : "") + (v4.enabled ? " (head split read in place: operand v)" : "");
+        push_step(std::move(s));
+        return out;
     }
 
     // ---------------------------------------------------------------- projections of one tensor as one matmul
@@ -2535,24 +2602,31 @@ class Planner {
         p.out_axis_stride = out.ss.strides[axis];
     }
 
-    PlanTensor visit_softmax(int v) {
-        const ValueInfo& info = g_.values[v];
-        KN_CHECK(info.dtype == DType::F32 || info.dtype == DType::F16, KN_ERR_UNSUPPORTED, "softmax needs f32 or f16");
-        // softmax(c * x + mask): the scale and the additive term (an attention mask, usually a broadcast view)
-        // are applied as the row is loaded instead of by an elementwise step of their own
-        float scale = 1.f;
+    // softmax(c * x + mask): the scale and the additive term (an attention mask, usually a broadcast view)
+    // are applied as the row is loaded instead of by an elementwise step of their own
+    struct SoftmaxInput {
+        float scale;
         PlanTensor in;
         std::optional<PlanTensor> term;
+    };
+    SoftmaxInput softmax_input(int v) {
+        const ValueInfo& info = g_.values[v];
         const int input = info.inputs[0];
         const ValueInfo& ii = g_.values[input];
         if (ii.op == OpKind::Binary && ii.binary_op == BinaryOp::Add && ii.dtype == info.dtype && fusable(input) && !map_[input] &&
             !match_epilogue(input)) {
             auto [s0, t0] = visit_scalable(ii.inputs[0]);
             auto [s1, t1] = visit_scalable(ii.inputs[1]);
-            if (s1 == 1.f && t0.ss.shape == t1.ss.shape) { scale = s0; in = t0; term = t1; }
-            else if (s0 == 1.f && t0.ss.shape == t1.ss.shape) { scale = s1; in = t1; term = t0; }
+            if (s1 == 1.f && t0.ss.shape == t1.ss.shape) return {s0, t0, t1};
+            if (s0 == 1.f && t0.ss.shape == t1.ss.shape) return {s1, t1, t0};
         }
-        if (!term) std::tie(scale, in) = visit_scalable(input);
+        auto [scale, in] = visit_scalable(input);
+        return {scale, in, std::nullopt};
+    }
+    PlanTensor visit_softmax(int v) {
+        const ValueInfo& info = g_.values[v];
+        KN_CHECK(info.dtype == DType::F32 || info.dtype == DType::F16, KN_ERR_UNSUPPORTED, "softmax needs f32 or f16");
+        const auto [scale, in, term] = softmax_input(v);
         PlanTensor out = alloc_shared(shape_of(v), info.dtype, v);
         Step s;
         s.kind = StepKind::Softmax;
