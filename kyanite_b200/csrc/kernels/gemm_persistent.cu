@@ -506,12 +506,22 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 //   - the next kernel is released at once, so that it can do the same.
 // The partial tile goes to shared memory (row pitch bn + 4 floats: conflict-free for 16-byte accesses), CTA r of the
 // cluster sums rows [r * per, (r + 1) * per) in slice order, adds the addends and stores along the rows; any strides, any
-// alignment.  At most 128 registers a thread: two CTAs to an SM, this kernel's and the next one's among them.
-// us a launch, before (persistent kernel, K slices through a scratch buffer and a second kernel) -> now: 120 x 768 x 768
-// 11.6 -> 7.1, 120 x 768 x 3072 16.6 -> 9.7, 333 x 4096 x 4096 f16 33.7 -> 20.7, 333 x 4096 x 11008 f16 58.7 -> 38.5,
-// 333 x 11008 x 4096 f16 52.7 -> 40.6 (kernel_bench's linear_short*), 3x3 convolution of 32 x 32 positions, 640 -> 640 channels 37.5 -> 26.6.
-constexpr int kGsThreads = 256;
+// alignment.  Stored rows are bound by instructions (eight epilogue warps, each address and predicate counts) and, with
+// slices, by the 16 bytes per cycle that an SM reads from other SMs' shared memory.  Hence four columns of a fixed column
+// group per thread, rows a constant step apart, variants of the loop by addends and slices, and addends that differ by row
+// requested four rows ahead, the first of them under the MMAs.  (Item by item, with addresses, addends and predicates worked
+// out for each, a tile's way out took 5 000 to 25 000 of the kernel's 20 000 to 60 000 cycles; sent as 16-byte remote stores
+// instead of read, the partial sums of four slices and more took half as long again.)
+// The producer's and the issuer's warps are not epilogue warps: set-up of the epilogue would otherwise follow the last MMA.
+// At most 96 registers a thread: two CTAs to an SM, this kernel's and the next one's among them.
+// us a launch, before the epilogue by column groups -> now: 120 x 2304 x 768 9.7 -> 8.4, 120 x 3072 x 768 + GELU 10.8 -> 10.3,
+// 333 x 4096 x 4096 f16 21.0 -> 17.2, 333 x 4096 x 11008 f16 38.6 -> 36.0, 333 x 11008 x 4096 f16 40.4 -> 33.3,
+// 4096 x 320 x 320 + bias + skip 16.6 -> 8.0, 4096 x 320 x 1280 + bias + skip 21.8 -> 13.9, 3x3 convolution of 32 x 32
+// positions, 640 -> 640 channels 26.4 -> 24.0.
+constexpr int kGsThreads = 320;   // eight epilogue warps, the producer's and the issuer's
+constexpr int kGsEpilogue = 256;
 constexpr int kGsMaxSlices = 8;   // the largest portable cluster
+constexpr int kGsBatch = 4;       // rows that a thread of the epilogue has in flight
 
 struct GemmSlicesParams {
     GemmPersistentParams g;
@@ -567,7 +577,7 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         *abandon = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {
+    if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_addr), "r"((uint32_t)q.tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -585,35 +595,34 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const int a_row0 = mt * kGpBlockM, b_row0 = nt * p.bn;
 
     bool good = true;
-    if (warp == 0 && lane == 0) {
-        // ---------------- producer
+    if (warp == 8) {
+        // ---------------- producer.  Lane s fills stage s first: one pass over the set-up arithmetic for all stages
         const int first = min(stages, k_count);
-        OperandCursor<HALF, false> constant(p, a_row0, b_row0, bt, k_begin), other = constant;
-        for (int s = 0; s < first; s++) {
-            const uint32_t dst = base + (uint32_t)s * stage_bytes, bar = full_bar + 8u * s;
-            mbar_expect_tx(bar, stage_bytes);
-            if (q.a_const) constant.load_a(p, &map_a, dst, bar, a_row0, bt);
-            if (q.b_const) constant.load_b(p, &map_b, dst + kGpATileBytes, bar, b_row0, bt);
-            constant.next(p);
+        OperandCursor<HALF, false> cursor(p, a_row0, b_row0, bt, k_begin + lane);
+        const uint32_t my_dst = base + (uint32_t)lane * stage_bytes, my_bar = full_bar + 8u * lane;
+#pragma unroll 1
+        for (int pass = 0; pass < 2; pass++) {   // the constant operand, then the other
+            if (pass == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+            if (lane < first) {
+                if (pass == 0) mbar_expect_tx(my_bar, stage_bytes);
+                if ((q.a_const != 0) == (pass == 0)) cursor.load_a(p, &map_a, my_dst, my_bar, a_row0, bt);
+                if ((q.b_const != 0) == (pass == 0)) cursor.load_b(p, &map_b, my_dst + kGpATileBytes, my_bar, b_row0, bt);
+            }
         }
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        for (int s = 0; s < first; s++) {
-            const uint32_t dst = base + (uint32_t)s * stage_bytes, bar = full_bar + 8u * s;
-            if (!q.a_const) other.load_a(p, &map_a, dst, bar, a_row0, bt);
-            if (!q.b_const) other.load_b(p, &map_b, dst + kGpATileBytes, bar, b_row0, bt);
-            other.next(p);
+        if (lane == first - 1) {   // its cursor is the last one requested
+            int s = 0, round = 1;
+#pragma unroll 1
+            for (int k = first; k < k_count; k++) {
+                cursor.next(p);
+                if (!mbar_wait(empty_bar + 8u * s, (uint32_t)((round & 1) ^ 1), abandon, p.status, 31)) break;
+                const uint32_t dst = base + (uint32_t)s * stage_bytes, bar = full_bar + 8u * s;
+                mbar_expect_tx(bar, stage_bytes);
+                cursor.load_a(p, &map_a, dst, bar, a_row0, bt);
+                cursor.load_b(p, &map_b, dst + kGpATileBytes, bar, b_row0, bt);
+                if (++s == stages) { s = 0; round++; }
+            }
         }
-        int s = 0, round = 1;
-        for (int k = first; k < k_count; k++) {
-            if (!mbar_wait(empty_bar + 8u * s, (uint32_t)((round & 1) ^ 1), abandon, p.status, 31)) break;
-            const uint32_t dst = base + (uint32_t)s * stage_bytes, bar = full_bar + 8u * s;
-            mbar_expect_tx(bar, stage_bytes);
-            other.load_a(p, &map_a, dst, bar, a_row0, bt);
-            other.load_b(p, &map_b, dst + kGpATileBytes, bar, b_row0, bt);
-            other.next(p);
-            if (++s == stages) { s = 0; round++; }
-        }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 9 && lane == 0) {
         // ---------------- MMA issuer (the instruction descriptor of gemm_persistent_kernel)
         // (the clock of a bounded wait starts when the kernels in front are done, however long they take)
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -636,15 +645,66 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         if (good) mma_commit(acc_full);
     }
     __syncwarp();
-    asm volatile("griddepcontrol.wait;" ::: "memory");   // (the addends and the output belong to earlier kernels until here)
-    // the accumulator is complete, and with it every read of the stages: they become the partial tile
-    if (lane == 0) good = mbar_wait(acc_full, 0, abandon, p.status, 33, kWaitCycles, 2000) && good;
+
+    // The result's rows of this CTA: a thread of the epilogue takes four columns of every row_step-th row
+    const int rows = (int)min((int64_t)kGpBlockM, p.m - (int64_t)mt * kGpBlockM), per = (rows + splits - 1) / splits;
+    const int my_rows = max(0, min(per, rows - sp * per));
+    const int cols = (int)min((int64_t)p.bn, p.n - (int64_t)nt * p.bn), groups = (cols + 3) >> 2;
+    const int row_step = kGsEpilogue / groups, row0 = threadIdx.x / groups, col = (threadIdx.x - row0 * groups) * 4, valid = min(4, cols - col);
+    const bool mine = row0 < row_step;
+    using T = typename std::conditional<HALF, __half, float>::type;
+    using Four = typename std::conditional<HALF, uint2, float4>::type;   // four elements
+    auto whole = [&](const float* addend, const int64_t* st, bool aligned) { return addend == nullptr || aligned || st[2] == 0; };
+    const bool vec = q.out_vec != 0 && (cols & 3) == 0 && whole(p.add1, p.s1, q.add1_vec) && whole(p.add2, p.s2, q.add2_vec);
+    // An addend that all rows share is read once, any other a batch of rows ahead (the first batch under the MMAs), as
+    // `extra` and, if there are two, `extra2`
+    const bool rows1 = p.add1 && p.s1[1] != 0, rows2 = p.add2 && p.s2[1] != 0;
+    const int extras = (rows1 ? 1 : 0) + (rows2 ? 1 : 0);
+    const T *add1 = nullptr, *add2 = nullptr, *extra = nullptr, *extra2 = nullptr;
+    const int64_t extra_row = rows1 ? p.s1[1] : p.s2[1], extra2_row = p.s2[1];
+    const bool extra_one = (rows1 ? p.s1[2] : p.s2[2]) == 0, extra2_one = p.s2[2] == 0;   // one value per row
+    T* out = nullptr;
+    float shared[4] = {0.f, 0.f, 0.f, 0.f};
+    Four next[kGsBatch], next2[kGsBatch];
+    auto four = [&](const T* from, bool one) {
+        if (!one) return *(const Four*)from;
+        Four v;
+        T* e = (T*)&v;
+        e[0] = *from, e[1] = e[0], e[2] = e[0], e[3] = e[0];
+        return v;
+    };
+    auto fetch = [&](int row) {
+#pragma unroll
+        for (int i = 0; i < kGsBatch; i++) {
+            const int r = row + i * row_step;
+            if (r < my_rows) {
+                next[i] = four(extra + r * extra_row, extra_one);
+                if (extras > 1) next2[i] = four(extra2 + r * extra2_row, extra2_one);
+            }
+        }
+    };
+    if (warp < kGsEpilogue / 32) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // (the addends and the output belong to earlier kernels until here)
+        const int64_t m = (int64_t)mt * kGpBlockM + sp * per, n = (int64_t)nt * p.bn + col;
+        out = (T*)q.out + bt * q.so[0] + m * q.so[1] + n * q.so[2];
+        if (p.add1) add1 = (const T*)p.add1 + bt * p.s1[0] + m * p.s1[1] + n * p.s1[2];
+        if (p.add2) add2 = (const T*)p.add2 + bt * p.s2[0] + m * p.s2[1] + n * p.s2[2];
+        extra = rows1 ? add1 : add2, extra2 = add2;
+        if (mine && vec) {
+            if (p.add1 && !rows1) add_four(shared, add1, p.s1[2], q.add1_vec != 0, 4);
+            if (p.add2 && !rows2) add_four(shared, add2, p.s2[2], q.add2_vec != 0, 4);
+            if (extras) fetch(row0);
+        }
+        // the accumulator is complete, and with it every read of the stages: they become the partial tile
+        if (lane == 0) good = mbar_wait(acc_full, 0, abandon, p.status, 33, kWaitCycles, 1000) && good;
+    }
     good = __syncthreads_and(good ? 1 : 0) != 0;
-    if (good) {
+    if (good && warp < kGsEpilogue / 32) {
         tc_fence_after();
         const int quarter = warp & 3;
         const uint32_t row_addr = base + (uint32_t)(quarter * 32 + lane) * pitch;
-        for (int c = warp >> 2; c < (p.bn >> 5); c += kGsThreads / 128) {
+#pragma unroll 1
+        for (int c = warp >> 2; c < (p.bn >> 5); c += kGsEpilogue / 128) {
             uint32_t v[32];
             tmem_load_32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c * 32), v);
 #pragma unroll
@@ -655,80 +715,145 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
         tc_fence_before();
     }
-    __syncthreads();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)q.tmem_cols) : "memory");
     if (splits > 1) cluster_sync_all();   // every slice's partial tile lies in its CTA's shared memory
+    else __syncthreads();
+    if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)q.tmem_cols) : "memory");
 
-    {
-        const int rows = (int)min((int64_t)kGpBlockM, p.m - (int64_t)mt * kGpBlockM), per = (rows + splits - 1) / splits;
-        const int row_end = good ? min(rows, (sp + 1) * per) : 0;
-        const int64_t col_tile = (int64_t)nt * p.bn;
-        const int cols = (int)min((int64_t)p.bn, p.n - col_tile);
-        // lanes of a warp: 8, 16 or 32 groups of four columns, the rest of the warp further rows
-        const int group_bits = p.bn <= 32 ? 3 : (p.bn <= 64 ? 4 : 5), warp_rows = 32 >> group_bits;
-        const int my_group = lane & ((1 << group_bits) - 1), my_row = lane >> group_bits;
-        using T = typename std::conditional<HALF, __half, float>::type;
-        const T* add1 = (const T*)p.add1;
-        const T* add2 = (const T*)p.add2;
-        T* out = (T*)q.out;
-        // items of a warp: (rows, column group); two at a time, so that the reads of both are in flight together (one at a
-        // time the sum of three slices of 128 x 256 took 6 us, of which the reads are 1)
-        const int col_groups = (cols + (4 << group_bits) - 1) / (4 << group_bits);
-        const int step_rows = (kGsThreads / 32) * warp_rows;
-        const int row_steps = max(0, (row_end - sp * per - warp * warp_rows + step_rows - 1) / step_rows);
-        auto fetch = [&](int row, int c, float (&part)[kGsMaxSlices][4]) {
-            if (row >= row_end || c >= cols) return;
-            const uint32_t local = base + (uint32_t)row * pitch + (uint32_t)c * 4u;
+    auto activate = [&](float (&y)[4]) {
+#pragma unroll 1
+        for (int j = 0; j < 4; j++) {   // (rolled: the error function would be most of the epilogue's code)
+            const float t = apply_activation(y[0], p.act);
+            y[0] = y[1], y[1] = y[2], y[2] = y[3], y[3] = t;
+        }
+    };
+    // four columns of a row of a slice's partial tile, from this CTA's rows on
+    const uint32_t from = base + (uint32_t)(sp * per) * pitch + (uint32_t)col * 4u;
+    auto partial = [&](float (&x)[4], uint32_t at) {
+        if (splits == 1) asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(at));
+        else asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(at));
+    };
+    const int end = good && mine && warp < kGsEpilogue / 32 ? my_rows : 0;
+    // kGsBatch rows at a time, with eight reads of partial sums in flight: of S slices and the rows that leaves.  What this
+    // loop costs is instructions (two warps a scheduler), so what does not change in it is decided outside
+    auto store_rows = [&](auto most, auto added) {
+        constexpr int S = decltype(most)::value, R = S == 1 ? kGsBatch : 8 / S, EXTRAS = decltype(added)::value;
+        uint32_t peer[S];
 #pragma unroll
-            for (int s = 0; s < kGsMaxSlices; s++)
-                if (s < splits)
-                    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                 : "=f"(part[s][0]), "=f"(part[s][1]), "=f"(part[s][2]), "=f"(part[s][3])
-                                 : "r"(map_to_cta(local, (uint32_t)s)));
-        };
-        auto finish = [&](int row, int c, const float (&part)[kGsMaxSlices][4]) {
-            if (row >= row_end || c >= cols) return;
-            const int64_t m = (int64_t)mt * kGpBlockM + row, n = col_tile + c;
-            const int valid = min(4, cols - c);
-            float v[4] = {part[0][0], part[0][1], part[0][2], part[0][3]};
+        for (int s = 0; s < S; s++) peer[s] = S == 1 ? from : map_to_cta(from, (uint32_t)min(s, splits - 1));
+#pragma unroll 1
+        for (int row = row0; row < end; row += kGsBatch * row_step) {
+            float y[kGsBatch][4];
+            bool in[kGsBatch];
 #pragma unroll
-            for (int s = 1; s < kGsMaxSlices; s++)
-                if (s < splits) v[0] += part[s][0], v[1] += part[s][1], v[2] += part[s][2], v[3] += part[s][3];
-            if (add1) add_four(v, add1 + bt * p.s1[0] + m * p.s1[1] + n * p.s1[2], p.s1[2], q.add1_vec != 0, valid);
-            if (add2) add_four(v, add2 + bt * p.s2[0] + m * p.s2[1] + n * p.s2[2], p.s2[2], q.add2_vec != 0, valid);
+            for (int i = 0; i < kGsBatch; i++) in[i] = row + i * row_step < end;
 #pragma unroll
-            for (int j = 0; j < 4; j++) v[j] = apply_activation(v[j], p.act);
-            T* dst = out + bt * q.so[0] + m * q.so[1] + n * q.so[2];
-            if (q.out_vec != 0 && valid == 4) {
-                if (HALF) {
-                    const __half2 lo = __floats2half2_rn(v[0], v[1]), hi = __floats2half2_rn(v[2], v[3]);
+            for (int i = 0; i < kGsBatch; i += R) {
+                float x[R][S][4];
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+#pragma unroll
+                    for (int s = 0; s < S; s++)
+                        if (in[i + r] && (S <= 2 || s < splits)) partial(x[r][s], peer[s] + (uint32_t)(row + (i + r) * row_step) * pitch);
+                }
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) y[i + r][j] = x[r][0][j];
+#pragma unroll
+                    for (int s = 1; s < S; s++) {
+                        if (S > 2 && s >= splits) break;
+#pragma unroll
+                        for (int j = 0; j < 4; j++) y[i + r][j] += x[r][s][j];
+                    }
+                }
+                if constexpr (S == 4) {
+#pragma unroll 1
+                    for (int s = S; s < splits; s++) {   // (of more than four slices, with two addends: no registers for eight)
+#pragma unroll
+                        for (int r = 0; r < R; r++)
+                            if (in[i + r]) partial(x[r][0], map_to_cta(from, (uint32_t)s) + (uint32_t)(row + (i + r) * row_step) * pitch);
+#pragma unroll
+                        for (int r = 0; r < R; r++) {
+#pragma unroll
+                            for (int j = 0; j < 4; j++) y[i + r][j] += x[r][0][j];
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < kGsBatch; i++) {
+                auto add = [&](const Four& a) {
+                    if constexpr (HALF) {
+                        const float2 lo = __half22float2(*(const __half2*)&a.x), hi = __half22float2(*(const __half2*)&a.y);
+                        y[i][0] += lo.x, y[i][1] += lo.y, y[i][2] += hi.x, y[i][3] += hi.y;
+                    } else {
+                        y[i][0] += a.x, y[i][1] += a.y, y[i][2] += a.z, y[i][3] += a.w;
+                    }
+                };
+#pragma unroll
+                for (int j = 0; j < 4; j++) y[i][j] += shared[j];
+                if constexpr (EXTRAS > 0) add(next[i]);
+                if constexpr (EXTRAS > 1) add(next2[i]);
+            }
+            if constexpr (EXTRAS > 0) fetch(row + kGsBatch * row_step);
+            if (p.act == (int)Activation::Relu) {
+#pragma unroll
+                for (int i = 0; i < kGsBatch; i++) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) y[i][j] = fmaxf(y[i][j], 0.f);
+                }
+            } else if (p.act != (int)Activation::None) {
+#pragma unroll
+                for (int i = 0; i < kGsBatch; i++)
+                    if (in[i]) activate(y[i]);
+            }
+            T* dst = out + (int64_t)row * q.so[1];
+#pragma unroll
+            for (int i = 0; i < kGsBatch; i++, dst += (int64_t)row_step * q.so[1]) {
+                if (!in[i]) continue;
+                if constexpr (HALF) {
+                    const __half2 lo = __floats2half2_rn(y[i][0], y[i][1]), hi = __floats2half2_rn(y[i][2], y[i][3]);
                     *(uint2*)dst = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
                 } else {
-                    *(float4*)dst = make_float4(v[0], v[1], v[2], v[3]);
+                    *(float4*)dst = make_float4(y[i][0], y[i][1], y[i][2], y[i][3]);
                 }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (j < valid) dst[j * q.so[2]] = (T)v[j];
             }
-        };
-        int row = sp * per + warp * warp_rows + my_row, group = 0;
-        auto advance = [&]() {
-            if (++group == col_groups) group = 0, row += step_rows;
-        };
-        for (int left = row_steps * col_groups; left > 0; left -= 2) {
-            float first[kGsMaxSlices][4], second[kGsMaxSlices][4];
-            const int row1 = row, c1 = ((group << group_bits) + my_group) * 4;
-            advance();
-            const int row2 = left > 1 ? row : row_end, c2 = ((group << group_bits) + my_group) * 4;
-            advance();
-            fetch(row1, c1, first);
-            fetch(row2, c2, second);
-            finish(row1, c1, first);
-            finish(row2, c2, second);
         }
+    };
+    auto store_all = [&](auto most) {
+        if (extras == 0) store_rows(most, std::integral_constant<int, 0>());
+        else if (extras == 1) store_rows(most, std::integral_constant<int, 1>());
+        else if constexpr (decltype(most)::value <= 4) store_rows(most, std::integral_constant<int, 2>());
+        else store_rows(std::integral_constant<int, 4>(), std::integral_constant<int, 2>());
+    };
+    if (!vec) {   // any strides, any alignment, columns that are no multiple of four
+#pragma unroll 1
+        for (int row = row0; row < end; row += row_step) {
+            float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+            for (int s = 0; s < splits; s++) {
+                float x[4];
+                partial(x, (splits == 1 ? from : map_to_cta(from, (uint32_t)s)) + (uint32_t)row * pitch);
+#pragma unroll
+                for (int j = 0; j < 4; j++) y[j] += x[j];
+            }
+            if (add1) add_four(y, add1 + row * p.s1[1], p.s1[2], q.add1_vec != 0, valid);
+            if (add2) add_four(y, add2 + row * p.s2[1], p.s2[2], q.add2_vec != 0, valid);
+            activate(y);
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (j < valid) out[row * q.so[1] + j * q.so[2]] = (T)y[j];
+        }
+    } else if (splits == 1) {
+        store_all(std::integral_constant<int, 1>());
+    } else if (splits == 2) {
+        store_all(std::integral_constant<int, 2>());
+    } else if (splits <= 4) {
+        store_all(std::integral_constant<int, 4>());
+    } else {
+        store_all(std::integral_constant<int, 8>());
     }
-    __syncthreads();
+    __syncwarp();
     if (splits > 1) cluster_sync_all();   // nobody leaves while its partial tile may still be read
 }
 
@@ -975,10 +1100,12 @@ int gemm_persistent_launch(const void* launch, cudaStream_t stream) {
 // Tile width and K slices for gemm_slices_kernel; slices = 0: the matmul is for the persistent kernel.
 //
 // The line: less than one round of the chip in the persistent kernel's tiles (at most 148 of 128 rows x its block width).
-// Within it the cheapest total wins, in SM cycles: a K block costs its MMAs (bn / 2 cycles each, four of them) or its bytes at the 60 per
-// cycle that an SM was measured to take from L2, whichever is longer; storing and summing a partial tile costs by its width,
-// a cluster some 1 200 cycles more, a CTA 2 500 before its first MMA.  A round holds fewer CTAs than there are SMs when
-// they come in clusters, which lie inside a GPC (kClusterCtas).
+// Within it the cheapest total wins, in SM cycles as clock stamps in the kernel show them: a K block costs its MMAs (bn / 2
+// cycles each, four of them) or its bytes at the 65 per cycle that an SM takes from L2, whichever is longer; a CTA 2 500 before
+// and 1 300 after its first and last MMAs; the partial tile's way to shared memory 4.5 a column and its way out 25 a column, or,
+// with slices, two cluster barriers and the bytes that come from other CTAs, of which an SM takes some 16 per cycle
+// (120 x 2304 x 768: 2 slices of 32 columns 8.4 us, 5 of 96 9.0; 640 x 1024 x 2880: 6 slices of 256 columns 16.7 us, 3 of 128
+// 18.6).  A round holds fewer CTAs than there are SMs when they come in clusters, which lie inside a GPC (kClusterCtas).
 GemmSlices gemm_slices_choose(const GemmParams& g) {
     // CTAs of one per SM that fit the chip at once, by the size of their clusters (cudaOccupancyMaxActiveClusters)
     static const int kClusterCtas[kGsMaxSlices + 1] = {0, 148, 148, 135, 132, 130, 132, 105, 120};
@@ -997,12 +1124,13 @@ GemmSlices gemm_slices_choose(const GemmParams& g) {
         if (g.b4.enabled && g.b4.rd % bn != 0 && g.b4.rd < g.n) continue;
         const int64_t tiles = m_tiles * ((g.n + bn - 1) / bn) * g.batch;
         if (tiles > (1 << 24)) continue;
-        const double block = std::max(2.0 * bn, (kGpATileBytes + 128.0 * bn) / 60.0);
+        const double block = std::max({350.0, 2.0 * bn, (kGpATileBytes + 128.0 * bn) / 65.0});
         for (int64_t want = 1; want <= kGsMaxSlices && want <= k_blocks; want++) {
             const int64_t per = (k_blocks + want - 1) / want, slices = (k_blocks + per - 1) / per;
             if (slices != want) continue;
             const double rounds = std::ceil((double)(tiles * slices) / kClusterCtas[slices]);
-            const double cost = rounds * (2500.0 + per * block + (slices > 1 ? 24.0 * bn + 1200.0 : 16.0 * bn));
+            const double store = slices > 1 ? 3600.0 + 26.0 * bn * (double)(slices - 1) / (double)slices : 25.0 * bn;
+            const double cost = rounds * (3800.0 + per * block + 4.5 * bn + store);
             if (best.slices == 0 || cost < best_cost) {
                 best_cost = cost;
                 best.slices = (int)slices;

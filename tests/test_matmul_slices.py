@@ -106,3 +106,30 @@ def test_behind_a_long_kernel():
     with CudaExecutor(0, g, 0, math_mode=MATH_TF32) as ex:
         got = ex.evaluate([np.ones(1, np.float16), inputs[0]])
     assert_tensors_match(expected, got[1:], 2e-3, 2e-3, abs_scaled=True)
+
+
+# the ways an addend reaches the rows: shared by all, one value per row, one per element, along the rows instead of the columns
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,m,n,k", [(1, 129, 96, 64), (1, 250, 320, 1280), (2, 100, 132, 768), (1, 120, 96, 4096)])
+@pytest.mark.parametrize("kinds", ["row", "row_element", "element_column", "element_element", "across", "row_across"])
+def test_addends(b, m, n, k, kinds):
+    from kyanite_b200.executor import CudaExecutor
+    r = np.random.Generator(np.random.PCG64(m + n))
+    g = Graph()
+    y = g.batched_mat_mul(g.input(shape(b, m, k)), g.permute(g.constant_tensor((r.standard_normal((b, n, k)) / np.sqrt(k)).astype(np.float32)), [0, 2, 1]))
+    inputs = [r.standard_normal((b, m, k)).astype(np.float32)]
+    for kind in kinds.split("_"):
+        if kind in ("row", "column"):
+            y = g.add(y, g.constant_tensor(r.standard_normal((b, m, 1) if kind == "row" else (b, 1, n)).astype(np.float32)))
+        else:
+            s = (b, n, m) if kind == "across" else (b, m, n)
+            t = g.input(shape(*s))
+            inputs.append(r.standard_normal(s).astype(np.float32))
+            y = g.add(y, g.permute(t, [0, 2, 1]) if kind == "across" else t)
+    g.output(y)
+    assert tile(g)
+    with CudaExecutor(0, g, 0, math_mode=MATH_TF32) as ex:
+        got = ex.evaluate(inputs)
+    expected = cpu_eval_graph(g.to_bytes(), 0, inputs)
+    # k products of operands rounded to 11 bits, each off by 2^-11 of itself: a sum of size 1 is off by 2^-11, five times that covers the largest of them
+    assert np.abs(got[0].astype(np.float64) - expected[0]).max() <= 5 * 2.0 ** -11 * max(1.0, np.abs(expected[0]).max() / 3)
