@@ -118,7 +118,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     const int e_chunks = p.dv >> 5;       // of which the first go through shared memory
     asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing above touches global memory
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---------------- producer
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
@@ -164,7 +164,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             }
             if (t + (int)gridDim.x < p.total) request_q(t + (int)gridDim.x);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---------------- MMA issuer: f32 accumulate, TF32 x TF32, both K-major, M = 128
         const uint32_t idesc_s = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(p.half_n >> 3) << 17) | ((uint32_t)(kAtBlockM >> 4) << 24);
         // (bit 16: the B operand is MN-major, its N index contiguous)

@@ -105,7 +105,7 @@ attn_softmax_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const uint32_t tmem_base = *tmem_slot;
     asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing above touches global memory
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---------------- producer
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
@@ -125,7 +125,7 @@ attn_softmax_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                                 h * p.half_n, b2, b3);
             }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---------------- MMA issuer: f32 accumulate, TF32 x TF32, both K-major, M = 128, N = half_n
         const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(p.half_n >> 3) << 17) | ((uint32_t)(kAsBlockM >> 4) << 24);
         int local = 0;

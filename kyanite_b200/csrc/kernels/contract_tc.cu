@@ -139,7 +139,7 @@ tc_contract_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         n0_img = tn * p.nb;
     }
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---------------- producer
         for (int it = 0; it < k_count; it++) {
             const int s = it % stages;
@@ -157,7 +157,7 @@ tc_contract_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 tma_load_3d(b_base + s * b_tile_bytes, &map_b, full_bar + 8u * s, cb * kBlockK, ncol0, tap);
             }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---------------- MMA issuer
         // instruction descriptor: f32 accumulate, tf32 x tf32, both K-major, M = 128, N = bn
         const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(kBlockM >> 4) << 24);
@@ -444,7 +444,7 @@ tc_conv_cl_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     // this grid's CTAs retire (its prologue then overlaps our tail) ...
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---------------- producer
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
@@ -506,7 +506,7 @@ tc_conv_cl_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             const uint32_t parity = ((it / stages) & 1) ^ 1;
             if (mbar_wait(empty_bar + 8u * st, parity, abandon, p.status, 1)) prefetch_residual();
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---------------- MMA issuer: M = 128 output channels.  The windows of the CTA's sub-tiles lie
         // back to back in the stage, (hb + R - 1) groups of 8 pixels each, so ONE instruction per tap and
         // K step covers all of them: its N spans per_cta * hb + (per_cta - 1) * (R - 1) groups, and the

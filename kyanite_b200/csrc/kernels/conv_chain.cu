@@ -196,7 +196,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap map_tiles, const __grid_co
     const uint32_t tmem_acc = *tmem_slot;
     const uint32_t tmem_held = tmem_acc + (uint32_t)p.n_mma;      // n_mma is a multiple of 16
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---------------- filter producer: tiles are consumed in the order they are stored; the filter
         // is a constant of the plan, so nothing here waits for the previous kernel
         // Within a layer the tiles may be consumed in any order (they all accumulate into the same
@@ -226,7 +226,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap map_tiles, const __grid_co
             }
             layer_base += n;
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---------------- MMA issuer
         const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(p.n_mma >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         int slot = 0, round = 0;

@@ -140,7 +140,7 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
 
     if (warp == 8) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---------------- producer
             const uint32_t qk_bytes = (uint32_t)(p.qk_blocks * kFlBlockBytes), v_bytes = (uint32_t)(p.v_panels * kFlBlockBytes);
             mbar_expect_tx(q_full, qk_bytes);
@@ -159,7 +159,7 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
         }
     } else if (warp == 9) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---------------- MMA issuer: f32 accumulate, M = 128; Q and the keys K-major, V with its columns contiguous
             // (bit 16: the MN-major B operand)
             const uint32_t fmt = HALF ? 0u : 2u;

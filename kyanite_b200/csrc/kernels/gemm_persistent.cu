@@ -236,7 +236,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     auto slice_blocks = [&](int sp) { return min(p.k_iters_slice, p.k_iters - sp * p.k_iters_slice); };
 
     if (threadIdx.x == 0) dbg_mark(p, 0, 1);
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---------------- producer
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
@@ -263,10 +263,10 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 if (++s == stages) { s = 0; round++; }
             }
         }
-    } else if (warp == 1 && lane == 0 && PAIR && rank != 0) {
+    } else if (PAIR && warp == 1 && rank != 0) {
         // the peer issues no MMAs (the leader's instructions drive both tensor cores)
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---------------- MMA issuer
         // instruction descriptor: f32 accumulate; A and B formats 2 = TF32 (kind::tf32) or 0 = F16 (kind::f16); both
         // K-major; N, M
@@ -596,33 +596,37 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
     bool good = true;
     if (warp == 8) {
-        // ---------------- producer.  Lane s fills stage s first: one pass over the set-up arithmetic for all stages
+        // ---------------- producer.  Lane s fills stage s first: one pass over the set-up arithmetic for all stages (stage by
+        // stage in one thread, launches of 120 rows took 5 to 20 % longer)
         const int first = min(stages, k_count);
-        OperandCursor<HALF, false> cursor(p, a_row0, b_row0, bt, k_begin + lane);
-        const uint32_t my_dst = base + (uint32_t)lane * stage_bytes, my_bar = full_bar + 8u * lane;
+        {
+            const OperandCursor<HALF, false> cursor(p, a_row0, b_row0, bt, k_begin + lane);
+            const uint32_t dst = base + (uint32_t)lane * stage_bytes, bar = full_bar + 8u * lane;
 #pragma unroll 1
-        for (int pass = 0; pass < 2; pass++) {   // the constant operand, then the other
-            if (pass == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
-            if (lane < first) {
-                if (pass == 0) mbar_expect_tx(my_bar, stage_bytes);
-                if ((q.a_const != 0) == (pass == 0)) cursor.load_a(p, &map_a, my_dst, my_bar, a_row0, bt);
-                if ((q.b_const != 0) == (pass == 0)) cursor.load_b(p, &map_b, my_dst + kGpATileBytes, my_bar, b_row0, bt);
+            for (int pass = 0; pass < 2; pass++) {   // the constant operand, then the other
+                if (pass == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+                if (lane < first) {
+                    if (pass == 0) mbar_expect_tx(bar, stage_bytes);
+                    if ((q.a_const != 0) == (pass == 0)) cursor.load_a(p, &map_a, dst, bar, a_row0, bt);
+                    if ((q.b_const != 0) == (pass == 0)) cursor.load_b(p, &map_b, dst + kGpATileBytes, bar, b_row0, bt);
+                }
             }
         }
-        if (lane == first - 1) {   // its cursor is the last one requested
+        if (k_count > first && elect_one()) {
+            OperandCursor<HALF, false> cursor(p, a_row0, b_row0, bt, k_begin + first);
             int s = 0, round = 1;
 #pragma unroll 1
             for (int k = first; k < k_count; k++) {
-                cursor.next(p);
                 if (!mbar_wait(empty_bar + 8u * s, (uint32_t)((round & 1) ^ 1), abandon, p.status, 31)) break;
                 const uint32_t dst = base + (uint32_t)s * stage_bytes, bar = full_bar + 8u * s;
                 mbar_expect_tx(bar, stage_bytes);
                 cursor.load_a(p, &map_a, dst, bar, a_row0, bt);
                 cursor.load_b(p, &map_b, dst + kGpATileBytes, bar, b_row0, bt);
+                cursor.next(p);
                 if (++s == stages) { s = 0; round++; }
             }
         }
-    } else if (warp == 9 && lane == 0) {
+    } else if (warp == 9 && elect_one()) {
         // ---------------- MMA issuer (the instruction descriptor of gemm_persistent_kernel)
         // (the clock of a bounded wait starts when the kernels in front are done, however long they take)
         asm volatile("griddepcontrol.wait;" ::: "memory");

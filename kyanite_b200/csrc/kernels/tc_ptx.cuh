@@ -12,6 +12,24 @@ constexpr long long kWaitCycles = 4000000000ll;   // ~2 s at 2 GHz
 // ---------------------------------------------------------------- PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// One lane of a converged warp.  The role loops (bulk copies, MMAs) run in it: their operands have to be in uniform registers,
+// and only behind `elect.sync` does the compiler know that one thread is active.  Behind `lane == 0` it emits a loop over the
+// active lanes around every such instruction.  lane == 0 -> elect.sync: the 144 MMAs (N = 80) of a layer of conv_chain_kernel
+// with one 8 x 8 board 13 350 -> 11 470 cycles, 72 of a 64-channel layer 8 600 -> 6 500 (two boards, N = 144, are bound by
+// shared memory and stay at 13 330); 2048 x 11008 x 4096 in f16 138 -> 125 us; 16384 x 3072 x 768 + GELU 139.6 -> 133.0 us.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    __syncwarp();   // (every lane of the warp calls this)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(one)
+        :
+        : "memory");
+    return one != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
