@@ -12,7 +12,7 @@ constexpr long long kWaitCycles = 4000000000ll;   // ~2 s at 2 GHz
 // ---------------------------------------------------------------- PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// One lane of a converged warp.  The role loops (bulk copies, MMAs) run in it: their operands have to be in uniform registers,
+// One lane of a converged warp.  The role loops (bulk copies, MMAs) run in it, but for the filter requests of conv_chain_kernel: their operands have to be in uniform registers,
 // and only behind `elect.sync` does the compiler know that one thread is active.  Behind `lane == 0` it emits a loop over the
 // active lanes around every such instruction.  lane == 0 -> elect.sync: the 144 MMAs (N = 80) of a layer of conv_chain_kernel
 // with one 8 x 8 board 13 350 -> 11 470 cycles, 72 of a 64-channel layer 8 600 -> 6 500 (two boards, N = 144, are bound by
