@@ -220,7 +220,7 @@ struct TileArgs {
 //    64 x  64, 8 x 4 per thread, KG 2  four times the tiles
 // Plain multiply-adds: the packed form (fma.rn.f32x2) issues at half the rate and measured 5 % slower, K blocks of 64
 // spilled registers.  4096 positions x 128 channels x 1152: 48 to 52 us
-// (kernel_bench's conv_exact); 19200 x 256 x 2304: 800 us (two tiles a SM, three
+// (36 by contract_cols_kernel, which kernel_bench's conv_exact takes now); 19200 x 256 x 2304: 800 us (two tiles a SM, three
 // rounds of 148 for 300 tiles).
 // `Index` counts along K: 64 bits for reductions that 32 do not hold.
 template <class Problem, int BM, int BN, int TN, int KG, class Index>

@@ -21,7 +21,7 @@
 //
 // Measured, scores matmul + softmax + copies + context matmul planned node by node -> this step (kernel_bench's
 // attention_causal_f16, attention_latent and attention_short_f16): 32 heads of 2048 causal rows, f16, d = 128:
-// 122 + 155 + 15 + 57 -> 98 us, 10 of them flash_finite_kernel; 8 heads of 4096 rows, f32, d = 40: 117 + 198 + 99 -> 134 us;
+// 122 + 155 + 15 + 57 -> 93 us, 10 of them flash_finite_kernel; 8 heads of 4096 rows, f32, d = 40: 117 + 198 + 99 -> 122 us;
 // 32 heads of 333 causal rows, f16, d = 128: 215 -> 20 us.
 // What bounds it: a block is some 6 000 cycles of a CTA (scores seen 1 200 after the issuer starts them, read 1 000, maximum
 // 300, exponentials 1 800, context MMAs 1 300 at 80 cycles an instruction with A from tensor memory), two CTAs in turn.
