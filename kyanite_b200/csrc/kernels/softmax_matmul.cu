@@ -50,7 +50,6 @@ __global__ void __launch_bounds__(GROUPS * 128) softmax_matmul_kernel(const __gr
     const int blocks = (p.n + kSmKeys - 1) / kSmKeys, pitch = blocks * kSmKeys + 4, block_floats = kSmKeys * p.dv;
     float* const values = (float*)smem;                                   // up to two blocks of [128 keys][columns]
     float* const prob = values + (blocks > 1 ? 2 : 1) * block_floats;     // [rows][pitch]
-    float* const inverse = prob + kRows * pitch;                          // [rows]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned bt = blockIdx.x / (unsigned)p.tiles;
     const int row0 = (int)(blockIdx.x - bt * (unsigned)p.tiles) * kRows;
@@ -117,8 +116,10 @@ __global__ void __launch_bounds__(GROUPS * 128) softmax_matmul_kernel(const __gr
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        // (divided here and not after the product, which would be out of range for values of V within `sum` of the largest f32)
+#pragma unroll 4
+        for (int c = lane; c < p.n; c += 32) e[c] /= sum;
         for (int c = p.n + lane; c < blocks * kSmKeys; c += 32) e[c] = 0.f;
-        if (lane == 0) inverse[warp + i * kWarps] = 1.f / sum;
     }
 
     // lanes 1..3 pick the row, 0 and 4 and the warp the columns (which reads are served in one pass: see contract_simt.cu)
@@ -175,7 +176,6 @@ __global__ void __launch_bounds__(GROUPS * 128) softmax_matmul_kernel(const __gr
     for (int i = 0; i < RPT; i++) {
         const int r = ty + i * 8;
         if (row0 + r >= p.m) continue;
-        const float inv = inverse[r];
 #pragma unroll
         for (int c = 0; c < PANELS; c++) {
             if (c * 16 + tx >= chunks) continue;
@@ -185,14 +185,14 @@ __global__ void __launch_bounds__(GROUPS * 128) softmax_matmul_kernel(const __gr
                 const float4 t = others[(g * kRows + r) * chunks + c * 16 + tx];
                 o.x += t.x, o.y += t.y, o.z += t.z, o.w += t.w;
             }
-            *(float4*)(out + (int64_t)(row0 + r) * p.sc[2] + (c * 16 + tx) * 4) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+            *(float4*)(out + (int64_t)(row0 + r) * p.sc[2] + (c * 16 + tx) * 4) = o;
         }
     }
 }
 
 int shared_bytes(int64_t n, int64_t dv, int64_t rows) {
     const int64_t blocks = (n + kSmKeys - 1) / kSmKeys;
-    return (int)(((blocks > 1 ? 2 : 1) * kSmKeys * dv + rows * (blocks * kSmKeys + 4) + rows) * 4);
+    return (int)(((blocks > 1 ? 2 : 1) * kSmKeys * dv + rows * (blocks * kSmKeys + 4)) * 4);
 }
 
 template <int PANELS, int RPT, int GROUPS>

@@ -71,3 +71,22 @@ def test_masked_rows_and_values_that_are_not_finite():
         expected, = cpu_eval_graph(g.to_bytes(), 0, [x, v])
     np.testing.assert_array_equal(np.isnan(got), np.isnan(expected))
     np.testing.assert_allclose(got, expected, rtol=1e-4, atol=1e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,split", [(1, 2, False), (16, 40, False), (20, 300, True), (2600, 77, False)])
+def test_values_near_the_end_of_the_range(m, n, split):
+    """The probabilities are divided by their sum before the product: a weighted mean is no larger than the largest value."""
+    b, dv, heads = 2, 8, 2
+    g = graph(b, m, n, dv, None, heads if split else 0, split)
+    rng = np.random.default_rng(m + n)
+    x = np.zeros((b, m, n), np.float32)
+    v = (rng.uniform(2e38, 3e38, (b, n, dv)) * np.where(np.arange(dv) < 4, 1.0, rng.choice([-1.0, 1.0], (b, n, dv)))).astype(np.float32)
+    operand = v.transpose(1, 0, 2).reshape(n, heads * dv) if split else v
+    with CudaExecutor(0, g, 0, math_mode=MATH_TF32) as ex:
+        got, = ex.evaluate([x, operand])
+    expected = np.broadcast_to(v.astype(np.float64).mean(axis=1, keepdims=True), (b, m, dv))
+    if split:
+        expected = expected.transpose(1, 0, 2).reshape(m, heads * dv)
+    # equal probabilities, rounded once, and f32 sums of at most 300 terms: 300 * 2^-24 of the terms' mean size
+    np.testing.assert_allclose(got, expected, rtol=0, atol=300 * 2.0 ** -24 * 3e38)
