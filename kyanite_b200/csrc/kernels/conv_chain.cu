@@ -4,8 +4,8 @@
 // every layer of the run back to back without ever leaving its SM: the activations live in shared
 // memory (as the B operand of the next layer's MMAs), the skip connection of a residual block lives in
 // tensor memory next to the accumulator, and per layer only the filter streams in from L2 through a
-// small ring (one request per filter tap: up to four 16 KB tiles, stored by the planner in the swizzled
-// byte order of shared memory so a linear bulk copy delivers them).  Compared with one launch per layer
+// small ring (a request is one filter tap or, of narrow layers, a row of three: up to six 16 KB tiles, stored by the
+// planner in the swizzled byte order of shared memory so a linear bulk copy delivers them).  Compared with one launch per layer
 // this removes, per layer, the launch, the pipeline fill, the activation round trip through L2 and the
 // output store.
 //
@@ -62,7 +62,7 @@ struct ChainKernelParams {
     int32_t n_img, c_in, k, h, w;
     int32_t n_layers, per_cta, gx, gy, wp, q_first, r_first, n_mma, rows_alloc, slots, tmem_cols, c_blocks_max;
     int32_t total_tiles;
-    int32_t group;   // filter tiles per request and per ring slot
+    int32_t group;   // filter tiles that a ring slot holds
     long long* trace; // KN_CHAIN_TRACE only: per layer 8 clock64 stamps of CTA 0, in pinned host memory
     uint8_t flags[kMaxChainLayers];
     uint8_t c_blocks[kMaxChainLayers];
@@ -118,6 +118,23 @@ constexpr uint32_t kSleepNs = 20000u;
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+
+// The order in which a layer's filter tiles are consumed, and how many come at a time: the layer has `n` of them, the CTA
+// begins at tile `first` and wraps around; a request is what fits a ring slot and divides the layer (slots full of tiles,
+// rows of three taps, or single taps; a first layer of 32 channels before layers of 64 has nine tiles for slots of six: three
+// at a time).
+struct LayerTiles {
+    int n, first, request;
+    __device__ LayerTiles(const ChainKernelParams& p, int l) {
+        const int blocks = p.c_blocks[l];
+        const bool pointwise = (p.flags[l] & kChainFlagPointwise) != 0;
+        n = (pointwise ? 1 : 9) * blocks;
+        request = n % p.group == 0 ? p.group : (!pointwise && 3 * blocks <= p.group ? 3 * blocks : blocks);
+        // (CTAs begin at whole taps of the widest layer where the layer consists of those)
+        const int unit = n % p.c_blocks_max == 0 ? p.c_blocks_max : 1;
+        first = (int)((blockIdx.x * 5u) % (uint32_t)(n / unit)) * unit;
+    }
+};
 
 // E: epilogue warps per TMEM lane quarter; CW: accumulator columns per epilogue chunk (16 or 8); TRACE: whether the
 // first CTA stamps its phases
@@ -209,24 +226,29 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap map_tiles, const __grid_co
         int layer_base = 0, slot = 0, round = 0;
         bool ok = true;
         for (int l = 0; l < p.n_layers && ok; l++) {
-            const int n = ((p.flags[l] & kChainFlagPointwise) ? 1 : 9) * p.c_blocks[l];
-            const int g = n % p.group == 0 ? p.group : 1;      // tiles per request
-            const int groups = n / g;
-            int idx = (int)((blockIdx.x * 5u) % (uint32_t)groups);
-            for (int i = 0; i < groups; i++) {
+            const LayerTiles tiles(p, l);
+            int idx = tiles.first;
+            for (int left = tiles.n; left > 0; left -= tiles.request) {
                 if (round > 0) {
                     if (!mbar_wait(empty_bar + 8u * slot, (uint32_t)((round & 1) ^ 1), abandon, p.status, 11, kWaitCycles, kSleepNs)) { ok = false; break; }
                 }
                 const uint32_t bar = full_bar + 8u * slot;
-                mbar_expect_tx(bar, (uint32_t)g * kTileBytes);
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(ring_base + (uint32_t)slot * slot_bytes), "l"(p.tiles + (size_t)(layer_base + idx * g) * (kTileBytes / 4)),
-                               "r"((uint32_t)g * kTileBytes), "r"(bar)
-                             : "memory");
-                if (++idx == groups) idx = 0;
+                mbar_expect_tx(bar, (uint32_t)tiles.request * kTileBytes);
+                uint32_t dst = ring_base + (uint32_t)slot * slot_bytes;
+                auto copy = [&](int count) {
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                 ::"r"(dst), "l"(p.tiles + (size_t)(layer_base + idx) * (kTileBytes / 4)), "r"((uint32_t)count * kTileBytes), "r"(bar)
+                                 : "memory");
+                    dst += (uint32_t)count * kTileBytes;
+                    idx += count;
+                    if (idx == tiles.n) idx = 0;
+                };
+                const int head = min(tiles.request, tiles.n - idx);
+                copy(head);
+                if (head < tiles.request) copy(tiles.request - head);   // (the request that wraps around)
                 if (++slot == p.slots) { slot = 0; round++; }
             }
-            layer_base += n;
+            layer_base += tiles.n;
         }
     } else if (warp == 1 && elect_one()) {
         // ---------------- MMA issuer
@@ -249,21 +271,17 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap map_tiles, const __grid_co
             const int cbl = p.c_blocks[l];
             uint32_t accumulate = 0;
             const bool pointwise = (p.flags[l] & kChainFlagPointwise) != 0;
-            const int n = (pointwise ? 1 : 9) * cbl;
-            const int g = n % p.group == 0 ? p.group : 1;
-            const int groups = n / g;
-            // the producer's order: start at group (blockIdx.x * 5) % groups, wrap around
-            int tile = (int)((blockIdx.x * 5u) % (uint32_t)groups) * g;
-            int tap = tile / cbl, cb = tile - tap * cbl;
+            const LayerTiles tiles(p, l);
+            int tap = tiles.first / cbl, cb = tiles.first - tap * cbl;
             if (pointwise) tap = 4;     // the centre tap: the operand starts at the pixel itself
-            for (int i = 0; i < groups && ok; i++) {
+            for (int left = tiles.n; left > 0 && ok; left -= tiles.request) {
                 long long tw = 0;
                 if (trace) tw = clock64();
                 ok = mbar_wait(full_bar + 8u * slot, (uint32_t)(round & 1), abandon, p.status, 13, kWaitCycles, kSleepNs);
                 if (!ok) break;
                 if (trace) full_wait += clock64() - tw;
                 tc_fence_after();
-                for (int u = 0; u < g; u++) {
+                for (int u = 0; u < tiles.request; u++) {
                     const int r = tap >= 6 ? 2 : (tap >= 3 ? 1 : 0), s = tap - 3 * r;
                     const uint32_t row0 = (uint32_t)(p.r_first + (r - 1) * p.wp + (s - 1));
                     const uint64_t da = smem_desc_sw128(ring_base + (uint32_t)slot * slot_bytes + (uint32_t)u * kTileBytes);
@@ -588,8 +606,8 @@ std::shared_ptr<void> chain_prepare(const ConvChainParams& c, uint32_t* status_w
         for (int d = 0; d < 4; d++) p.head_s_out[i][d] = c.head_s_out[i][d];
     }
     p.head_begin[c.n_heads] = c.head_begin[c.n_heads];
-    // one request per filter tap (all channel blocks of the tap, up to 64 KB): large requests stream at
-    // about twice the rate of single 16 KB tiles
+    // slots of one filter tap (all its channel blocks, up to 64 KB) or three taps (up to 96 KB): large requests stream at about
+    // twice the rate of single 16 KB tiles
     p.group = g.group;
     p.slots = g.slots / p.group;
     // KN_CHAIN_TRACE=1 in the environment: the traced variant of the kernel stamps clock64 per layer in its first CTA

@@ -194,3 +194,48 @@ def test_heads_match_oracle_and_separate_kernels(name):
         # scale (see test_chain_matches_oracle_and_per_layer_kernels), and a softmax turns an absolute logit
         # difference into the same RELATIVE difference of its outputs, so those are held to 2.5e-3.
         assert_tensors_match(ex.evaluate([x]), fused, 2.5e-3, 2.5e-3, abs_scaled=True)
+
+
+def order_sensitive_heads():
+    """Two 3x3 layers of 64 channels that copy their input, then a 1x1 layer of 2^24 (channel 0) + 32 x 0.125 (channels 32 to 63):
+    2^24 + 4 if the second block of 32 channels is summed first, 2^24 if every piece of it is added to 2^24 and lost."""
+    g = Graph()
+    cur = g.input(shape(BATCH, 64, 8, 8))
+    same = np.zeros((64, 64, 3, 3), np.float32)
+    same[np.arange(64), np.arange(64), 1, 1] = 1
+    for _ in range(2):
+        cur = g.relu(g.conv(cur, g.constant_tensor(same), 1, 1, 1, 1))
+    head = np.zeros((5, 64, 1, 1), np.float32)
+    head[:, 0] = 2.0 ** 12
+    head[:, 32:] = 0.125
+    g.output(g.conv(cur, g.constant_tensor(head), 1, 1, 0, 0))
+    return g
+
+
+@pytest.mark.gpu
+def test_heads_are_summed_in_one_order():
+    from kyanite_b200.executor import CudaExecutor
+    g, batch = order_sensitive_heads(), 37
+    assert "heads=5" in steps(plan_describe(g, batch, MATH_TF32))[0]
+    x = np.zeros((batch, 64, 8, 8), np.float32)
+    x[:, 0] = 2.0 ** 12
+    x[:, 32:] = 1
+    with CudaExecutor(0, g, batch, math_mode=MATH_TF32) as ex:
+        got, = ex.evaluate([x])
+    assert np.abs(got - 2.0 ** 24).max() <= 4
+    np.testing.assert_array_equal(got, np.broadcast_to(got[:1], got.shape))   # whatever its place in the batch
+
+
+# layers of other widths than the chain's widest, whose tiles come in requests of their own: the first one (32, 64 and 96 channels
+# of 32, 64 and 128), every number of boards per CTA and every starting tap
+@pytest.mark.gpu
+@pytest.mark.parametrize("channels,c_in,h,batch", [(64, 7, 8, 11), (64, 40, 9, 20), (32, 30, 8, 19), (128, 33, 8, 10), (128, 70, 7, 9), (96, 20, 8, 4), (40, 64, 6, 12)])
+def test_requests_of_every_width(channels, c_in, h, batch):
+    from kyanite_b200.executor import CudaExecutor
+    g = tower_with_heads(channels, h, h, c_in, [5], [True], seed=channels + c_in)
+    x = rng(c_in).standard_normal((batch, c_in, h, h)).astype(np.float32)
+    assert "heads=5" in steps(plan_describe(g, batch, MATH_TF32))[0]
+    expected = cpu_eval_graph(g.to_bytes(), batch, [x])
+    with CudaExecutor(0, g, batch, math_mode=MATH_TF32) as ex:
+        # (the bounds of test_heads_match_oracle_and_separate_kernels)
+        assert_tensors_match(expected, ex.evaluate([x]), 4e-3, 4e-3, abs_scaled=True)
