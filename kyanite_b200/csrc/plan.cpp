@@ -1466,6 +1466,9 @@ class Planner {
         float unused;
         const int y = peel_positive_scale(si.inputs[0], &unused);   // scores and softmax are one step already
         if (y >= 0 && g_.values[y].op == OpKind::MatMul && attn_softmax_fits(batch, m, n, shape_of(g_.values[y].inputs[0])[2])) return std::nullopt;
+        if (g_.values[vin].op == OpKind::Permute && g_.values[vin].permutation == std::vector<int>{0, 2, 1} && !map_[vin] &&
+            match_head_chain(g_.values[vin].inputs[0]))
+            return std::nullopt;   // a transposed head split: the matmul reads it in place, planned as a tensor it would be copied
         GemmOperand4D v4{};
         PlanTensor values;
         int64_t ob = 0, orows = 0, ocols = 0;

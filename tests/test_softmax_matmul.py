@@ -38,6 +38,14 @@ def test_route():
     assert len(steps(graph(12, 120, 77, 64), MATH_F32)) == 2
 
 
+def test_transposed_head_split_is_read_in_place():
+    g = Graph()
+    split = g.view(g.permute(g.view(g.input(shape(200, 128)), shape(2, 100, 4, 32)), [0, 2, 1, 3]), shape(8, 100, 32))
+    g.output(g.batched_mat_mul(g.softmax(g.input(shape(8, 70, 32)), 2), g.permute(split, [0, 2, 1])))
+    plan = steps(g, MATH_TF32)
+    assert len(plan) == 2 and "Softmax" in plan[0] and "read in place: operand b" in plan[1], plan
+
+
 CASES = [(1, 1, 1, 4, None, 0, False), (2, 15, 127, 40, "input", 0, False), (2, 17, 129, 64, None, 0, False), (3, 33, 33, 68, "causal", 0, False),
          (4, 16, 1024, 128, None, 2, False), (8, 1000, 77, 80, None, 8, True), (40, 130, 200, 36, "input", 0, False), (6, 50, 300, 24, "input", 3, True), (12, 120, 120, 64, None, 12, True), (2, 130, 257, 80, None, 1, False)]
 
