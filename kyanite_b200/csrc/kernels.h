@@ -267,7 +267,7 @@ int launch_layernorm_f16(const RowParams& p, cudaStream_t stream);
 int launch_gather(const GatherParams& p, cudaStream_t stream);
 int launch_im2col(const Im2colParams& p, cudaStream_t stream);
 int launch_gemm_simt(const GemmParams& p, cudaStream_t stream);
-constexpr int64_t kSoftmaxMatmulMaxKeys = 1024, kSoftmaxMatmulMaxCols = 128;
+constexpr int64_t kSoftmaxMatmulMaxKeys = 128, kSoftmaxMatmulMaxCols = 128;
 int launch_softmax_matmul(const GemmParams& p, cudaStream_t stream);   // p.row_softmax == 4
 int launch_conv_simt(const ConvParams& p, cudaStream_t stream);
 int launch_host_copy(const HostCopyParams& p, cudaStream_t stream);

@@ -1450,7 +1450,8 @@ class Planner {
     }
 
     // matmul(softmax([c *] X [+ term]), V) of f32 values where the matmul keeps f32 operands in the default mode: softmax and product are one step
-    // (kernels/softmax_matmul.cu), with the head merge that follows, if there is one (`heads` > 0, as above).
+    // (kernels/softmax_matmul.cu), with the head merge that follows, if there is one (`heads` > 0, as above).  Up to 128 keys:
+    // beyond, the separate steps are faster (figures there).
     std::optional<PlanTensor> try_softmax_matmul(int v, int64_t heads) {
         const ValueInfo& mi = g_.values[v];
         if (mi.op != OpKind::MatMul || mi.dtype != DType::F32 || opts_.math_mode != KN_MATH_TF32 || shape_of(v).size() != 3) return std::nullopt;

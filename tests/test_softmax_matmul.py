@@ -34,6 +34,7 @@ def test_route():
     assert len(steps(graph(12, 60, 60, 64, "input", heads=6, split=True), MATH_TF32)) == 1
     assert len(steps(graph(3, 20, 30, 6), MATH_TF32)) > 1          # columns that are no whole 16-byte pieces
     assert len(steps(graph(3, 20, 1025, 8), MATH_TF32)) > 1        # rows too long to keep
+    assert len(steps(graph(3, 20, 128, 8), MATH_TF32)) == 1 and len(steps(graph(3, 20, 129, 8), MATH_TF32)) == 2
     assert "softmax(x)" not in plan_describe(graph(64, 512, 512, 64), 0, MATH_TF32)   # for the tensor cores
     assert len(steps(graph(12, 120, 77, 64), MATH_F32)) == 2
 
@@ -47,7 +48,8 @@ def test_transposed_head_split_is_read_in_place():
 
 
 CASES = [(1, 1, 1, 4, None, 0, False), (2, 15, 127, 40, "input", 0, False), (2, 17, 129, 64, None, 0, False), (3, 33, 33, 68, "causal", 0, False),
-         (4, 16, 1024, 128, None, 2, False), (8, 1000, 77, 80, None, 8, True), (40, 130, 200, 36, "input", 0, False), (6, 50, 300, 24, "input", 3, True), (12, 120, 120, 64, None, 12, True), (2, 130, 257, 80, None, 1, False)]
+         (4, 16, 1024, 128, None, 2, False), (8, 1000, 77, 80, None, 8, True), (40, 130, 200, 36, "input", 0, False), (6, 50, 300, 24, "input", 3, True),
+         (5, 31, 125, 128, "input", 0, False), (40, 130, 126, 100, None, 8, True), (4, 9, 128, 88, None, 4, True), (2, 5, 5, 72, "causal", 0, False), (12, 120, 120, 64, None, 12, True), (2, 130, 257, 80, None, 1, False)]
 
 
 @pytest.mark.gpu
@@ -98,3 +100,20 @@ def test_values_near_the_end_of_the_range(m, n, split):
         expected = expected.transpose(1, 0, 2).reshape(m, heads * dv)
     # equal probabilities, rounded once, and f32 sums of at most 300 terms: 300 * 2^-24 of the terms' mean size
     np.testing.assert_allclose(got, expected, rtol=0, atol=300 * 2.0 ** -24 * 3e38)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,m,n,dv", [(12, 4, 128, 64), (4, 1, 77, 128), (12, 120, 120, 64), (12, 1, 1024, 32), (4, 33, 700, 88)])
+def test_error_against_64_bits(b, m, n, dv):
+    """Of a term: exponential 2 ulp at most (half an ulp on average), division and product half an ulp each, and some ten additions on
+    its way into the sum, whose errors are independent; the scores' own rounding (of up to 6) is 2^-22 at most: 3.6 units of 2^-24
+    in all.  (One running sum over 256 of 1024 keys is 5.8 units off.)"""
+    g = graph(b, m, n, dv)
+    rng = np.random.default_rng(n)
+    x, v = rng.standard_normal((b, m, n)).astype(np.float32) * 2, rng.standard_normal((b, n, dv)).astype(np.float32)
+    s = x.astype(np.float64) * 0.7
+    e = np.exp(s - s.max(axis=2, keepdims=True))
+    expected = e / e.sum(axis=2, keepdims=True) @ v.astype(np.float64)
+    with CudaExecutor(0, g, 0, math_mode=MATH_TF32) as ex:
+        got, = ex.evaluate([x, v])
+    assert np.linalg.norm(got - expected) <= 3.6 * 2.0 ** -24 * np.linalg.norm(expected)
