@@ -818,16 +818,23 @@ int launch_scalar(const ScalarParams& p, cudaStream_t stream) {
         }
     }
     // V consecutive 16-byte positions per thread spread a micro-op's decoding over more elements; fewer give a small tensor
-    // threads enough to cover its loads, which a program issues one after the other.  Four where that leaves every SM two
-    // rounds of 1024 threads, two where it leaves one.  Before, four wherever the extent allowed: 1.3 M elements, scale + shift + SiLU
-    // in f32 9.5 -> 7.5 us, their sum with a second tensor 6.5 -> 4.8; 2048 x 4096 in f16, sum 12.3 -> 9.6, half of a rotary embedding
-    // 14.1 -> 11.4.
-    auto enough = [&](int64_t elements, int64_t rounds) { return p.total / elements >= rounds * 148 * 1024; };
+    // threads enough to cover its loads, which a program issues one after the other.  Against four wherever the extent allows:
+    // 1.3 M elements, scale + shift + SiLU in f32 9.5 -> 7.5 us, their sum with a second tensor 6.5 -> 4.8; 2048 x 4096 in f16, sum
+    // 12.3 -> 9.6, half of a rotary embedding 14.1 -> 11.4.
+    // `rounds` of 1024 threads an SM, with `elements` each:
+    auto enough = [&](int64_t elements, double rounds) { return (double)p.total / (double)elements >= rounds * 148 * 1024; };
+    // Programs in f32 (or of both types) over tensors that are read as one row: what the chip holds at once is 1.52 M elements with
+    // two positions a thread (five blocks an SM) and 2.42 M with four (four blocks).  Four where two would start a second
+    // round of blocks and four does not (sum in f32, 1.86 M: 6.9 us with four, 7.2 with two; 1.4 M: 6.6 and 5.2; 2.5 M: 8.7 and 8.5),
+    // and from 1.75 rounds on (4.3 M: 12.2 and 13.1; 3.9 M: 11.4 and 11.1).  With a broadcast operand two are as good there
+    // (4.3 M: 18.9 us with four, 16.4 with two).
+    const bool four = enough(16, 2) || (p.rank == 1 && (enough(16, 1.75) || (p.total > 148 * 5 * 256 * 8 && p.total <= 148 * 4 * 256 * 16)));
     if (p.vec4 == 2) {
         // (as many as the innermost extent and the spill slots, n_regs * V * 4 KB of shared memory per block, allow)
         const int64_t inner4 = p.dims[p.rank - 1] / 4;
-        if (inner4 % 4 == 0 && p.n_regs <= 4 && enough(16, 2)) return launch_acc<4, false>(p, stream);
-        if (inner4 % 2 == 0 && enough(8, 1)) return launch_acc<2, false>(p, stream);
+        // (two from one block an SM on: 0.37 M elements, scale + shift in f32 4.9 us with one, 4.1 with two; sum 3.1 with either)
+        if (inner4 % 4 == 0 && p.n_regs <= 4 && four) return launch_acc<4, false>(p, stream);
+        if (inner4 % 2 == 0 && enough(8, 0.25)) return launch_acc<2, false>(p, stream);
         return launch_acc<1, false>(p, stream);
     } else if (p.vec4 == 5) {
         // an accumulator program over f16 only: packed halves, eight per position (the innermost extent is a multiple
@@ -839,7 +846,7 @@ int launch_scalar(const ScalarParams& p, cudaStream_t stream) {
     } else if (p.vec4 == 4) {
         // f16 / f32 mix as an accumulator program: the innermost extent is a multiple of 8 (the planner's condition)
         const int64_t inner4 = p.dims[p.rank - 1] / 4;
-        if (inner4 % 4 == 0 && p.n_regs <= 4 && enough(16, 2)) return launch_acc<4, true>(p, stream);
+        if (inner4 % 4 == 0 && p.n_regs <= 4 && four) return launch_acc<4, true>(p, stream);
         return launch_acc<2, true>(p, stream);
     } else if (p.vec4 == 3) {
         const int64_t total8 = p.total >> 3;
