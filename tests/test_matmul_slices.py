@@ -133,3 +133,55 @@ def test_addends(b, m, n, k, kinds):
     expected = cpu_eval_graph(g.to_bytes(), 0, inputs)
     # k products of operands rounded to 11 bits, each off by 2^-11 of itself: a sum of size 1 is off by 2^-11, five times that covers the largest of them
     assert np.abs(got[0].astype(np.float64) - expected[0]).max() <= 5 * 2.0 ** -11 * max(1.0, np.abs(expected[0]).max() / 3)
+
+
+# how many slices the planner takes, and with it which of the kernel's row loops runs (1, 2, up to 4, up to 8)
+COUNTS = [
+    # (half, b, m, n, k, slices)
+    (False, 1, 250, 320, 96, 1), (False, 1, 129, 2304, 768, 2), (False, 3, 190, 768, 768, 2), (False, 1, 250, 1280, 768, 3),
+    (False, 1, 120, 1000, 520, 4), (False, 1, 129, 768, 768, 5), (False, 1, 120, 384, 768, 8),
+    (True, 1, 129, 2304, 2048, 2), (True, 1, 333, 768, 1280, 3), (True, 1, 120, 1000, 1280, 4), (True, 1, 129, 136, 1280, 7),
+]
+
+
+def count(g):
+    slices = re.search(r"splitk=(\d+) in a cluster", tile(g))
+    return int(slices.group(1)) if slices else 1
+
+
+@pytest.mark.parametrize("half,b,m,n,k,slices", COUNTS)
+def test_slice_counts(half, b, m, n, k, slices):
+    assert count(build(b, m, n, k, half)[0]) == slices
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("half,b,m,n,k,slices", [c for c in COUNTS if c[0]])
+def test_slice_counts_f16(half, b, m, n, k, slices):
+    """(a sum or an activation of f16 values rounds once more and is a step of its own)"""
+    from kyanite_b200.executor import CudaExecutor
+    g, inputs = build(b, m, n, k, half, seed=n)
+    expected = cpu_eval_graph(g.to_bytes(), 0, inputs)
+    with CudaExecutor(0, g, 0, math_mode=MATH_TF32) as ex:
+        assert_tensors_match(expected, ex.evaluate(inputs), 2e-3, 2e-3, abs_scaled=True)   # (as in test_matches_oracle)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("act", ["none", "relu", "gelu"])
+@pytest.mark.parametrize("elements", [0, 1, 2])
+@pytest.mark.parametrize("half,b,m,n,k,slices", [c for c in COUNTS if not c[0]])
+def test_row_loops(half, b, m, n, k, slices, elements, act):
+    """Every number of slices with no, one and two addends that differ by row (with one of them, a bias too)."""
+    from kyanite_b200.configs import _gelu
+    from kyanite_b200.executor import CudaExecutor
+    r = np.random.Generator(np.random.PCG64(n + elements))
+    g, inputs = build(b, m, n, k, bias=elements == 1, seed=n)
+    y = g.outputs.pop()
+    for _ in range(elements):
+        y = g.add(y, g.input(shape(b, m, n)))
+        inputs.append(r.standard_normal((b, m, n)).astype(np.float32))
+    y = {"none": lambda: y, "relu": lambda: g.relu(y), "gelu": lambda: _gelu(g, y)}[act]()
+    g.output(y)
+    assert count(g) == slices and len([l for l in plan_describe(g, 0, MATH_TF32).splitlines() if l.startswith("step")]) == 1
+    expected = cpu_eval_graph(g.to_bytes(), 0, inputs)
+    with CudaExecutor(0, g, 0, math_mode=MATH_TF32) as ex:
+        assert_tensors_match(expected, ex.evaluate(inputs), 2e-3, 2e-3, abs_scaled=True)   # (as in test_matches_oracle)
