@@ -752,6 +752,7 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             for (int i = 0; i < kGsBatch; i++) in[i] = row + i * row_step < end;
 #pragma unroll
             for (int i = 0; i < kGsBatch; i += R) {
+                if (i > 0 && !in[i]) break;   // (few rows a thread: eight slices of 134 x 32 results 5.9 -> 5.6 us, 5.6 before there were batches)
                 float x[R][S][4];
 #pragma unroll
                 for (int r = 0; r < R; r++) {
