@@ -568,7 +568,7 @@ static bool softmax_vec4_ok(const RowParams& p) {
 #define KN_ROW_VEC4_CASE(KERNEL, TPR, N)                     \
     case N: launch_pdl(KERNEL<TPR, N>, dim3(grid), dim3(256), (size_t)(0), stream, p); break;
 
-#define KN_ROW_DISPATCH(KERNEL, VEC4, STREAMING, OK)                                                            \
+#define KN_ROW_DISPATCH(KERNEL, VEC4, STREAMING, OK, LONG)   /* LONG: threads for a row of 1025 .. 8192 */      \
     if (p.rows == 0 || p.len == 0) return 0;                                                                   \
     if (p.rows > 0x7FFFFFFFll) return (int)cudaErrorInvalidValue;                                              \
     const int64_t len = p.len;                                                                                 \
@@ -611,9 +611,9 @@ static bool softmax_vec4_ok(const RowParams& p) {
         else launch_pdl(KERNEL<32, 32>, dim3(grid), dim3(256), (size_t)(0), stream, p);                                                      \
     } else if (len <= 8192) {                                                                                  \
         const unsigned grid = (unsigned)p.rows;                                                                \
-        if (len <= 2048) launch_pdl(KERNEL<256, 8>, dim3(grid), dim3(256), (size_t)(0), stream, p);                                          \
-        else if (len <= 4096) launch_pdl(KERNEL<256, 16>, dim3(grid), dim3(256), (size_t)(0), stream, p);                                    \
-        else launch_pdl(KERNEL<256, 32>, dim3(grid), dim3(256), (size_t)(0), stream, p);                                                     \
+        if (len <= 2048) launch_pdl(KERNEL<LONG, 2048 / LONG>, dim3(grid), dim3(LONG), (size_t)(0), stream, p);\
+        else if (len <= 4096) launch_pdl(KERNEL<LONG, 4096 / LONG>, dim3(grid), dim3(LONG), (size_t)(0), stream, p);\
+        else launch_pdl(KERNEL<LONG, 8192 / LONG>, dim3(grid), dim3(LONG), (size_t)(0), stream, p);            \
     } else {                                                                                                   \
         launch_pdl(STREAMING, dim3((unsigned)p.rows), dim3(256), (size_t)(0), stream, p);                                                    \
     }                                                                                                          \
@@ -623,14 +623,7 @@ int launch_softmax(const RowParams& p, cudaStream_t stream) {
     if (p.half) return launch_softmax_f16(p, stream);
     // Longer rows without 16-byte alignment (a policy over 9 x 9 boards: rows of 5 913 elements): 512 threads a row, four to
     // sixteen elements each, requested at once.  101 rows of 5 913: 11.5 -> 6.2 us (256 threads, 32 elements each).
-    if (p.rows > 0 && p.rows <= 0x7FFFFFFFll && p.len > 1024 && p.len <= 8192 && !softmax_vec4_ok(p)) {
-        const dim3 grid((unsigned)p.rows), block(512);
-        if (p.len <= 2048) launch_pdl(softmax_cached_kernel<512, 4>, grid, block, (size_t)0, stream, p);
-        else if (p.len <= 4096) launch_pdl(softmax_cached_kernel<512, 8>, grid, block, (size_t)0, stream, p);
-        else launch_pdl(softmax_cached_kernel<512, 16>, grid, block, (size_t)0, stream, p);
-        return (int)cudaGetLastError();
-    }
-    KN_ROW_DISPATCH(softmax_cached_kernel, softmax_vec4_kernel, softmax_streaming_kernel, softmax_vec4_ok)
+    KN_ROW_DISPATCH(softmax_cached_kernel, softmax_vec4_kernel, softmax_streaming_kernel, softmax_vec4_ok, 512)
 }
 
 int launch_layernorm(const RowParams& p, cudaStream_t stream) {
@@ -670,7 +663,7 @@ int launch_layernorm(const RowParams& p, cudaStream_t stream) {
         KN_LN_CLUSTER(2) KN_LN_CLUSTER(4) KN_LN_CLUSTER(8)
 #undef KN_LN_CLUSTER
     }
-    KN_ROW_DISPATCH(layernorm_cached_kernel, layernorm_vec4_kernel, layernorm_streaming_kernel, row_vec4_ok)
+    KN_ROW_DISPATCH(layernorm_cached_kernel, layernorm_vec4_kernel, layernorm_streaming_kernel, row_vec4_ok, 256)
 }
 
 int launch_reduce(const ReduceParams& p, cudaStream_t stream) {
