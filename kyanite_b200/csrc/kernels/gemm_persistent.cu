@@ -10,9 +10,9 @@
 // the producer is already loading and the MMA thread already multiplying tile i + 1.  For the short-K
 // shapes of transformer layers (K = 768: 24 K-blocks per tile) fill and drain were most of a tile's time.
 //
-//   warp 0 lane 0   TMA producer: per K block the 128 x 32 A tile and the BN x 32 B tile (K-major, 128-byte
+//   warp 0, a lane  TMA producer: per K block the 128 x 32 A tile and the BN x 32 B tile (K-major, 128-byte
 //                   swizzle, rounded to TF32 by the copy engine), ring of stages with full / empty mbarriers
-//   warp 1 lane 0   MMA issuer: four tcgen05.mma.kind::tf32 (K = 8) per stage into accumulator `tile & 1`;
+//   warp 1, a lane  MMA issuer: four tcgen05.mma.kind::tf32 (K = 8) per stage into accumulator `tile & 1`;
 //                   waits for that accumulator to be drained, signals it full with tcgen05.commit
 //   warps 2..5      epilogue: thread <-> accumulator lane <-> output row; 32 columns at a time
 //
@@ -513,7 +513,8 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 // out for each, a tile's way out took 5 000 to 25 000 of the kernel's 20 000 to 60 000 cycles; sent as 16-byte remote stores
 // instead of read, the partial sums of four slices and more took half as long again.)
 // The producer's and the issuer's warps are not epilogue warps: set-up of the epilogue would otherwise follow the last MMA.
-// At most 96 registers a thread: two CTAs to an SM, this kernel's and the next one's among them.
+// At most 96 registers a thread: two CTAs to an SM, this kernel's and the next one's among them.  The f32 loops over rows with two
+// addends that differ by row do not fit that (104 bytes of stack, nearly all of it theirs).
 // us a launch, before the epilogue by column groups -> now: 120 x 2304 x 768 9.7 -> 8.4, 120 x 3072 x 768 + GELU 10.8 -> 10.3,
 // 333 x 4096 x 4096 f16 21.0 -> 17.2, 333 x 4096 x 11008 f16 38.6 -> 36.0, 333 x 11008 x 4096 f16 40.4 -> 33.3,
 // 4096 x 320 x 320 + bias + skip 16.6 -> 8.0, 4096 x 320 x 1280 + bias + skip 21.8 -> 13.9, 3x3 convolution of 32 x 32
@@ -532,22 +533,15 @@ struct GemmSlicesParams {
     int32_t tmem_cols;
 };
 
-template <typename T>
-__device__ __forceinline__ void add_four(float (&v)[4], const T* src, int64_t col_stride, bool vec, int valid) {
+__device__ __forceinline__ void add_four(float (&v)[4], const float* src, int64_t col_stride, bool vec, int valid) {
     if (vec && valid == 4) {
-        if (sizeof(T) == 4) {
-            const float4 a = *(const float4*)src;
-            v[0] += a.x, v[1] += a.y, v[2] += a.z, v[3] += a.w;
-        } else {
-            const uint2 a = *(const uint2*)src;
-            const float2 lo = __half22float2(*(const __half2*)&a.x), hi = __half22float2(*(const __half2*)&a.y);
-            v[0] += lo.x, v[1] += lo.y, v[2] += hi.x, v[3] += hi.y;
-        }
+        const float4 a = *(const float4*)src;
+        v[0] += a.x, v[1] += a.y, v[2] += a.z, v[3] += a.w;
         return;
     }
 #pragma unroll
     for (int j = 0; j < 4; j++)
-        if (j < valid) v[j] += (float)src[j * col_stride];
+        if (j < valid) v[j] += src[j * col_stride];
 }
 
 template <bool HALF>
@@ -657,26 +651,19 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const int row_step = kGsEpilogue / groups, row0 = threadIdx.x / groups, col = (threadIdx.x - row0 * groups) * 4, valid = min(4, cols - col);
     const bool mine = row0 < row_step;
     using T = typename std::conditional<HALF, __half, float>::type;
-    using Four = typename std::conditional<HALF, uint2, float4>::type;   // four elements
     auto whole = [&](const float* addend, const int64_t* st, bool aligned) { return addend == nullptr || aligned || st[2] == 0; };
     const bool vec = q.out_vec != 0 && (cols & 3) == 0 && whole(p.add1, p.s1, q.add1_vec) && whole(p.add2, p.s2, q.add2_vec);
     // An addend that all rows share is read once, any other a batch of rows ahead (the first batch under the MMAs), as
     // `extra` and, if there are two, `extra2`
     const bool rows1 = p.add1 && p.s1[1] != 0, rows2 = p.add2 && p.s2[1] != 0;
-    const int extras = (rows1 ? 1 : 0) + (rows2 ? 1 : 0);
-    const T *add1 = nullptr, *add2 = nullptr, *extra = nullptr, *extra2 = nullptr;
+    const int extras = (rows1 ? 1 : 0) + (rows2 ? 1 : 0);   // (results of f16 have no addends: the sum would round once more)
+    const float *add1 = nullptr, *add2 = nullptr, *extra = nullptr, *extra2 = nullptr;
     const int64_t extra_row = rows1 ? p.s1[1] : p.s2[1], extra2_row = p.s2[1];
     const bool extra_one = (rows1 ? p.s1[2] : p.s2[2]) == 0, extra2_one = p.s2[2] == 0;   // one value per row
     T* out = nullptr;
     float shared[4] = {0.f, 0.f, 0.f, 0.f};
-    Four next[kGsBatch], next2[kGsBatch];
-    auto four = [&](const T* from, bool one) {
-        if (!one) return *(const Four*)from;
-        Four v;
-        T* e = (T*)&v;
-        e[0] = *from, e[1] = e[0], e[2] = e[0], e[3] = e[0];
-        return v;
-    };
+    float4 next[kGsBatch], next2[kGsBatch];
+    auto four = [&](const float* from, bool one) { return one ? make_float4(*from, *from, *from, *from) : *(const float4*)from; };
     auto fetch = [&](int row) {
 #pragma unroll
         for (int i = 0; i < kGsBatch; i++) {
@@ -691,8 +678,8 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         asm volatile("griddepcontrol.wait;" ::: "memory");   // (the addends and the output belong to earlier kernels until here)
         const int64_t m = (int64_t)mt * kGpBlockM + sp * per, n = (int64_t)nt * p.bn + col;
         out = (T*)q.out + bt * q.so[0] + m * q.so[1] + n * q.so[2];
-        if (p.add1) add1 = (const T*)p.add1 + bt * p.s1[0] + m * p.s1[1] + n * p.s1[2];
-        if (p.add2) add2 = (const T*)p.add2 + bt * p.s2[0] + m * p.s2[1] + n * p.s2[2];
+        if (p.add1) add1 = p.add1 + bt * p.s1[0] + m * p.s1[1] + n * p.s1[2];
+        if (p.add2) add2 = p.add2 + bt * p.s2[0] + m * p.s2[1] + n * p.s2[2];
         extra = rows1 ? add1 : add2, extra2 = add2;
         if (mine && vec) {
             if (p.add1 && !rows1) add_four(shared, add1, p.s1[2], q.add1_vec != 0, 4);
@@ -787,14 +774,7 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             }
 #pragma unroll
             for (int i = 0; i < kGsBatch; i++) {
-                auto add = [&](const Four& a) {
-                    if constexpr (HALF) {
-                        const float2 lo = __half22float2(*(const __half2*)&a.x), hi = __half22float2(*(const __half2*)&a.y);
-                        y[i][0] += lo.x, y[i][1] += lo.y, y[i][2] += hi.x, y[i][3] += hi.y;
-                    } else {
-                        y[i][0] += a.x, y[i][1] += a.y, y[i][2] += a.z, y[i][3] += a.w;
-                    }
-                };
+                auto add = [&](const float4& a) { y[i][0] += a.x, y[i][1] += a.y, y[i][2] += a.z, y[i][3] += a.w; };
 #pragma unroll
                 for (int j = 0; j < 4; j++) y[i][j] += shared[j];
                 if constexpr (EXTRAS > 0) add(next[i]);
@@ -826,7 +806,8 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
     };
     auto store_all = [&](auto most) {
-        if (extras == 0) store_rows(most, std::integral_constant<int, 0>());
+        if constexpr (HALF) store_rows(most, std::integral_constant<int, 0>());
+        else if (extras == 0) store_rows(most, std::integral_constant<int, 0>());
         else if (extras == 1) store_rows(most, std::integral_constant<int, 1>());
         else if constexpr (decltype(most)::value <= 4) store_rows(most, std::integral_constant<int, 2>());
         else store_rows(std::integral_constant<int, 4>(), std::integral_constant<int, 2>());
@@ -996,8 +977,9 @@ std::shared_ptr<void> gemm_persistent_prepare(const GemmParams& g, uint32_t* sta
     l->half = half;
     p.n_tiles = (int)((g.n + p.bn - 1) / p.bn);
     // CTA pairs: at least one 256-row tile per pair of SMs, and a reduction long enough
-    // for the mainloop to matter (measured, f32: 11 % faster at 24 K blocks and more, even at 16, 8 to 17 % slower at
-    // 2 to 10, where a tile is mostly epilogue and the pair's hand-offs cost more than the operand traffic they save).
+    // for the mainloop to matter (pairs against one CTA a tile, 16384 x 768, 16384 x 3072, 4096 x 4096 and 8192 x 1024 results in f32
+    // and f16: 1.13 to 1.25 of the time at 2 and 4 K blocks, where a tile is mostly epilogue and the pair's hand-offs cost more
+    // than the operand traffic they save, 0.96 to 1.11 at 12, 0.90 to 1.04 at 16, 0.86 to 0.99 at 20 and 24).
     // KN_GEMM_PAIR=0 in the environment switches pairs off, KN_GEMM_PAIR=1 drops the K condition (A/B measurements).
     // (no K slices; the A operand may be a head split or merge read in place, 42.3 -> 38.5 us on the BERT output
     // projection; with convolution windows as the A operand pairs measured no faster, 127.4 against 126.3 us, and a B
@@ -1148,6 +1130,7 @@ GemmSlices gemm_slices_choose(const GemmParams& g) {
 
 std::shared_ptr<void> gemm_slices_prepare(const GemmParams& g, uint32_t* status_word) {
     if (g.slices < 1 || g.slices > kGsMaxSlices || g.slices_bn < 32 || g.slices_bn > 256 || g.slices_bn % 32 != 0) return nullptr;
+    if (g.half && (g.add1 != nullptr || g.add2 != nullptr)) return nullptr;
     auto l = std::make_shared<GemmSlicesLaunch>();
     memset(&l->p, 0, sizeof(l->p));
     GemmPersistentParams& p = l->p.g;
