@@ -447,11 +447,15 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
 //    64 x 64, 8 x 8 per thread, two groups, 128 threads, three CTAs per SM: the registers allow no more, and twelve warps an
 //             SM hide the shared reads that eight of a 128 x 128 tile do not (equal where those fill the chip, 0.66 against
 //             0.56 where they do not)
+//    the same with four groups, 256 threads: at most 148 CTAs, one to an SM (as fast as two groups there, 64 boards 36.7 us with
+//             either, and closer to 64 bits: sums over a quarter of a K block)
 //    32 x 32, 4 x 4 per thread, four groups: for problems of a few tiles, where it is the number of CTAs that counts
 // What a small problem costs is latency, so: the constant operand is requested ahead of the dependency wait, for as many
 // stages as there are; rows are located once, in a table, and not by divisions in the loop; slices of a tile send their sums to
-// the CTA that stores them (one cluster barrier, no remote reads).
-// One 8 x 8 board, 128 -> 128 channels, 3 x 3: 12.1 us on contract_simt_kernel, 5.5 us here; 64 boards 48 -> 36 us, 256 boards 112 us
+// the CTA that stores them (two cluster barriers: one that the peers have started, waited for at the first remote store, and
+// one that the sums have arrived; no remote reads).
+// One 8 x 8 board, 128 -> 128 channels, 3 x 3: 12.1 us on contract_simt_kernel, 5.5 us here
+// (in a chain; by itself 7.4, kernel_bench's conv_exact_board); 64 boards 48 -> 36 us, 256 boards 112 us
 // (0.61 of the rate); 12 heads of 120 x 64 x 120 (probabilities . V) 14.1 -> 4.8 us.
 template <int BM, int BN, int TM, int TN, int KG, int ST>
 struct ColsLayout {
@@ -463,12 +467,6 @@ struct ColsLayout {
     static constexpr int kReceived = (kUnits + 8) * 16;                         // sums sent by the other slices
     static constexpr int kBytes = kFront + kReceived + BM * (int)sizeof(RowAt) + BM * 24;
 };
-
-__device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*(uint64_t*)&a), "l"(*(uint64_t*)&b), "l"(*(uint64_t*)&c));
-    return *(float2*)&d;
-}
 
 struct ColsArgs {
     int slices;
@@ -730,20 +728,6 @@ contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant
             store(mm, nn, v);
         }
     }
-}
-
-// Dynamic shared memory above 48 KB is opted in to once per device and kernel.
-template <class Kernel>
-int allow_shared(Kernel kernel, int bytes, bool (&done)[64], std::mutex& mu) {
-    int device = 0;
-    cudaGetDevice(&device);
-    std::lock_guard<std::mutex> lock(mu);
-    if (device >= 0 && device < 64 && !done[device]) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) return (int)e;
-        done[device] = true;
-    }
-    return 0;
 }
 
 template <class Problem, int BM, int BN, int TM, int TN, int KG, int ST, int OCC>

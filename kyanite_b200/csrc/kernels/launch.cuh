@@ -11,6 +11,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstdint>
+#include <mutex>
 #include <utility>
 
 namespace kn {
@@ -33,6 +35,27 @@ inline void launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     (void)cudaLaunchKernelEx(&cfg, kernel, Params(std::forward<Args>(args))...);   // a failure stays in cudaGetLastError()
+}
+
+// Dynamic shared memory above 48 KB is opted in to once per device and kernel.
+template <class Kernel>
+int allow_shared(Kernel kernel, int bytes, bool (&done)[64], std::mutex& mu) {
+    int device = 0;
+    cudaGetDevice(&device);
+    std::lock_guard<std::mutex> lock(mu);
+    if (device >= 0 && device < 64 && !done[device]) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return (int)e;
+        done[device] = true;
+    }
+    return 0;
+}
+
+// Two multiply-adds in one instruction (fma.rn.f32x2).
+__device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*(uint64_t*)&a), "l"(*(uint64_t*)&b), "l"(*(uint64_t*)&c));
+    return *(float2*)&d;
 }
 
 }  // namespace kn

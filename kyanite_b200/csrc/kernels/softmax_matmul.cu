@@ -11,8 +11,8 @@
 //
 // What bounds it is latency (scores and V from L2, softmax, product, store; the arithmetic of 12 heads of 120 rows and keys is
 // 1 us).  Softmax, product and the copy that merges the heads as three launches -> this one: 12 heads of 120 rows and keys,
-// 64 columns 9.7 -> 4.8 us; 8 heads of 1024 rows, 77 keys, 80 columns 21.3 -> 10.5 us.  With more keys in blocks of 128, two of
-// them in flight, it lost to the separate steps: 12 heads of 16 rows, 88 columns, 256 keys 13.6 us against 6.5, 1024 keys 49
+// 64 columns 9.7 -> 4.8 us; 8 heads of 1024 rows, 77 keys, 80 columns 21.3 -> 10.5 us (in a graph of eight such calls; launched by
+// itself 6.2 and 11.0, kernel_bench's softmax_values_short*).  With more keys in blocks of 128, two of them in flight, it lost to the separate steps: 12 heads of 16 rows, 88 columns, 256 keys 13.6 us against 6.5, 1024 keys 49
 // against 12; one CTA reads all of V, where contract_cols_kernel spreads the keys over a cluster.
 #include <cuda_runtime.h>
 
@@ -26,12 +26,6 @@ namespace kn {
 
 namespace {
 
-
-__device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(*(uint64_t*)&a), "l"(*(uint64_t*)&b), "l"(*(uint64_t*)&c));
-    return *(float2*)&d;
-}
 
 struct SoftmaxMatmulParams {
     const float *x, *term, *v;   // term may be null
@@ -190,16 +184,7 @@ template <int PANELS, int RPT, int GROUPS>
 int launch_rows(const SoftmaxMatmulParams& q, unsigned grid, cudaStream_t stream) {
     static std::mutex mu;
     static bool done[64] = {false};
-    int device = 0;
-    cudaGetDevice(&device);
-    {   // (the opt-in to more than 48 KB is per device)
-        std::lock_guard<std::mutex> lock(mu);
-        if (device >= 0 && device < 64 && !done[device]) {
-            cudaError_t e = cudaFuncSetAttribute(softmax_matmul_kernel<PANELS, RPT, GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
-            if (e != cudaSuccess) return (int)e;
-            done[device] = true;
-        }
-    }
+    if (int e = allow_shared(softmax_matmul_kernel<PANELS, RPT, GROUPS>, 128 * 1024, done, mu)) return e;
     launch_pdl(softmax_matmul_kernel<PANELS, RPT, GROUPS>, dim3(grid), dim3(GROUPS * 128), (size_t)shared_bytes(q.n, q.dv, 8 * RPT, GROUPS), stream, q);
     return (int)cudaGetLastError();
 }
