@@ -7,7 +7,7 @@ over its algorithmic bytes (memory-bound steps) or TFLOP/s over its FLOP (contra
     python -m kyanite_b200.kernel_bench --case softmax  # one case (this is what the ncu captures run)
 
 Working sets are several times the 126 MB L2, so back-to-back launches still stream from HBM (those of the short calls,
-`*_short*`, and of `conv_exact` lie in it, as the calls' own do).  Peaks come
+`*_short*`, and of `conv_exact*` and `softmax_ragged` lie in it, as the calls' own do).  Peaks come
 from MEASURED_PEAKS.json at the repository root when present (copy bandwidth, bf16 GEMM burst; TF32 is
 taken as half the bf16 figure, f16 operands as the bf16 figure itself), else the fallback 6650 GB/s / 1590 TFLOP/s.
 """
@@ -64,6 +64,14 @@ def case_softmax_long(rng):
     return g, 0, [rng.standard_normal((65536, 2048)).astype(np.float32)]
 
 
+def case_softmax_ragged(rng):
+    """A policy over 9 x 9 boards: softmax over [101, 5913], rows without 16-byte alignment."""
+    g = Graph()
+    x = g.input(shape(101, 5913))
+    g.output(g.softmax(x, 1))
+    return g, 0, [rng.standard_normal((101, 5913)).astype(np.float32)]
+
+
 def case_layernorm(rng):
     """Post-LN with residual: layernorm(a + b) over [262144, 768] (16 BERT batches of 32 x 512 tokens)."""
     g = Graph()
@@ -81,6 +89,14 @@ def case_layernorm_group(rng):
     x = g.input(shape(64, 81920))
     g.output(g.layernorm(x, 1, 1e-5))
     return g, 0, [rng.standard_normal((64, 81920)).astype(np.float32)]
+
+
+def case_layernorm_group_short(rng):
+    """A group norm of the UNet-shaped graph at batch 1: 32 rows of 40 960 elements."""
+    g = Graph()
+    x = g.input(shape(32, 40960))
+    g.output(g.layernorm(x, 1, 1e-5))
+    return g, 0, [rng.standard_normal((32, 40960)).astype(np.float32)]
 
 
 def case_reduce(rng):
@@ -172,6 +188,18 @@ def _blockwise_attention_case(heads, rows, keys, d, half=False, causal=False):
         return g, 0, [rng.standard_normal((heads, n, d)).astype(dtype.np) for n in (rows, keys, keys)]
     build.__doc__ = (f"Attention by key blocks: {heads} heads of {rows} rows, {keys} keys, d = {d}" + (", f16" if half else "") +
                      (", causal" if causal else ""))
+    return build
+
+
+def _softmax_values_case(heads, rows, keys, d):
+    def build(rng):
+        g = Graph()
+        x, v = g.input(shape(heads, rows, keys)), g.input(shape(keys, heads * d))
+        v = g.view(g.permute(g.view(v, shape(1, keys, heads, d)), [0, 2, 1, 3]), shape(heads, keys, d))
+        y = g.batched_mat_mul(g.softmax(g.mul(x, g.scalar(1.0 / math.sqrt(d))), 2), v)
+        g.output(g.view(g.permute(g.view(y, shape(1, heads, rows, d)), [0, 2, 1, 3]), shape(rows, heads * d)))
+        return g, 0, [rng.standard_normal(s).astype(np.float32) for s in ((heads, rows, keys), (keys, heads * d))]
+    build.__doc__ = f"softmax(scores) . V in f32, heads split and merged: {heads} heads of {rows} rows, {keys} keys, {d} columns"
     return build
 
 
@@ -274,8 +302,10 @@ CASES = {
     "residual_add": case_residual_add,
     "softmax": case_softmax,
     "softmax_long": case_softmax_long,
+    "softmax_ragged": case_softmax_ragged,
     "layernorm": case_layernorm,
     "layernorm_group": case_layernorm_group,
+    "layernorm_group_short": case_layernorm_group_short,
     "reduce": case_reduce,
     "gather": case_gather,
     "permute_copy": case_permute_copy,
@@ -310,6 +340,9 @@ CASES = {
     "linear_short_ffn_f16": _linear_f16_case(333, 11008, 4096),
     "linear_short_down_f16": _linear_f16_case(333, 4096, 11008),
     "conv_exact": _conv_case(64, 128, 8, 8, 128, 3, 1, 1, "Residual tower's convolution in exact f32: 4096 positions, 128 -> 128 channels"),
+    "conv_exact_board": _conv_case(1, 128, 8, 8, 128, 3, 1, 1, "The same convolution for one board: 64 positions"),
+    "softmax_values_short": _softmax_values_case(12, 120, 120, 64),
+    "softmax_values_short_cross": _softmax_values_case(8, 1024, 77, 80),
 }
 
 
@@ -350,8 +383,9 @@ def run_case(name: str, launches: int, device: int):
             if flops > 0:
                 # f16 operands: the dense f16 / bf16 rate (the measured bf16 GEMM figure); f32 storage: TF32, half of it
                 # (exact f32: 148 SMs x 128 lanes x 1.965 GHz)
-                peak = 74.4 if _is_exact(name) else (2.0 * tf32 if _is_f16(name) else tf32)
-                rec.update(bound="fma" if _is_exact(name) else "tensor", achieved=round(flops / us / 1e6, 1), unit="TFLOP/s", peak=peak,
+                fma = _is_exact(name) or desc.startswith("softmax(x) . V")
+                peak = 74.4 if fma else (2.0 * tf32 if _is_f16(name) else tf32)
+                rec.update(bound="fma" if fma else "tensor", achieved=round(flops / us / 1e6, 1), unit="TFLOP/s", peak=peak,
                            frac=round(flops / us / 1e6 / peak, 3))
             else:
                 rec.update(bound="hbm", achieved=round(alg_bytes / us / 1e3, 1), unit="GB/s", peak=hbm,
