@@ -7,10 +7,10 @@
 // row block: up to 512 columns), and its epilogue warps turn the rows into probabilities on the way out: the scores
 // never reach memory.
 //
-//   warp 0 lane 0   producer: the Q tile [128 x K] and the K matrix [keys x K] of the work item, as 128-byte-wide K
+//   warp 0, a lane  producer: the Q tile [128 x K] and the K matrix [keys x K] of the work item, as 128-byte-wide K
 //                   blocks (128-byte swizzle, rounded to TF32 by the copy engine), through 4-D tensor maps: an
 //                   operand may be an attention head split read in place (GemmOperand4D, kernels.h)
-//   warp 1 lane 0   MMA issuer: per half of the keys (at most 256 accumulator columns per instruction) and K block,
+//   warp 1, a lane  MMA issuer: per half of the keys (at most 256 accumulator columns per instruction) and K block,
 //                   four tcgen05.mma.kind::tf32; tcgen05.commit frees the operand buffer and signals the accumulator
 //   warps 2..9      epilogue, thread <-> accumulator lane <-> query row, two warps per lane quarter sharing a row's
 //                   columns.  Three sweeps over the row in tensor memory, 32 columns at a time: the maximum; then

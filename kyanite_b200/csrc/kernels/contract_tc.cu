@@ -3,10 +3,10 @@
 // act(acc + add1 + add2).
 //
 // One CTA computes one 128 x BN output tile:
-//   warp 0 / lane 0   TMA producer: per K block one `cp.async.bulk.tensor` for the 128 x 32 A tile and
+//   warp 0, one lane  TMA producer: per K block one `cp.async.bulk.tensor` for the 128 x 32 A tile and
 //                     one for the BN x 32 B tile, both K-major with the 128-byte swizzle, into a
 //                     ring of shared-memory stages guarded by full/empty mbarriers
-//   warp 1 / lane 0   MMA issuer: four `tcgen05.mma.kind::tf32` (K = 8 each) per stage into a
+//   warp 1, one lane  MMA issuer: four `tcgen05.mma.kind::tf32` (K = 8 each) per stage into a
 //                     128-lane x BN-column f32 accumulator in TMEM; `tcgen05.commit` frees the stage
 //   warps 2..5        epilogue: `tcgen05.ld` the accumulator (one output row per thread), add the
 //                     optional addends, activation, store through the output's element strides

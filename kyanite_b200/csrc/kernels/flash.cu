@@ -10,9 +10,9 @@
 //
 //   warps 0..7      softmax: a row per lane quarter and lane, its 128 columns on two warps of 64 (the maximum and, at the
 //                   end, the sum are exchanged through shared memory)
-//   warp 8 lane 0   producer: Q once, keys and values of a block through one buffer each; the next block's keys are
+//   warp 8, a lane  producer: Q once, keys and values of a block through one buffer each; the next block's keys are
 //                   requested when the score MMAs have read this block's, under the exponentials
-//   warp 9 lane 0   MMA issuer
+//   warp 9, a lane  MMA issuer
 //
 // Inside a CTA the phases of a block follow one another (scores, exponentials, context); what fills the tensor cores and
 // the special-function unit meanwhile is the SM's second CTA: 256 columns of tensor memory, some 100 KB of shared memory
