@@ -20,7 +20,7 @@
 //              pattern is anchored at a 1024-byte boundary, so the descriptor's base-offset field stays 0
 //              (measured: a non-zero base offset permutes the channels).
 //
-// Warp roles (64 + 128 E threads): warp 0 lane 0 streams filter tiles; warp 1 lane 0 issues the MMAs of a layer
+// Warp roles (64 + 128 E threads): warp 0 lane 0 streams filter tiles; an elected lane of warp 1 issues the MMAs of a layer
 // once its input is complete; the other 4 E warps are the epilogue (E warps per TMEM lane quarter, taking the
 // 16-column chunks of the accumulator in turn; E = 3 when the chunk count divides by three, as the 9 chunks of
 // two 8x8 boards do, else 2): accumulator + bias (+ held skip tensor) -> ReLU -> written back as the
@@ -259,6 +259,12 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap map_tiles, const __grid_co
         for (int l = 0; l < p.n_layers && ok; l++) {
             long long t0 = 0, full_wait = 0;
             if (trace) t0 = clock64();
+            const int cbl = p.c_blocks[l];
+            uint32_t accumulate = 0;
+            const bool pointwise = (p.flags[l] & kChainFlagPointwise) != 0;
+            const LayerTiles tiles(p, l);   // (divisions: ahead of the wait)
+            int tap = tiles.first / cbl, cb = tiles.first - tap * cbl;
+            if (pointwise) tap = 4;     // the centre tap: the operand starts at the pixel itself
             // the layer's input is complete in shared memory and the accumulator has been read out
             ok = mbar_wait(act_bar, (uint32_t)(l & 1), abandon, p.status, 12, kWaitCycles, kSleepNs);
             if (!ok) break;
@@ -268,12 +274,6 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap map_tiles, const __grid_co
             // to hide that kernel's launch and set-up, late enough that its CTAs do not sit on this SM (blocked
             // in griddepcontrol.wait) for the whole run.
             if (l == p.n_layers - 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-            const int cbl = p.c_blocks[l];
-            uint32_t accumulate = 0;
-            const bool pointwise = (p.flags[l] & kChainFlagPointwise) != 0;
-            const LayerTiles tiles(p, l);
-            int tap = tiles.first / cbl, cb = tiles.first - tap * cbl;
-            if (pointwise) tap = 4;     // the centre tap: the operand starts at the pixel itself
             for (int left = tiles.n; left > 0 && ok; left -= tiles.request) {
                 long long tw = 0;
                 if (trace) tw = clock64();
@@ -529,8 +529,10 @@ bool tc_chain_geometry(int h, int w, int64_t n_img, int c_blocks, ChainGeometry*
             if (requests < 2) break;
             g.slots = requests * g.group;
             g.smem_bytes = fixed + act_bytes + g.slots * kTileBytes;
-            // per layer: 36 tiles x 4 MMAs (an MMA costs ~70 cycles up to N = 128, then grows with N), plus
-            // the epilogue over the columns; CTAs run in waves of one per SM
+            // per layer: 36 tiles x 4 MMAs, plus the epilogue over the columns; CTAs run in waves of one per SM.  (What an MMA
+            // costs is from before the issue loop ran in an elected lane; it is 80 cycles for 80 columns and 93 for 144 now.
+            // For four channel blocks both give the same geometry, for every board from 5 x 5 to 13 x 13 and up to 2048
+            // images; for one and two blocks, whose layers have fewer MMAs, the geometry has not been measured again.)
             const double mma = std::max(70.0, 0.47 * g.n_mma + 16.0);
             const double per_layer = 144.0 * mma + 22.0 * g.n_mma + 900.0;
             const int64_t ctas = (n_img + g.per_cta - 1) / g.per_cta;
