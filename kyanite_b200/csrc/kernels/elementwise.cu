@@ -832,9 +832,11 @@ int launch_scalar(const ScalarParams& p, cudaStream_t stream) {
     if (p.vec4 == 2) {
         // (as many as the innermost extent and the spill slots, n_regs * V * 4 KB of shared memory per block, allow)
         const int64_t inner4 = p.dims[p.rank - 1] / 4;
-        // (two from one block an SM on: 0.37 M elements, scale + shift in f32 4.9 us with one, 4.1 with two; sum 3.1 with either)
+        // (two from 0.6 rounds on: 0.75 M elements, sum in f32 3.8 us with one, 3.4 with two; 0.6 M 3.6 with either.  Two from a
+        // quarter of a round on gained 5 to 15 % for scale + shift by itself, 0.4 to 0.6 M, and lost 1.4 us a step between the
+        // convolutions of a denoising step, 0.66 M)
         if (inner4 % 4 == 0 && p.n_regs <= 4 && four) return launch_acc<4, false>(p, stream);
-        if (inner4 % 2 == 0 && enough(8, 0.25)) return launch_acc<2, false>(p, stream);
+        if (inner4 % 2 == 0 && enough(8, 0.6)) return launch_acc<2, false>(p, stream);
         return launch_acc<1, false>(p, stream);
     } else if (p.vec4 == 5) {
         // an accumulator program over f16 only: packed halves, eight per position (the innermost extent is a multiple
