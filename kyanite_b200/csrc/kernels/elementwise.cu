@@ -832,11 +832,12 @@ int launch_scalar(const ScalarParams& p, cudaStream_t stream) {
     if (p.vec4 == 2) {
         // (as many as the innermost extent and the spill slots, n_regs * V * 4 KB of shared memory per block, allow)
         const int64_t inner4 = p.dims[p.rank - 1] / 4;
-        // (two from 0.6 rounds on: 0.75 M elements, sum in f32 3.8 us with one, 3.4 with two; 0.6 M 3.6 with either.  Two from a
-        // quarter of a round on gained 5 to 15 % for scale + shift by itself, 0.4 to 0.6 M, and lost 1.4 us a step between the
-        // convolutions of a denoising step, 0.66 M)
+        // (two from 0.6 rounds on: 0.75 M elements, sum in f32 3.8 us with one, 3.4 with two; and where they make one or two blocks
+        // an SM, 0.3 to 0.6 M: scale + shift of 0.47 M 5.1 us with one, 4.5 with two, sum 3.3 with either.  In between one:
+        // 0.66 M took 1.4 us more a step with two between the convolutions of a denoising step)
+        const bool two = enough(8, 0.6) || (enough(8, 0.25) && p.total <= 148 * 2 * 256 * 8);
         if (inner4 % 4 == 0 && p.n_regs <= 4 && four) return launch_acc<4, false>(p, stream);
-        if (inner4 % 2 == 0 && enough(8, 0.6)) return launch_acc<2, false>(p, stream);
+        if (inner4 % 2 == 0 && two) return launch_acc<2, false>(p, stream);
         return launch_acc<1, false>(p, stream);
     } else if (p.vec4 == 5) {
         // an accumulator program over f16 only: packed halves, eight per position (the innermost extent is a multiple

@@ -36,7 +36,8 @@ CASES = [
     (F16, F16, 67, 1032),     # one: rows of an odd number of positions
     (F32, F32, 4673, 1040),   # four positions of four floats, from 4.85 M elements on
     (F32, F32, 697, 1048),    # two, from 0.73 M on
-    (F32, F32, 61, 1044),
+    (F32, F32, 301, 1048), (F32, F32, 577, 1048),   # and from 0.3 M to 0.6 M
+    (F32, F32, 587, 1048), (F32, F32, 61, 1044),    # one
     (F16, F32, 4673, 1040),   # of both types: four from 4.85 M on, else two
     (F16, F32, 697, 1048),
 ]
