@@ -447,8 +447,9 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
 //    64 x 64, 8 x 8 per thread, two groups, 128 threads, three CTAs per SM: the registers allow no more, and twelve warps an
 //             SM hide the shared reads that eight of a 128 x 128 tile do not (equal where those fill the chip, 0.66 against
 //             0.56 where they do not)
-//    the same with four groups, 256 threads: at most 148 CTAs, one to an SM (as fast as two groups there, 64 boards 36.7 us with
-//             either, and closer to 64 bits: sums over a quarter of a K block)
+//    the same with four groups, 256 threads, where at most 148 CTAs of it come out cheapest: no slower than two groups in 44 of
+//             45 matmuls and convolutions, 4 % slower in one (639 x 127 x 2077: 41.3 us, 39.6), and closer to 64 bits (sums over a
+//             quarter of a K block)
 //    32 x 32, 4 x 4 per thread, four groups: for problems of a few tiles, where it is the number of CTAs that counts
 // What a small problem costs is latency, so: the constant operand is requested ahead of the dependency wait, for as many
 // stages as there are; rows are located once, in a table, and not by divisions in the loop; slices of a tile send their sums to
