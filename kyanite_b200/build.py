@@ -35,6 +35,7 @@ SOURCES = [
     "kernels/contract_simt.cu",
     "kernels/contract_tc.cu",
     "kernels/conv_chain.cu",
+    "kernels/conv_chain_pair.cu",
     "kernels/gemm_persistent.cu",
     "kernels/attn_softmax.cu",
     "kernels/attention.cu",

@@ -213,7 +213,9 @@ struct ConvChainParams {
     const float* tiles;   // filter tiles [tile][128 output channels][32 input channels] in the 128-byte-swizzled
                           // order of shared memory, TF32, layers back to back;
                           // within a layer tile = tap * c_blocks + channel block, tap = r * 3 + s
+                          // (pair: [CTA of the pair][channel block][tap][its half of the output channels][32])
     const float* bias;    // [layer][128]
+    int32_t pair;         // the kernel on CTA pairs takes it
     int32_t n, c_in, k, h, w;
     int32_t n_layers;
     int64_t s_in[4], s_out[4];

@@ -1,19 +1,20 @@
 // A run of 3x3 stride-1 same-padding convolutions (a residual tower) as ONE kernel for sm_100a.
 //
-// A 3x3 convolution of an image reads that image only, so a CTA that owns a few whole images can run
+// A 3x3 convolution of an image reads that image only, so a CTA that owns a whole image can run
 // every layer of the run back to back without ever leaving its SM: the activations live in shared
 // memory (as the B operand of the next layer's MMAs), the skip connection of a residual block lives in
 // tensor memory next to the accumulator, and per layer only the filter streams in from L2 through a
 // small ring (a request is one filter tap or, of narrow layers, a row of three: up to six 16 KB tiles, stored by the
 // planner in the swizzled byte order of shared memory so a linear bulk copy delivers them).  Compared with one launch per layer
 // this removes, per layer, the launch, the pipeline fill, the activation round trip through L2 and the
-// output store.
+// output store.  Images of up to 128 padded positions run on CTA pairs instead (conv_chain_pair.cu, which reads and
+// copies half as many bytes per MMA); this kernel takes the larger ones, one image per CTA.
 //
 // Accumulator orientation: D[output channel = TMEM lane][padded position = column].
 //   A operand  filter tile [128 output channels x 32 input channels], K-major, 128-byte swizzle, copied
 //              with `cp.async.bulk` from a tile array the planner lays out tap by tap
 //   B operand  the activation buffer: per 32-channel block, one 128-byte row per padded position, same
-//              swizzle.  The images are stored as one tall zero-padded image (ChainGeometry, tc.h), so
+//              swizzle.  The image is stored zero-padded (ChainGeometry, tc.h), so
 //              filter tap (r, s) is the same operand started `(r-1) * wp + (s-1)` rows further on.  Such a
 //              start is 128-byte but not 1024-byte aligned.  The tensor core resolves the swizzle from the
 //              absolute shared-memory address (16-byte chunk index XOR address bits 7..9), and the buffer's
@@ -22,8 +23,7 @@
 //
 // Warp roles (64 + 128 E threads): warp 0 lane 0 streams filter tiles; an elected lane of warp 1 issues the MMAs of a layer
 // once its input is complete; the other 4 E warps are the epilogue (E warps per TMEM lane quarter, taking the
-// 16-column chunks of the accumulator in turn; E = 3 when the chunk count divides by three, as the 9 chunks of
-// two 8x8 boards do, else 2): accumulator + bias (+ held skip tensor) -> ReLU -> written back as the
+// 16-column chunks of the accumulator in turn; E = 3 when the chunk count divides by three, else 2): accumulator + bias (+ held skip tensor) -> ReLU -> written back as the
 // next layer's operand (rounded to TF32, zeros at padding positions) and, if a later layer adds it,
 // into the held-tensor columns of TMEM in full f32; a layer flagged to store writes its result to global
 // memory.  The last layer may be a pointwise (1x1) layer that computes several convolutions of the last
@@ -60,7 +60,7 @@ struct ChainKernelParams {
     const float* tiles;
     int64_t s_in[4], s_out[4];
     int32_t n_img, c_in, k, h, w;
-    int32_t n_layers, per_cta, gx, gy, wp, q_first, r_first, n_mma, rows_alloc, slots, tmem_cols, c_blocks_max;
+    int32_t n_layers, wp, q_first, r_first, n_mma, rows_alloc, slots, tmem_cols, c_blocks_max;
     int32_t total_tiles;
     int32_t group;   // filter tiles that a ring slot holds
     long long* trace; // KN_CHAIN_TRACE only: per layer 8 clock64 stamps of CTA 0, in pinned host memory
@@ -73,43 +73,6 @@ struct ChainKernelParams {
     int64_t head_s_out[kMaxChainHeads][4];
     uint8_t head_relu[kMaxChainHeads];
 };
-
-__device__ __forceinline__ void tmem_store_16(uint32_t taddr, const uint32_t (&v)[16]) {   // caller waits (tcgen05.wait::st)
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-          "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-        : "memory");
-}
-
-__device__ __forceinline__ void tmem_load_16_nowait(uint32_t taddr, uint32_t (&v)[16]) {   // caller waits (tcgen05.wait::ld)
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr)
-        : "memory");
-}
-
-__device__ __forceinline__ void tmem_store_8(uint32_t taddr, const uint32_t (&v)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_load_8_nowait(uint32_t taddr, uint32_t (&v)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                 : "r"(taddr)
-                 : "memory");
-}
-template <int CW> __device__ __forceinline__ void tmem_store_chunk(uint32_t taddr, const uint32_t (&v)[CW]) {
-    if constexpr (CW == 16) tmem_store_16(taddr, v); else tmem_store_8(taddr, v);
-}
-template <int CW> __device__ __forceinline__ void tmem_load_chunk_nowait(uint32_t taddr, uint32_t (&v)[CW]) {
-    if constexpr (CW == 16) tmem_load_16_nowait(taddr, v); else tmem_load_8_nowait(taddr, v);
-}
 
 // Suspend-time hint of the kernel's mbarrier waits: a waiting thread is woken when the phase completes, so the hint
 // only bounds how long it sleeps between two looks at the abandon flag.
@@ -136,11 +99,11 @@ struct LayerTiles {
     }
 };
 
-// E: epilogue warps per TMEM lane quarter; CW: accumulator columns per epilogue chunk (16 or 8); TRACE: whether the
-// first CTA stamps its phases
-template <int E, int CW, bool TRACE>
+// E: epilogue warps per TMEM lane quarter; TRACE: whether the first CTA stamps its phases
+template <int E, bool TRACE>
 __global__ void __launch_bounds__(64 + 128 * E, 1)
 conv_chain_kernel(const __grid_constant__ CUtensorMap map_tiles, const __grid_constant__ ChainKernelParams p) {
+    constexpr int CW = 16;   // accumulator columns per epilogue chunk
     constexpr int kChainThreads = 64 + 128 * E;
     constexpr int kEpilogueThreads = 128 * E;
     static_assert(kChainThreads >= kChainThreadsMin, "set-up loops assume at least 320 threads");
@@ -181,18 +144,14 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap map_tiles, const __grid_co
         const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
         for (uint32_t i = threadIdx.x; i < act_bytes / 16u; i += kChainThreads) z[i] = zero;
     }
-    // column -> pixel table: bit 31 real pixel, bits 16..23 image within the CTA, 8..15 y, 0..7 x
+    // column -> pixel table: bit 31 real pixel, bits 8..15 y, 0..7 x
     if (threadIdx.x < 256) {
         const int n = threadIdx.x;
         uint32_t info = 0;
         if (n < p.n_mma) {
             const int q = n + p.q_first;
             const int row = q / p.wp, col = q - row * p.wp;
-            const int iy = row / (p.h + 1), ry = row - iy * (p.h + 1);
-            const int ix = col / (p.w + 1), cx = col - ix * (p.w + 1);
-            const int img = iy * p.gx + ix;
-            if (cx != 0 && ry != 0 && iy < p.gy && (int64_t)blockIdx.x * p.per_cta + img < p.n_img)
-                info = 0x80000000u | ((uint32_t)img << 16) | ((uint32_t)(ry - 1) << 8) | (uint32_t)(cx - 1);
+            if (col != 0 && row != 0 && row <= p.h) info = 0x80000000u | ((uint32_t)(row - 1) << 8) | (uint32_t)(col - 1);
         }
         colinfo[n] = info;
     }
@@ -309,7 +268,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap map_tiles, const __grid_co
         const int half = (warp - 2) >> 2;      // which of the quarter's E warps this is: it takes chunks half, half + E, ...
         const int ch = quarter * 32 + lane;
         const uint32_t lane_bits = (uint32_t)(quarter * 32) << 16;
-        const int64_t img0 = (int64_t)blockIdx.x * p.per_cta;
+        const int64_t img = blockIdx.x;
         const bool has_block = (ch >> 5) < p.c_blocks_max;     // narrower layers: no operand rows for these channels
         const uint32_t chunk = (uint32_t)(ch >> 2) & 7u;
         // this channel's 4 bytes inside a 128-byte row of its 32-channel block, before the swizzle
@@ -342,7 +301,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap map_tiles, const __grid_co
                 const uint32_t info = colinfo[c * CW + j];
                 float x = 0.f;
                 if ((info >> 31) && ch < p.c_in)
-                    x = p.in[(img0 + ((info >> 16) & 0xFF)) * p.s_in[0] + (int64_t)ch * p.s_in[1] + (int64_t)((info >> 8) & 0xFF) * p.s_in[2] +
+                    x = p.in[img * p.s_in[0] + (int64_t)ch * p.s_in[1] + (int64_t)((info >> 8) & 0xFF) * p.s_in[2] +
                              (int64_t)(info & 0xFF) * p.s_in[3]];
                 v[j] = __float_as_uint(x);
                 if (has_block) store_operand(my_rows + (uint32_t)c * (CW * 128u), j, x);
@@ -453,7 +412,7 @@ conv_chain_kernel(const __grid_constant__ CUtensorMap map_tiles, const __grid_co
                         for (int j = 0; j < CW; j++) {
                             if ((mask >> j) & 1u) {
                                 const uint32_t info = colinfo[c * CW + j];
-                                o_ptr[(img0 + ((info >> 16) & 0xFF)) * o_s0 + (int64_t)((info >> 8) & 0xFF) * o_s2 +
+                                o_ptr[img * o_s0 + (int64_t)((info >> 8) & 0xFF) * o_s2 +
                                       (int64_t)(info & 0xFF) * o_s3] = __uint_as_float(v[j]);
                             }
                         }
@@ -502,49 +461,24 @@ static int round_up_int(int x, int to) { return (x + to - 1) / to * to; }
 
 bool tc_chain_geometry(int h, int w, int64_t n_img, int c_blocks, ChainGeometry* out) {
     if (h < 1 || w < 1 || h > 254 || w > 254 || n_img < 1 || c_blocks < 1 || c_blocks > 4) return false;
-    ChainGeometry best{};
-    double best_cost = 1e300;
-    // gx images side by side, gy such rows of images below one another
-    for (int gx = 1; gx <= 16; gx++) {
-        for (int gy = 1; gy <= 16; gy++) {
-            ChainGeometry g{};
-            g.gx = gx;
-            g.gy = gy;
-            g.per_cta = gx * gy;
-            g.wp = gx * (w + 1);
-            g.q_first = g.wp + 1;
-            g.r_first = round_up_int(g.q_first, 8);
-            const int q_last = ((gy - 1) * (h + 1) + h) * g.wp + (gx - 1) * (w + 1) + w;
-            g.n_mma = round_up_int(q_last - g.q_first + 1, 16);
-            if (g.n_mma > 256) break;
-            g.rows_alloc = round_up_int(g.r_first + g.n_mma + g.wp + 2, 8);
-            const int act_bytes = c_blocks * g.rows_alloc * 128;
-            const int fixed = 1024 /* alignment */ + 16 * 8 + 32 + 1024 /* column table */ + 128 /* chunk masks */ + 24 /* poller's verdict */ + 128 /* dummy rows */;
-            // the ring holds whole taps (c_blocks tiles each), or rows of three taps where narrow layers leave room for two of
-            // those: a request costs the MMA issuer some 170 cycles (17 layers, one board a CTA: 64 channels 87.2 -> 83.6 us on
-            // 8 x 8 and 97.4 -> 92.2 on 9 x 9, 32 channels 70.4 -> 60.1)
-            const int room = (227 * 1024 - fixed - act_bytes) / kTileBytes;
-            g.group = c_blocks <= 2 && room >= 6 * c_blocks ? 3 * c_blocks : c_blocks;
-            const int requests = std::min(4, room / g.group);
-            if (requests < 2) break;
-            g.slots = requests * g.group;
-            g.smem_bytes = fixed + act_bytes + g.slots * kTileBytes;
-            // per layer: 36 tiles x 4 MMAs, plus the epilogue over the columns; CTAs run in waves of one per SM.  (What an MMA
-            // costs is from before the issue loop ran in an elected lane; it is 80 cycles for 80 columns and 93 for 144 now.
-            // For four channel blocks both give the same geometry, for every board from 5 x 5 to 13 x 13 and up to 2048
-            // images; for one and two blocks, whose layers have fewer MMAs, the geometry has not been measured again.)
-            const double mma = std::max(70.0, 0.47 * g.n_mma + 16.0);
-            const double per_layer = 144.0 * mma + 22.0 * g.n_mma + 900.0;
-            const int64_t ctas = (n_img + g.per_cta - 1) / g.per_cta;
-            const double cost = (double)((ctas + 147) / 148) * per_layer;
-            if (cost < best_cost) {
-                best_cost = cost;
-                best = g;
-            }
-        }
-    }
-    if (best.per_cta == 0) return false;
-    if (out) *out = best;
+    ChainGeometry g{};
+    g.wp = w + 1;
+    g.q_first = g.wp + 1;
+    g.r_first = round_up_int(g.q_first, 8);
+    g.n_mma = round_up_int(h * g.wp + w - g.q_first + 1, 16);
+    if (g.n_mma > 256) return false;
+    g.rows_alloc = round_up_int(g.r_first + g.n_mma + g.wp + 2, 8);
+    const int act_bytes = c_blocks * g.rows_alloc * 128;
+    const int fixed = 1024 /* alignment */ + 16 * 8 + 32 + 1024 /* column table */ + 128 /* chunk masks */ + 24 /* poller's verdict */ + 128 /* dummy rows */;
+    // the ring holds whole taps (c_blocks tiles each), or rows of three taps where narrow layers leave room for two of
+    // those: a request costs the MMA issuer some 170 cycles
+    const int room = (227 * 1024 - fixed - act_bytes) / kTileBytes;
+    g.group = c_blocks <= 2 && room >= 6 * c_blocks ? 3 * c_blocks : c_blocks;
+    const int requests = std::min(4, room / g.group);
+    if (requests < 2) return false;
+    g.slots = requests * g.group;
+    g.smem_bytes = fixed + act_bytes + g.slots * kTileBytes;
+    if (out) *out = g;
     return true;
 }
 
@@ -555,6 +489,31 @@ struct ChainLaunch {
     int smem_bytes;
     int epilogue_warps;   // per lane quarter: the kernel variant
 };
+
+// KN_CHAIN_TRACE=1 in the environment: the traced variant of the kernel stamps clock64 per layer in its first CTA
+// (MMA issuer: wait for the layer's input, all MMAs issued; first epilogue warp: accumulator ready, chunks
+// finished) and the table is printed when the process exits.  A measuring aid: the stamps cost a few percent.
+long long* chain_trace_table(int n_layers) {
+    if (!getenv("KN_CHAIN_TRACE") || n_layers > kMaxChainLayers) return nullptr;
+    static long long* table = nullptr;
+    static int layers = 0;
+    if (!table && cudaHostAlloc((void**)&table, (size_t)kMaxChainLayers * 64, cudaHostAllocMapped) == cudaSuccess) {
+        atexit([] {
+            const long long* d = table;
+            fprintf(stderr, "convolution chain, CTA 0, SM clock cycles per layer\n"
+                            "layer  wait_input  issue_mmas  (of which filter waits)  accumulator_wait  epilogue_chunks  layer_period\n");
+            for (int i = 0; i < layers; i++)
+                fprintf(stderr, "%5d  %10lld  %10lld  %23lld  %16lld  %15lld  %12lld\n", i, d[i * 8 + 1] - d[i * 8 + 0],
+                        d[i * 8 + 2] - d[i * 8 + 1], d[i * 8 + 3], d[i * 8 + 5] - d[i * 8 + 4], d[i * 8 + 6] - d[i * 8 + 5],
+                        i ? d[i * 8 + 1] - d[(i - 1) * 8 + 1] : 0);
+        });
+    }
+    if (table) {
+        memset(table, 0, (size_t)kMaxChainLayers * 64);
+        layers = n_layers;
+    }
+    return table;
+}
 
 std::shared_ptr<void> chain_prepare(const ConvChainParams& c, uint32_t* status_word) {
     auto l = std::make_shared<ChainLaunch>();
@@ -585,9 +544,6 @@ std::shared_ptr<void> chain_prepare(const ConvChainParams& c, uint32_t* status_w
     p.h = c.h;
     p.w = c.w;
     p.n_layers = c.n_layers;
-    p.per_cta = g.per_cta;
-    p.gx = g.gx;
-    p.gy = g.gy;
     p.wp = g.wp;
     p.q_first = g.q_first;
     p.r_first = g.r_first;
@@ -612,44 +568,15 @@ std::shared_ptr<void> chain_prepare(const ConvChainParams& c, uint32_t* status_w
     // twice the rate of single 16 KB tiles
     p.group = g.group;
     p.slots = g.slots / p.group;
-    // KN_CHAIN_TRACE=1 in the environment: the traced variant of the kernel stamps clock64 per layer in its first CTA
-    // (MMA issuer: wait for the layer's input, all MMAs issued; first epilogue warp: accumulator ready, chunks
-    // finished) and the table is printed when the process exits.  A measuring aid: the stamps cost a few percent.
-    if (getenv("KN_CHAIN_TRACE") && p.n_layers <= kMaxChainLayers) {
-        static long long* table = nullptr;
-        static int layers = 0;
-        if (!table && cudaHostAlloc((void**)&table, (size_t)kMaxChainLayers * 64, cudaHostAllocMapped) == cudaSuccess) {
-            atexit([] {
-                const long long* d = table;
-                fprintf(stderr, "conv_chain_kernel, CTA 0, SM clock cycles per layer\n"
-                                "layer  wait_input  issue_mmas  (of which filter waits)  accumulator_wait  epilogue_chunks  layer_period\n");
-                for (int i = 0; i < layers; i++)
-                    fprintf(stderr, "%5d  %10lld  %10lld  %23lld  %16lld  %15lld  %12lld\n", i, d[i * 8 + 1] - d[i * 8 + 0],
-                            d[i * 8 + 2] - d[i * 8 + 1], d[i * 8 + 3], d[i * 8 + 5] - d[i * 8 + 4], d[i * 8 + 6] - d[i * 8 + 5],
-                            i ? d[i * 8 + 1] - d[(i - 1) * 8 + 1] : 0);
-            });
-        }
-        if (table) {
-            memset(table, 0, (size_t)kMaxChainLayers * 64);
-            layers = p.n_layers;
-            p.trace = table;
-        }
-    }
+    p.trace = chain_trace_table(p.n_layers);
     int64_t dims[3] = {32, 128, p.total_tiles}, strides[3] = {1, 32, 128 * 32};
     int box[3] = {32, 128, 1};
     l->map_tiles = tc_make_map(c.tiles, 3, dims, strides, box, true);
-    l->grid = dim3((unsigned)((c.n + g.per_cta - 1) / g.per_cta), 1, 1);
+    l->grid = dim3((unsigned)c.n, 1, 1);
     l->smem_bytes = g.smem_bytes;
-    // Epilogue variants: the accumulator's columns are shared out in chunks among E warps per lane quarter.  Three
-    // warps taking 16-column chunks when the chunk count divides by three (two 8x8 boards: 9 chunks, three each
-    // instead of five and four), else two.  Four or six warps taking 8-column chunks exist as variants and measured
-    // slower (two boards: 315 / 327 us against 314.5): the epilogue is bound by instruction issue, not by latency.
-    // KN_CHAIN_EPILOGUE=<E> in the environment picks one (measuring).
+    // Epilogue variants: the accumulator's 16-column chunks are shared out among three warps per lane quarter when their count
+    // divides by three, else two.  (Four or six with chunks of 8 columns measured slower: the epilogue is bound by instruction issue.)
     l->epilogue_warps = ((g.n_mma / 16) % 3 == 0) ? 3 : 2;
-    if (const char* e = getenv("KN_CHAIN_EPILOGUE")) {
-        const int v = atoi(e);
-        if (v == 2 || v == 3 || v == 4 || v == 6) l->epilogue_warps = v;
-    }
     return l;
 }
 
@@ -663,10 +590,8 @@ int chain_launch(const void* launch, cudaStream_t stream) {
         std::lock_guard<std::mutex> lock(mu);
         if (device >= 0 && device < 64 && !done[device]) {
             const void* variants[] = {
-                (const void*)conv_chain_kernel<2, 16, false>, (const void*)conv_chain_kernel<3, 16, false>,
-                (const void*)conv_chain_kernel<4, 8, false>,  (const void*)conv_chain_kernel<6, 8, false>,
-                (const void*)conv_chain_kernel<2, 16, true>,  (const void*)conv_chain_kernel<3, 16, true>,
-                (const void*)conv_chain_kernel<4, 8, true>,   (const void*)conv_chain_kernel<6, 8, true>,
+                (const void*)conv_chain_kernel<2, false>, (const void*)conv_chain_kernel<3, false>,
+                (const void*)conv_chain_kernel<2, true>,  (const void*)conv_chain_kernel<3, true>,
             };
             for (const void* v : variants) {
                 cudaError_t e = cudaFuncSetAttribute(v, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -687,14 +612,9 @@ int chain_launch(const void* launch, cudaStream_t stream) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     void* args[] = {(void*)&l.map_tiles, (void*)&l.p};
-    const void* kernel = nullptr;
     const bool t = l.p.trace != nullptr;
-    switch (l.epilogue_warps) {
-        case 6: kernel = t ? (const void*)conv_chain_kernel<6, 8, true> : (const void*)conv_chain_kernel<6, 8, false>; break;
-        case 4: kernel = t ? (const void*)conv_chain_kernel<4, 8, true> : (const void*)conv_chain_kernel<4, 8, false>; break;
-        case 3: kernel = t ? (const void*)conv_chain_kernel<3, 16, true> : (const void*)conv_chain_kernel<3, 16, false>; break;
-        default: kernel = t ? (const void*)conv_chain_kernel<2, 16, true> : (const void*)conv_chain_kernel<2, 16, false>; break;
-    }
+    const void* kernel = l.epilogue_warps == 3 ? (t ? (const void*)conv_chain_kernel<3, true> : (const void*)conv_chain_kernel<3, false>)
+                                               : (t ? (const void*)conv_chain_kernel<2, true> : (const void*)conv_chain_kernel<2, false>);
     return (int)cudaLaunchKernelExC(&cfg, kernel, args);
 }
 

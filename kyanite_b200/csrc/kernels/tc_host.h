@@ -53,5 +53,9 @@ int flash_attention_launch(const void* launch, cudaStream_t stream);
 // Convolution chain (kernels/conv_chain.cu): launch data built once the device pointers are known.
 std::shared_ptr<void> chain_prepare(const ConvChainParams& c, uint32_t* status_word);
 int chain_launch(const void* launch, cudaStream_t stream);
+// The same on CTA pairs (kernels/conv_chain_pair.cu), for ConvChainParams::pair.
+std::shared_ptr<void> chain_pair_prepare(const ConvChainParams& c, uint32_t* status_word);
+int chain_pair_launch(const void* launch, cudaStream_t stream);
+long long* chain_trace_table(int n_layers);   // pinned words for KN_CHAIN_TRACE, else null
 
 }  // namespace kn

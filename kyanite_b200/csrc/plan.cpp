@@ -2969,12 +2969,12 @@ class Planner {
         p.w = first.conv.w;
         const size_t n_layers = len + (heads.empty() ? 0 : 1);
         p.n_layers = (int32_t)n_layers;
-        int64_t n_tiles = 0;
+        int blocks = (p.k + 31) / 32;
         for (size_t a = 0; a < len; a++) {
             const ConvParams& c = steps[layers[a].step].conv;
             KN_CHECK(c.k == p.k && (a == 0 || c.c == p.k), KN_ERR_INTERNAL, "convolution chain with changing width");
             p.c_blocks[a] = (uint8_t)((c.c + 31) / 32);
-            n_tiles += 9 * p.c_blocks[a];
+            blocks = std::max<int>(blocks, p.c_blocks[a]);
             p.flags[a] = (uint8_t)((c.act == (int32_t)Activation::Relu ? kChainFlagRelu : 0) |
                                    (layers[a].res_operand >= 0 ? kChainFlagAddHeld : 0) | (hold[a] ? kChainFlagHold : 0));
             s.flops += steps[layers[a].step].flops;
@@ -2983,30 +2983,41 @@ class Planner {
         if (!heads.empty()) {
             p.c_blocks[len] = (uint8_t)((p.k + 31) / 32);
             p.flags[len] = kChainFlagPointwise;
-            n_tiles += p.c_blocks[len];
         }
-        // filter tiles: [tile][128][32] f32 (already TF32), zero beyond the real channels
-        auto tiles = std::make_shared<std::vector<uint8_t>>((size_t)n_tiles * 128 * 32 * 4, 0);
+        int head_channels = 0;
+        for (auto& h : heads) head_channels += steps[h.step].conv.k;
+        ChainPairGeometry pair;
+        p.pair = tc_chain_pair_geometry(p.h, p.w, p.n, blocks, p.k, head_channels, &pair);
+        // filter tiles (already TF32, zero beyond the real channels), stored exactly as they sit in shared memory (rows of 128
+        // bytes whose 16-byte chunks are XOR-swizzled with the row number), so that a linear bulk copy delivers them
+        std::vector<int64_t> layer_rows(n_layers + 1, 0);   // first row of 32 floats of a layer
+        auto tile_rows = [&](size_t a) { return p.pair ? (a < len ? pair.n_trunk : pair.n_last) : 128; };
+        for (size_t a = 0; a < n_layers; a++) layer_rows[a + 1] = layer_rows[a] + (int64_t)(a < len ? 9 : 1) * p.c_blocks[a] * tile_rows(a);
+        const int64_t n_rows = layer_rows[n_layers];
+        // where input channel `ch` of output channel `k` at a tap goes
+        auto tile_pos = [&](size_t a, int tap, int k, int ch) {
+            const int taps = a < len ? 9 : 1, cb = ch / 32, col = ch % 32;
+            int64_t row;
+            if (p.pair) {
+                const int half = tile_rows(a) / 2;
+                row = layer_rows[a] + ((int64_t)((k / half) * p.c_blocks[a] + cb) * taps + tap) * half + k % half;
+            } else {
+                row = layer_rows[a] + (int64_t)(tap * p.c_blocks[a] + cb) * 128 + k;
+            }
+            return row * 32 + ((((col >> 2) ^ (int)(row & 7)) << 2) | (col & 3));   // (tiles begin at multiples of eight rows)
+        };
+        auto tiles = std::make_shared<std::vector<uint8_t>>((size_t)n_rows * 32 * 4, 0);
         auto bias = std::make_shared<std::vector<uint8_t>>(n_layers * 128 * 4, 0);
         float* tp = (float*)tiles->data();
         float* bp = (float*)bias->data();
-        int64_t tile = 0;
         for (size_t a = 0; a < len; a++) {
             const Step& st = steps[layers[a].step];
             const ConvParams& c = st.conv;
             const int64_t c_pad = (c.c + 3) / 4 * 4;
             const float* src = (const float*)plan_.buffers[st.operands[1].buf].owned->data();   // [tap][K][c_pad]
             for (int tap = 0; tap < 9; tap++)
-                for (int cb = 0; cb < p.c_blocks[a]; cb++, tile++)
-                    for (int k = 0; k < c.k; k++)
-                        for (int ch = cb * 32; ch < std::min<int>(c.c, cb * 32 + 32); ch++)
-                        {
-                            // stored exactly as the tile sits in shared memory (rows of 128 bytes whose 16-byte
-                            // chunks are XOR-swizzled with the row number), so a linear bulk copy delivers it
-                            const int col = ch - cb * 32;
-                            const int64_t pos = (int64_t)k * 32 + ((((col >> 2) ^ (k & 7)) << 2) | (col & 3));
-                            tp[tile * 128 * 32 + pos] = src[((int64_t)tap * c.k + k) * c_pad + ch];
-                        }
+                for (int k = 0; k < c.k; k++)
+                    for (int ch = 0; ch < c.c; ch++) tp[tile_pos(a, tap, k, ch)] = src[((int64_t)tap * c.k + k) * c_pad + ch];
             if (layers[a].bias_operand >= 0) {
                 const PlanTensor& b = st.operands[layers[a].bias_operand];
                 const float* bsrc = (const float*)plan_.buffers[b.buf].host_data;
@@ -3029,9 +3040,7 @@ class Planner {
                     memcpy(&bits, &v, 4);
                     if ((bits & 0x7F800000u) != 0x7F800000u) bits = (bits + 0x1000u) & 0xFFFFE000u;
                     memcpy(&v, &bits, 4);
-                    const int row = row0 + k, cb = ch / 32, col = ch % 32;
-                    const int64_t pos = (int64_t)row * 32 + ((((col >> 2) ^ (row & 7)) << 2) | (col & 3));
-                    tp[(tile + cb) * 128 * 32 + pos] = v;
+                    tp[tile_pos(len, 0, row0 + k, ch)] = v;
                 }
             if (heads[hi].bias_operand >= 0) {
                 const PlanTensor& b = st.operands[heads[hi].bias_operand];
@@ -3046,7 +3055,7 @@ class Planner {
             s.flops += st.flops;
         }
         p.head_begin[heads.size()] = row0;
-        PlanTensor t_tiles = alloc_const({n_tiles, 128, 32}, DType::F32, s.value, nullptr, tiles);
+        PlanTensor t_tiles = alloc_const({n_rows, 32}, DType::F32, s.value, nullptr, tiles);
         PlanTensor t_bias = alloc_const({(int64_t)n_layers, 128}, DType::F32, s.value, nullptr, bias);
         // operand 1 is the trunk's result; when nothing reads it, it is neither stored nor allocated (the slot
         // then repeats the first head's output)
@@ -3061,7 +3070,7 @@ class Planner {
             p.s_out[d] = last.operands[2].ss.strides[d];
         }
         s.desc = "convchain layers=" + std::to_string(len) + " n=" + std::to_string(p.n) + " c=" + std::to_string(p.c_in) + " hw=" +
-                 std::to_string(p.h) + "x" + std::to_string(p.w) + " k=" + std::to_string(p.k) + " rs=3x3 tf32";
+                 std::to_string(p.h) + "x" + std::to_string(p.w) + " k=" + std::to_string(p.k) + " rs=3x3 tf32" + (p.pair ? " on CTA pairs" : "");
         if (!heads.empty()) {
             s.desc += " heads=";
             for (size_t hi = 0; hi < heads.size(); hi++) s.desc += (hi ? "+" : "") + std::to_string(p.head_begin[hi + 1] - p.head_begin[hi]);

@@ -34,17 +34,11 @@ bool flash_attention_fits(int64_t batch, int64_t m, int64_t n, int64_t k, int64_
 // Output tile of the convolution kernel: wb x hb x nb output positions (product 128).
 bool tc_conv_tile(int oh, int ow, int* wb, int* hb, int* nb);
 
-// Shared-memory layout of the convolution-chain kernel (kernels/conv_chain.cu).  The images of one CTA
-// are stored as one large zero-padded image, `gx` images side by side and `gy` such rows of images below
-// one another: a row has `wp = gx * (w + 1)` positions (the position in front of each image row is the
-// zero left of it and, being adjacent in memory, the zero right of the image row before it), there are
-// `h + 1` rows per row of images (the first is the zero row shared with the images above), and one more
-// zero row at the end.  With that, filter tap (r, s) of every output position is the position
-// `(r - 1) * wp + (s - 1)` further on, a constant shift of the operand's start address.  Two 8x8 boards
-// side by side need 144 accumulator columns (128 of them real pixels), stacked they would need 160.
+// Shared-memory layout of the convolution-chain kernel (kernels/conv_chain.cu), one image per CTA.  The image is stored zero-padded:
+// a row has `wp = w + 1` positions (the position in front of each image row is the zero left of it and, being adjacent in memory,
+// the zero right of the image row before it), and there is a zero row above and below.  With that, filter tap (r, s) of every
+// output position is the position `(r - 1) * wp + (s - 1)` further on, a constant shift of the operand's start address.
 struct ChainGeometry {
-    int per_cta;      // images per CTA = gx * gy
-    int gx, gy;
     int wp;           // positions per padded row
     int q_first;      // padded position of output column 0 (the first real pixel)
     int r_first;      // shared-memory row that holds position q_first: q_first rounded up to a multiple of 8, so
@@ -52,11 +46,23 @@ struct ChainGeometry {
     int n_mma;        // accumulator columns: padded positions q_first .. q_first + n_mma - 1
     int rows_alloc;   // 128-byte rows per 32-channel block of the activation buffer
     int slots;        // 16 KB filter tiles in flight
-    int group;        // filter tiles per request (a whole tap = the layer's channel blocks)
+    int group;        // filter tiles per request (a whole tap = the layer's channel blocks, or three taps)
     int smem_bytes;
 };
 // False if images of this size do not fit (then every layer stays its own step).  `c_blocks` = 32-channel
 // blocks of the widest layer.  Pure host arithmetic.
 bool tc_chain_geometry(int h, int w, int64_t n_img, int c_blocks, ChainGeometry* out);
+
+// The same on CTA pairs (kernels/conv_chain_pair.cu): 128 accumulator lanes per CTA are the positions of its images, which are
+// stored as one large zero-padded image, `gx` images side by side (wp = gx * (w + 1)) and `gy` such rows of images below one
+// another (h + 1 rows each, the first being the zero row shared with the images above).
+struct ChainPairGeometry {
+    int per_cta, gx, gy, wp;   // images per CTA = gx * gy
+    int pitch;                 // operand rows between groups of eight accumulator lanes: 9 where an image row is a group, else 8
+    int n_trunk, n_last;       // accumulator columns of a 3x3 layer and of the pointwise last layer (0: none)
+    int rows_alloc, slots, slot_bytes, smem_bytes;
+};
+// False if they do not fit.  `k`: output channels of the 3x3 layers; `head_channels`: of the pointwise last layer, 0 if there is none.
+bool tc_chain_pair_geometry(int h, int w, int64_t n_img, int blocks, int k, int head_channels, ChainPairGeometry* out);
 
 }  // namespace kn
