@@ -2,29 +2,27 @@
 // probabilities ever leaving the SM, one CTA per (batch entry, 128 query rows).  Operands in f32 storage (TF32 on load,
 // kind::tf32) or f16 storage (kind::f16); statistics, sums and both accumulators are f32 in either.
 //
-// The keys are taken 128 at a time.  A block's scores are one accumulator of 128 columns in tensor memory; its
+// The keys are taken 64 at a time.  A block's scores are one of two accumulators of 64 columns in tensor memory; its
 // probabilities take the place of the scores (f16: packed, half the columns) and are the A operand of the second MMA, whose
 // accumulator of up to 128 columns is kept over all blocks.  Exponentials are taken against a reference that follows the
 // row's running maximum only when that has risen by more than 8 (in powers of two): then the row's accumulator and sum are
-// rescaled, which after the first few blocks hardly ever happens; the quotient does not depend on the reference.
+// rescaled (once the block before has been added), which after the first few blocks hardly ever happens; the quotient does
+// not depend on the reference.
 //
-//   warps 0..7      softmax: a row per lane quarter and lane, its 128 columns on two warps of 64 (the maximum and, at the
-//                   end, the sum are exchanged through shared memory)
-//   warp 8, a lane  producer: Q once, keys and values of a block through one buffer each; the next block's keys are
-//                   requested when the score MMAs have read this block's, under the exponentials
-//   warp 9, a lane  MMA issuer
+//   warps 0..3      softmax: a row per thread, all 64 columns of it, so nothing is exchanged
+//   warp 4, a lane  producer: Q once, keys and values of a block through two buffers each (one where two do not fit)
+//   warp 5, a lane  MMA issuer: the next block's score MMAs go ahead of this block's context MMAs, under its exponentials
 //
-// Inside a CTA the phases of a block follow one another (scores, exponentials, context); what fills the tensor cores and
-// the special-function unit meanwhile is the SM's second CTA: 256 columns of tensor memory, some 100 KB of shared memory
-// (head dimensions up to 64 in f32 or 128 in f16; larger ones run one CTA per SM).  Two CTAs of 320 threads leave a thread 96
-// registers, of which a row's 64 scores take two thirds: every variant spills 240 to 280 bytes.
+// Two CTAs share an SM: 256 columns of tensor memory, some 100 KB of shared memory (head dimensions up to 64 in f32 or 128 in
+// f16; larger ones run one CTA per SM), 192 threads with 160 registers: a row's 64 scores stay in them.  (With blocks of 128
+// keys, one accumulator, and a row on two warps the phases of a block followed one another: 6 000 cycles of a CTA for 128 keys,
+// 5 000 now, 240 to 280 bytes of registers spilled, a barrier of all warps for every maximum.)
 //
-// Measured, scores matmul + softmax + copies + context matmul planned node by node -> this step (kernel_bench's
-// attention_causal_f16, attention_latent and attention_short_f16): 32 heads of 2048 causal rows, f16, d = 128:
-// 122 + 155 + 15 + 57 -> 93 us, 10 of them flash_finite_kernel; 8 heads of 4096 rows, f32, d = 40: 117 + 198 + 99 -> 122 us;
-// 32 heads of 333 causal rows, f16, d = 128: 215 -> 20 us.
-// What bounds it: a block is some 6 000 cycles of a CTA (scores seen 1 200 after the issuer starts them, read 1 000, maximum
-// 300, exponentials 1 800, context MMAs 1 300 at 80 cycles an instruction with A from tensor memory), two CTAs in turn.
+// Measured (kernel_bench's attention_causal_f16, attention_latent and attention_short_f16), one accumulator of 128 keys -> now:
+// 32 heads of 2048 causal rows, f16, d = 128: 94 -> 69 us, 10 of them flash_finite_kernel; 8 heads of 4096 rows, f32, d = 40:
+// 119 -> 74 us; 32 heads of 333 causal rows, f16, d = 128: 19.5 -> 16.4 us.
+// What bounds it: f32, the context MMAs (80 cycles for 8 keys with A from tensor memory, whatever the number of columns: 1 300 of
+// the 2 500 cycles that an SM takes for 128 keys) next to the exponentials (1 024 at 16 a cycle).
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -46,9 +44,10 @@ namespace {
 
 using namespace tcp;
 
-constexpr int kFlThreads = 320;
-constexpr int kFlRows = 128, kFlKeys = 128;
-constexpr int kFlBlockBytes = 128 * 128;   // 128 rows of 128 bytes
+constexpr int kFlThreads = 192;
+constexpr int kFlRows = 128, kFlKeys = 64;
+constexpr int kFlTableKeys = 128;          // keys of a block in the planner's table of a constant term
+constexpr int kFlQBytes = kFlRows * 128, kFlKeyBytes = kFlKeys * 128;   // a panel: rows of 128 bytes
 constexpr int kFlTmemCols = 256, kFlOutCol = 128;
 constexpr float kLog2e = 1.44269504088896340736f;
 constexpr float kRiseLimit = 8.0f;
@@ -56,7 +55,8 @@ constexpr float kHalfSumBelow = -1024.f;   // f16 values are one apart here
 constexpr uint32_t kFlSleepNs = 1000;
 
 struct FlashParams {
-    int32_t m, n, batch, m_tiles, key_blocks;
+    int32_t m, n, batch, m_tiles, key_blocks, table_blocks;
+    int32_t key_slots, value_slots;  // buffers of a block's keys, of its values: one or two
     int32_t qk_blocks, qk_steps;     // 128-byte blocks of a row of Q; instructions of 32 bytes along it
     int32_t dv, v_panels, out_cols;  // columns of V, 128-byte panels of them, N of the context MMAs
     int32_t a_bi, b_bi, v_bi;        // batch entry bt -> map coordinates (bt % bi, bt / bi)
@@ -96,27 +96,29 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     constexpr int kElems = HALF ? 64 : 32;   // elements per 128 bytes
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t k_base = base + (uint32_t)(p.qk_blocks * kFlBlockBytes);
-    const uint32_t v_base = k_base + (uint32_t)(p.qk_blocks * kFlBlockBytes);
-    const uint32_t exch = v_base + (uint32_t)(p.v_panels * kFlBlockBytes);
-    float* exchange = (float*)(gen_base + (exch - base));   // [2 column halves][128 rows]
-    const uint32_t q_full = exch + 1024u, k_full = q_full + 8u, s_full = q_full + 16u, v_full = q_full + 24u, p_ready = q_full + 32u,
-                   pv_done = q_full + 40u, slot_addr = q_full + 48u;
+    const uint32_t k_bytes = (uint32_t)(p.qk_blocks * kFlKeyBytes), v_bytes = (uint32_t)(p.v_panels * kFlKeyBytes);
+    const uint32_t k_base = base + (uint32_t)(p.qk_blocks * kFlQBytes);
+    const uint32_t v_base = k_base + (uint32_t)p.key_slots * k_bytes;
+    const uint32_t bars = v_base + (uint32_t)p.value_slots * v_bytes;
+    // (of two: one per parity of the block)
+    const uint32_t q_full = bars, pv_done = bars + 8u, k_full = bars + 24u, v_full = bars + 40u, s_full = bars + 56u, p_ready = bars + 72u, slot_addr = bars + 88u;
     volatile uint32_t* tmem_slot = (volatile uint32_t*)(gen_base + (slot_addr - base));
     volatile int* abandon = (volatile int*)(gen_base + (slot_addr + 4u - base));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
-        mbar_init(k_full, 1);
-        mbar_init(s_full, 1);
-        mbar_init(v_full, 1);
-        mbar_init(p_ready, 8);
-        mbar_init(pv_done, 1);
+        for (uint32_t b = 0; b < 16u; b += 8u) {
+            mbar_init(pv_done + b, 1);
+            mbar_init(k_full + b, 1);
+            mbar_init(v_full + b, 1);
+            mbar_init(s_full + b, 1);
+            mbar_init(p_ready + b, 4);
+        }
         *abandon = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 8) {
+    if (warp == 4) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_addr), "r"((uint32_t)kFlTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -128,37 +130,48 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
     // the last row blocks first: under a causal mask they have the most keys
     const int bt = (int)(blockIdx.x % (unsigned)p.batch), mt = p.m_tiles - 1 - (int)(blockIdx.x / (unsigned)p.batch);
-    const int16_t* blocks_of = TERM && p.term_blocks ? p.term_blocks + (int64_t)mt * (p.key_blocks + 1) : nullptr;   // (a constant)
-    int n_blocks = blocks_of ? (int)blocks_of[0] : p.key_blocks;
+    const int16_t* blocks_of = TERM && p.term_blocks ? p.term_blocks + (int64_t)mt * (p.table_blocks + 1) : nullptr;   // (a constant)
+    constexpr int kTableStep = kFlTableKeys / kFlKeys;
+    int n_table = blocks_of ? (int)blocks_of[0] : p.table_blocks;
     auto block_cols = [&](int j) { return min(kFlKeys, (p.n - j * kFlKeys + 31) & ~31); };   // (past n: zero fill, masked below)
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (TERM && p.not_finite && n_blocks < p.key_blocks) {   // up to the last masked block that does not give exact zeros
-        const int32_t* flags = p.not_finite + (int64_t)bt * p.key_blocks;
+    if (TERM && p.not_finite && n_table < p.table_blocks) {   // up to the last masked block that does not give exact zeros
+        const int32_t* flags = p.not_finite + (int64_t)bt * p.table_blocks;
         int last = 0;
-        for (int j = n_blocks + lane; j < p.key_blocks; j += 32) last = flags[j] != 0 ? j + 1 : last;
-        n_blocks = max(n_blocks, __reduce_max_sync(0xffffffffu, last));
+        for (int j = n_table + lane; j < p.table_blocks; j += 32) last = flags[j] != 0 ? j + 1 : last;
+        n_table = max(n_table, __reduce_max_sync(0xffffffffu, last));
     }
+    const int n_blocks = min(n_table * kTableStep, p.key_blocks);
 
-    if (warp == 8) {
+    if (warp == 4) {
         if (elect_one()) {
             // ---------------- producer
-            const uint32_t qk_bytes = (uint32_t)(p.qk_blocks * kFlBlockBytes), v_bytes = (uint32_t)(p.v_panels * kFlBlockBytes);
-            mbar_expect_tx(q_full, qk_bytes);
+            const uint32_t q_bytes = (uint32_t)(p.qk_blocks * kFlQBytes);
+            mbar_expect_tx(q_full, q_bytes);
             for (int b = 0; b < p.qk_blocks; b++)
-                tma_load_4d(base + (uint32_t)(b * kFlBlockBytes), &map_q, q_full, b * kElems, mt * kFlRows, bt % p.a_bi, bt / p.a_bi);
+                tma_load_4d(base + (uint32_t)(b * kFlQBytes), &map_q, q_full, b * kElems, mt * kFlRows, bt % p.a_bi, bt / p.a_bi);
             const int k2 = bt % p.b_bi, k3 = bt / p.b_bi, v2 = bt % p.v_bi, v3 = bt / p.v_bi;
-            for (int j = 0; j < n_blocks; j++) {
-                if (j > 0 && !mbar_wait(s_full, (uint32_t)((j - 1) & 1), abandon, p.status, 51, kWaitCycles, kFlSleepNs)) break;
-                mbar_expect_tx(k_full, qk_bytes);
+            auto keys = [&](int j) -> bool {
+                const int used = j - p.key_slots;   // the block whose keys lay there: its scores are complete
+                if (used >= 0 && !mbar_wait(s_full + 8u * (used & 1), (uint32_t)((used >> 1) & 1), abandon, p.status, 51, kWaitCycles, kFlSleepNs)) return false;
+                const uint32_t to = k_base + (p.key_slots == 2 ? (uint32_t)(j & 1) * k_bytes : 0u);
+                mbar_expect_tx(k_full + 8u * (j & 1), k_bytes);
                 for (int b = 0; b < p.qk_blocks; b++)
-                    tma_load_4d(k_base + (uint32_t)(b * kFlBlockBytes), &map_k, k_full, b * kElems, j * kFlKeys, k2, k3);
-                if (j > 0 && !mbar_wait(pv_done, (uint32_t)((j - 1) & 1), abandon, p.status, 52, kWaitCycles, kFlSleepNs)) break;
-                mbar_expect_tx(v_full, v_bytes);
+                    tma_load_4d(to + (uint32_t)(b * kFlKeyBytes), &map_k, k_full + 8u * (j & 1), b * kElems, j * kFlKeys, k2, k3);
+                return true;
+            };
+            bool ok = keys(0);
+            for (int j = 0; j < n_blocks && ok; j++) {
+                if (j + 1 < n_blocks && !keys(j + 1)) break;
+                const int used = j - p.value_slots;
+                if (used >= 0 && !mbar_wait(pv_done + 8u * (used & 1), (uint32_t)((used >> 1) & 1), abandon, p.status, 52, kWaitCycles, kFlSleepNs)) break;
+                const uint32_t to = v_base + (p.value_slots == 2 ? (uint32_t)(j & 1) * v_bytes : 0u);
+                mbar_expect_tx(v_full + 8u * (j & 1), v_bytes);
                 for (int b = 0; b < p.v_panels; b++)
-                    tma_load_4d(v_base + (uint32_t)(b * kFlBlockBytes), &map_v, v_full, b * kElems, j * kFlKeys, v2, v3);
+                    tma_load_4d(to + (uint32_t)(b * kFlKeyBytes), &map_v, v_full + 8u * (j & 1), b * kElems, j * kFlKeys, v2, v3);
             }
         }
-    } else if (warp == 9) {
+    } else if (warp == 5) {
         if (elect_one()) {
             // ---------------- MMA issuer: f32 accumulate, M = 128; Q and the keys K-major, V with its columns contiguous
             // (bit 16: the MN-major B operand)
@@ -168,74 +181,72 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             // MN-major B: panels of 128 bytes of columns lie `leading byte offset` apart, groups of keys `stride byte
             // offset`: eight keys and the 128-byte swizzle for 16-bit elements, four and the swizzle in 32-byte pieces for
             // 32-bit ones (see attention.cu)
-            const uint64_t v_desc = ((uint64_t)(kFlBlockBytes >> 4) << 16) | ((uint64_t)((HALF ? 1024 : 512) >> 4) << 32) | ((uint64_t)1 << 46) |
+            const uint64_t v_desc = ((uint64_t)(kFlKeyBytes >> 4) << 16) | ((uint64_t)((HALF ? 1024 : 512) >> 4) << 32) | ((uint64_t)1 << 46) |
                                     ((uint64_t)(HALF ? 2 : 1) << 61);
             constexpr int kStepKeys = HALF ? 16 : 8, kStepCols = 8;   // keys of an instruction; their columns in tensor memory
-            const bool ok = mbar_wait(q_full, 0, abandon, p.status, 53, kWaitCycles, kFlSleepNs);
-            for (int j = 0; j < n_blocks && ok; j++) {
-                const uint32_t parity = (uint32_t)(j & 1);
-                const int cols = block_cols(j);
-                if (!mbar_wait(k_full, parity, abandon, p.status, 54, kWaitCycles, kFlSleepNs)) break;
-                // (the probabilities of the block before lie where the scores go)
-                if (j > 0 && !mbar_wait(pv_done, parity ^ 1u, abandon, p.status, 55, kWaitCycles, kFlSleepNs)) break;
+            auto scores = [&](int j) -> bool {
+                const uint32_t b = (uint32_t)(j & 1);
+                if (!mbar_wait(k_full + 8u * b, (uint32_t)((j >> 1) & 1), abandon, p.status, 54, kWaitCycles, kFlSleepNs)) return false;
+                // (the probabilities of the block before the last lie where the scores go)
+                if (j > 1 && !mbar_wait(pv_done + 8u * b, (uint32_t)(((j - 2) >> 1) & 1), abandon, p.status, 55, kWaitCycles, kFlSleepNs)) return false;
                 tc_fence_after();
-                const uint32_t idesc_s = idesc | ((uint32_t)(cols >> 3) << 17);
+                const uint32_t idesc_s = idesc | ((uint32_t)(block_cols(j) >> 3) << 17);
+                const uint32_t from = k_base + (p.key_slots == 2 ? b * k_bytes : 0u);
                 for (int s = 0; s < p.qk_steps; s++) {
-                    const uint32_t at = (uint32_t)((s >> 2) * kFlBlockBytes);
-                    const uint64_t da = smem_desc_sw128(base + at) + 2u * (s & 3), db = smem_desc_sw128(k_base + at) + 2u * (s & 3);
-                    if (HALF) mma_f16(tmem_s, da, db, idesc_s, s != 0 ? 1u : 0u);
-                    else mma_tf32(tmem_s, da, db, idesc_s, s != 0 ? 1u : 0u);
+                    const uint64_t da = smem_desc_sw128(base + (uint32_t)((s >> 2) * kFlQBytes)) + 2u * (s & 3);
+                    const uint64_t db = smem_desc_sw128(from + (uint32_t)((s >> 2) * kFlKeyBytes)) + 2u * (s & 3);
+                    if (HALF) mma_f16(tmem_s + b * kFlKeys, da, db, idesc_s, s != 0 ? 1u : 0u);
+                    else mma_tf32(tmem_s + b * kFlKeys, da, db, idesc_s, s != 0 ? 1u : 0u);
                 }
-                mma_commit(s_full);
-                if (!mbar_wait(v_full, parity, abandon, p.status, 56, kWaitCycles, kFlSleepNs)) break;
-                if (!mbar_wait(p_ready, parity, abandon, p.status, 57, kWaitCycles, kFlSleepNs)) break;
+                mma_commit(s_full + 8u * b);
+                return true;
+            };
+            bool ok = mbar_wait(q_full, 0, abandon, p.status, 53, kWaitCycles, kFlSleepNs) && scores(0);
+            for (int j = 0; j < n_blocks && ok; j++) {
+                const uint32_t b = (uint32_t)(j & 1), parity = (uint32_t)((j >> 1) & 1);
+                if (j + 1 < n_blocks && !scores(j + 1)) break;   // under this block's exponentials
+                if (!mbar_wait(v_full + 8u * b, parity, abandon, p.status, 56, kWaitCycles, kFlSleepNs)) break;
+                if (!mbar_wait(p_ready + 8u * b, parity, abandon, p.status, 57, kWaitCycles, kFlSleepNs)) break;
                 tc_fence_after();
+                const uint32_t from = v_base + (p.value_slots == 2 ? b * v_bytes : 0u);
+                const int cols = block_cols(j);
                 for (int s = 0; s < cols / kStepKeys; s++) {
-                    const uint64_t db = v_desc | (uint64_t)(((v_base + (uint32_t)(s * kStepKeys * 128)) & 0x3FFFFu) >> 4);
-                    if (HALF) mma_f16_a_tmem(tmem_o, tmem_s + (uint32_t)(s * kStepCols), db, idesc_o, (j | s) != 0 ? 1u : 0u);
-                    else mma_tf32_a_tmem(tmem_o, tmem_s + (uint32_t)(s * kStepCols), db, idesc_o, (j | s) != 0 ? 1u : 0u);
+                    const uint64_t db = v_desc | (uint64_t)(((from + (uint32_t)(s * kStepKeys * 128)) & 0x3FFFFu) >> 4);
+                    if (HALF) mma_f16_a_tmem(tmem_o, tmem_s + b * kFlKeys + (uint32_t)(s * kStepCols), db, idesc_o, (j | s) != 0 ? 1u : 0u);
+                    else mma_tf32_a_tmem(tmem_o, tmem_s + b * kFlKeys + (uint32_t)(s * kStepCols), db, idesc_o, (j | s) != 0 ? 1u : 0u);
                 }
-                mma_commit(pv_done);
+                mma_commit(pv_done + 8u * b);
             }
         }
     } else {
         // ---------------- softmax
-        const int quarter = warp & 3, half = warp >> 2;
-        const int row_in_tile = quarter * 32 + lane, row = mt * kFlRows + row_in_tile;
+        const int quarter = warp, row_in_tile = quarter * 32 + lane, row = mt * kFlRows + row_in_tile;
         const uint32_t lane_bits = (uint32_t)(quarter * 32) << 16;
-        const uint32_t my_s = tmem_s + lane_bits + (uint32_t)(half * 64), my_o = tmem_o + lane_bits;
+        const uint32_t my_o = tmem_o + lane_bits;
         using T = typename std::conditional<HALF, __half, float>::type;
         const T* term_row = TERM ? (const T*)p.term + bt * p.term_s[0] + (int64_t)min(row, p.m - 1) * p.term_s[1] : nullptr;
-        // (the warps meet at barriers, so they must agree on going on: one lane waits, then all vote)
-        auto wait_agreed = [&](uint32_t bar, uint32_t parity, uint32_t code) -> bool {
+        auto wait = [&](uint32_t bar, uint32_t parity, uint32_t code) -> bool {   // one lane polls
             uint32_t good = 1;
             if (lane == 0) good = mbar_wait(bar, parity, abandon, p.status, code, kWaitCycles, kFlSleepNs) ? 1u : 0u;
             good = __shfl_sync(0xffffffffu, good, 0);
-            uint32_t all_good;
-            asm volatile(
-                "{\n\t.reg .pred p, q;\n\t"
-                "setp.ne.u32 p, %1, 0;\n\t"
-                "bar.red.and.pred q, 1, 256, p;\n\t"
-                "selp.u32 %0, 1, 0, q;\n\t}"
-                : "=r"(all_good)
-                : "r"(good)
-                : "memory");
             tc_fence_after();
-            return all_good != 0;
+            return good != 0;
         };
         // x in units of its exponent: with a term  x = scale * s + term, exponent (x - ref) * log2(e); without one x = s
         const float unit = TERM ? kLog2e : p.scale * kLog2e;
         float seen = -INFINITY, ref = 0.f, sum = 0.f;
         bool ok = true;
         for (int j = 0; j < n_blocks; j++) {
-            if (!wait_agreed(s_full, (uint32_t)(j & 1), 58)) { ok = false; break; }
+            const uint32_t b = (uint32_t)(j & 1);
+            const uint32_t my_s = tmem_s + lane_bits + b * kFlKeys;
+            if (!wait(s_full + 8u * b, (uint32_t)((j >> 1) & 1), 58)) { ok = false; break; }
             uint32_t v[2][32];
             tmem_load_32_nowait(my_s, v[0]);
             tmem_load_32_nowait(my_s + 32u, v[1]);
             tmem_loads_done();
-            const int col0 = j * kFlKeys + half * 64;
+            const int col0 = j * kFlKeys;
             if (TERM) {
-                const int kind = blocks_of == nullptr ? 1 : (int)blocks_of[1 + j];
+                const int kind = blocks_of == nullptr ? 1 : (int)blocks_of[1 + j / kTableStep];
                 if (kind != 1) {
                     const float same = kind == 2 ? -INFINITY : 0.f;
 #pragma unroll
@@ -289,13 +300,6 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             float top = -INFINITY;
 #pragma unroll
             for (int i = 0; i < 64; i++) top = fmaxf(top, __uint_as_float(v[i >> 5][i & 31]));
-            exchange[half * 128 + row_in_tile] = top;
-            // (also: every score of the block has been read.  In f16 the other half's warps store their probabilities over
-            // columns that this half's have just read, so the barrier orders tensor-memory accesses too)
-            tc_fence_before();
-            asm volatile("bar.sync 2, 256;" ::: "memory");
-            tc_fence_after();
-            top = fmaxf(top, exchange[(half ^ 1) * 128 + row_in_tile]);
             // a row whose scores were all -infinity so far has no reference yet (and zeros in its sum and output)
             const bool first = seen == -INFINITY;
             seen = fmaxf(seen, top);
@@ -306,7 +310,8 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 ref = next;
                 sum *= factor;
                 if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
-                    for (int c = half; c < (p.out_cols + 31) >> 5; c += 2) {
+                    if (!wait(pv_done + 8u * (b ^ 1u), (uint32_t)(((j - 1) >> 1) & 1), 59)) { ok = false; break; }   // (the block before is still being added)
+                    for (int c = 0; c < (p.out_cols + 31) >> 5; c++) {
                         uint32_t o[32];
                         tmem_load_32(my_o + (uint32_t)(c * 32), o);
 #pragma unroll
@@ -339,7 +344,7 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 }
             }
             if (HALF) {
-                tmem_store_32(tmem_s + lane_bits + (uint32_t)(half * 32), v[0]);
+                tmem_store_32(my_s, v[0]);
             } else {
                 tmem_store_32(my_s, v[0]);
                 tmem_store_32(my_s + 32u, v[1]);
@@ -347,14 +352,12 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             tmem_stores_done();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) arrive_one(p_ready);
+            if (lane == 0) arrive_one(p_ready + 8u * b);
         }
-        if (ok && wait_agreed(pv_done, (uint32_t)((n_blocks - 1) & 1), 59)) {
-            exchange[half * 128 + row_in_tile] = sum;
-            asm volatile("bar.sync 2, 256;" ::: "memory");
-            const float inv = 1.f / (sum + exchange[(half ^ 1) * 128 + row_in_tile]);
+        if (ok && wait(pv_done + 8u * ((n_blocks - 1) & 1), (uint32_t)(((n_blocks - 1) >> 1) & 1), 59)) {
+            const float inv = 1.f / sum;
             T* dst = (T*)p.out + (bt / p.out_heads) * p.out_s[0] + (bt % p.out_heads) * p.out_s[1] + (int64_t)row * p.out_s[2];
-            for (int c = half; c < (p.dv + 31) >> 5; c += 2) {
+            for (int c = 0; c < (p.dv + 31) >> 5; c++) {
                 uint32_t o[32];
                 tmem_load_32(my_o + (uint32_t)(c * 32), o);
 #pragma unroll
@@ -382,7 +385,7 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         tc_fence_before();
     }
     __syncthreads();
-    if (warp == 8) {
+    if (warp == 4) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_s), "r"((uint32_t)kFlTmemCols) : "memory");
     }
@@ -404,14 +407,14 @@ __global__ void __launch_bounds__(256) flash_finite_kernel(const __grid_constant
     pdl_enter();
     constexpr int kSize = HALF ? 2 : 4;
     const int j = (int)(blockIdx.x % (unsigned)p.key_blocks), bt = (int)(blockIdx.x / (unsigned)p.key_blocks);
-    const int rows = min(kFlKeys, p.n - j * kFlKeys);
+    const int rows = min(kFlTableKeys, p.n - j * kFlTableKeys);
     auto exponent_full = [](uint32_t w) {
         return HALF ? (w & 0x7C00u) == 0x7C00u || (w & 0x7C000000u) == 0x7C000000u : (w & 0x7F800000u) == 0x7F800000u;
     };
     bool found = false;
 #pragma unroll
     for (int o = 0; o < 2; o++) {
-        const char* base = (const char*)p.base[o] + ((bt % p.bi[o]) * p.s_x[o] + (bt / p.bi[o]) * p.s_y[o] + (int64_t)j * kFlKeys * p.s_row[o]) * kSize;
+        const char* base = (const char*)p.base[o] + ((bt % p.bi[o]) * p.s_x[o] + (bt / p.bi[o]) * p.s_y[o] + (int64_t)j * kFlTableKeys * p.s_row[o]) * kSize;
         const int chunks = p.cols[o] * kSize / 16, row_step = 256 / chunks, chunk_step = 256 % chunks;
         int r = threadIdx.x / chunks, c = threadIdx.x % chunks;
 #pragma unroll 8
@@ -435,9 +438,10 @@ struct FlashLaunch {
     bool half;
 };
 
-int flash_smem_bytes(int64_t k, int64_t dv, bool half) {
-    const int64_t elems = half ? 64 : 32;
-    return (int)(1024 + (2 * ((k + elems - 1) / elems) + (dv + elems - 1) / elems) * kFlBlockBytes + 1024 + 64);
+// Shared memory with `key_slots` and `value_slots` buffers
+int flash_smem_bytes(int64_t k, int64_t dv, bool half, int key_slots, int value_slots) {
+    const int64_t elems = half ? 64 : 32, k_panels = (k + elems - 1) / elems, v_panels = (dv + elems - 1) / elems;
+    return (int)(1024 + k_panels * kFlQBytes + (key_slots * k_panels + value_slots * v_panels) * kFlKeyBytes + 128);
 }
 
 }  // namespace
@@ -445,7 +449,7 @@ int flash_smem_bytes(int64_t k, int64_t dv, bool half) {
 bool flash_attention_fits(int64_t batch, int64_t m, int64_t n, int64_t k, int64_t dv, bool half) {
     if (batch < 1 || m < 1 || n < 1 || k < 8 || dv < 8) return false;
     if (k > 128 || dv > 128 || k % 8 != 0 || dv % 8 != 0 || n > (1 << 21) || m > (1 << 24)) return false;
-    return batch * ((m + kFlRows - 1) / kFlRows) < (1ll << 30) && flash_smem_bytes(k, dv, half) <= 227 * 1024;
+    return batch * ((m + kFlRows - 1) / kFlRows) < (1ll << 30) && flash_smem_bytes(k, dv, half, 1, 1) <= 227 * 1024;
 }
 
 std::shared_ptr<void> flash_attention_prepare(const GemmParams& g, uint32_t* status_word) {
@@ -463,6 +467,7 @@ std::shared_ptr<void> flash_attention_prepare(const GemmParams& g, uint32_t* sta
     p.batch = (int)g.batch;
     p.m_tiles = (int)((g.m + kFlRows - 1) / kFlRows);
     p.key_blocks = (int)((g.n + kFlKeys - 1) / kFlKeys);
+    p.table_blocks = (int)((g.n + kFlTableKeys - 1) / kFlTableKeys);
     p.qk_blocks = (int)((g.k + elems - 1) / elems);
     p.qk_steps = (int)((g.k + elems / 4 - 1) / (elems / 4));
     p.dv = (int)g.values_cols;
@@ -481,13 +486,13 @@ std::shared_ptr<void> flash_attention_prepare(const GemmParams& g, uint32_t* sta
     FiniteParams& f = l->finite;
     memset(&f, 0, sizeof(f));
     f.n = p.n;
-    f.key_blocks = p.key_blocks;
+    f.key_blocks = p.table_blocks;
     f.flags = (int32_t*)g.scratch;
     // an operand [batch, rows, k] as a 4-D map (K offset, row, x, y): a head split read in place as it is, a plain one with
     // x = the batch entry (bi = batch + 1: coordinates (bt, 0))
-    auto operand = [&](const GemmOperand4D& o, const void* base, int64_t rows, int64_t cols, int64_t s_batch, int64_t s_row, int64_t s_col,
+    auto operand = [&](const GemmOperand4D& o, const void* base, int box_rows, int64_t rows, int64_t cols, int64_t s_batch, int64_t s_row, int64_t s_col,
                        bool mn_major, CUtensorMap* map, int32_t* bi, int scanned) {
-        int box[4] = {(int)elems, kFlRows, 1, 1};
+        int box[4] = {(int)elems, box_rows, 1, 1};
         int64_t dims[4] = {cols, rows, g.batch, 1}, strides[4] = {1, s_row, s_batch, align};
         if (o.enabled) {
             if (o.kd != cols || o.rd < rows || o.strides[0] != 1) return false;
@@ -509,11 +514,17 @@ std::shared_ptr<void> flash_attention_prepare(const GemmParams& g, uint32_t* sta
         else *map = tc_make_map(base, 4, dims, strides, box, true);
         return true;
     };
-    if (!operand(g.a4, g.a, g.m, g.k, g.sa[0], g.sa[1], g.sa[2], false, &l->map_q, &p.a_bi, -1)) return nullptr;
-    if (!operand(g.b4, g.b, g.n, g.k, g.sb[0], g.sb[2], g.sb[1], false, &l->map_k, &p.b_bi, 0)) return nullptr;
-    if (!operand(g.v4, g.values, g.n, g.values_cols, g.values_strides[0], g.values_strides[1], g.values_strides[2], true, &l->map_v, &p.v_bi, 1))
+    if (!operand(g.a4, g.a, kFlRows, g.m, g.k, g.sa[0], g.sa[1], g.sa[2], false, &l->map_q, &p.a_bi, -1)) return nullptr;
+    if (!operand(g.b4, g.b, kFlKeys, g.n, g.k, g.sb[0], g.sb[2], g.sb[1], false, &l->map_k, &p.b_bi, 0)) return nullptr;
+    if (!operand(g.v4, g.values, kFlKeys, g.n, g.values_cols, g.values_strides[0], g.values_strides[1], g.values_strides[2], true, &l->map_v, &p.v_bi, 1))
         return nullptr;
-    l->smem_bytes = flash_smem_bytes(g.k, g.values_cols, half);
+    // two buffers of each where two CTAs of it share an SM (or none would with one)
+    const int half_sm = 113 * 1024, whole_sm = 227 * 1024;
+    p.key_slots = p.value_slots = 1;
+    const int limit = flash_smem_bytes(g.k, g.values_cols, half, 1, 1) <= half_sm ? half_sm : whole_sm;
+    if (flash_smem_bytes(g.k, g.values_cols, half, 1, 2) <= limit) p.value_slots = 2;
+    if (flash_smem_bytes(g.k, g.values_cols, half, 2, p.value_slots) <= limit) p.key_slots = 2;
+    l->smem_bytes = flash_smem_bytes(g.k, g.values_cols, half, p.key_slots, p.value_slots);
     l->grid = (unsigned)(g.batch * p.m_tiles);
     return l;
 }
@@ -536,7 +547,7 @@ int flash_attention_launch(const void* launch, cudaStream_t stream) {
         }
     }
     if (l.finite.flags) {
-        const dim3 blocks((unsigned)l.p.batch * (unsigned)l.p.key_blocks);
+        const dim3 blocks((unsigned)l.p.batch * (unsigned)l.p.table_blocks);
         launch_pdl(l.half ? flash_finite_kernel<true> : flash_finite_kernel<false>, blocks, dim3(256), (size_t)0, stream, l.finite);
     }
     const dim3 grid(l.grid), block(kFlThreads);
