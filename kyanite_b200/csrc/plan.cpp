@@ -2320,6 +2320,7 @@ class Planner {
                                      !(opts_.flags & KN_FLAG_NO_PERSISTENT_GEMM);
         const bool long_k = C * R * S >= 2048 && (may_be_implicit || N * OH * OW * R * S * C * 4 <= (256ll << 20));
         if (!strided && !few_positions && !pointwise && !long_k) return std::nullopt;
+        if (pointwise && !strided && py == 0 && px == 0 && becomes_chain_head(ci, x)) return std::nullopt;
         if (N < 1 || N > 65535 || OH * OW < 64 || K < 16 || K % 4 != 0 || C < 1 || R * S > 64) return std::nullopt;
         if (2.0 * (double)N * OH * OW * K * C * R * S < 2e8) return std::nullopt;
         const ValueInfo& wi = g_.values[ci.inputs[1]];
@@ -2853,6 +2854,35 @@ class Planner {
                 if (t.buf == buf) return true;
         }
         return false;
+    }
+
+    // Will fuse_conv_chains take this 1x1 convolution of `x` into the chain that produces x?  As a matmul of its own it would read the
+    // trunk's result, which then had to be stored as well, and get a transposing copy behind it (tower of 128 channels, 2048 boards:
+    // 25 + 8 us of a 1.5 ms call).  (The last two steps that lead to x are a chain's layers, and all 1x1 convolutions of x fit its
+    // pointwise layer.)
+    bool becomes_chain_head(const ValueInfo& ci, const PlanTensor& x) const {
+        if (opts_.math_mode != KN_MATH_TF32 || (opts_.flags & KN_FLAG_NO_CONV_CHAIN)) return false;
+        const Step* last = nullptr;
+        const Step* before = nullptr;
+        PlanTensor wanted = x;
+        for (size_t i = plan_.steps.size(); i-- > 0 && !before;) {
+            const Step& s = plan_.steps[i];
+            if (s.kind != StepKind::Conv || s.operands.size() < 3 || !s.operands[2].same_storage(wanted)) continue;
+            ChainLayer l;
+            if (!chain_candidate(s, l)) return false;
+            (last ? before : last) = &s;
+            wanted = s.operands[0];
+        }
+        if (!before) return false;
+        int64_t channels = 0;
+        for (int u : users_[ci.inputs[0]]) {
+            const ValueInfo& o = g_.values[u];
+            if (o.op != OpKind::Conv || o.inputs[0] != ci.inputs[0]) continue;
+            const ValueInfo& f = g_.values[o.inputs[1]];
+            if (f.op != OpKind::Constant || shape_of(o.inputs[1])[2] != 1 || shape_of(o.inputs[1])[3] != 1) return false;
+            channels += shape_of(o.inputs[1])[0];
+        }
+        return channels <= 128;
     }
 
     void fuse_conv_chains() {

@@ -3,6 +3,7 @@ layout changes.  Bounds: those of test_conv_chain.py (operands rounded to TF32, 
 import numpy as np
 import pytest
 
+from kyanite_b200.configs import resnet_tower
 from kyanite_b200.executor import MATH_TF32, plan_describe
 from kyanite_b200.graph import BATCH, Graph, shape
 from oracle.cpu_eval import assert_tensors_match, cpu_eval_graph
@@ -67,3 +68,12 @@ def test_infinity_and_nan_stay_in_their_image():
     others = [i for i in range(9) if i not in (4, 7)]
     np.testing.assert_array_equal(got[others], clean[others])
     assert not np.isfinite(got[4][:, 2:5, 2:5]).any() and not np.isfinite(got[7][:, 0:2, 6:8]).any()
+
+
+def test_heads_of_large_batches_join_the_chain():
+    """A 1x1 convolution large enough to be a matmul of its own stays with the chain whose result it reads, if all of them fit."""
+    g, _ = resnet_tower()
+    d = steps(plan_describe(g, 2048, MATH_TF32))
+    assert "heads=73+32 (trunk result not stored)" in d[0] and len(d) == 5
+    d = steps(plan_describe(tower_with_heads(128, 8, 8, 8, [100, 40], [False] * 2), 2048, MATH_TF32))
+    assert len([l for l in d if "conv via im2col" in l]) == 2 and "heads=" not in d[0]
