@@ -39,6 +39,7 @@ SOURCES = [
     "kernels/gemm_persistent.cu",
     "kernels/attn_softmax.cu",
     "kernels/attention.cu",
+    "kernels/conv_chain_exact.cu",
     "kernels/flash.cu",
 ]
 

@@ -219,7 +219,7 @@ struct Executor {
                     break;
                 default: fail(KN_ERR_INTERNAL, "unknown step kind");
             }
-            if (s.tensor_core)
+            if (s.tensor_core || s.kind == StepKind::ConvChain)
                 tc_prepare_step(s, status_dev, plan->opts.flags, (plan->opts.flags & KN_FLAG_TRACE_GEMM) ? status_host + 4 : nullptr);
             launches += s.launches;
         }

@@ -213,7 +213,8 @@ struct ConvChainParams {
     const float* tiles;   // filter tiles [tile][128 output channels][32 input channels] in the 128-byte-swizzled
                           // order of shared memory, TF32, layers back to back;
                           // within a layer tile = tap * c_blocks + channel block, tap = r * 3 + s
-                          // (pair: [CTA of the pair][channel block][tap][its half of the output channels][32])
+                          // (pair: [CTA of the pair][channel block][tap][its half of the output channels][32];
+                          // exact: [CTA of the cluster][input channel, padded to whole chunks][tap][its output channels], f32)
     const float* bias;    // [layer][128]
     int32_t pair;         // the kernel on CTA pairs takes it
     int32_t n, c_in, k, h, w;
@@ -249,6 +250,7 @@ struct AllReduceParams {
     uint8_t dtype;     // DType: F32 or F16
 };
 
+    int32_t exact;        // the one in exact f32 does
 // ---- small transfers between device memory and pinned host memory (kernels/host_copy.cu)
 constexpr int kMaxHostCopies = 8;
 struct HostCopyParams {

@@ -699,8 +699,8 @@ struct TcLaunch {
     ConvClParams cl;
     dim3 grid;
     int smem_bytes;
-    std::shared_ptr<void> chain;  // ConvChain step: launch data of kernels/conv_chain.cu
-    bool chain_pair = false;      // (of kernels/conv_chain_pair.cu)
+    std::shared_ptr<void> chain;  // ConvChain step: launch data of kernels/conv_chain*.cu
+    int (*launch_chain)(const void*, cudaStream_t) = nullptr;
     std::shared_ptr<void> gemm_p; // matmul taken by the persistent kernel (kernels/gemm_persistent.cu)
     std::shared_ptr<void> gemm_s; // matmul of few tiles, K slices summed inside a cluster (kernels/gemm_persistent.cu)
     std::shared_ptr<void> attn;   // matmul with a row softmax (kernels/attn_softmax.cu)
@@ -897,8 +897,10 @@ bool tc_conv_tile(int oh, int ow, int* wb, int* hb, int* nb) {
 void tc_prepare_step(Step& step, uint32_t* status_word, int flags, uint32_t* trace_words) {
     auto launch = std::make_shared<TcLaunch>();
     if (step.kind == StepKind::ConvChain) {
-        launch->chain = step.chain.pair ? chain_pair_prepare(step.chain, status_word) : chain_prepare(step.chain, status_word);
-        launch->chain_pair = step.chain.pair != 0;
+        launch->chain = step.chain.exact  ? chain_exact_prepare(step.chain, status_word)
+                        : step.chain.pair ? chain_pair_prepare(step.chain, status_word)
+                                          : chain_prepare(step.chain, status_word);
+        launch->launch_chain = step.chain.exact ? chain_exact_launch : (step.chain.pair ? chain_pair_launch : chain_launch);
         step.tc = launch;
         return;
     }
@@ -1125,7 +1127,7 @@ static int launch_splitk_reduce(const SplitKReduceParams& r, cudaStream_t stream
 
 int tc_launch_step(const Step& step, cudaStream_t stream) {
     const TcLaunch& l = *step.tc;
-    if (l.chain) return l.chain_pair ? chain_pair_launch(l.chain.get(), stream) : chain_launch(l.chain.get(), stream);
+    if (l.chain) return l.launch_chain(l.chain.get(), stream);
     if (l.flash) return flash_attention_launch(l.flash.get(), stream);
     if (l.attention) return attention_launch(l.attention.get(), stream);
     if (l.attn) return attn_softmax_launch(l.attn.get(), stream);

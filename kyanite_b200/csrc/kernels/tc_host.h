@@ -56,6 +56,9 @@ int chain_launch(const void* launch, cudaStream_t stream);
 // The same on CTA pairs (kernels/conv_chain_pair.cu), for ConvChainParams::pair.
 std::shared_ptr<void> chain_pair_prepare(const ConvChainParams& c, uint32_t* status_word);
 int chain_pair_launch(const void* launch, cudaStream_t stream);
+// In exact f32 on a cluster per image (kernels/conv_chain_exact.cu), for ConvChainParams::exact.
+std::shared_ptr<void> chain_exact_prepare(const ConvChainParams& c, uint32_t* status_word);
+int chain_exact_launch(const void* launch, cudaStream_t stream);
 long long* chain_trace_table(int n_layers);   // pinned words for KN_CHAIN_TRACE, else null
 
 }  // namespace kn

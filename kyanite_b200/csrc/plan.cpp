@@ -2811,17 +2811,21 @@ class Planner {
         if (w.ss.strides[0] != c_pad || (c.c > 1 && w.ss.strides[1] != 1) || w.ss.strides[2] != 3 * c.k * c_pad ||
             w.ss.strides[3] != c.k * c_pad)
             return false;
-        for (size_t o = 3; o < s.operands.size(); o++) {
-            const PlanTensor& a = s.operands[o];
-            const BufferInfo& ab = plan_.buffers[a.buf];
-            if (per_channel(a) && ab.kind == BufKind::Const && ab.host_data != nullptr && l.bias_operand < 0)
-                l.bias_operand = (int)o;
-            else if (l.res_operand < 0)
-                l.res_operand = (int)o;
-            else
-                return false;
-        }
-        return true;
+        return chain_addends(s, l);
+    }
+
+    // The same for exact f32, whose filters are planner-made constants [3][3][C][K] (filter_rows)
+    bool exact_chain_candidate(const Step& s, ChainLayer& l) const {
+        if (s.kind != StepKind::Conv || s.tensor_core) return false;
+        const ConvParams& c = s.conv;
+        if (c.r != 3 || c.s != 3 || c.pad_y != 1 || c.pad_x != 1 || c.stride_y != 1 || c.stride_x != 1 || c.oh != c.h || c.ow != c.w) return false;
+        if (c.act != (int32_t)Activation::None && c.act != (int32_t)Activation::Relu) return false;
+        if (c.k % 8 != 0 || s.operands[0].dtype != DType::F32 || s.operands[2].dtype != DType::F32) return false;
+        const PlanTensor& w = s.operands[1];
+        const BufferInfo& wb = plan_.buffers[w.buf];
+        if (wb.kind != BufKind::Const || !wb.owned || w.offset != 0 || (int64_t)wb.owned->size() != (int64_t)9 * c.c * c.k * 4) return false;
+        if (w.ss.strides[0] != 1 || (c.c > 1 && w.ss.strides[1] != c.k) || w.ss.strides[2] != (int64_t)3 * c.c * c.k || w.ss.strides[3] != (int64_t)c.c * c.k) return false;
+        return chain_addends(s, l);
     }
 
     // A later 1x1 convolution of the chain's last result, with constant filter and bias: it can run as
@@ -2886,7 +2890,7 @@ class Planner {
     }
 
     void fuse_conv_chains() {
-        if (opts_.math_mode != KN_MATH_TF32 || (opts_.flags & KN_FLAG_NO_CONV_CHAIN)) return;
+        if (opts_.flags & KN_FLAG_NO_CONV_CHAIN) return;
         std::vector<Step>& steps = plan_.steps;
         std::vector<Step> result;
         std::vector<uint8_t> consumed(steps.size(), 0);   // 1x1 convolutions that became heads of an earlier chain
@@ -2901,7 +2905,10 @@ class Planner {
             for (size_t j = i; j < steps.size() && layers.size() < (size_t)kMaxChainLayers; j++) {
                 ChainLayer l;
                 l.step = j;
-                if (!chain_candidate(steps[j], l)) break;
+                if (!(exact ? exact_chain_candidate(steps[j], l) : chain_candidate(steps[j], l))) break;
+                if (exact && (steps[j].conv.k != steps[i].conv.k ||
+                              !conv_chain_exact_geometry(steps[i].conv.h, steps[i].conv.w, steps[i].conv.n, steps[i].conv.c, steps[i].conv.k, nullptr)))
+                    break;
                 if (!layers.empty()) {
                     const Step& prev = steps[j - 1];
                     if (!steps[j].operands[0].same_storage(prev.operands[2])) break;
@@ -2919,6 +2926,21 @@ class Planner {
                     if (layers[a].res_operand >= 0 && !s.operands[layers[a].res_operand].same_storage(held)) break;
                     for (size_t b = a + 1; b < layers.size(); b++) {
                         const Step& later = steps[layers[b].step];
+    // a constant per channel is the bias, one other addend the skip tensor
+    bool chain_addends(const Step& s, ChainLayer& l) const {
+        for (size_t o = 3; o < s.operands.size(); o++) {
+            const PlanTensor& a = s.operands[o];
+            const BufferInfo& ab = plan_.buffers[a.buf];
+            if (per_channel(a) && ab.kind == BufKind::Const && ab.host_data != nullptr && l.bias_operand < 0)
+                l.bias_operand = (int)o;
+            else if (l.res_operand < 0)
+                l.res_operand = (int)o;
+            else
+                return false;
+        }
+        return true;
+    }
+
                         if (layers[b].res_operand >= 0 && later.operands[layers[b].res_operand].same_storage(s.operands[2])) hold[a] = 1;
                     }
                     if (hold[a]) held = s.operands[2];
@@ -2938,7 +2960,7 @@ class Planner {
                 }
                 // the tensor held at the end must not be required after a cut (it never is: cuts only shorten)
             }
-            if (len < 2) {
+            if (len < (exact ? 4u : 2u)) {   // (an exact chain takes some 8 us to begin: cluster, zeroed activations, input)
                 result.push_back(std::move(steps[i]));
                 i++;
                 continue;
@@ -2946,7 +2968,7 @@ class Planner {
             // 1x1 convolutions of the chain's result anywhere later in the plan become heads of a pointwise
             // last layer (their inputs are the result and constants, so they can run this early)
             std::vector<ChainHead> heads;
-            if (len < (size_t)kMaxChainLayers) {
+            if (!exact && len < (size_t)kMaxChainLayers) {
                 const Step& last = steps[layers[len - 1].step];
                 int channels = 0;
                 for (size_t j = layers[len - 1].step + 1; j < steps.size() && heads.size() < (size_t)kMaxChainHeads; j++) {
@@ -2989,7 +3011,7 @@ class Planner {
         const Step& last = steps[layers[len - 1].step];
         Step s;
         s.kind = StepKind::ConvChain;
-        s.tensor_core = true;
+        s.tensor_core = first.tensor_core;
         s.value = last.value;
         ConvChainParams& p = s.chain;
         p.n = first.conv.n;
@@ -3017,37 +3039,44 @@ class Planner {
         int head_channels = 0;
         for (auto& h : heads) head_channels += steps[h.step].conv.k;
         ChainPairGeometry pair;
-        p.pair = tc_chain_pair_geometry(p.h, p.w, p.n, blocks, p.k, head_channels, &pair);
+        ChainExactGeometry ex;
+        p.exact = !first.tensor_core;
+        p.pair = !p.exact && tc_chain_pair_geometry(p.h, p.w, p.n, blocks, p.k, head_channels, &pair);
+        if (p.exact) KN_CHECK(conv_chain_exact_geometry(p.h, p.w, p.n, p.c_in, p.k, &ex), KN_ERR_INTERNAL, "exact convolution chain does not fit");
         // filter tiles (already TF32, zero beyond the real channels), stored exactly as they sit in shared memory (rows of 128
         // bytes whose 16-byte chunks are XOR-swizzled with the row number), so that a linear bulk copy delivers them
-        std::vector<int64_t> layer_rows(n_layers + 1, 0);   // first row of 32 floats of a layer
+        std::vector<int64_t> layer_at(n_layers + 1, 0);   // first value of a layer
+            const bool exact = steps[i].kind == StepKind::Conv && !steps[i].tensor_core;
         auto tile_rows = [&](size_t a) { return p.pair ? (a < len ? pair.n_trunk : pair.n_last) : 128; };
-        for (size_t a = 0; a < n_layers; a++) layer_rows[a + 1] = layer_rows[a] + (int64_t)(a < len ? 9 : 1) * p.c_blocks[a] * tile_rows(a);
-        const int64_t n_rows = layer_rows[n_layers];
+        auto padded_inputs = [&](size_t a) { return (int64_t)((a == 0 ? p.c_in : p.k) + ex.chunk - 1) / ex.chunk * ex.chunk; };
+        for (size_t a = 0; a < n_layers; a++)
+            layer_at[a + 1] = layer_at[a] + (p.exact ? padded_inputs(a) * 9 * p.k : (int64_t)(a < len ? 9 : 1) * p.c_blocks[a] * tile_rows(a) * 32);
         // where input channel `ch` of output channel `k` at a tap goes
-        auto tile_pos = [&](size_t a, int tap, int k, int ch) {
+        auto tile_pos = [&](size_t a, int tap, int k, int ch) -> int64_t {
+            if (p.exact) return layer_at[a] + (((k / ex.cols) * padded_inputs(a) + ch) * 9 + tap) * ex.cols + k % ex.cols;
             const int taps = a < len ? 9 : 1, cb = ch / 32, col = ch % 32;
-            int64_t row;
+            int64_t row;   // (tiles begin at multiples of eight rows)
             if (p.pair) {
                 const int half = tile_rows(a) / 2;
-                row = layer_rows[a] + ((int64_t)((k / half) * p.c_blocks[a] + cb) * taps + tap) * half + k % half;
+                row = ((int64_t)((k / half) * p.c_blocks[a] + cb) * taps + tap) * half + k % half;
             } else {
-                row = layer_rows[a] + (int64_t)(tap * p.c_blocks[a] + cb) * 128 + k;
+                row = (int64_t)(tap * p.c_blocks[a] + cb) * 128 + k;
             }
-            return row * 32 + ((((col >> 2) ^ (int)(row & 7)) << 2) | (col & 3));   // (tiles begin at multiples of eight rows)
+            return layer_at[a] + row * 32 + ((((col >> 2) ^ (int)(row & 7)) << 2) | (col & 3));
         };
-        auto tiles = std::make_shared<std::vector<uint8_t>>((size_t)n_rows * 32 * 4, 0);
+        auto tiles = std::make_shared<std::vector<uint8_t>>((size_t)layer_at[n_layers] * 4, 0);
         auto bias = std::make_shared<std::vector<uint8_t>>(n_layers * 128 * 4, 0);
         float* tp = (float*)tiles->data();
         float* bp = (float*)bias->data();
         for (size_t a = 0; a < len; a++) {
             const Step& st = steps[layers[a].step];
             const ConvParams& c = st.conv;
-            const int64_t c_pad = (c.c + 3) / 4 * 4;
-            const float* src = (const float*)plan_.buffers[st.operands[1].buf].owned->data();   // [tap][K][c_pad]
+            const float* src = (const float*)plan_.buffers[st.operands[1].buf].owned->data();   // [tap][K][C, padded to 4]; exact: [tap][C][K]
+            const int64_t tap_stride = p.exact ? (int64_t)c.c * c.k : (int64_t)c.k * ((c.c + 3) / 4 * 4);
+            const int64_t k_stride = p.exact ? 1 : (c.c + 3) / 4 * 4, c_stride = p.exact ? c.k : 1;
             for (int tap = 0; tap < 9; tap++)
                 for (int k = 0; k < c.k; k++)
-                    for (int ch = 0; ch < c.c; ch++) tp[tile_pos(a, tap, k, ch)] = src[((int64_t)tap * c.k + k) * c_pad + ch];
+                    for (int ch = 0; ch < c.c; ch++) tp[tile_pos(a, tap, k, ch)] = src[tap * tap_stride + k * k_stride + ch * c_stride];
             if (layers[a].bias_operand >= 0) {
                 const PlanTensor& b = st.operands[layers[a].bias_operand];
                 const float* bsrc = (const float*)plan_.buffers[b.buf].host_data;
@@ -3085,7 +3114,7 @@ class Planner {
             s.flops += st.flops;
         }
         p.head_begin[heads.size()] = row0;
-        PlanTensor t_tiles = alloc_const({n_rows, 32}, DType::F32, s.value, nullptr, tiles);
+        PlanTensor t_tiles = alloc_const({layer_at[n_layers]}, DType::F32, s.value, nullptr, tiles);
         PlanTensor t_bias = alloc_const({(int64_t)n_layers, 128}, DType::F32, s.value, nullptr, bias);
         // operand 1 is the trunk's result; when nothing reads it, it is neither stored nor allocated (the slot
         // then repeats the first head's output)
@@ -3100,7 +3129,7 @@ class Planner {
             p.s_out[d] = last.operands[2].ss.strides[d];
         }
         s.desc = "convchain layers=" + std::to_string(len) + " n=" + std::to_string(p.n) + " c=" + std::to_string(p.c_in) + " hw=" +
-                 std::to_string(p.h) + "x" + std::to_string(p.w) + " k=" + std::to_string(p.k) + " rs=3x3 tf32" + (p.pair ? " on CTA pairs" : "");
+                 std::to_string(p.h) + "x" + std::to_string(p.w) + " k=" + std::to_string(p.k) + " rs=3x3" + (p.exact ? " exact, " + std::to_string(ex.cluster) + " CTAs per image" : p.pair ? " tf32 on CTA pairs" : " tf32");
         if (!heads.empty()) {
             s.desc += " heads=";
             for (size_t hi = 0; hi < heads.size(); hi++) s.desc += (hi ? "+" : "") + std::to_string(p.head_begin[hi + 1] - p.head_begin[hi]);

@@ -65,4 +65,15 @@ struct ChainPairGeometry {
 // False if they do not fit.  `k`: output channels of the 3x3 layers; `head_channels`: of the pointwise last layer, 0 if there is none.
 bool tc_chain_pair_geometry(int h, int w, int64_t n_img, int blocks, int k, int head_channels, ChainPairGeometry* out);
 
+// Exact f32 chains (kernels/conv_chain_exact.cu): a cluster of CTAs per image, each with `cols` of the output channels.
+struct ChainExactGeometry {
+    int cluster, cols, items, k_groups;   // items: (image row, 8 output channels) of a CTA; k_groups of threads share the input channels
+    int chunk, slots;                     // input channels of a weight chunk; chunks in flight
+    int channels, act_floats;             // input channels that shared memory holds, floats of one
+    int units;                            // results of a thread, in groups of four
+    int smem_bytes;
+};
+// False where the layers are better launched one by one: images that do not fit, or more of them than the chip holds clusters.
+bool conv_chain_exact_geometry(int h, int w, int64_t n_img, int c_in, int k, ChainExactGeometry* out);
+
 }  // namespace kn

@@ -1,0 +1,51 @@
+"""Runs of 3x3 convolutions in exact f32 as one launch (kernels/conv_chain_exact.cu), at every number of CTAs per image."""
+import numpy as np
+import pytest
+
+from kyanite_b200.executor import FLAG_NO_CONV_CHAIN, MATH_F32, MATH_TF32, plan_describe
+from oracle.cpu_eval import cpu_eval_graph
+from test_conv_chain import rng, steps, tower
+
+
+def chains(g, batch, mode=MATH_F32, flags=0):
+    return [l for l in steps(plan_describe(g, batch, mode, flags=flags)) if "ConvChain" in l]
+
+
+@pytest.mark.parametrize("channels,batch,ctas", [(128, 7, 16), (128, 9, 8), (128, 33, 4), (128, 45, 2), (128, 74, 2), (128, 148, 1), (64, 1, 8), (64, 16, 4), (32, 34, 2)])
+def test_ctas_per_image(channels, batch, ctas):
+    g = tower(channels, 2, 8, 8, 21)
+    line, = chains(g, batch)
+    assert f"exact, {ctas} CTAs per image" in line and "/tc" not in line
+    assert not chains(g, batch, flags=FLAG_NO_CONV_CHAIN)
+
+
+def test_route():
+    assert not chains(tower(128, 2, 8, 8, 21), 149)                          # more images than one round
+    assert not chains(tower(128, 2, 8, 8, 21), 40)                           # wide layers, a round of which little is used
+    assert not chains(tower(64, 1, 8, 8, 21), 4)                             # three layers
+    assert chains(tower(64, 2, 8, 8, 21), 1, MATH_TF32)                      # fewer than 128 positions keep f32 operands
+    assert not chains(tower(36, 2, 8, 8, 21), 4)                             # channels that are no multiple of eight
+    assert not chains(tower(64, 2, 9, 9, 21), 4)                             # rows that are too long
+
+
+CASES = [  # channels, input channels, blocks, h, w, batch
+    (128, 21, 2, 8, 8, 6), (128, 128, 2, 8, 8, 7), (128, 5, 2, 8, 8, 9), (128, 21, 2, 8, 8, 21), (128, 21, 2, 8, 8, 50), (128, 3, 2, 8, 8, 110),
+    (64, 21, 2, 7, 7, 2), (64, 64, 2, 8, 8, 12), (64, 9, 2, 16, 8, 3), (64, 1, 2, 8, 8, 75), (96, 30, 2, 7, 7, 33), (32, 100, 2, 8, 7, 20), (40, 1, 2, 5, 8, 90),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("channels,c_in,blocks,h,w,batch", CASES)
+@pytest.mark.parametrize("residual", [True, False])
+def test_matches_oracle(channels, c_in, blocks, h, w, batch, residual):
+    from kyanite_b200.executor import CudaExecutor
+    g = tower(channels, blocks, h, w, c_in, seed=channels + h, residual=residual, relu=residual)
+    if not chains(g, batch):
+        pytest.skip("launched one by one")
+    x = rng(c_in).standard_normal((batch, c_in, h, w)).astype(np.float32)
+    expected, = cpu_eval_graph(g.to_bytes(), batch, [x])
+    with CudaExecutor(0, g, batch, math_mode=MATH_F32) as ex:
+        got, = ex.evaluate([x])
+        # five layers of f32 sums of up to 1152 terms in another order: 1e-5 of the scale
+        assert np.abs(got.astype(np.float64) - expected).max() <= 1e-5 * np.abs(expected).max()
+        np.testing.assert_array_equal(got, ex.evaluate([x])[0])
