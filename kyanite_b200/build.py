@@ -36,10 +36,10 @@ SOURCES = [
     "kernels/contract_tc.cu",
     "kernels/conv_chain.cu",
     "kernels/conv_chain_pair.cu",
+    "kernels/conv_chain_exact.cu",
     "kernels/gemm_persistent.cu",
     "kernels/attn_softmax.cu",
     "kernels/attention.cu",
-    "kernels/conv_chain_exact.cu",
     "kernels/flash.cu",
 ]
 

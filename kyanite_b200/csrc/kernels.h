@@ -217,6 +217,7 @@ struct ConvChainParams {
                           // exact: [CTA of the cluster][input channel, padded to whole chunks][tap][its output channels], f32)
     const float* bias;    // [layer][128]
     int32_t pair;         // the kernel on CTA pairs takes it
+    int32_t exact;        // the one in exact f32 does
     int32_t n, c_in, k, h, w;
     int32_t n_layers;
     int64_t s_in[4], s_out[4];
@@ -250,7 +251,6 @@ struct AllReduceParams {
     uint8_t dtype;     // DType: F32 or F16
 };
 
-    int32_t exact;        // the one in exact f32 does
 // ---- small transfers between device memory and pinned host memory (kernels/host_copy.cu)
 constexpr int kMaxHostCopies = 8;
 struct HostCopyParams {

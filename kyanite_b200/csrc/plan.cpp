@@ -2796,6 +2796,21 @@ class Planner {
         return true;
     }
 
+    // a constant per channel is the bias, one other addend the skip tensor
+    bool chain_addends(const Step& s, ChainLayer& l) const {
+        for (size_t o = 3; o < s.operands.size(); o++) {
+            const PlanTensor& a = s.operands[o];
+            const BufferInfo& ab = plan_.buffers[a.buf];
+            if (per_channel(a) && ab.kind == BufKind::Const && ab.host_data != nullptr && l.bias_operand < 0)
+                l.bias_operand = (int)o;
+            else if (l.res_operand < 0)
+                l.res_operand = (int)o;
+            else
+                return false;
+        }
+        return true;
+    }
+
     bool chain_candidate(const Step& s, ChainLayer& l) const {
         if (s.kind != StepKind::Conv || !s.tensor_core) return false;
         const ConvParams& c = s.conv;
@@ -2902,6 +2917,7 @@ class Planner {
             }
             // longest run starting at i
             std::vector<ChainLayer> layers;
+            const bool exact = steps[i].kind == StepKind::Conv && !steps[i].tensor_core;
             for (size_t j = i; j < steps.size() && layers.size() < (size_t)kMaxChainLayers; j++) {
                 ChainLayer l;
                 l.step = j;
@@ -2926,21 +2942,6 @@ class Planner {
                     if (layers[a].res_operand >= 0 && !s.operands[layers[a].res_operand].same_storage(held)) break;
                     for (size_t b = a + 1; b < layers.size(); b++) {
                         const Step& later = steps[layers[b].step];
-    // a constant per channel is the bias, one other addend the skip tensor
-    bool chain_addends(const Step& s, ChainLayer& l) const {
-        for (size_t o = 3; o < s.operands.size(); o++) {
-            const PlanTensor& a = s.operands[o];
-            const BufferInfo& ab = plan_.buffers[a.buf];
-            if (per_channel(a) && ab.kind == BufKind::Const && ab.host_data != nullptr && l.bias_operand < 0)
-                l.bias_operand = (int)o;
-            else if (l.res_operand < 0)
-                l.res_operand = (int)o;
-            else
-                return false;
-        }
-        return true;
-    }
-
                         if (layers[b].res_operand >= 0 && later.operands[layers[b].res_operand].same_storage(s.operands[2])) hold[a] = 1;
                     }
                     if (hold[a]) held = s.operands[2];
@@ -3046,7 +3047,6 @@ class Planner {
         // filter tiles (already TF32, zero beyond the real channels), stored exactly as they sit in shared memory (rows of 128
         // bytes whose 16-byte chunks are XOR-swizzled with the row number), so that a linear bulk copy delivers them
         std::vector<int64_t> layer_at(n_layers + 1, 0);   // first value of a layer
-            const bool exact = steps[i].kind == StepKind::Conv && !steps[i].tensor_core;
         auto tile_rows = [&](size_t a) { return p.pair ? (a < len ? pair.n_trunk : pair.n_last) : 128; };
         auto padded_inputs = [&](size_t a) { return (int64_t)((a == 0 ? p.c_in : p.k) + ex.chunk - 1) / ex.chunk * ex.chunk; };
         for (size_t a = 0; a < n_layers; a++)
