@@ -27,6 +27,7 @@ SOURCES = [
     "host_copy.cpp",
     "executor.cu",
     "kernels/elementwise.cu",
+    "kernels/elementwise_fixed.cu",
     "kernels/rows.cu",
     "kernels/rows_f16.cu",
     "kernels/softmax_matmul.cu",

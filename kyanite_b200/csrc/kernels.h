@@ -54,6 +54,7 @@ struct ScalarParams {
     // documents the micro-op format); `n_regs` = number of spill slots it uses (0..8).
     int32_t n_micro, n_regs;
     ScalarInstr micro[SCALAR_MAX_INSTR + 2 * SCALAR_MAX_OPERANDS];
+    int32_t fixed;   // vec4 == 2 or 5: the number of the compiled program that this is (kernels/elementwise_fixed.cu), or 0
 };
 
 // ---- reduce: replaces autokernel/reduce.{rs,cu}
@@ -262,6 +263,9 @@ struct HostCopyParams {
 
 // All launchers enqueue on `stream` and return the cudaError_t of the launch as int.
 int launch_scalar(const ScalarParams& p, cudaStream_t stream);
+// Programs that are compiled (kernels/elementwise_fixed.cu): the number of the one that `p`'s accumulator program is, or 0
+int scalar_fixed_program(const ScalarParams& p, bool half);
+int launch_scalar_fixed(const ScalarParams& p, cudaStream_t stream);
 int launch_reduce(const ReduceParams& p, cudaStream_t stream);
 int launch_softmax(const RowParams& p, cudaStream_t stream);      // dispatches on p.half
 int launch_layernorm(const RowParams& p, cudaStream_t stream);

@@ -805,6 +805,7 @@ bool as_transpose(const ScalarParams& p, TransposeParams& q) {
 
 int launch_scalar(const ScalarParams& p, cudaStream_t stream) {
     if (p.total == 0) return 0;
+    if (p.fixed) return launch_scalar_fixed(p, stream);
     if (p.vec4 != 2 && p.vec4 != 4 && p.vec4 != 5) {
         TransposeParams q;
         if (as_transpose(p, q)) {
