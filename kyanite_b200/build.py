@@ -34,6 +34,7 @@ SOURCES = [
     "kernels/gather.cu",
     "kernels/host_copy.cu",
     "kernels/contract_simt.cu",
+    "kernels/dense_chain.cu",
     "kernels/contract_tc.cu",
     "kernels/conv_chain.cu",
     "kernels/conv_chain_pair.cu",

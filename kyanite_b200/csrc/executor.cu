@@ -107,7 +107,12 @@ struct Executor {
     cudaStream_t side_stream = nullptr;          // capture-time fork for early output copies
     bool profile = false;
     std::vector<float> step_us;
-    int launches = 0;
+    int launches = 0;                            // of the steps one by one
+    struct DenseChain {
+        size_t first, last;                      // steps
+        DenseChainParams p;
+    };
+    std::vector<DenseChain> dense_chains;        // steps that are launched together, in order
     Comm* comm = nullptr;              // not owned; AllReduce steps sum over its ranks (null: a world of one)
 
     ~Executor() {
@@ -223,6 +228,101 @@ struct Executor {
                 tc_prepare_step(s, status_dev, plan->opts.flags, (plan->opts.flags & KN_FLAG_TRACE_GEMM) ? status_host + 4 : nullptr);
             launches += s.launches;
         }
+        find_dense_chains();
+    }
+
+    // Runs of small dense layers (and the softmax behind them) that one kernel takes, see kernels/dense_chain.cu: plain f32
+    // matmuls with constant weights, each of which reads what the one before computed and nobody else reads.  The steps stay what
+    // they are for whoever launches or times them one by one.
+    void find_dense_chains() {
+        dense_chains.clear();
+        const std::vector<Step>& steps = plan->steps;
+        auto constant = [&](const PlanTensor& t) { return plan->buffers[t.buf].kind == BufKind::Const; };
+        auto is_layer = [&](const Step& s) {
+            if (s.kind != StepKind::Gemm) return false;
+            const GemmParams& g = s.gemm;
+            return g.batch == 1 && !g.half && !g.round_tf32 && g.conv_operand == 0 && g.row_softmax == 0 && !g.values && !g.a4.enabled && !g.b4.enabled &&
+                   !g.add2 && constant(s.operands[1]) && (g.add1 == nullptr || (g.s1[1] == 0 && constant(s.operands[3]))) &&
+                   (g.act == (int32_t)Activation::None || g.act == (int32_t)Activation::Relu) && g.m >= 1 && g.k >= 1 && g.k <= kDenseChainMaxK &&
+                   g.n >= 1 && g.n <= kDenseChainMaxN && (g.n == 1 || g.sc[2] == 1) && s.operands[2].dtype == DType::F32;
+        };
+        // step i's result is read by step i + 1 and by nothing else
+        auto read_next_only = [&](size_t i) {
+            const int buf = steps[i].operands[2].buf;
+            if (plan->buffers[buf].always_live) return false;
+            for (size_t j = 0; j < steps.size(); j++)
+                for (const PlanTensor& t : steps[j].operands)
+                    if (t.buf == buf && j != i && j != i + 1) return false;
+            return true;
+        };
+        auto bytes_of = [&](const PlanTensor& t) {   // [first, last) of what it covers
+            int64_t low = 0, high = 1;
+            for (int d = 0; d < t.ss.rank(); d++) {
+                const int64_t reach = (t.ss.shape[d] - 1) * t.ss.strides[d];
+                (reach < 0 ? low : high) += reach;
+            }
+            const uint8_t* at = device_ptr(t);
+            return std::make_pair(at + low * 4, at + high * 4);
+        };
+        for (size_t i = 0; i < steps.size(); i++) {
+            if (!is_layer(steps[i])) continue;
+            DenseChain c{};
+            DenseChainParams& p = c.p;
+            int weights = 0;
+            size_t j = i;
+            for (; j < steps.size() && p.n_layers < kDenseChainLayers && is_layer(steps[j]); j++) {
+                const GemmParams& g = steps[j].gemm;
+                if (j > i) {
+                    const GemmParams& before = steps[j - 1].gemm;
+                    if (g.a != before.c || g.m != before.m || g.k != before.n || (g.m > 1 && g.sa[1] != before.sc[1]) || (g.k > 1 && g.sa[2] != 1) || !read_next_only(j - 1)) break;
+                }
+                const int more = dense_chain_weights((int)g.k, (int)g.n);
+                if (weights + more > kDenseChainWeights) break;
+                DenseLayer& d = p.layer[p.n_layers++];
+                d.w = g.b, d.w_k = g.sb[1], d.w_n = g.sb[2];
+                d.bias = g.add1, d.bias_n = g.s1[2];
+                d.k = (int)g.k, d.n = (int)g.n;
+                d.relu = g.act == (int32_t)Activation::Relu;
+                d.at = weights;
+                weights += more;
+            }
+            if (p.n_layers == 0) continue;
+            c.first = i;
+            c.last = i + (size_t)p.n_layers - 1;
+            const GemmParams &g0 = steps[i].gemm, &g1 = steps[c.last].gemm;
+            p.in = g0.a, p.rows = g0.m, p.in_row = g0.sa[1], p.in_col = g0.sa[2];
+            p.out = g1.c, p.out_row = g1.sc[1];
+            const PlanTensor* result = &steps[c.last].operands[2];
+            if (c.last + 1 < steps.size() && steps[c.last + 1].kind == StepKind::Softmax && read_next_only(c.last)) {
+                const RowParams& r = steps[c.last + 1].row;
+                if (r.in0 == g1.c && !r.in1 && !r.half && r.rows == g1.m && r.len == g1.n && r.scale == 1.f && (r.len == 1 || (r.in_axis_stride == 1 && r.out_axis_stride == 1)) &&
+                    (r.rows == 1 || (r.outer_rank == 1 && r.in_strides[0] == g1.sc[1]))) {
+                    p.softmax = 1;
+                    p.out = r.out;
+                    p.out_row = r.rows == 1 ? 0 : r.out_strides[0];
+                    c.last++;
+                    result = &steps[c.last].operands[1];
+                }
+            }
+            // (the result may have been given the memory of what the first layer reads)
+            const auto in = bytes_of(steps[i].operands[0]), out = bytes_of(*result);
+            if (c.last == c.first || (in.first < out.second && out.first < in.second)) continue;
+            dense_chains.push_back(c);
+            i = c.last;
+        }
+    }
+
+    // Step i of the list, as part of a run of all of them
+    void launch_at(size_t i) {
+        for (const DenseChain& c : dense_chains) {
+            if (i < c.first || i > c.last) continue;
+            if (i == c.first) {
+                const int err = launch_dense_chain(c.p, stream);
+                if (err != 0) fail(KN_ERR_CUDA, std::string("launch of dense layers failed: ") + cudaGetErrorString((cudaError_t)err));
+            }
+            return;
+        }
+        launch_step(plan->steps[i]);
     }
 
     void launch_step(const Step& s) {
@@ -283,7 +383,7 @@ struct Executor {
                 cudaGraph_t graph = nullptr;
                 KN_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
                 try {
-                    for (const Step& s : plan->steps) launch_step(s);
+                    for (size_t i = 0; i < plan->steps.size(); i++) launch_at(i);
                 } catch (...) {
                     cudaStreamEndCapture(stream, &graph);
                     if (graph) cudaGraphDestroy(graph);
@@ -296,7 +396,7 @@ struct Executor {
             }
             KN_CUDA(cudaGraphLaunch(graph_exec, stream));
         } else {
-            for (const Step& s : plan->steps) launch_step(s);
+            for (size_t i = 0; i < plan->steps.size(); i++) launch_at(i);
         }
     }
 
@@ -392,7 +492,7 @@ struct Executor {
             launch_copies(up);
             bool forked = false;
             for (size_t i = 0; i < n_steps; i++) {
-                launch_step(plan->steps[i]);
+                launch_at(i);
                 if (i + 1 == n_steps) break;
                 for (size_t o = 0; o < producer.size(); o++) {
                     if (producer[o] != (int)i || bytes_out[o] == 0 || by_kernel[o]) continue;

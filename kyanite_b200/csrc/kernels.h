@@ -181,6 +181,24 @@ struct GemmParams {
     int64_t conv_strides[3];   // element strides of the image tensor: image, row, pixel (channels are contiguous)
 };
 
+// ---- a run of small dense layers and the softmax behind them in one launch (kernels/dense_chain.cu): the executor's way of
+// launching such Gemm and Softmax steps
+constexpr int kDenseChainLayers = 4, kDenseChainMaxK = 256, kDenseChainMaxN = 128, kDenseChainWeights = 7424;
+struct DenseLayer {
+    const float *w, *bias;            // [k][n] with strides w_k, w_n; bias or null
+    int64_t w_k, w_n, bias_n;
+    int32_t k, n, relu, at;           // at: where its weights lie in shared memory
+};
+struct DenseChainParams {
+    const float* in;                  // [rows][k of the first layer]
+    float* out;                       // [rows][n of the last], columns contiguous
+    int64_t rows, in_row, in_col, out_row;
+    int32_t n_layers, softmax;
+    DenseLayer layer[kDenseChainLayers];
+};
+int dense_chain_weights(int k, int n);   // floats of shared memory that a layer's weights take
+int launch_dense_chain(const DenseChainParams& p, cudaStream_t stream);
+
 // ---- 2D convolution (cross-correlation, zero padding) with fused epilogue
 // out = act(conv(in, filter) + add1 + add2); replaces cudnnConvolutionBiasActivationForward
 // (kn-cuda-sys/src/wrapper/operation.rs:162-240).

@@ -1,0 +1,80 @@
+"""Small dense layers that follow one another, and a softmax behind them, in one launch (kernels/dense_chain.cu): the executor's way
+of running such steps, which the plan still lists one by one.  It computes in f32 whatever the mode, so in the default mode, where
+64 rows and more would have their operands rounded to 11 bits, results at f32's precision also show that it ran."""
+import numpy as np
+import pytest
+
+from kyanite_b200.executor import MATH_F32, MATH_TF32
+from kyanite_b200.graph import BATCH, Graph, UnaryOp, shape
+
+
+def rng(seed):
+    return np.random.Generator(np.random.PCG64(seed))
+
+
+def layers(widths, softmax, bias=True, seed=0, probe=None):
+    r = rng(seed)
+    g = Graph()
+    y = x = g.input(shape(BATCH, widths[0]))
+    weights = []
+    for i, (k, n) in enumerate(zip(widths, widths[1:])):
+        w, b = (r.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32), r.standard_normal((1, n)).astype(np.float32)
+        weights.append((w, b if bias else np.zeros((1, n), np.float32)))
+        y = g.linear(y, g.constant_tensor(w))
+        if bias:
+            y = g.add(y, g.constant_tensor(b))
+        if i + 2 < len(widths):
+            y = g.relu(y)
+        if probe == i:
+            g.output(g.unary(UnaryOp.TANH, y))
+    g.output(g.softmax(y, 1) if softmax else y)
+    return g, weights
+
+
+def want(x, weights, softmax):
+    y = x.astype(np.float64)
+    for i, (w, b) in enumerate(weights):
+        y = y @ w.T.astype(np.float64) + b
+        if i + 1 < len(weights):
+            y = np.maximum(y, 0)
+    if softmax:
+        y = np.exp(y - y.max(1, keepdims=True))
+        y /= y.sum(1, keepdims=True)
+    return y
+
+
+CASES = [  # widths of the layers, softmax, bias
+    ([16, 32, 32, 4], True, True), ([256, 3], True, True), ([5, 9, 8, 1], False, True), ([1, 96, 33], True, False), ([7, 31, 64, 8, 2], True, True),
+    ([20, 8, 40], False, True), ([33, 100], True, True),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 7, 64, 2369])
+@pytest.mark.parametrize("widths,softmax,bias", CASES)
+@pytest.mark.parametrize("mode", [MATH_F32, MATH_TF32])
+def test_values(rows, widths, softmax, bias, mode):
+    from kyanite_b200.executor import CudaExecutor
+    g, weights = layers(widths, softmax, bias, seed=len(widths))
+    x = rng(rows).standard_normal((rows, widths[0])).astype(np.float32)
+    expected = want(x, weights, softmax)
+    with CudaExecutor(0, g, rows, math_mode=mode) as ex:
+        got, = ex.evaluate([x])
+        # a few layers of f32 sums of at most 256 terms
+        assert np.abs(got - expected).max() <= 4e-6 * np.abs(expected).max()
+        ex.set_profile(True)                       # (one by one: the steps themselves)
+        alone, = ex.evaluate([x])
+        ex.set_profile(False)
+        assert np.abs(alone - expected).max() <= 4e-3 * np.abs(expected).max()
+        np.testing.assert_array_equal(got, ex.evaluate([x])[0])
+
+
+@pytest.mark.gpu
+def test_a_result_that_is_read_elsewhere_is_stored():
+    from kyanite_b200.executor import CudaExecutor
+    g, weights = layers([16, 32, 32, 4], True, probe=1)
+    x = rng(1).standard_normal((9, 16)).astype(np.float32)
+    with CudaExecutor(0, g, 9, math_mode=MATH_F32) as ex:
+        hidden, got = ex.evaluate([x])
+    h = np.tanh(np.maximum(want(x, weights[:2], False), 0))
+    assert np.abs(hidden - h).max() <= 4e-6 and np.abs(got - want(x, weights, True)).max() <= 4e-6
