@@ -5,7 +5,7 @@
 // the pipeline, the shared-memory layout and the operand descriptors are the same.
 //
 // Compared with the one-tile-per-CTA kernel in contract_tc.cu, a CTA here stays on its SM and walks over
-// output tiles, and tensor memory holds TWO accumulators: while the four epilogue warps drain tile i
+// output tiles, and tensor memory holds TWO accumulators: while the epilogue warps drain tile i
 // (tcgen05.ld -> addends / activation -> swizzled staging tile in shared memory -> bulk tensor store),
 // the producer is already loading and the MMA thread already multiplying tile i + 1.  For the short-K
 // shapes of transformer layers (K = 768: 24 K-blocks per tile) fill and drain were most of a tile's time.
@@ -14,7 +14,12 @@
 //                   swizzle, rounded to TF32 by the copy engine), ring of stages with full / empty mbarriers
 //   warp 1, a lane  MMA issuer: four tcgen05.mma.kind::tf32 (K = 8) per stage into accumulator `tile & 1`;
 //                   waits for that accumulator to be drained, signals it full with tcgen05.commit
-//   warps 2..5      epilogue: thread <-> accumulator lane <-> output row; 32 columns at a time
+//   warps 2..9      epilogue: two groups of four, thread <-> accumulator lane <-> output row; the groups take 32 columns each in
+//                   turn.  One group is as fast while the next tile's MMAs hide it; where a CTA has few tiles or the epilogue
+//                   computes (GELU) it is not: 16384 x 768 x 768 + bias 38.8 us with one group and 36.5 with two, 16384 x 3072 x
+//                   768 + GELU 136.9 and 129.8, 2048 x 4096 x 4096 of halves 51.9 and 51.3 (without an epilogue to speak of, 2048 x
+//                   11008 x 4096 of halves, 129.8 and 130.3).  One warp of a group polls for the accumulator, the rest sleep at
+//                   a barrier: with all of them polling, long reductions lost 1% to the power it took.
 //
 // Large matmuls with a long reduction run on CTA PAIRS (template parameter PAIR, clusters of two): `cta_group::2`
 // instructions compute a 256 x BN tile on two SMs, each CTA loading its own 128 rows of A and half of B (see the
@@ -47,7 +52,8 @@ namespace {
 
 using namespace tcp;
 
-constexpr int kGpThreads = 192;
+constexpr int kGpEpilogueGroups = 2;   // of four warps, which take the accumulator's 32-column chunks in turn
+constexpr int kGpThreads = 64 + 128 * kGpEpilogueGroups;
 constexpr int kGpBlockM = 128;
 constexpr int kGpBlockK = 32;
 constexpr int kGpATileBytes = kGpBlockM * 128;
@@ -201,7 +207,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(acc_full + 8u * b, 1);
-            mbar_init(acc_empty + 8u * b, PAIR ? 256 : 128);   // (pair: the epilogue threads of both CTAs arrive on the leader's)
+            mbar_init(acc_empty + 8u * b, (PAIR ? 8 : 4) * kGpEpilogueGroups);   // (a warp each; pair: those of both CTAs arrive on the leader's)
         }
         *abandon = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -320,12 +326,14 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         const int quarter = warp & 3;
         const int row_in_tile = quarter * 32 + lane;
         const uint32_t lane_bits = (uint32_t)(quarter * 32) << 16;
-        const bool issuer = threadIdx.x == 64;   // the thread that talks to the copy engine
+        const int group = (warp - 2) >> 2;       // has chunks group, group + 2, ... and a staging tile of its own
+        const bool issuer = ((threadIdx.x - 64) & 127) == 0;   // the thread of the group that talks to the copy engine
         // swizzled position of this row's 16-byte chunk c inside a staging tile: chunk ^ (row & 7)
         const uint32_t row_base = (uint32_t)row_in_tile * 128u;
         const uint32_t row_phase = (uint32_t)row_in_tile & 7u;
-        int local = 0, stage_buf = 0;
+        int local = 0;
         bool ok = true;
+        const uint32_t staging = staging_base + (uint32_t)group * kGpStageTileBytes;
         for (int t = worker; t < p.total_tiles && ok; t += n_workers, local++) {
             int mt, nt, bt, sp;
             tile_coords(t, mt, nt, bt, sp);
@@ -333,31 +341,31 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             const int buf = local & 1;
             {
                 uint32_t good = 1;
-                if (lane == 0) good = mbar_wait(acc_full + 8u * buf, (uint32_t)((local >> 1) & 1), abandon, p.status, 24) ? 1u : 0u;
+                if (lane == 0 && (warp - 2) % 4 == 0) good = mbar_wait(acc_full + 8u * buf, (uint32_t)((local >> 1) & 1), abandon, p.status, 24) ? 1u : 0u;
                 good = __shfl_sync(0xffffffffu, good, 0);
-                // the loop below synchronises the four epilogue warps with each other, so they must agree on
+                // the loop below synchronises the group's four warps with each other, so they must agree on
                 // entering it: vote (every epilogue thread gets here, its wait being bounded)
                 uint32_t all_good;
                 asm volatile(
                     "{\n\t.reg .pred p, q;\n\t"
                     "setp.ne.u32 p, %1, 0;\n\t"
-                    "bar.red.and.pred q, 2, 128, p;\n\t"
+                    "bar.red.and.pred q, %2, 128, p;\n\t"
                     "selp.u32 %0, 1, 0, q;\n\t}"
                     : "=r"(all_good)
-                    : "r"(good)
+                    : "r"(good), "r"(3 + group)
                     : "memory");
                 if (!all_good) { ok = false; break; }
                 while (!mbar_try_wait(acc_full + 8u * buf, (uint32_t)((local >> 1) & 1))) {}
             }
             tc_fence_after();
-            const bool eclk = p.clocks != nullptr && blockIdx.x == 0 && local < kGpClockTiles && issuer;
+            const bool eclk = p.clocks != nullptr && blockIdx.x == 0 && local < kGpClockTiles && threadIdx.x == 64;
             long long store_wait = 0;
             if (eclk) p.clocks[local * 8 + 4] = clock64();
             if (issuer) dbg_mark(p, 4, 1);
             const int64_t row = (int64_t)mt * kGpBlockM + row_in_tile;
             const bool row_ok = row < p.m;
             const int chunks = (p.bn + 31) >> 5;
-            for (int c = 0; c < chunks; c++) {
+            for (int c = group; c < chunks; c += kGpEpilogueGroups) {
                 const int col0 = nt * p.bn + c * 32;
                 if (col0 >= p.n) break;                       // uniform: nothing of this chunk is inside the matrix
                 uint32_t v[32];
@@ -404,7 +412,18 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                         }
                         continue;
                     }
-                    if (mode == 1) {
+                    const float* cols = add + bt * st[0] + (int64_t)col0 * st[2];
+                    if (mode == 1 && st[2] == 1 && col0 + 32 <= p.n && ((uintptr_t)cols & 15) == 0) {
+                        // (every lane reads the same 128 bytes; a shuffle per column takes four times as long)
+#pragma unroll
+                        for (int q = 0; q < 8; q++) {
+                            const float4 a4 = __ldg((const float4*)cols + q);
+                            v[4 * q] = __float_as_uint(__uint_as_float(v[4 * q]) + a4.x);
+                            v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + a4.y);
+                            v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + a4.z);
+                            v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + a4.w);
+                        }
+                    } else if (mode == 1) {
                         const int64_t col = col0 + lane;
                         const float mine = col < p.n ? __ldg(add + bt * st[0] + col * st[2]) : 0.f;
 #pragma unroll
@@ -438,16 +457,16 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 #pragma unroll
                     for (int j = 0; j < 32; j++) v[j] = __float_as_uint(gelu_erf_tensor_core(__uint_as_float(v[j])));
                 }
-                // the staging tile about to be written was handed to the copy engine two chunks ago
+                // the staging tile about to be written was handed to the copy engine with the group's last chunk
                 if (issuer) {
                     const long long t0 = eclk ? clock64() : 0;
-                    asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                     if (eclk) store_wait += clock64() - t0;
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
                 if (HALF && p.out_half) {
                     // f16 output: rows of 32 halves = 64 bytes, plain row-major (the store map has no swizzle)
-                    const uint32_t stile = staging_base + (uint32_t)stage_buf * kGpStageTileBytes + (uint32_t)row_in_tile * 64u;
+                    const uint32_t stile = staging + (uint32_t)row_in_tile * 64u;
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         uint32_t h[4];
@@ -461,7 +480,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                                      : "memory");
                     }
                 } else {
-                    const uint32_t stile = staging_base + (uint32_t)stage_buf * kGpStageTileBytes + row_base;
+                    const uint32_t stile = staging + row_base;
 #pragma unroll
                     for (int q = 0; q < 8; q++)
                         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stile + (((uint32_t)q ^ row_phase) << 4)),
@@ -469,19 +488,22 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                                      : "memory");
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
                 if (issuer) {
-                    tma_store_3d(&map_c, staging_base + (uint32_t)stage_buf * kGpStageTileBytes, col0, mt * kGpBlockM, bt * p.splits + sp);
+                    tma_store_3d(&map_c, staging, col0, mt * kGpBlockM, bt * p.splits + sp);
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     dbg_mark(p, 5, (uint32_t)(c + 1));
                 }
-                stage_buf ^= 1;
             }
             if (eclk) p.clocks[local * 8 + 5] = clock64(), p.clocks[local * 8 + 6] = store_wait;
             // every tcgen05.ld of this accumulator has completed (tmem_load_32 waits): the MMA thread may reuse it
+            // (the arrival hands over nothing in memory: no release at cluster scope, which waits for all of a thread's stores)
             tc_fence_before();
-            if (PAIR) mbar_arrive_cluster(map_to_cta(acc_empty + 8u * buf, 0));
-            else mbar_arrive_local(acc_empty + 8u * buf);
+            __syncwarp();
+            if (lane == 0) {
+                if (PAIR) mbar_arrive_remote(map_to_cta(acc_empty + 8u * buf, 0));
+                else mbar_arrive_local(acc_empty + 8u * buf);
+            }
         }
         if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // shared memory must outlive the stores
         if (issuer) dbg_mark(p, 6, 1);
@@ -840,7 +862,7 @@ gemm_slices_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         store_all(std::integral_constant<int, 8>());
     }
     __syncwarp();
-    if (splits > 1) cluster_sync_all();   // nobody leaves while its partial tile may still be read
+    if (splits > 1) cluster_sync_relaxed();   // nobody leaves while its partial tile may still be read (what was read has been used)
 }
 
 struct GemmSlicesLaunch {

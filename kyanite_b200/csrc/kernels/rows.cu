@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(512) layernorm_cluster_kernel(const __grid_con
         if (e < end) out[e] = make_float4(v[i].x / denom, v[i].y / denom, v[i].z / denom, v[i].w / denom);
     }
     // no CTA leaves while another may still read its partial sums
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // (what was read has been used)
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
