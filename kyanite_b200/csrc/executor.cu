@@ -174,6 +174,7 @@ struct Executor {
                     s.gather.out = ptr[2];
                     break;
                 case StepKind::Gemm:
+                    s.gemm.status = status_dev;
                     s.gemm.a = (const float*)ptr[0];
                     s.gemm.b = (const float*)ptr[1];
                     s.gemm.c = (float*)ptr[2];
@@ -196,6 +197,7 @@ struct Executor {
                     }
                     break;
                 case StepKind::Conv:
+                    s.conv.status = status_dev;
                     s.conv.in = (const float*)ptr[0];
                     s.conv.filter = (const float*)ptr[1];
                     s.conv.out = (float*)ptr[2];

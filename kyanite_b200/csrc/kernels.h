@@ -179,6 +179,7 @@ struct GemmParams {
     int32_t conv_operand;
     int32_t conv_c, conv_h, conv_w, conv_ow, conv_r, conv_s, conv_pad_y, conv_pad_x;
     int64_t conv_strides[3];   // element strides of the image tensor: image, row, pixel (channels are contiguous)
+    uint32_t* status;          // word that a kernel raises when a bounded wait expires
 };
 
 // ---- a run of small dense layers and the softmax behind them in one launch (kernels/dense_chain.cu): the executor's way of
@@ -213,6 +214,7 @@ struct ConvParams {
     int32_t act;
     int32_t round_tf32;
     int32_t f_const;     // the filter is a constant: it may be read before the kernels in front have finished
+    uint32_t* status;    // word that a kernel raises when a bounded wait expires
 };
 
 // ---- a run of stride-1 3x3 same-padding convolutions executed by ONE kernel, activations resident

@@ -16,6 +16,7 @@
 
 #include "epilogue.cuh"
 #include "launch.cuh"
+#include "tc_ptx.cuh"
 
 namespace kn {
 
@@ -453,9 +454,10 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
 //    32 x 32, 4 x 4 per thread, four groups: for problems of a few tiles, where it is the number of CTAs that counts
 // What a small problem costs is latency, so: the constant operand is requested ahead of the dependency wait, for as many
 // stages as there are; rows are located once, in a table, and not by divisions in the loop; slices of a tile send their sums to
-// the CTA that stores them (two cluster barriers: one that the peers have started, waited for at the first remote store, and
-// one that the sums have arrived; no remote reads).
-// One 8 x 8 board, 128 -> 128 channels, 3 x 3: 12.1 us on contract_simt_kernel, 5.5 us here
+// the CTA that stores them (a cluster barrier that the peers have started, waited for at the first remote store, and a barrier in
+// the receiver's memory that counts the bytes of the sums, `st.async`: a second cluster barrier has to release what it hands
+// over, which takes some 1000 cycles; no remote reads).
+// One 8 x 8 board, 128 -> 128 channels, 3 x 3: 12.1 us on contract_simt_kernel, 5.2 us here (5.6 with a second cluster barrier)
 // (in a chain; by itself 7.4, kernel_bench's conv_exact_board); 64 boards 48 -> 36 us, 256 boards 112 us
 // (0.61 of the rate); 12 heads of 120 x 64 x 120 (probabilities . V) 14.1 -> 4.8 us.
 template <int BM, int BN, int TM, int TN, int KG, int ST>
@@ -466,7 +468,8 @@ struct ColsLayout {
     static constexpr int kFront = ST * kStage > kTile ? ST * kStage : kTile;   // stages, then (in their place) the partial tiles
     static constexpr int kUnits = BM * BN / 4;                                  // groups of four columns
     static constexpr int kReceived = (kUnits + 8) * 16;                         // sums sent by the other slices
-    static constexpr int kBytes = kFront + kReceived + BM * (int)sizeof(RowAt) + BM * 24;
+    static constexpr int kBarrier = kFront + kReceived + BM * (int)sizeof(RowAt) + BM * 24;   // counts the bytes of sums that arrive
+    static constexpr int kBytes = kBarrier + 16;
 };
 
 struct ColsArgs {
@@ -489,10 +492,21 @@ contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant
     typename Problem::Line* const lines = (typename Problem::Line*)(rows + BM);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int slices = args.slices;
-    if (slices > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (waited for before the first remote store)
+    const int slice = (int)(blockIdx.z % (unsigned)slices);
+    // units of four columns of the result, of which each slice stores `share`
+    const int share = (L::kUnits + slices - 1) / slices;
+    const uint32_t arrived = smem_addr(smem + L::kBarrier);
+    if (slices > 1) {
+        if (threadIdx.x == 0) {
+            tcp::mbar_init(arrived, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            tcp::mbar_expect_tx(arrived, (uint32_t)(max(0, min(share, L::kUnits - slice * share)) * slices) * 16u);
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (waited for before the first remote store)
+    }
     const int64_t M = prob.rows(), N = prob.cols();
     const int inner = (int)prob.inner(), taps = prob.taps();
-    const int slice = (int)(blockIdx.z % (unsigned)slices);
     const int64_t batch = blockIdx.z / (unsigned)slices;
     const int64_t m0 = (int64_t)blockIdx.x * BM, n0 = (int64_t)blockIdx.y * BN;
     const int tid = threadIdx.x;
@@ -672,9 +686,7 @@ contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant
                 make_float4(acc[i][2 * j].x, acc[i][2 * j].y, acc[i][2 * j + 1].x, acc[i][2 * j + 1].y);
     __syncthreads();
     if (slices > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    // units of four columns, in the order in which the result's contiguous axis comes first; of several slices, each
-    // stores `share` of them
-    const int share = (L::kUnits + slices - 1) / slices;
+    // units of four columns, in the order in which the result's contiguous axis comes first
     auto place = [&](int u, int& mm, int& nn) {
         mm = args.rows_fast ? u % BM : u / (BN / 4);
         nn = (args.rows_fast ? u / BM : u % (BN / 4)) * 4;
@@ -709,14 +721,20 @@ contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant
             store(mm, nn, v);
         } else {
             const int owner = u / share;
-            uint32_t to;
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_addr(received + slice * share + u - owner * share)), "r"(owner));
-            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+            const uint32_t to = tcp::map_to_cta(smem_addr(received + slice * share + u - owner * share), (uint32_t)owner);
+            asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                         ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(tcp::map_to_cta(arrived, (uint32_t)owner))
+                         : "memory");
         }
     }
     if (slices > 1) {
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const long long start = clock64();
+        while (!tcp::mbar_try_wait_cluster(arrived, 0)) {
+            if (clock64() - start > tcp::kWaitCycles) {
+                atomicMax(prob.p.status, 71u);
+                return;
+            }
+        }
         for (int u = tid; u < share && slice * share + u < L::kUnits; u += NT) {
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
