@@ -30,6 +30,7 @@ SOURCES = [
     "kernels/elementwise_fixed.cu",
     "kernels/rows.cu",
     "kernels/rows_f16.cu",
+    "kernels/group_norm.cu",
     "kernels/softmax_matmul.cu",
     "kernels/gather.cu",
     "kernels/host_copy.cu",

@@ -213,6 +213,13 @@ struct Executor {
                     s.rms.out = ptr[1];
                     s.rms.gain = ptr.size() > 2 ? (const float*)ptr[2] : nullptr;
                     break;
+                case StepKind::GroupNorm:
+                    s.group_norm.in = (const float*)ptr[0];
+                    s.group_norm.out = (float*)ptr[1];
+                    s.group_norm.scale = (const float*)ptr[2];
+                    s.group_norm.shift = (const float*)ptr[3];
+                    s.group_norm.status = status_dev;
+                    break;
                 case StepKind::AllReduce:
                     s.all_reduce.in = ptr[0];
                     s.all_reduce.out = ptr[1];
@@ -340,6 +347,7 @@ struct Executor {
             case StepKind::ConvChain: err = tc_launch_step(s, stream); break;
             case StepKind::Im2col: err = launch_im2col(s.im2col, stream); break;
             case StepKind::RmsNorm: err = launch_rmsnorm(s.rms, stream); break;
+            case StepKind::GroupNorm: err = launch_group_norm(s.group_norm, stream); break;
             case StepKind::AllReduce: {
                 const AllReduceParams& a = s.all_reduce;
                 if (comm != nullptr && comm->world > 1)

@@ -90,6 +90,21 @@ struct RowParams {
 // ---- root-mean-square norm over the innermost axis:  out = x / sqrt(mean(x^2) + eps) * gain.  The IR has no such
 // operation; the planner recognises the pow / mean / sqrt / div / mul subgraph (with the value casts around it in
 // half-storage graphs) and this one kernel takes the place of five elementwise and reduce steps.
+// ---- group normalisation with scale, shift and SiLU (kernels/group_norm.cu)
+struct GroupNormParams {
+    const float* in;
+    float* out;
+    const float *scale, *shift;      // per channel, `*_stride` apart
+    int64_t scale_stride, shift_stride;
+    int64_t in_image, in_position;   // channels-last (in_last): elements between images and positions; else planes of hw
+    int64_t out_image, out_position;
+    int32_t images, channels, group_channels, groups, hw;
+    int32_t cluster;                 // CTAs of a group
+    int32_t in_last, out_last, silu;
+    float eps;
+    uint32_t* status;                // word that the kernel raises when a bounded wait expires
+};
+
 struct RmsNormParams {
     const void* in;          // [rows, len], rows `in_row_stride` elements apart, f32 or f16
     void* out;               // [rows, len] dense, f32 or f16
@@ -289,6 +304,8 @@ int launch_scalar_fixed(const ScalarParams& p, cudaStream_t stream);
 int launch_reduce(const ReduceParams& p, cudaStream_t stream);
 int launch_softmax(const RowParams& p, cudaStream_t stream);      // dispatches on p.half
 int launch_layernorm(const RowParams& p, cudaStream_t stream);
+int launch_group_norm(const GroupNormParams& p, cudaStream_t stream);  // kernels/group_norm.cu
+int group_norm_cluster(int64_t groups, int64_t values);   // 0: a group is too large
 int launch_rmsnorm(const RmsNormParams& p, cudaStream_t stream);  // kernels/rows_f16.cu
 int launch_softmax_f16(const RowParams& p, cudaStream_t stream);  // kernels/rows_f16.cu
 int launch_layernorm_f16(const RowParams& p, cudaStream_t stream);

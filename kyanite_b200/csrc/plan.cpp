@@ -16,7 +16,7 @@
 namespace kn {
 
 const char* step_kind_name(StepKind k) {
-    static const char* names[] = {"Scalar", "Reduce", "Softmax", "Layernorm", "Gather", "Gemm", "Conv", "ConvChain", "Im2col", "AllReduce", "RmsNorm"};
+    static const char* names[] = {"Scalar", "Reduce", "Softmax", "Layernorm", "Gather", "Gemm", "Conv", "ConvChain", "Im2col", "AllReduce", "RmsNorm", "GroupNorm"};
     return (int)k < (int)StepKind::COUNT ? names[(int)k] : "?";
 }
 
@@ -86,6 +86,27 @@ void coalesce_axes(std::vector<int64_t>& dims, std::vector<std::vector<int64_t>>
     }
     dims = std::move(nd);
     strides = std::move(ns);
+}
+
+// Puts the axes of an elementwise step into the order of the first result's memory (operand `result`), which need not be the
+// graph's: channels-last tensors are read and written in whole rows then.
+void order_axes(std::vector<int64_t>& dims, std::vector<std::vector<int64_t>>& strides, size_t result) {
+    const std::vector<int64_t>& by = strides[result];
+    std::vector<size_t> order;
+    for (size_t d = 0; d < dims.size(); d++) {
+        if (dims[d] > 1 && by[d] <= 0) return;
+        if (dims[d] > 1) order.push_back(d);
+    }
+    if (order.empty() || by[order.back()] == 1) return;   // (it ends in the contiguous axis already)
+    std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return by[a] > by[b]; });
+    std::vector<int64_t> nd;
+    for (size_t d : order) nd.push_back(dims[d]);
+    for (auto& s : strides) {
+        std::vector<int64_t> ns;
+        for (size_t d : order) ns.push_back(s[d]);
+        s = ns;
+    }
+    dims = nd;
 }
 
 // slot reference while a scalar program is being built: loads and instructions are numbered
@@ -266,6 +287,7 @@ class Planner {
         std::vector<int64_t> dims = shape;
         std::vector<std::vector<int64_t>> strides;
         for (auto& t : s.operands) strides.push_back(t.ss.strides);
+        order_axes(dims, strides, (size_t)block.loads.size());
         coalesce_axes(dims, strides);
         KN_CHECK((int)dims.size() <= DEV_MAX_RANK, KN_ERR_UNSUPPORTED,
                  "elementwise step needs more than 8 non-mergeable axes");
@@ -540,6 +562,7 @@ class Planner {
         if (auto fused = try_merged_attention(v)) return *fused;
         if (auto fused = try_fused_contraction(v)) return *fused;
         if (auto fused = try_fused_rmsnorm(v)) return *fused;
+        if (auto fused = try_fused_group_norm(v)) return *fused;
         const ValueInfo& info = g_.values[v];
         std::vector<int64_t> shape = shape_of(v);
         switch (info.op) {
@@ -554,7 +577,21 @@ class Planner {
             case OpKind::View: {
                 PlanTensor in = visit(info.inputs[0]);
                 if (auto s = in.ss.view(shape)) return in.with(*s);
-                PlanTensor dense = alloc_shared(in.ss.shape, in.dtype, v);
+                // (of an image whose channels are contiguous: kept so where that can be viewed, as in the enlargements of an
+                // image by broadcasting along new axes)
+                PlanTensor dense;
+                if (in.ss.rank() >= 4 && in.ss.shape[1] > 1 && in.ss.strides[1] == 1) {
+                    std::vector<int64_t> memory{in.ss.shape[0]};
+                    std::vector<int> back{0, in.ss.rank() - 1};
+                    for (int d = 2; d < in.ss.rank(); d++) memory.push_back(in.ss.shape[d]), back.push_back(d - 1);
+                    memory.push_back(in.ss.shape[1]);
+                    const StridedShape kept = StridedShape::simple(memory).permute(back);
+                    if (kept.view(shape)) {
+                        dense = alloc_shared(memory, in.dtype, v);
+                        dense = dense.with(dense.ss.permute(back));
+                    }
+                }
+                if (dense.buf < 0) dense = alloc_shared(in.ss.shape, in.dtype, v);
                 emit_copy(in, dense, v);
                 auto s = dense.ss.view(shape);
                 KN_CHECK(s.has_value(), KN_ERR_INTERNAL, "view of a dense tensor failed");
@@ -580,7 +617,7 @@ class Planner {
             case OpKind::Concat: {
                 std::vector<PlanTensor> ins;
                 for (int i : info.inputs) ins.push_back(visit(i));
-                PlanTensor out = alloc_shared(shape, info.dtype, v);
+                PlanTensor out = alloc_concat(v, ins);
                 int64_t start = 0;
                 for (auto& in : ins) {
                     int64_t n = in.ss.shape[info.axis];
@@ -622,6 +659,18 @@ class Planner {
             }
             default: fail(KN_ERR_INTERNAL, "unknown operation");
         }
+    }
+
+    // Where a concatenation goes: channels-last if it joins the channels of images that all are (each part is a copy of whole
+    // rows then, and so is what a convolution or a group norm reads), else plain
+    PlanTensor alloc_concat(int v, const std::vector<PlanTensor>& parts) {
+        const ValueInfo& info = g_.values[v];
+        const std::vector<int64_t> sh = shape_of(v);
+        bool last = info.dtype == DType::F32 && info.axis == 1 && sh.size() == 4 && sh[1] % 4 == 0 && sh[2] * sh[3] > 1;
+        for (const PlanTensor& t : parts) last = last && t.ss.strides[1] == 1 && t.ss.shape[1] % 4 == 0 && t.ss.strides[3] != 1;
+        if (!last) return alloc_shared(sh, info.dtype, v);
+        PlanTensor out = alloc_shared({sh[0], sh[2], sh[3], sh[1]}, info.dtype, v);
+        return out.with(out.ss.permute({0, 3, 1, 2}));
     }
 
     // ---------------------------------------------------------------- elementwise fusion
@@ -1828,7 +1877,7 @@ class Planner {
             x = channels_last(x, ci.inputs[0]);
             w = tap_major_filter(w, ci.inputs[1]);
             // keep the activation channels-last while it flows from convolution to convolution
-            if (root_shape == native && native[1] % 4 == 0 && feeds_tensor_core_conv(root)) {
+            if (root_shape == native && native[1] % 4 == 0 && (feeds_tensor_core_conv(root) || feeds_group_norm(root))) {
                 out = alloc_shared({native[0], native[2], native[3], native[1]}, DType::F32, root);
                 out = out.with(out.ss.permute({0, 3, 1, 2}));
             }
@@ -1981,6 +2030,109 @@ class Planner {
         auto rs = out.ss.view(root_shape);
         KN_CHECK(rs.has_value(), KN_ERR_INTERNAL, "view of a dense contraction output failed");
         return out.with(*rs);
+    }
+
+    // Group normalisation: view [N, groups, rest] -> layernorm -> view -> * scale -> + shift (-> times its own sigmoid), scale and
+    // shift one value per channel.  One launch that reads and writes plain or channels-last memory, where the
+    // nodes by themselves need plain memory, an elementwise step and a transposing copy on either side.
+    std::optional<PlanTensor> try_fused_group_norm(int root) {
+        auto is_binary = [&](int v, BinaryOp op) { return g_.values[v].op == OpKind::Binary && g_.values[v].binary_op == op; };
+        if (g_.values[root].dtype != DType::F32 || shape_of(root).size() != 4) return std::nullopt;
+        int sum = root;
+        bool silu = false;
+        if (is_binary(root, BinaryOp::Mul)) {
+            for (int side = 0; side < 2 && !silu; side++) {
+                const int s = g_.values[root].inputs[side], o = g_.values[root].inputs[1 - side];
+                const ValueInfo& si = g_.values[s];
+                silu = si.op == OpKind::Unary && si.unary_op == UnaryOp::Sigmoid && si.inputs[0] == o && fusable(s) && !map_[s] &&
+                       g_.is_hidden_with_uses(o, 2) && !map_[o];
+                if (silu) sum = o;
+            }
+            if (!silu) return std::nullopt;
+        }
+        if (!is_binary(sum, BinaryOp::Add)) return std::nullopt;
+        int scale = -1, shift = -1, norm = -1, x = -1;
+        for (int side = 0; side < 2 && x < 0; side++) {
+            const int mul = g_.values[sum].inputs[side];
+            if (!is_binary(mul, BinaryOp::Mul) || !fusable(mul) || map_[mul]) continue;
+            for (int inner = 0; inner < 2 && x < 0; inner++) {
+                const int view = g_.values[mul].inputs[inner];
+                if (g_.values[view].op != OpKind::View || !fusable(view) || map_[view]) continue;
+                norm = g_.values[view].inputs[0];
+                const ValueInfo& ni = g_.values[norm];
+                if (ni.op != OpKind::Layernorm || ni.dtype != DType::F32 || ni.axis != 2 || !fusable(norm) || map_[norm]) continue;
+                const int grouped = ni.inputs[0];
+                if (g_.values[grouped].op != OpKind::View || !fusable(grouped) || map_[grouped]) continue;
+                if (shape_of(g_.values[grouped].inputs[0]) != shape_of(root) || shape_of(norm).size() != 3) continue;
+                x = g_.values[grouped].inputs[0];
+                scale = g_.values[mul].inputs[1 - inner];
+                shift = g_.values[sum].inputs[1 - side];
+            }
+        }
+        if (x < 0) return std::nullopt;
+        const std::vector<int64_t> sh = shape_of(root), ns = shape_of(norm);
+        const int64_t N = sh[0], C = sh[1], hw = sh[2] * sh[3], groups = ns[1];
+        if (N < 1 || hw < 1 || groups < 1 || ns[0] != N || C % groups != 0 || ns[2] != C / groups * hw) return std::nullopt;
+        if (hw % 4 != 0 || C % 4 != 0 || N * groups > (1 << 24) || group_norm_cluster(N * groups, C / groups * hw) == 0) return std::nullopt;
+        // one value per channel, known without a step that reads the sum
+        auto channel_value = [&](int v, PlanTensor* t) {
+            const ValueInfo* i = &g_.values[v];
+            if (i->op == OpKind::Broadcast) i = &g_.values[i->inputs[0]];
+            if (i->op != OpKind::Constant || i->dtype != DType::F32) return false;
+            *t = visit(v);
+            return per_channel(*t);
+        };
+        PlanTensor st, ht;
+        if (!channel_value(scale, &st) || !channel_value(shift, &ht)) return std::nullopt;
+
+        // from here on steps are emitted
+        PlanTensor in = visit(x);
+        auto plain = [&](const PlanTensor& t) {
+            const auto& s = t.ss.strides;
+            return s[3] == 1 && (sh[2] == 1 || s[2] == sh[3]) && s[1] == hw && (N == 1 || s[0] % 4 == 0) && t.offset % 4 == 0;
+        };
+        auto last = [&](const PlanTensor& t) {
+            const auto& s = t.ss.strides;
+            return s[1] == 1 && s[3] > 0 && s[3] % 4 == 0 && s[3] < (1ll << 31) && (sh[2] == 1 || s[2] == sh[3] * s[3]) && (N == 1 || s[0] % 4 == 0) && t.offset % 4 == 0;
+        };
+        bool convolutions = !users_[root].empty();   // what reads the result wants its channels contiguous
+        for (int u : users_[root]) convolutions = convolutions && g_.values[u].op == OpKind::Conv && g_.values[u].inputs[0] == root;
+        const bool in_last = !plain(in) && last(in) && convolutions;
+        if (!in_last && !plain(in)) in = ensure_simple_copy(in, x);
+        const bool out_last = in_last || convolutions;
+        PlanTensor out;
+        if (out_last) {
+            out = alloc_shared({N, sh[2], sh[3], C}, DType::F32, root);
+            out = out.with(out.ss.permute({0, 3, 1, 2}));
+        } else {
+            out = alloc_shared(sh, DType::F32, root);
+        }
+        Step s;
+        s.kind = StepKind::GroupNorm;
+        s.value = root;
+        GroupNormParams& p = s.group_norm;
+        p.images = (int32_t)N;
+        p.channels = (int32_t)C;
+        p.groups = (int32_t)groups;
+        p.group_channels = (int32_t)(C / groups);
+        p.hw = (int32_t)hw;
+        p.cluster = group_norm_cluster(N * groups, C / groups * hw);
+        p.in_last = in_last;
+        p.out_last = out_last;
+        p.silu = silu;
+        p.eps = g_.values[norm].eps;
+        p.in_image = N == 1 ? 0 : in.ss.strides[0];
+        p.in_position = in_last ? in.ss.strides[3] : 1;
+        p.out_image = out.ss.strides[0];
+        p.out_position = out_last ? out.ss.strides[3] : 1;
+        p.scale_stride = st.ss.strides[1];
+        p.shift_stride = ht.ss.strides[1];
+        s.operands = {in, out, st, ht};
+        s.writes = {0, 1, 0, 0};
+        s.desc = "groupnorm n=" + std::to_string(N) + " c=" + std::to_string(C) + " groups=" + std::to_string(groups) + " hw=" + std::to_string(hw) +
+                 (silu ? " silu" : "") + (in_last ? " channels-last" : out_last ? " to channels-last" : "");
+        push_step(std::move(s));
+        return out;
     }
 
     // ---------------------------------------------------------------- root-mean-square norm
@@ -2471,6 +2623,15 @@ class Planner {
         if (ci.stride_y != 1 || ci.stride_x != 1) return false;
         std::vector<int64_t> o = shape_of(conv);
         return o[0] * o[2] * o[3] >= kConvTilePositions && o[1] >= 4;
+    }
+    // is it read by a group norm that a convolution follows (try_fused_group_norm), which takes it channels-last as well?
+    bool feeds_group_norm(int v) {
+        for (int u : users_[v]) {
+            if (g_.values[u].op != OpKind::View || users_[u].size() != 1 || shape_of(u).size() != 3) continue;
+            const int norm = users_[u][0];
+            if (g_.values[norm].op == OpKind::Layernorm && g_.values[norm].axis == 2 && users_[norm].size() == 1 && g_.values[users_[norm][0]].op == OpKind::View) return true;
+        }
+        return false;
     }
     bool feeds_tensor_core_conv(int v) {
         for (int u : users_[v])

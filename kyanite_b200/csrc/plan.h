@@ -49,7 +49,7 @@ struct PlanTensor {
 
 struct TcLaunch;   // tensor maps and launch geometry of a tensor-core step (kernels/contract_tc.cu)
 
-enum class StepKind : uint8_t { Scalar = 0, Reduce, Softmax, Layernorm, Gather, Gemm, Conv, ConvChain, Im2col, AllReduce, RmsNorm, COUNT };
+enum class StepKind : uint8_t { Scalar = 0, Reduce, Softmax, Layernorm, Gather, Gemm, Conv, ConvChain, Im2col, AllReduce, RmsNorm, GroupNorm, COUNT };
 const char* step_kind_name(StepKind k);
 
 struct Step {
@@ -74,6 +74,7 @@ struct Step {
     Im2colParams im2col{};
     AllReduceParams all_reduce{};
     RmsNormParams rms{};
+    GroupNormParams group_norm{};
 };
 
 struct Plan {
