@@ -245,9 +245,12 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             tmem_load_32_nowait(my_s + 32u, v[1]);
             tmem_loads_done();
             const int col0 = j * kFlKeys;
+            bool plain = false;   // a block whose term is zero throughout: scores as without a term
             if (TERM) {
                 const int kind = blocks_of == nullptr ? 1 : (int)blocks_of[1 + j / kTableStep];
-                if (kind != 1) {
+                if (kind == 0 && p.scale > 0.f) {
+                    plain = true;
+                } else if (kind != 1) {
                     const float same = kind == 2 ? -INFINITY : 0.f;
 #pragma unroll
                     for (int i = 0; i < 64; i++) v[i >> 5][i & 31] = __float_as_uint(fmaf(p.scale, __uint_as_float(v[i >> 5][i & 31]), same));
@@ -300,6 +303,7 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             float top = -INFINITY;
 #pragma unroll
             for (int i = 0; i < 64; i++) top = fmaxf(top, __uint_as_float(v[i >> 5][i & 31]));
+            if (plain) top *= p.scale;
             // a row whose scores were all -infinity so far has no reference yet (and zeros in its sum and output)
             const bool first = seen == -INFINITY;
             seen = fmaxf(seen, top);
@@ -320,29 +324,30 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     }
                 }
             }
-            const float shift = -ref * unit;
+            auto exponentials = [&](auto exponent) {
 #pragma unroll
-            for (int c = 0; c < 2; c++) {
+                for (int c = 0; c < 2; c++) {
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    const float x0 = __uint_as_float(v[c][i]), x1 = __uint_as_float(v[c][i + 1]);
-                    // (with a term the difference first: the lowest finite value times log2(e) would overflow)
-                    const float e0 = exp2_approx(TERM ? (x0 - ref) * unit : fmaf(x0, unit, shift));
-                    const float e1 = exp2_approx(TERM ? (x1 - ref) * unit : fmaf(x1, unit, shift));
-                    if (HALF) {
-                        sum += e0 + e1;
-                        const __half2 h = __floats2half2_rn(e0, e1);
-                        v[0][c * 16 + (i >> 1)] = *(const uint32_t*)&h;
-                    } else {
-                        // rounded to the operand's eleven bits here, so that the sum is of what the MMAs see
-                        uint32_t r0, r1;
-                        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r0) : "f"(e0));
-                        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r1) : "f"(e1));
-                        sum += __uint_as_float(r0) + __uint_as_float(r1);
-                        v[c][i] = r0, v[c][i + 1] = r1;
+                    for (int i = 0; i < 32; i += 2) {
+                        const float e0 = exp2_approx(exponent(__uint_as_float(v[c][i]))), e1 = exp2_approx(exponent(__uint_as_float(v[c][i + 1])));
+                        if (HALF) {
+                            sum += e0 + e1;
+                            const __half2 h = __floats2half2_rn(e0, e1);
+                            v[0][c * 16 + (i >> 1)] = *(const uint32_t*)&h;
+                        } else {
+                            // rounded to the operand's eleven bits here, so that the sum is of what the MMAs see
+                            uint32_t r0, r1;
+                            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r0) : "f"(e0));
+                            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r1) : "f"(e1));
+                            sum += __uint_as_float(r0) + __uint_as_float(r1);
+                            v[c][i] = r0, v[c][i + 1] = r1;
+                        }
                     }
                 }
-            }
+            };
+            const float shift = -ref * unit, factor = plain ? p.scale * unit : unit;
+            if (TERM && !plain) exponentials([&](float x) { return (x - ref) * unit; });   // (the lowest finite value times log2(e) would overflow)
+            else exponentials([&](float x) { return fmaf(x, factor, shift); });
             if (HALF) {
                 tmem_store_32(my_s, v[0]);
             } else {
