@@ -20,6 +20,7 @@
 #include <algorithm>
 
 #include "../kernels.h"
+#include "../scalar_ops.h"
 #include "launch.cuh"
 #include "tc_ptx.cuh"
 
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(kMaxThreads) group_norm_kernel(const __grid_co
         sq = lanes_sum<kMaxCluster>(n > 0.f ? part.y + delta * delta * n : 0.f);
     }
     const float denom = sqrtf(sq / (float)(pieces * V) + p.eps), inverse = 1.f / denom;
-    const bool normal = denom > 1e-15f && denom < 1e15f;
+    const bool normal = divides_by(denom);
     float* out = p.out + img * p.out_image + (OUT_LAST ? c0 : (int64_t)c0 * p.hw);
     const float *scale = p.scale + c0 * p.scale_stride, *shift = p.shift + c0 * p.shift_stride;
     const bool dense = OUT_LAST && p.scale_stride == 1 && p.shift_stride == 1 && ((uintptr_t)scale | (uintptr_t)shift) % (4 * V) == 0;
@@ -169,10 +170,7 @@ __global__ void __launch_bounds__(kMaxThreads) group_norm_kernel(const __grid_co
 #pragma unroll
         for (int j = 0; j < V; j++) {
             const float d = x[i][j] - mean;
-            // d / denom: the product with the inverse and one correction by its remainder (Markstein, 1990), as exact as a division
-            // and without its branches
-            const float q = d * inverse;
-            y[j] = normal ? fmaf(fmaf(-q, denom, d), inverse, q) : d / denom;
+            y[j] = normal ? divide_by(d, denom, inverse) : d / denom;
             y[j] = __fadd_rn(__fmul_rn(y[j], a[j]), b[j]);
             if (p.silu) y[j] *= 1.0f / (1.0f + expf(-y[j]));
         }

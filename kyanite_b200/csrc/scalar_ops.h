@@ -23,6 +23,15 @@
 
 namespace kn {
 
+// x / y for many x and one y whose inverse is at hand: the product and one correction by its remainder (Markstein, 1990), as exact
+// as a division where neither y nor the quotient is near the ends of the range, and without a division's branches, which leave a
+// thread's quotients one behind the other.
+KN_HD bool divides_by(float y) { return y > 1e-15f && y < 1e15f; }
+KN_HD float divide_by(float x, float y, float inverse) {
+    const float q = x * inverse;
+    return fmaf(fmaf(-q, y, x), inverse, q);
+}
+
 KN_HD float bits_to_f32(uint64_t b) {
     uint32_t u = (uint32_t)b;
     float f;
