@@ -2478,16 +2478,20 @@ class Planner {
         const bool long_k = C * R * S >= 2048 && (may_be_implicit || N * OH * OW * R * S * C * 4 <= (256ll << 20));
         if (!strided && !few_positions && !pointwise && !long_k) return std::nullopt;
         if (pointwise && !strided && py == 0 && px == 0 && becomes_chain_head(ci, x)) return std::nullopt;
-        if (N < 1 || N > 65535 || OH * OW < 64 || K < 16 || K % 4 != 0 || C < 1 || R * S > 64) return std::nullopt;
-        if (2.0 * (double)N * OH * OW * K * C * R * S < 2e8) return std::nullopt;
+        if (N < 1 || N > 65535 || OH * OW < 64 || K % 4 != 0 || C < 1 || R * S > 64) return std::nullopt;
+        // Few channels of a long reduction (an image's last convolution): the convolution kernel has a CTA per 128 positions that goes
+        // through all of K; where that leaves half of the SMs idle, slices of K over clusters.  320 -> 4 channels of 64 x 64 39.4 -> 11.3
+        // us, 512 -> 12 of 16 x 16 59.9 -> 8.1; at the line, 256 -> 12 of 74 x 128, 33.5 -> 19.5.
+        const bool narrow = K < 16 && !pointwise && long_k && may_be_implicit && OH * OW % 128 == 0 && N * OH * OW <= 74 * 128;
+        if (!narrow && (K < 16 || 2.0 * (double)N * OH * OW * K * C * R * S < 2e8)) return std::nullopt;
         const ValueInfo& wi = g_.values[ci.inputs[1]];
         if (wi.op != OpKind::Constant || !w.ss.has_simple_strides() || w.offset != 0) return std::nullopt;
         // Two orientations.  positions x channels: the result is channels-last in memory, which the next
         // tensor-core convolution wants.  If the value the graph asks for (a view of the result, say the
         // [N, groups, ...] view a group norm takes) cannot be expressed on that layout, channels x positions:
         // the filter is the A operand (shared by the batch), the result is plain NCHW.
-        const bool nchw = !StridedShape({N, K, OH, OW}, {OH * OW * K, 1, OW * K, K}).view(shape_of(root)).has_value();
-        if (nchw && (K < 64 || OH * OW < 16 || (OH * OW) % 4 != 0)) return std::nullopt;
+        const bool nchw = narrow || !StridedShape({N, K, OH, OW}, {OH * OW * K, 1, OW * K, K}).view(shape_of(root)).has_value();
+        if (nchw && ((K < 64 && !narrow) || OH * OW < 16 || (OH * OW) % 4 != 0)) return std::nullopt;
         // addends as [N, OH*OW, K] or [N, K, OH*OW]
         ConvGemm g;
         for (const PlanTensor& t : addends) {
