@@ -208,11 +208,40 @@ __global__ void __launch_bounds__(256) im2col_kernel(const __grid_constant__ Im2
     }
 }
 
+// Few channels (the image itself): a thread per position and tap, C4 pieces of four channels each.  Lanes run along the result, which
+// is written in whole lines; what they read of one another's windows comes from L1.  The kernel above would leave 28 of 32 lanes of
+// each store without a channel: 64 images of 3 x 32 x 32 91.2 us there, 4.7
+// here.
+template <int C4>
+__global__ void __launch_bounds__(256) im2col_few_kernel(const __grid_constant__ Im2colParams p, uint32_t total) {
+    pdl_enter();
+    const uint32_t e = blockIdx.x * 256u + threadIdx.x;
+    if (e >= total) return;
+    const uint32_t taps = (uint32_t)(p.r * p.s), positions = (uint32_t)(p.oh * p.ow);
+    const uint32_t at = e / taps, tap = e - at * taps, n = at / positions, pos = at - n * positions;
+    const uint32_t oy = pos / (uint32_t)p.ow, ox = pos - oy * (uint32_t)p.ow, r = tap / (uint32_t)p.s, q = tap - r * (uint32_t)p.s;
+    const int iy = (int)oy * p.stride_y + (int)r - p.pad_y, ix = (int)ox * p.stride_x + (int)q - p.pad_x;
+    const bool inside = iy >= 0 && iy < p.h && ix >= 0 && ix < p.w;
+    const float* src = p.in + n * p.s_in[0] + (inside ? iy * p.s_in[2] + ix * p.s_in[3] : 0);
+    float v[C4 * 4];
+#pragma unroll
+    for (int c = 0; c < C4 * 4; c++) v[c] = inside && c < p.c ? __ldg(src + c * p.s_in[1]) : 0.f;
+#pragma unroll
+    for (int c = 0; c < C4; c++) ((float4*)p.col)[(int64_t)e * C4 + c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+}
+
 }  // namespace
 
 int launch_im2col(const Im2colParams& p, cudaStream_t stream) {
     const int64_t positions = (int64_t)p.oh * p.ow;
     if (p.n == 0 || positions == 0 || p.c_pad == 0) return 0;
+    const int64_t windows = positions * p.r * p.s * p.n;
+    if (p.c_pad <= 8 && p.c_pad % 4 == 0 && windows < (1ll << 31) && (uintptr_t)p.col % 16 == 0) {
+        const dim3 grid((unsigned)((windows + 255) / 256));
+        if (p.c_pad == 4) launch_pdl(im2col_few_kernel<1>, grid, dim3(256), (size_t)0, stream, p, (uint32_t)windows);
+        else launch_pdl(im2col_few_kernel<2>, grid, dim3(256), (size_t)0, stream, p, (uint32_t)windows);
+        return (int)cudaGetLastError();
+    }
     const int64_t p_tiles = (positions + 31) / 32, c_tiles = (p.c_pad + kIm2colC - 1) / kIm2colC;
     const int64_t blocks = p_tiles * c_tiles * p.r * p.s * p.n;
     if (blocks >= (1ll << 31)) return (int)cudaErrorInvalidValue;
