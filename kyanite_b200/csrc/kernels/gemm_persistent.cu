@@ -52,8 +52,6 @@ namespace {
 
 using namespace tcp;
 
-constexpr int kGpEpilogueGroups = 2;   // of four warps, which take the accumulator's 32-column chunks in turn
-constexpr int kGpThreads = 64 + 128 * kGpEpilogueGroups;
 constexpr int kGpBlockM = 128;
 constexpr int kGpBlockK = 32;
 constexpr int kGpATileBytes = kGpBlockM * 128;
@@ -62,6 +60,7 @@ constexpr int kGpStageTileBytes = 128 * 128;   // epilogue staging: 128 rows x 3
 
 struct GemmPersistentParams {
     int32_t bn, stages, k_iters;
+    int32_t groups;           // of epilogue warps, which share two staging tiles
     int32_t a_batch, b_batch;        // 1, or 0 when every batch entry uses the same A / B (batch stride 0)
     int32_t splits, k_iters_slice;   // split K: slice sp of a tile covers K blocks [sp * k_iters_slice, ...) and is stored
                                      // as matrix `batch * splits + sp` of the output map (the partial-sum buffer)
@@ -177,8 +176,10 @@ struct OperandCursor {
 // shared-memory pipe carries a third fewer bytes per multiply-add than with one CTA per tile (that pipe, not the
 // tensor pipe, bounds the one-CTA kernel at about 0.83 of the tensor rate).  CTA 0 of the pair (the leader) issues the
 // MMAs; the loads of both CTAs complete on the leader's barriers; `tcgen05.commit` reaches the barriers of both.
-template <bool HALF, bool PAIR>   // operand storage: f16 (kind::f16) or f32 (kind::tf32); one CTA per tile or a CTA pair
-__global__ void __launch_bounds__(kGpThreads, 1)
+// operand storage: f16 (kind::f16) or f32 (kind::tf32); one CTA per tile or a CTA pair; groups of four epilogue warps, which take the
+// accumulator's 32-column chunks in turn
+template <bool HALF, bool PAIR, int GROUPS>
+__global__ void __launch_bounds__(64 + 128 * GROUPS, 1)
 gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                        const __grid_constant__ CUtensorMap map_c, const __grid_constant__ GemmPersistentParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -207,7 +208,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(acc_full + 8u * b, 1);
-            mbar_init(acc_empty + 8u * b, (PAIR ? 8 : 4) * kGpEpilogueGroups);   // (a warp each; pair: those of both CTAs arrive on the leader's)
+            mbar_init(acc_empty + 8u * b, (PAIR ? 8 : 4) * GROUPS);   // (a warp each; pair: those of both CTAs arrive on the leader's)
         }
         *abandon = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -326,14 +327,18 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         const int quarter = warp & 3;
         const int row_in_tile = quarter * 32 + lane;
         const uint32_t lane_bits = (uint32_t)(quarter * 32) << 16;
-        const int group = (warp - 2) >> 2;       // has chunks group, group + 2, ... and a staging tile of its own
+        const int group = GROUPS == 1 ? 0 : (warp - 2) >> 2;   // of two: has chunks group, group + 2, ... and a staging tile of its own
         const bool issuer = ((threadIdx.x - 64) & 127) == 0;   // the thread of the group that talks to the copy engine
         // swizzled position of this row's 16-byte chunk c inside a staging tile: chunk ^ (row & 7)
         const uint32_t row_base = (uint32_t)row_in_tile * 128u;
         const uint32_t row_phase = (uint32_t)row_in_tile & 7u;
         int local = 0;
         bool ok = true;
-        const uint32_t staging = staging_base + (uint32_t)group * kGpStageTileBytes;
+        auto group_sync = [&]() {   // (of a barrier that the instruction names: one from a register takes longer)
+            if (group == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+            else asm volatile("bar.sync 2, 128;" ::: "memory");
+        };
+        uint32_t staging = staging_base + (uint32_t)group * kGpStageTileBytes;
         for (int t = worker; t < p.total_tiles && ok; t += n_workers, local++) {
             int mt, nt, bt, sp;
             tile_coords(t, mt, nt, bt, sp);
@@ -346,14 +351,10 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 // the loop below synchronises the group's four warps with each other, so they must agree on
                 // entering it: vote (every epilogue thread gets here, its wait being bounded)
                 uint32_t all_good;
-                asm volatile(
-                    "{\n\t.reg .pred p, q;\n\t"
-                    "setp.ne.u32 p, %1, 0;\n\t"
-                    "bar.red.and.pred q, %2, 128, p;\n\t"
-                    "selp.u32 %0, 1, 0, q;\n\t}"
-                    : "=r"(all_good)
-                    : "r"(good), "r"(3 + group)
-                    : "memory");
+                if (group == 0)
+                    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 3, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(all_good) : "r"(good) : "memory");
+                else
+                    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 4, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(all_good) : "r"(good) : "memory");
                 if (!all_good) { ok = false; break; }
                 while (!mbar_try_wait(acc_full + 8u * buf, (uint32_t)((local >> 1) & 1))) {}
             }
@@ -365,7 +366,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             const int64_t row = (int64_t)mt * kGpBlockM + row_in_tile;
             const bool row_ok = row < p.m;
             const int chunks = (p.bn + 31) >> 5;
-            for (int c = group; c < chunks; c += kGpEpilogueGroups) {
+            for (int c = group; c < chunks; c += GROUPS) {
                 const int col0 = nt * p.bn + c * 32;
                 if (col0 >= p.n) break;                       // uniform: nothing of this chunk is inside the matrix
                 uint32_t v[32];
@@ -457,13 +458,13 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 #pragma unroll
                     for (int j = 0; j < 32; j++) v[j] = __float_as_uint(gelu_erf_tensor_core(__uint_as_float(v[j])));
                 }
-                // the staging tile about to be written was handed to the copy engine with the group's last chunk
+                // the staging tile about to be written was handed to the copy engine with the group's last chunk, or the one before
                 if (issuer) {
                     const long long t0 = eclk ? clock64() : 0;
-                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(GROUPS == 1 ? 1 : 0) : "memory");
                     if (eclk) store_wait += clock64() - t0;
                 }
-                asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+                group_sync();
                 if (HALF && p.out_half) {
                     // f16 output: rows of 32 halves = 64 bytes, plain row-major (the store map has no swizzle)
                     const uint32_t stile = staging + (uint32_t)row_in_tile * 64u;
@@ -488,12 +489,13 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                                      : "memory");
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+                group_sync();
                 if (issuer) {
                     tma_store_3d(&map_c, staging, col0, mt * kGpBlockM, bt * p.splits + sp);
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     dbg_mark(p, 5, (uint32_t)(c + 1));
                 }
+                if (GROUPS == 1) staging = staging == staging_base ? staging_base + kGpStageTileBytes : staging_base;
             }
             if (eclk) p.clocks[local * 8 + 5] = clock64(), p.clocks[local * 8 + 6] = store_wait;
             // every tcgen05.ld of this accumulator has completed (tmem_load_32 waits): the MMA thread may reuse it
@@ -1052,6 +1054,10 @@ std::shared_ptr<void> gemm_persistent_prepare(const GemmParams& g, uint32_t* sta
         p.clocks = table;
     }
     const int stage_bytes = kGpATileBytes + (pair ? p.bn / 2 : p.bn) * 128;
+    // One group where a tile has few K blocks and nothing to compute, so that its stores bound it: they leave in the order of the
+    // columns then.  384 x 512 x 512 x 64: one group 85.6 us, two 94.2, two with a staging tile more each 100; one group
+    // chosen in the kernel instead of compiled 92.
+    p.groups = !pair && p.k_iters <= 8 && g.act == 0 ? 1 : 2;
     const int fixed = 1024 + 2 * kGpStageTileBytes + 16 * 8 + 64 + 64;
     p.stages = std::max(2, std::min(6, (227 * 1024 - fixed) / stage_bytes));
     l->smem_bytes = fixed + p.stages * stage_bytes;
@@ -1073,8 +1079,9 @@ int gemm_persistent_launch(const void* launch, cudaStream_t stream) {
     {
         std::lock_guard<std::mutex> lock(mu);
         if (device >= 0 && device < 64 && !done[device]) {
-            const void* variants[] = {(const void*)gemm_persistent_kernel<false, false>, (const void*)gemm_persistent_kernel<true, false>,
-                                      (const void*)gemm_persistent_kernel<false, true>, (const void*)gemm_persistent_kernel<true, true>};
+            const void* variants[] = {(const void*)gemm_persistent_kernel<false, false, 1>, (const void*)gemm_persistent_kernel<true, false, 1>,
+                                      (const void*)gemm_persistent_kernel<false, false, 2>, (const void*)gemm_persistent_kernel<true, false, 2>,
+                                      (const void*)gemm_persistent_kernel<false, true, 2>, (const void*)gemm_persistent_kernel<true, true, 2>};
             for (const void* v : variants) {
                 cudaError_t e = cudaFuncSetAttribute(v, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
                 if (e != cudaSuccess) return (int)e;
@@ -1086,7 +1093,7 @@ int gemm_persistent_launch(const void* launch, cudaStream_t stream) {
         // clusters of two CTAs, still with the programmatic edge to the previous kernel
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = l.grid;
-        cfg.blockDim = dim3(kGpThreads);
+        cfg.blockDim = dim3(64u + 128u * (unsigned)l.p.groups);   // (two: see gemm_persistent_prepare)
         cfg.dynamicSmemBytes = (size_t)l.smem_bytes;
         cfg.stream = stream;
         cudaLaunchAttribute attr[2];
@@ -1098,11 +1105,14 @@ int gemm_persistent_launch(const void* launch, cudaStream_t stream) {
         attr[1].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 2;
-        if (l.half) return (int)cudaLaunchKernelEx(&cfg, gemm_persistent_kernel<true, true>, l.map_a, l.map_b, l.map_c, l.p);
-        return (int)cudaLaunchKernelEx(&cfg, gemm_persistent_kernel<false, true>, l.map_a, l.map_b, l.map_c, l.p);
+        if (l.half) return (int)cudaLaunchKernelEx(&cfg, gemm_persistent_kernel<true, true, 2>, l.map_a, l.map_b, l.map_c, l.p);
+        return (int)cudaLaunchKernelEx(&cfg, gemm_persistent_kernel<false, true, 2>, l.map_a, l.map_b, l.map_c, l.p);
     }
-    if (l.half) launch_pdl(gemm_persistent_kernel<true, false>, dim3(l.grid), dim3(kGpThreads), (size_t)(l.smem_bytes), stream, l.map_a, l.map_b, l.map_c, l.p);
-    else launch_pdl(gemm_persistent_kernel<false, false>, dim3(l.grid), dim3(kGpThreads), (size_t)(l.smem_bytes), stream, l.map_a, l.map_b, l.map_c, l.p);
+    auto launch_groups = [&](auto kernel) {
+        launch_pdl(kernel, dim3(l.grid), dim3(64u + 128u * (unsigned)l.p.groups), (size_t)(l.smem_bytes), stream, l.map_a, l.map_b, l.map_c, l.p);
+    };
+    if (l.p.groups == 1) launch_groups(l.half ? gemm_persistent_kernel<true, false, 1> : gemm_persistent_kernel<false, false, 1>);
+    else launch_groups(l.half ? gemm_persistent_kernel<true, false, 2> : gemm_persistent_kernel<false, false, 2>);
     return (int)cudaGetLastError();
 }
 
