@@ -631,11 +631,12 @@ int launch_softmax(const RowParams& p, cudaStream_t stream) {
 
 int launch_layernorm(const RowParams& p, cudaStream_t stream) {
     if (p.half) return launch_layernorm_f16(p, stream);
-    // Rows of 257..1024 elements that do not fill the chip as a warp each: what bounds them is the chain of one thread's work, so a
-    // row is a block of 256 threads up to two rows per SM and of 128 up to twelve.  120 rows of 768: a warp each 4.85 us, 128 threads
-    // 2.99, 256 threads 2.55; 333 rows 5.4, 3.07 and 3.20; 1024 rows 5.4, 3.7 and 4.35; 4096 rows 5.8, 8.0 and 10.8.
+    // Rows of 257..1024 elements that do not fill the chip as a warp each: what bounds them is the chain of one thread's work, so up
+    // to twelve rows per SM a row is a block of 128 threads, and up to two per SM, of more than 512 elements, of 256.  120 rows of 768:
+    // a warp each 4.85 us, 128 threads 2.99, 256 threads 2.55; 333 rows 5.4, 3.07 and 3.20; 1024 rows 5.4, 3.7 and 4.35; 4096 rows
+    // 5.8, 8.0 and 10.8.  333 rows of 320: 3.4, 2.8 and 3.0.
     if (p.len > 256 && p.len <= 1024 && p.rows > 0 && p.rows <= 148 * 12 && row_vec4_ok_len(p, 1024)) {
-        if (p.rows <= 148 * 2) launch_pdl(layernorm_vec4_kernel<256, 1>, dim3((unsigned)p.rows), dim3(256), (size_t)0, stream, p);
+        if (p.rows <= 148 * 2 && p.len > 512) launch_pdl(layernorm_vec4_kernel<256, 1>, dim3((unsigned)p.rows), dim3(256), (size_t)0, stream, p);
         else if (p.len <= 512) launch_pdl(layernorm_vec4_kernel<128, 1>, dim3((unsigned)p.rows), dim3(128), (size_t)0, stream, p);
         else launch_pdl(layernorm_vec4_kernel<128, 2>, dim3((unsigned)p.rows), dim3(128), (size_t)0, stream, p);
         return (int)cudaGetLastError();
