@@ -43,8 +43,8 @@ BATCH = 256
 # 0 bytes written back); the two alternate in the trunk, so the mean is quoted.
 TRUNK_CONV_DRAM_BYTES = 13.24e6
 # DRAM bytes per launch of the convolution chain (all 33 tower layers) at batch 256, from one ncu capture
-# of this bench: 20.53 MB read (filters and input, once), 0 written back (the output stays in L2).
-CHAIN_DRAM_BYTES = 20.54e6
+# of this bench: 20.50 MB read (filters and input, once), 0 written back (the output stays in L2).
+CHAIN_DRAM_BYTES = 20.50e6
 WORKLOAD = "resnet_tower_f32_b256 (21x8x8 planes, stem + 16 residual blocks @128ch, policy 73x8x8 softmax, value 3 softmax)"
 
 
@@ -581,7 +581,7 @@ def main():
             flop, kind, desc = dominant[0][1], dominant[0][2], dominant[0][3]
             achieved = flop / (us * 1e-6) / 1e12
             chain = kind.startswith("ConvChain")
-            roofline = {"bound": "tensor", "kernel": ("conv_chain_kernel: " if chain else "tc_conv_cl_kernel: ") + desc,
+            roofline = {"bound": "tensor", "kernel": ("conv_chain_pair_kernel: " if chain else "tc_conv_cl_kernel: ") + desc,
                         "achieved": achieved, "peak": tensor_peak, "unit": "TFLOP/s", "frac": achieved / tensor_peak,
                         "traffic": CHAIN_DRAM_BYTES if chain else TRUNK_CONV_DRAM_BYTES,
                         "peak_source": f"{peaks['source']} bf16 burst / 2 (tf32)", "us_per_launch": us,
