@@ -329,7 +329,9 @@ static const int kClusterSizes[5] = {16, 8, 4, 2, 1}, kClustersFit[5] = {7, 15, 
 // us a layer, launched one by one -> as a chain, 8 x 8 boards. 128 channels, 7 boards (16 CTAs each) 11.0 -> 9.1, 4 8.9 -> 9.1; 15
 // (8) 14.8 -> 12.7, 10 12.3 -> 12.2; 33 (4) 22.6 -> 17.4, 20 17.4 -> 17.1, 16 14.9 -> 16.4; 64 (2) 37.3 -> 29.0, 46 34.8 -> 28.4, 40
 // 27.5 -> 28.2; 148 (1) 66.9 -> 55.6, 120 71.9 -> 55.9, 105 51.9 -> 55.9. 64 channels: faster at every size, 0.52 to 0.89 of the time,
-// at 0.46 and more of a round or with eight CTAs an image.
+// at 0.46 and more of a round or with eight CTAs an image. (Two batches of 22 boards at once: two chains of 0.67 of a round do not run
+// side by side, 1038 us against 1008 launched one by one, which is why 0.6 to 0.7 of a round, where a chain alone gains 0 to 6%, is
+// left out.)
 // Rows of 7 leave an eighth of a thread's work unused.
 bool conv_chain_exact_geometry(int h, int w, int64_t n_img, int c_in, int k, ChainExactGeometry* out) {
     if (w < 7 || w > W || h < 4 || h > 16 || n_img < 1 || c_in < 1 || c_in > 128 || k < 32 || k > 128 || k % 8 != 0) return false;
@@ -338,7 +340,7 @@ bool conv_chain_exact_geometry(int h, int w, int64_t n_img, int c_in, int k, Cha
         const int cluster = kClusterSizes[i];
         if (k % (8 * cluster) != 0 || n_img > kClustersFit[i]) continue;
         const double used = (double)(n_img * w) / (W * kClustersFit[i]);
-        if (k > 64 ? used < (cluster > 1 ? 0.6 : 0.72) : cluster < 8 && used < 0.45) return false;
+        if (k > 64 ? used < (cluster == 2 ? 0.6 : cluster == 1 ? 0.72 : 0.7) : cluster < 8 && used < 0.45) return false;
         g.cluster = cluster;
         g.cols = k / cluster;
         g.items = h * g.cols / 8;

@@ -11,7 +11,7 @@ def chains(g, batch, mode=MATH_F32, flags=0):
     return [l for l in steps(plan_describe(g, batch, mode, flags=flags)) if "ConvChain" in l]
 
 
-@pytest.mark.parametrize("channels,batch,ctas", [(128, 7, 16), (128, 9, 8), (128, 33, 4), (128, 45, 2), (128, 74, 2), (128, 148, 1), (64, 1, 8), (64, 16, 4), (32, 34, 2)])
+@pytest.mark.parametrize("channels,batch,ctas", [(128, 7, 16), (128, 11, 8), (128, 33, 4), (128, 45, 2), (128, 74, 2), (128, 148, 1), (64, 1, 8), (64, 16, 4), (32, 34, 2)])
 def test_ctas_per_image(channels, batch, ctas):
     g = tower(channels, 2, 8, 8, 21)
     line, = chains(g, batch)
@@ -29,7 +29,7 @@ def test_route():
 
 
 CASES = [  # channels, input channels, blocks, h, w, batch
-    (128, 21, 2, 8, 8, 6), (128, 128, 2, 8, 8, 7), (128, 5, 2, 8, 8, 9), (128, 21, 2, 8, 8, 21), (128, 21, 2, 8, 8, 50), (128, 3, 2, 8, 8, 110),
+    (128, 21, 2, 8, 8, 6), (128, 128, 2, 8, 8, 7), (128, 5, 2, 8, 8, 12), (128, 21, 2, 8, 8, 25), (128, 21, 2, 8, 8, 50), (128, 3, 2, 8, 8, 110),
     (64, 21, 2, 7, 7, 2), (64, 64, 2, 8, 8, 12), (64, 9, 2, 16, 8, 3), (64, 1, 2, 8, 8, 75), (96, 30, 2, 7, 7, 33), (32, 100, 2, 8, 7, 20), (40, 1, 2, 5, 8, 90),
 ]
 
