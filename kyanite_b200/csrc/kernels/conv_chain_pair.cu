@@ -50,6 +50,10 @@ using namespace tcp;
 constexpr int kEpilogueWarps = 4, kCols = 32 / kEpilogueWarps;
 constexpr int kEpilogueThreads = 128 * kEpilogueWarps, kThreads = 64 + kEpilogueThreads;
 constexpr uint32_t kSleepNs = 20000u;   // suspend-time hint of the waits
+// Rows of biases in shared memory.  A warp reads its first columns of a layer's row ahead of that layer's accumulator (behind the
+// wait 33 layers of 256 boards take 206.7 us, ahead of it 202.4), so the row is written two layers earlier: row (l + 2) % 3 once
+// accumulator l is complete, handed over with the operand of layer l + 1, which accumulator l + 1 has read.
+constexpr int kBiasRows = 3;
 
 struct ChainPairKernelParams {
     const float* in;
@@ -108,8 +112,8 @@ conv_chain_pair_kernel(const __grid_constant__ CUtensorMap map_trunk, const __gr
     const uint32_t block_bytes = (uint32_t)p.rows_alloc * 128u;
     const uint32_t act_bytes = (uint32_t)p.blocks * block_bytes;
     const uint32_t ring_base = base + act_bytes;
-    const uint32_t bias_base = ring_base + (uint32_t)p.slots * p.slot_bytes;     // 2 x 128 floats
-    const uint32_t bar_base = bias_base + 1024u;
+    const uint32_t bias_base = ring_base + (uint32_t)p.slots * p.slot_bytes;     // kBiasRows x 128 floats
+    const uint32_t bar_base = bias_base + kBiasRows * 512u;
     const uint32_t full_bar = bar_base, empty_bar = full_bar + 8u * p.slots, act_bar = empty_bar + 8u * p.slots;
     const uint32_t accum_bar = act_bar + 8u * 4u, slot_addr = accum_bar + 8u;
     float* bias_s = (float*)(gen_base + (bias_base - base));
@@ -135,7 +139,7 @@ conv_chain_pair_kernel(const __grid_constant__ CUtensorMap map_trunk, const __gr
         const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
         for (uint32_t i = threadIdx.x; i < act_bytes / 16u; i += kThreads) z[i] = zero;
     }
-    if (threadIdx.x < 128) bias_s[threadIdx.x] = p.bias[threadIdx.x];
+    if (threadIdx.x < 128 * min(2, p.n_layers)) bias_s[threadIdx.x] = p.bias[threadIdx.x];
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     cluster_sync_all();   // the peer's barriers are initialised before anything is sent to them
@@ -295,18 +299,19 @@ conv_chain_pair_kernel(const __grid_constant__ CUtensorMap map_trunk, const __gr
             // the next kernel of the stream may be scheduled once every CTA waits for its last layer: early enough to hide its
             // launch, late enough that its CTAs do not sit on this SM for the whole run
             if (last && warp == 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-            // the next layer's bias (its half of the table was last read a layer ago)
+            // the bias of the layer after the next (its row was last read by the layer before this one)
             float next_bias = 0.f;
             const int et = threadIdx.x - 64;
-            if (!last && et < 128) next_bias = p.bias[(l + 1) * 128 + et];
-            const float* layer_bias = bias_s + (l & 1) * 128;
+            const bool fetch_bias = l + 2 < p.n_layers && et < 128;
+            if (fetch_bias) next_bias = p.bias[(l + 2) * 128 + et];
+            const float* layer_bias = bias_s + l % kBiasRows * 128;
             float4 bias[kCols / 4];   // of the columns that come next
 #pragma unroll
             for (int j = 0; j < kCols; j += 4) bias[j / 4] = *(const float4*)(layer_bias + part * kCols + j);
             if (!mbar_wait(accum_bar, (uint32_t)(l & 1), abandon, p.status, 14, kWaitCycles, kSleepNs)) break;
             if (trace) p.trace[l * 8 + 5] = clock64();
             tc_fence_after();
-            if (!last && et < 128) bias_s[((l + 1) & 1) * 128 + et] = next_bias;
+            if (fetch_bias) bias_s[(l + 2) % kBiasRows * 128 + et] = next_bias;
             const int blocks = heads ? (n + 31) / 32 : p.blocks;
 #pragma unroll 1
             for (int cb = 0; cb < blocks; cb++) {
@@ -410,7 +415,7 @@ bool tc_chain_pair_geometry(int h, int w, int64_t n_img, int blocks, int k, int 
             g.n_last = round_up_int(head_channels, 16);
             g.rows_alloc = round_up_int(2 * g.wp + 2 + 15 * g.pitch + 8, 8);
             g.slot_bytes = std::max(3 * g.n_trunk, g.n_last) * 64;
-            const int fixed = 1024 /* alignment */ + 1024 /* bias */ + 16 * 8 + 5 * 8 + 32;
+            const int fixed = 1024 /* alignment */ + kBiasRows * 512 + 16 * 8 + 5 * 8 + 32;
             const int act_bytes = blocks * g.rows_alloc * 128;
             g.slots = std::min(8, (227 * 1024 - fixed - act_bytes) / g.slot_bytes);
             if (g.slots < 2) break;

@@ -70,6 +70,31 @@ def test_infinity_and_nan_stay_in_their_image():
     assert not np.isfinite(got[4][:, 2:5, 2:5]).any() and not np.isfinite(got[7][:, 0:2, 6:8]).any()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("channels", [16, 32, 72, 128])
+def test_every_layer_adds_its_own_bias(channels):
+    """Identity filters and small whole biases: each layer's bias counts, exactly, also with two executors at work at a time (the
+    table of biases in shared memory is written while earlier rows of it are read)."""
+    from kyanite_b200.executor import CudaExecutor
+    r, g, layers = rng(channels), Graph(), 30
+    biases = r.integers(-9, 10, (layers, channels)).astype(np.float32)
+    w = np.zeros((channels, channels, 3, 3), np.float32)
+    w[range(channels), range(channels), 1, 1] = 1
+    cur = g.input(shape(BATCH, channels, 8, 8))
+    for b in biases:
+        cur = g.add(g.conv(cur, g.constant_tensor(w), 1, 1, 1, 1), g.constant_tensor(b.reshape(1, channels, 1, 1)))
+    g.output(cur)
+    assert any("on CTA pairs" in l and "layers=%d" % layers in l for l in steps(plan_describe(g, 300, MATH_TF32)))
+    x = r.integers(-9, 10, (300, channels, 8, 8)).astype(np.float32)
+    want = x + biases.sum(0).reshape(1, channels, 1, 1)    # (at most 280: exact in TF32)
+    with CudaExecutor(0, g, 300, math_mode=MATH_TF32) as a, CudaExecutor(0, g, 300, math_mode=MATH_TF32) as b:
+        for _ in range(20):
+            a.evaluate_begin([x])
+            b.evaluate_begin([x])
+            np.testing.assert_array_equal(a.evaluate_end()[0], want)
+            np.testing.assert_array_equal(b.evaluate_end()[0], want)
+
+
 def test_heads_of_large_batches_join_the_chain():
     """A 1x1 convolution large enough to be a matmul of its own stays with the chain whose result it reads, if all of them fit."""
     g, _ = resnet_tower()
