@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kThreads) dense_chain_kernel(const __grid_cons
                 for (int c = 0; c < 4; c++) {
                     if (c >= groups) break;
                     const int n = c * 32 + lane;
-                    if (!last) values[warp][r][n] = y[r][c];   // (columns past n: weights and bias of zero)
+                    if (!last) values[warp][r][n] = n < d.n ? y[r][c] : 0.f;   // (past n: NaN where the row holds an infinity)
                     else if (n < d.n) p.out[(row0 + r) * p.out_row + n] = y[r][c];
                 }
             }

@@ -78,3 +78,21 @@ def test_a_result_that_is_read_elsewhere_is_stored():
         hidden, got = ex.evaluate([x])
     h = np.tanh(np.maximum(want(x, weights[:2], False), 0))
     assert np.abs(hidden - h).max() <= 4e-6 and np.abs(got - want(x, weights, True)).max() <= 4e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("widths", [[7, 9, 30, 3], [5, 33, 12], [8, 11, 6, 21]])
+@pytest.mark.parametrize("rows", [3, 2369])
+def test_infinities_stay_infinities(widths, rows):
+    """Positive weights and no activation: a row with an infinity is infinite in every column, behind layers of any width."""
+    from kyanite_b200.executor import CudaExecutor
+    g = Graph()
+    y = g.input(shape(BATCH, widths[0]))
+    for k, n in zip(widths, widths[1:]):
+        y = g.linear(y, g.constant_tensor(np.full((n, k), 0.25, np.float32)))
+    g.output(y)
+    x = np.ones((rows, widths[0]), np.float32)
+    x[1, 0], x[2, 3] = np.inf, -np.inf
+    with CudaExecutor(0, g, rows, math_mode=MATH_F32) as ex:
+        got, = ex.evaluate([x])
+    assert (got[1] == np.inf).all() and (got[2] == -np.inf).all() and np.isfinite(np.delete(got, [1, 2], 0)).all()
