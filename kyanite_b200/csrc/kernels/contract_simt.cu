@@ -454,9 +454,12 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
 //    32 x 32, 4 x 4 per thread, four groups: for problems of a few tiles, where it is the number of CTAs that counts
 // What a small problem costs is latency, so: the constant operand is requested ahead of the dependency wait, for as many
 // stages as there are; rows are located once, in a table, and not by divisions in the loop; slices of a tile send their sums to
-// the CTA that stores them (a cluster barrier that the peers have started, waited for at the first remote store, and a barrier in
-// the receiver's memory that counts the bytes of the sums, `st.async`: a second cluster barrier has to release what it hands
-// over, which takes some 1000 cycles; no remote reads).
+// the CTA that stores them (a cluster barrier that the peers have started, waited for at the first remote store; no remote reads).
+// COUNTED: that they have arrived is told by a barrier in the receiver's memory that counts their bytes (`st.async`), not by a
+// second cluster barrier, which has to release what it hands over and takes some 1000 cycles.  Only where a CTA has its SM to itself
+// or tiles are small: where two and more large tiles share an SM another CTA computes meanwhile, and the code with the counter
+// is the slower one even without slices (seven layers of 128 channels: 40 boards 178 -> 186 us with it, 95 373 -> 382,
+// 256 717 -> 723; 34 147.7 -> 147.7; eight boards of 256 channels 104 -> 106).
 // One 8 x 8 board, 128 -> 128 channels, 3 x 3: 12.1 us on contract_simt_kernel, 5.2 us here (5.6 with a second cluster barrier)
 // (in a chain; by itself 7.4, kernel_bench's conv_exact_board); 64 boards 48 -> 36 us, 256 boards 112 us
 // (0.61 of the rate); 12 heads of 120 x 64 x 120 (probabilities . V) 14.1 -> 4.8 us.
@@ -480,7 +483,7 @@ struct ColsArgs {
     bool wide_c;      // four columns of the result are one aligned 16-byte store
 };
 
-template <class Problem, int BM, int BN, int TM, int TN, int KG, int ST, int OCC>
+template <class Problem, int BM, int BN, int TM, int TN, int KG, int ST, int OCC, bool COUNTED>
 __global__ void __launch_bounds__(BM / TM * (BN / TN) * KG, OCC)
 contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant__ ColsArgs args) {
     using L = ColsLayout<BM, BN, TM, TN, KG, ST>;
@@ -493,16 +496,17 @@ contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int slices = args.slices;
     const int slice = (int)(blockIdx.z % (unsigned)slices);
-    // units of four columns of the result, of which each slice stores `share`
-    const int share = (L::kUnits + slices - 1) / slices;
     const uint32_t arrived = smem_addr(smem + L::kBarrier);
     if (slices > 1) {
-        if (threadIdx.x == 0) {
-            tcp::mbar_init(arrived, 1);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            tcp::mbar_expect_tx(arrived, (uint32_t)(max(0, min(share, L::kUnits - slice * share)) * slices) * 16u);
+        if (COUNTED) {
+            if (threadIdx.x == 0) {
+                const int share = (L::kUnits + slices - 1) / slices;
+                tcp::mbar_init(arrived, 1);
+                asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+                tcp::mbar_expect_tx(arrived, (uint32_t)(max(0, min(share, L::kUnits - slice * share)) * slices) * 16u);
+            }
+            __syncwarp();
         }
-        __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (waited for before the first remote store)
     }
     const int64_t M = prob.rows(), N = prob.cols();
@@ -686,7 +690,9 @@ contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant
                 make_float4(acc[i][2 * j].x, acc[i][2 * j].y, acc[i][2 * j + 1].x, acc[i][2 * j + 1].y);
     __syncthreads();
     if (slices > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    // units of four columns, in the order in which the result's contiguous axis comes first
+    // units of four columns, in the order in which the result's contiguous axis comes first; of several slices, each
+    // stores `share` of them
+    const int share = (L::kUnits + slices - 1) / slices;
     auto place = [&](int u, int& mm, int& nn) {
         mm = args.rows_fast ? u % BM : u / (BN / 4);
         nn = (args.rows_fast ? u / BM : u % (BN / 4)) * 4;
@@ -722,18 +728,26 @@ contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant
         } else {
             const int owner = u / share;
             const uint32_t to = tcp::map_to_cta(smem_addr(received + slice * share + u - owner * share), (uint32_t)owner);
-            asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
-                         ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(tcp::map_to_cta(arrived, (uint32_t)owner))
-                         : "memory");
+            if constexpr (COUNTED)
+                asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                             ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(tcp::map_to_cta(arrived, (uint32_t)owner))
+                             : "memory");
+            else
+                asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
         }
     }
     if (slices > 1) {
-        const long long start = clock64();
-        while (!tcp::mbar_try_wait_cluster(arrived, 0)) {
-            if (clock64() - start > tcp::kWaitCycles) {
-                atomicMax(prob.p.status, 71u);
-                return;
+        if constexpr (COUNTED) {
+            const long long start = clock64();
+            while (!tcp::mbar_try_wait_cluster(arrived, 0)) {
+                if (clock64() - start > tcp::kWaitCycles) {
+                    atomicMax(prob.p.status, 71u);
+                    return;
+                }
             }
+        } else {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         }
         for (int u = tid; u < share && slice * share + u < L::kUnits; u += NT) {
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -749,10 +763,10 @@ contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant
     }
 }
 
-template <class Problem, int BM, int BN, int TM, int TN, int KG, int ST, int OCC>
+template <class Problem, int BM, int BN, int TM, int TN, int KG, int ST, int OCC, bool COUNTED>
 int launch_cols_tile(const Problem& prob, int64_t M, int64_t N, int64_t batch, const ColsArgs& args, int at_least, cudaStream_t stream) {
     using L = ColsLayout<BM, BN, TM, TN, KG, ST>;
-    auto kernel = contract_cols_kernel<Problem, BM, BN, TM, TN, KG, ST, OCC>;
+    auto kernel = contract_cols_kernel<Problem, BM, BN, TM, TN, KG, ST, OCC, COUNTED>;
     static std::mutex mu;
     static bool done[64] = {false};
     const int smem = std::max(L::kBytes, at_least);
@@ -796,11 +810,11 @@ int launch_cols(const Problem& prob, int64_t M, int64_t N, int64_t batch, int64_
         consider(kSmall, small, slices);
         consider(large * slices <= 148 ? kLargeAlone : kLarge, large, slices);
     }
-    if (tile == kSmall) return launch_cols_tile<Problem, 32, 32, 4, 4, 4, 6, 2>(prob, M, N, batch, args, 0, stream);
-    if (tile == kLargeAlone) return launch_cols_tile<Problem, 64, 64, 8, 8, 4, 3, 1>(prob, M, N, batch, args, 0, stream);
+    if (tile == kSmall) return launch_cols_tile<Problem, 32, 32, 4, 4, 4, 6, 2, true>(prob, M, N, batch, args, 0, stream);
+    if (tile == kLargeAlone) return launch_cols_tile<Problem, 64, 64, 8, 8, 4, 3, 1, true>(prob, M, N, batch, args, 0, stream);
     // (two CTAs an SM are kept at two by the shared memory they ask for: three on some SMs and one on others took 81 us
     // instead of 57 for 1024 x 1024 x 1024)
-    return launch_cols_tile<Problem, 64, 64, 8, 8, 2, 3, 3>(prob, M, N, batch, args, per_sm == 2 ? 80 * 1024 : 0, stream);
+    return launch_cols_tile<Problem, 64, 64, 8, 8, 2, 3, 3, false>(prob, M, N, batch, args, per_sm == 2 ? 80 * 1024 : 0, stream);
 }
 
 template <class Problem, int BM, int BN, int TN, int KG, class Index = int>
