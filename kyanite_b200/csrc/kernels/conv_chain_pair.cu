@@ -101,8 +101,10 @@ __device__ __forceinline__ uint32_t operand_bits(uint32_t u) {
     return (u & 0x7F800000u) != 0x7F800000u ? u + 0x1000u : u;
 }
 
-// TRACE: whether the first CTA stamps its phases
-template <bool TRACE>
+// TRACE: whether the first CTA stamps its phases.  PARTIAL: the trunk's last channel block has columns that are no channels, which
+// are kept zero (a test of them in every variant costs 1.7 to 4 %: 157 -> 163.6 us for 17 layers of 64 channels, 101 boards of 9 x 9,
+// with the copies of the call)
+template <bool TRACE, bool PARTIAL>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_chain_pair_kernel(const __grid_constant__ CUtensorMap map_trunk, const __grid_constant__ CUtensorMap map_last,
                        const __grid_constant__ ChainPairKernelParams p) {
@@ -338,8 +340,15 @@ conv_chain_pair_kernel(const __grid_constant__ CUtensorMap map_trunk, const __gr
                             // (behind a ReLU there is no NaN, and infinity stays what it is without a test)
                             r[i] = relu ? (v[j + i] + 0x1000u) & 0xFFFFE000u : operand_bits(v[j + i]);
                         }
+                        if (PARTIAL && c0 + kCols > p.k) {   // (what the zeros of the filter make of an infinity is NaN)
+#pragma unroll
+                            for (int i = 0; i < 4; i++) r[i] = c0 + j + i < p.k ? r[i] : 0u;
+                        }
                         if (!last && real) store_operand(cb, (part * kCols + j) / 4, r[0], r[1], r[2], r[3]);
                     }
+                } else if (PARTIAL && l == 0 && !last && real) {   // (an input wider than the trunk: its last channels are in the operand)
+#pragma unroll
+                    for (int j = 0; j < kCols; j += 4) store_operand(cb, (part * kCols + j) / 4, 0u, 0u, 0u, 0u);
                 }
                 if (!last) block_done(cb);
                 if (trace && cb == 0) p.trace[l * 8 + 7] = clock64();
@@ -504,9 +513,11 @@ std::shared_ptr<void> chain_pair_prepare(const ConvChainParams& c, uint32_t* sta
 int chain_pair_launch(const void* launch, cudaStream_t stream) {
     const ChainPairLaunch& l = *(const ChainPairLaunch*)launch;
     static std::mutex mu;
-    static bool done[2][64] = {};
-    auto kernel = l.p.trace ? conv_chain_pair_kernel<true> : conv_chain_pair_kernel<false>;
-    if (int e = allow_shared(kernel, 227 * 1024, done[l.p.trace ? 1 : 0], mu)) return e;
+    static bool done[4][64] = {};
+    const bool trace = l.p.trace != nullptr, partial = l.p.k % 32 != 0;
+    auto kernel = trace ? (partial ? conv_chain_pair_kernel<true, true> : conv_chain_pair_kernel<true, false>)
+                        : (partial ? conv_chain_pair_kernel<false, true> : conv_chain_pair_kernel<false, false>);
+    if (int e = allow_shared(kernel, 227 * 1024, done[2 * trace + partial], mu)) return e;
     if (l.grid.x == 0) return 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = l.grid;

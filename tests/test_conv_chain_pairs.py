@@ -71,6 +71,27 @@ def test_infinity_and_nan_stay_in_their_image():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("channels,c_in", [(48, 60), (20, 8), (40, 64), (64, 100), (128, 128), (12, 3)])
+def test_infinity_reaches_its_neighbours_only(channels, c_in):
+    """Positive weights and no activation: within reach of an infinity every channel is infinite, nothing is NaN."""
+    from kyanite_b200.executor import CudaExecutor
+    g, layers = Graph(), 3
+    cur = g.input(shape(BATCH, c_in, 8, 8))
+    for c in [c_in] + [channels] * (layers - 1):
+        cur = g.conv(cur, g.constant_tensor(np.full((channels, c, 3, 3), 0.125, np.float32)), 1, 1, 1, 1)
+    g.output(cur)
+    assert any("on CTA pairs" in l for l in steps(plan_describe(g, 5, MATH_TF32)))
+    x = np.ones((5, c_in, 8, 8), np.float32)
+    x[3, c_in - 1, 2, 7] = np.inf
+    want = np.zeros((5, channels, 8, 8), bool)
+    want[3, :, :6, 4:] = True
+    with CudaExecutor(0, g, 5, math_mode=MATH_TF32) as ex:
+        got, = ex.evaluate([x])
+    np.testing.assert_array_equal(got == np.inf, want)
+    assert np.isfinite(got[~want]).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("channels", [16, 32, 72, 128])
 def test_every_layer_adds_its_own_bias(channels):
     """Identity filters and small whole biases: each layer's bias counts, exactly, also with two executors at work at a time (the
