@@ -198,6 +198,7 @@ conv_chain_exact_kernel(const __grid_constant__ ExactKernelParams p) {
             for (int i = 0; i < U; i++) b[i] = p.bias[l * 128 + channel[i]];
             const float* a_at = act + (works ? group * per_group : 0) * p.act_floats + row * kPitch;
             const int chunks = p.chunks[l];
+            ok = __all_sync(0xffffffffu, ok);   // (the lanes of a warp waited one by one, and vote in the loop)
             if (last && tid == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             for (int c = 0; c < chunks && ok; c++, a_at += p.chunk * p.act_floats) {
                 if (tid == 0) ok = load_next();
