@@ -263,6 +263,12 @@ conv_chain_exact_kernel(const __grid_constant__ ExactKernelParams p) {
                     : "memory");
                 if (!all) break;
             }
+            if (l == 0 && p.c_in > p.k && p.channels > p.k) {
+                // an input wider than the trunk: the channels that whole chunks add to the next layers are none of it (zero weights
+                // make NaN of an infinity)
+                for (int i = p.k * p.act_floats + tid; i < p.channels * p.act_floats; i += kWorkers) act[i] = 0.f;
+                sync_workers();
+            }
             // this CTA has read its input: the cluster may write the next layer's over it
             if (!last && tid < p.cluster) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(map_to_cta(ready, (uint32_t)tid)) : "memory");
             float4 y[U];

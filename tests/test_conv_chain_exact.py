@@ -4,6 +4,7 @@ import pytest
 
 from kyanite_b200.executor import FLAG_NO_CONV_CHAIN, MATH_F32, MATH_TF32, plan_describe
 from oracle.cpu_eval import cpu_eval_graph
+from kyanite_b200.graph import BATCH, Graph, shape
 from test_conv_chain import rng, steps, tower
 
 
@@ -49,3 +50,25 @@ def test_matches_oracle(channels, c_in, blocks, h, w, batch, residual):
         # five layers of f32 sums of up to 1152 terms in another order: 1e-5 of the scale
         assert np.abs(got.astype(np.float64) - expected).max() <= 1e-5 * np.abs(expected).max()
         np.testing.assert_array_equal(got, ex.evaluate([x])[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("channels,c_in,batch", [(48, 60, 100), (40, 64, 90), (80, 100, 70), (96, 128, 30), (128, 21, 7)])
+def test_infinity_reaches_its_neighbours_only(channels, c_in, batch):
+    """Positive weights and no activation: within reach of an infinity every channel is infinite, nothing is NaN.  (Whole chunks of
+    weights go past the channels of the trunk in most of these.)"""
+    from kyanite_b200.executor import CudaExecutor
+    g, layers = Graph(), 4
+    cur = g.input(shape(BATCH, c_in, 8, 8))
+    for c in [c_in] + [channels] * (layers - 1):
+        cur = g.conv(cur, g.constant_tensor(np.full((channels, c, 3, 3), 0.125, np.float32)), 1, 1, 1, 1)
+    g.output(cur)
+    assert chains(g, batch)
+    x = np.ones((batch, c_in, 8, 8), np.float32)
+    x[3, c_in - 1, 1, 7] = np.inf
+    want = np.zeros((batch, channels, 8, 8), bool)
+    want[3, :, :6, 3:] = True
+    with CudaExecutor(0, g, batch, math_mode=MATH_F32) as ex:
+        got, = ex.evaluate([x])
+    np.testing.assert_array_equal(got == np.inf, want)
+    assert np.isfinite(got[~want]).all()
