@@ -12,9 +12,10 @@
 // Weights stream through a ring by bulk copies, prefetched across layers.
 //
 // What bounds it: instruction issue.  An input channel is 288 packed multiply-adds a thread, which issue every other cycle, and some
-// 120 reads and moves beside them: 780 cycles for 576 (plain multiply-adds: 940).  Per layer some 4 000 cycles more: partial sums, the
-// wait for the slowest CTA of the cluster, remote stores at 16 bytes a cycle.  64 boards of 8 x 8, 128 channels: 36.5 us a layer
-// launched one by one, 29.0 here (0.56 of the multiply-add rate).
+// 120 reads and moves beside them: 780 cycles for 576 (plain multiply-adds: 940).  The rest of a layer is partial sums, the wait for
+// the slowest CTA of the cluster and remote stores at 16 bytes a cycle: some 7 000 of 58 000 cycles at two CTAs an image, and at
+// sixteen, whose arithmetic is 3 000, five sixths of them.  64 boards of 8 x 8, 128 channels: 36.5 us a layer launched one by one,
+// 29.7 here (0.55 of the multiply-add rate).
 //
 // Every wait is bounded; on expiry the executor's status word is raised and all roles leave.
 #include <cuda_runtime.h>
@@ -40,6 +41,12 @@ constexpr int kPitch = 12;       // floats of an image row in shared memory: x =
 constexpr int W = 8;             // positions of a row that a thread computes
 constexpr int kQuads = W / 4;    // groups of four positions
 constexpr int kSums = 8 * kQuads;            // partial sums of a thread, in float4
+// Products that a thread sums one behind the other, about: the sums of such segments of its input channels are summed by themselves, and
+// so are four groups' at a time.  With one sum over all of a thread's products chains were up to twice as far from 64 bits as
+// the layers launched one by one (nine layers of 128 channels: 130 boards 1.98 times, 46 1.44, 25 1.17); now 0.70 to 1.00 times.  A
+// segment's end costs 0.5 to 0.9 us a layer and moves 64 boards from 29.0 to 29.7 us a layer.  (At 72 products 64 boards took
+// 30.7; sums kept in tensor memory instead of shared memory no less.)
+constexpr int kSegment = 96;
 
 struct ExactKernelParams {
     const float* in;
@@ -50,6 +57,7 @@ struct ExactKernelParams {
     int32_t c_in, k, h, w;
     int32_t n_layers, cluster, cols, col_groups, k_groups, items;   // cols: output channels of a CTA; items = h * col_groups
     int32_t chunk, slots, channels;      // input channels of a weight chunk; ring slots; input channels that shared memory holds
+    int32_t segment;                     // chunks that are summed by themselves, or 0: all of them
     int32_t act_floats;                  // of a channel: (h + 2) * kPitch
     uint8_t flags[kMaxChainLayers];
     uint8_t chunks[kMaxChainLayers];     // weight chunks of the layer
@@ -62,8 +70,8 @@ __device__ __forceinline__ void store_async(uint32_t addr, uint32_t bar, float4 
                  : "memory");
 }
 
-// U: results of a thread, in groups of four (at most)
-template <int U>
+// U: results of a thread, in groups of four (at most).  SEGMENTED: a layer's input channels are more than one segment
+template <int U, bool SEGMENTED>
 __global__ void __launch_bounds__(kWorkers, 1)
 conv_chain_exact_kernel(const __grid_constant__ ExactKernelParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -187,69 +195,87 @@ conv_chain_exact_kernel(const __grid_constant__ ExactKernelParams p) {
         for (int l = 0; l < p.n_layers; l++) {
             const uint32_t flags = p.flags[l];
             const bool last = l == p.n_layers - 1;
-            if (l > 0) ok = mbar_wait_cluster(act_full, (uint32_t)((l - 1) & 1), abandon, p.status, 62);
-            float2 acc[W][4];
-#pragma unroll
-            for (int x = 0; x < W; x++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[x][j] = make_float2(0.f, 0.f);
             float b[U];
 #pragma unroll
             for (int i = 0; i < U; i++) b[i] = p.bias[l * 128 + channel[i]];
+            if (l > 0) ok = mbar_wait_cluster(act_full, (uint32_t)((l - 1) & 1), abandon, p.status, 62);
             const float* a_at = act + (works ? group * per_group : 0) * p.act_floats + row * kPitch;
             const int chunks = p.chunks[l];
             ok = __all_sync(0xffffffffu, ok);   // (the lanes of a warp waited one by one, and vote in the loop)
             if (last && tid == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-            for (int c = 0; c < chunks && ok; c++, a_at += p.chunk * p.act_floats) {
-                if (tid == 0) ok = load_next();
-                ok = ok && mbar_wait(full_bar + 8u * slot, (uint32_t)(round & 1), abandon, p.status, 63);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                if (works) {
-                    // Loads run one step ahead of their use: the weights of the next tap, the values of the next filter row
-                    const float* a_row = a_at;
-                    const float* w_at = (const float*)(smem + ring_at + slot * (int)chunk_bytes) + group * per_group * 9 * p.cols + cg * 8;
-                    float a[W + 2];
-                    float4 w0 = *(const float4*)w_at, w1 = *(const float4*)(w_at + 4);
-                    load_row(a, a_row);
+            int c = 0;
+            do {   // (a segment)
+                const int from_c = c, to = SEGMENTED ? min(chunks, c + p.segment) : chunks;
+                float2 acc[W][4];
+#pragma unroll
+                for (int x = 0; x < W; x++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[x][j] = make_float2(0.f, 0.f);
+                for (; c < to && ok; c++, a_at += p.chunk * p.act_floats) {
+                    if (tid == 0) ok = load_next();
+                    ok = ok && mbar_wait(full_bar + 8u * slot, (uint32_t)(round & 1), abandon, p.status, 63);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    if (works) {
+                        // Loads run one step ahead of their use: the weights of the next tap, the values of the next filter row
+                        const float* a_row = a_at;
+                        const float* w_at = (const float*)(smem + ring_at + slot * (int)chunk_bytes) + group * per_group * 9 * p.cols + cg * 8;
+                        float a[W + 2];
+                        float4 w0 = *(const float4*)w_at, w1 = *(const float4*)(w_at + 4);
+                        load_row(a, a_row);
 #pragma unroll 1
-                    for (int left = per_group; left > 0; left--) {
-                        const float* a_next = left > 1 ? a_row + p.act_floats : a_row;
+                        for (int left = per_group; left > 0; left--) {
+                            const float* a_next = left > 1 ? a_row + p.act_floats : a_row;
 #pragma unroll
-                        for (int dy = 0; dy < 3; dy++) {
-                            float b[W + 2];
-                            load_row(b, dy < 2 ? a_row + (dy + 1) * kPitch : a_next);
+                            for (int dy = 0; dy < 3; dy++) {
+                                float b[W + 2];
+                                load_row(b, dy < 2 ? a_row + (dy + 1) * kPitch : a_next);
 #pragma unroll
-                            for (int dx = 0; dx < 3; dx++) {
-                                if (dy * 3 + dx < 8 || left > 1) w_at += p.cols;   // (the chunk's last tap: read once more)
-                                const float4 n0 = *(const float4*)w_at, n1 = *(const float4*)(w_at + 4);
-                                const float2 w[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
+                                for (int dx = 0; dx < 3; dx++) {
+                                    if (dy * 3 + dx < 8 || left > 1) w_at += p.cols;   // (the chunk's last tap: read once more)
+                                    const float4 n0 = *(const float4*)w_at, n1 = *(const float4*)(w_at + 4);
+                                    const float2 w[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
 #pragma unroll
-                                for (int j = 0; j < 4; j++)
+                                    for (int j = 0; j < 4; j++)
 #pragma unroll
-                                    for (int x = 0; x < W; x++) acc[x][j] = fma_pair(make_float2(a[x + dx], a[x + dx]), w[j], acc[x][j]);
-                                w0 = n0, w1 = n1;
+                                        for (int x = 0; x < W; x++) acc[x][j] = fma_pair(make_float2(a[x + dx], a[x + dx]), w[j], acc[x][j]);
+                                    w0 = n0, w1 = n1;
+                                }
+#pragma unroll
+                                for (int x = 0; x < W + 2; x++) a[x] = b[x];
                             }
-#pragma unroll
-                            for (int x = 0; x < W + 2; x++) a[x] = b[x];
+                            a_row = a_next;
                         }
-                        a_row = a_next;
                     }
+                    __syncwarp();
+                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty_bar + 8u * slot) : "memory");
+                    if (++slot == p.slots) { slot = 0; round++; }
                 }
-                __syncwarp();
-                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty_bar + 8u * slot) : "memory");
-                if (++slot == p.slots) { slot = 0; round++; }
-            }
-            // partial sums, [quad of a channel][thread]
+                // partial sums, [quad of a channel][thread]
+                if (!SEGMENTED || from_c == 0) {
 #pragma unroll
-            for (int ch = 0; ch < 8; ch++)
+                    for (int ch = 0; ch < 8; ch++)
 #pragma unroll
-                for (int q = 0; q < kQuads; q++) {
-                    float v[4];
+                        for (int q = 0; q < kQuads; q++) {
+                            float v[4];
 #pragma unroll
-                    for (int x = 0; x < 4; x++) v[x] = ch & 1 ? acc[4 * q + x][ch / 2].y : acc[4 * q + x][ch / 2].x;
-                    partial[(ch * kQuads + q) * kWorkers + tid] = make_float4(v[0], v[1], v[2], v[3]);
+                            for (int x = 0; x < 4; x++) v[x] = ch & 1 ? acc[4 * q + x][ch / 2].y : acc[4 * q + x][ch / 2].x;
+                            partial[(ch * kQuads + q) * kWorkers + tid] = make_float4(v[0], v[1], v[2], v[3]);
+                        }
+                } else {
+#pragma unroll
+                    for (int ch = 0; ch < 8; ch++)
+#pragma unroll
+                        for (int q = 0; q < kQuads; q++) {
+                            float v[4];
+#pragma unroll
+                            for (int x = 0; x < 4; x++) v[x] = ch & 1 ? acc[4 * q + x][ch / 2].y : acc[4 * q + x][ch / 2].x;
+                            float4& at = partial[(ch * kQuads + q) * kWorkers + tid];
+                            const float4 t = at;
+                            at = make_float4(t.x + v[0], t.y + v[1], t.z + v[2], t.w + v[3]);
+                        }
                 }
+            } while (SEGMENTED && c < chunks && ok);
             if (tid == 0 && !last) mbar_expect_tx(act_full, (uint32_t)(n_units * p.cluster) * 16u);   // the next layer's input
             {   // (the workers agree on going on: none may be left waiting in a barrier)
                 uint32_t all;
@@ -276,8 +302,17 @@ conv_chain_exact_kernel(const __grid_constant__ ExactKernelParams p) {
             for (int i = 0; i < U; i++) {
                 if (!has_unit(i)) continue;
                 float4 s = partial[from[i]];
-#pragma unroll 8
-                for (int g = 1; g < p.k_groups; g++) {
+                int g = 1;
+#pragma unroll 2
+                for (; g + 4 <= p.k_groups; g += 4) {
+                    float4 t[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) t[q] = partial[from[i] + (g + q) * items];
+                    s.x += (t[0].x + t[1].x) + (t[2].x + t[3].x), s.y += (t[0].y + t[1].y) + (t[2].y + t[3].y);
+                    s.z += (t[0].z + t[1].z) + (t[2].z + t[3].z), s.w += (t[0].w + t[1].w) + (t[2].w + t[3].w);
+                }
+#pragma unroll 1
+                for (; g < p.k_groups; g++) {
                     const float4 t = partial[from[i] + g * items];
                     s.x += t.x, s.y += t.y, s.z += t.z, s.w += t.w;
                 }
@@ -333,9 +368,9 @@ struct ExactLaunch {
 static const int kClusterSizes[5] = {16, 8, 4, 2, 1}, kClustersFit[5] = {7, 15, 33, 74, 148};
 
 // The layers take the same time however many of the clusters of a round there are, so the rule looks at how full the round is:
-// us a layer, launched one by one -> as a chain, 8 x 8 boards. 128 channels, 7 boards (16 CTAs each) 11.0 -> 9.1, 4 8.9 -> 9.1; 15
-// (8) 14.8 -> 12.7, 10 12.3 -> 12.2; 33 (4) 22.6 -> 17.4, 20 17.4 -> 17.1, 16 14.9 -> 16.4; 64 (2) 37.3 -> 29.0, 46 34.8 -> 28.4, 40
-// 27.5 -> 28.2; 148 (1) 66.9 -> 55.6, 120 71.9 -> 55.9, 105 51.9 -> 55.9. 64 channels: faster at every size, 0.52 to 0.89 of the time,
+// us a layer, launched one by one -> as a chain, 8 x 8 boards (13 layers, the first of 21 channels). 128 channels, 6 boards (16 CTAs
+// each) 12.2 -> 7.8, 5 7.9 -> 7.8; 12 (8) 19.1 -> 11.0, 11 10.7 -> 11.0; 24 (4) 23.9 -> 15.3, 20 13.8 -> 15.3; 45 (2) 31.6 -> 26.6, 40
+// 23.0 -> 26.6; 120 (1) 68.4 -> 53.0, 112 64.0 -> 53.1, 110 49.0 -> 53.1. 64 channels: faster at every size, 0.42 to 0.87 of the time,
 // at 0.46 and more of a round or with eight CTAs an image. (Two batches of 22 boards at once: two chains of 0.67 of a round do not run
 // side by side, 1038 us against 1008 launched one by one, which is why 0.6 to 0.7 of a round, where a chain alone gains 0 to 6%, is
 // left out.)
@@ -405,6 +440,9 @@ std::shared_ptr<void> chain_exact_prepare(const ConvChainParams& c, uint32_t* st
     p.k_groups = g.k_groups;
     p.items = g.items;
     p.chunk = g.chunk;
+    const int chunks = (c.k + g.chunk - 1) / g.chunk, products = 9 * g.chunk / g.k_groups;   // of a thread in a chunk
+    const int segments = std::max((chunks * products + kSegment - 1) / kSegment, chunks * products > kSegment / 2 ? 2 : 1);
+    p.segment = segments > 1 ? (chunks + segments - 1) / segments : 0;
     p.slots = g.slots;
     p.channels = g.channels;
     p.act_floats = g.act_floats;
@@ -422,13 +460,15 @@ std::shared_ptr<void> chain_exact_prepare(const ConvChainParams& c, uint32_t* st
 int chain_exact_launch(const void* launch, cudaStream_t stream) {
     const ExactLaunch& l = *(const ExactLaunch*)launch;
     static std::mutex mu;
-    static bool done[2][64] = {};
-    auto kernel = l.units > 4 ? conv_chain_exact_kernel<8> : conv_chain_exact_kernel<4>;
+    static bool done[4][64] = {};
+    const bool segmented = l.p.segment != 0;
+    auto kernel = l.units > 4 ? (segmented ? conv_chain_exact_kernel<8, true> : conv_chain_exact_kernel<8, false>)
+                              : (segmented ? conv_chain_exact_kernel<4, true> : conv_chain_exact_kernel<4, false>);
     int device = 0;
     cudaGetDevice(&device);
     {
         std::lock_guard<std::mutex> lock(mu);
-        bool& set = done[l.units > 4][device & 63];
+        bool& set = done[2 * (l.units > 4) + segmented][device & 63];
         if (!set) {
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);

@@ -72,3 +72,44 @@ def test_infinity_reaches_its_neighbours_only(channels, c_in, batch):
         got, = ex.evaluate([x])
     np.testing.assert_array_equal(got == np.inf, want)
     assert np.isfinite(got[~want]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("channels,batch", [(128, 130), (128, 46), (128, 25), (128, 12), (128, 7), (64, 46)])
+def test_no_further_from_64_bits_than_one_by_one(channels, batch):
+    """Five layers; as many sums are compared as make the ratio repeat to 2 % from one set of weights to the next."""
+    from kyanite_b200.executor import CudaExecutor
+    g = tower(channels, 2, 8, 8, 21, seed=channels + batch)
+    assert chains(g, batch)
+    x = rng(batch).standard_normal((batch, 21, 8, 8)).astype(np.float32)
+    results = []
+    for flags in (0, FLAG_NO_CONV_CHAIN):
+        with CudaExecutor(0, g, batch, math_mode=MATH_F32, flags=flags) as ex:
+            results.append(ex.evaluate([x])[0].astype(np.float64))
+    want = in_64_bits(g, x)
+    chain, single = (np.sqrt(((r - want) ** 2).mean()) for r in results)
+    assert chain <= 1.03 * single
+
+
+def in_64_bits(g, x):
+    """The graph of `tower`: convolutions, sums and ReLUs, node by node."""
+    from kyanite_b200.graph import BinaryOp, OpKind
+    values = g.all_values()
+    at = {}
+    for i, v in enumerate(values):
+        info = g[v]
+        a = [at[k] for k in info.inputs]
+        if info.kind == OpKind.INPUT:
+            y = x.astype(np.float64)
+        elif info.kind == OpKind.CONSTANT:
+            y = np.asarray(info.tensor, np.float64)
+        elif info.kind == OpKind.CONV:
+            padded = np.pad(a[0], ((0, 0), (0, 0), (1, 1), (1, 1)))
+            windows = np.lib.stride_tricks.sliding_window_view(padded, (3, 3), (2, 3))
+            y = np.einsum("nchwrs,kcrs->nkhw", windows, a[1], optimize=True)
+        elif info.kind in (OpKind.BROADCAST, OpKind.VIEW):
+            y = a[0] if a[0].ndim == 4 else a[0].reshape([1] * 4)
+        else:
+            y = {BinaryOp.ADD: np.add, BinaryOp.MAX: np.maximum, BinaryOp.MIN: np.minimum}[info.binary_op](a[0], a[1])
+        at[i] = y
+    return at[values.index(g.outputs[0])]
