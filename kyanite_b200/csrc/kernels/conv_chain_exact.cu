@@ -374,7 +374,8 @@ static const int kClusterSizes[5] = {16, 8, 4, 2, 1}, kClustersFit[5] = {7, 15, 
 // at 0.46 and more of a round or with eight CTAs an image. (Two batches of 22 boards at once: two chains of 0.67 of a round do not run
 // side by side, 1038 us against 1008 launched one by one, which is why 0.6 to 0.7 of a round, where a chain alone gains 0 to 6%, is
 // left out.)
-// Rows of 7 leave an eighth of a thread's work unused.
+// Other heights: five boards of 16 x 8 take 1.4 times as long as a chain, six 0.80, 48 of 5 x 8 1.04, 60 0.85. Rows of 7 leave an eighth
+// of a thread's work unused: 140 boards of 7 x 7 1.05, 146 0.81.
 bool conv_chain_exact_geometry(int h, int w, int64_t n_img, int c_in, int k, ChainExactGeometry* out) {
     if (w < 7 || w > W || h < 4 || h > 16 || n_img < 1 || c_in < 1 || c_in > 128 || k < 32 || k > 128 || k % 8 != 0) return false;
     ChainExactGeometry g{};
@@ -382,7 +383,9 @@ bool conv_chain_exact_geometry(int h, int w, int64_t n_img, int c_in, int k, Cha
         const int cluster = kClusterSizes[i];
         if (k % (8 * cluster) != 0 || n_img > kClustersFit[i]) continue;
         const double used = (double)(n_img * w) / (W * kClustersFit[i]);
-        if (k > 64 ? used < (cluster == 2 ? 0.6 : cluster == 1 ? 0.72 : 0.7) : cluster < 8 && used < 0.45) return false;
+        const double least_used = cluster == 16 ? (h > 8 ? 0.8 : 0.7) : cluster == 8 ? 0.78 : cluster == 4 ? 0.7 : cluster == 2 ? (h == 8 ? 0.6 : 0.7) : 0.72;
+        if (k > 64 ? used < least_used : cluster < 8 && used < 0.45) return false;
+        if (k > 64 && cluster == 1 && n_img * h * w <= 7104) return false;   // (222 tiles of 64 x 64: three CTAs of half a tile's K an SM)
         g.cluster = cluster;
         g.cols = k / cluster;
         g.items = h * g.cols / 8;
