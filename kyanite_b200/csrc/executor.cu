@@ -107,12 +107,8 @@ struct Executor {
     cudaStream_t side_stream = nullptr;          // capture-time fork for early output copies
     bool profile = false;
     std::vector<float> step_us;
-    int launches = 0;                            // of the steps one by one
-    struct DenseChain {
-        size_t first, last;                      // steps
-        DenseChainParams p;
-    };
-    std::vector<DenseChain> dense_chains;        // steps that are launched together, in order
+    int launches = 0;                            // of one run of all steps
+    std::vector<DenseChainParams> dense_runs;    // of plan->dense_runs
     Comm* comm = nullptr;              // not owned; AllReduce steps sum over its ranks (null: a world of one)
 
     ~Executor() {
@@ -237,96 +233,49 @@ struct Executor {
                 tc_prepare_step(s, status_dev, plan->opts.flags, (plan->opts.flags & KN_FLAG_TRACE_GEMM) ? status_host + 4 : nullptr);
             launches += s.launches;
         }
-        find_dense_chains();
+        prepare_dense_runs();
     }
 
-    // Runs of small dense layers (and the softmax behind them) that one kernel takes, see kernels/dense_chain.cu: plain f32
-    // matmuls with constant weights, each of which reads what the one before computed and nobody else reads.  The steps stay what
-    // they are for whoever launches or times them one by one.
-    void find_dense_chains() {
-        dense_chains.clear();
-        const std::vector<Step>& steps = plan->steps;
-        auto constant = [&](const PlanTensor& t) { return plan->buffers[t.buf].kind == BufKind::Const; };
-        auto is_layer = [&](const Step& s) {
-            if (s.kind != StepKind::Gemm) return false;
-            const GemmParams& g = s.gemm;
-            return g.batch == 1 && !g.half && !g.round_tf32 && g.conv_operand == 0 && g.row_softmax == 0 && !g.values && !g.a4.enabled && !g.b4.enabled &&
-                   !g.add2 && constant(s.operands[1]) && (g.add1 == nullptr || (g.s1[1] == 0 && constant(s.operands[3]))) &&
-                   (g.act == (int32_t)Activation::None || g.act == (int32_t)Activation::Relu) && g.m >= 1 && g.k >= 1 && g.k <= kDenseChainMaxK &&
-                   g.n >= 1 && g.n <= kDenseChainMaxN && (g.n == 1 || g.sc[2] == 1) && s.operands[2].dtype == DType::F32;
-        };
-        // step i's result is read by step i + 1 and by nothing else
-        auto read_next_only = [&](size_t i) {
-            const int buf = steps[i].operands[2].buf;
-            if (plan->buffers[buf].always_live) return false;
-            for (size_t j = 0; j < steps.size(); j++)
-                for (const PlanTensor& t : steps[j].operands)
-                    if (t.buf == buf && j != i && j != i + 1) return false;
-            return true;
-        };
-        auto bytes_of = [&](const PlanTensor& t) {   // [first, last) of what it covers
-            int64_t low = 0, high = 1;
-            for (int d = 0; d < t.ss.rank(); d++) {
-                const int64_t reach = (t.ss.shape[d] - 1) * t.ss.strides[d];
-                (reach < 0 ? low : high) += reach;
-            }
-            const uint8_t* at = device_ptr(t);
-            return std::make_pair(at + low * 4, at + high * 4);
-        };
-        for (size_t i = 0; i < steps.size(); i++) {
-            if (!is_layer(steps[i])) continue;
-            DenseChain c{};
-            DenseChainParams& p = c.p;
+    // What the runs of dense layers are launched with (Plan::dense_runs).  The steps stay what they are for whoever times them one by one.
+    void prepare_dense_runs() {
+        dense_runs.clear();
+        for (const DenseRun& r : plan->dense_runs) {
+            DenseChainParams p{};
+            p.softmax = r.softmax;
+            const size_t layers_end = r.last + (r.softmax ? 0 : 1);
             int weights = 0;
-            size_t j = i;
-            for (; j < steps.size() && p.n_layers < kDenseChainLayers && is_layer(steps[j]); j++) {
-                const GemmParams& g = steps[j].gemm;
-                if (j > i) {
-                    const GemmParams& before = steps[j - 1].gemm;
-                    if (g.a != before.c || g.m != before.m || g.k != before.n || (g.m > 1 && g.sa[1] != before.sc[1]) || (g.k > 1 && g.sa[2] != 1) || !read_next_only(j - 1)) break;
-                }
-                const int more = dense_chain_weights((int)g.k, (int)g.n);
-                if (weights + more > kDenseChainWeights) break;
+            for (size_t i = r.first; i < layers_end; i++) {
+                const GemmParams& g = plan->steps[i].gemm;
                 DenseLayer& d = p.layer[p.n_layers++];
                 d.w = g.b, d.w_k = g.sb[1], d.w_n = g.sb[2];
                 d.bias = g.add1, d.bias_n = g.s1[2];
                 d.k = (int)g.k, d.n = (int)g.n;
                 d.relu = g.act == (int32_t)Activation::Relu;
                 d.at = weights;
-                weights += more;
+                weights += dense_chain_weights(d.k, d.n);
+                launches -= plan->steps[i].launches;
             }
-            if (p.n_layers == 0) continue;
-            c.first = i;
-            c.last = i + (size_t)p.n_layers - 1;
-            const GemmParams &g0 = steps[i].gemm, &g1 = steps[c.last].gemm;
+            const GemmParams &g0 = plan->steps[r.first].gemm, &g1 = plan->steps[layers_end - 1].gemm;
             p.in = g0.a, p.rows = g0.m, p.in_row = g0.sa[1], p.in_col = g0.sa[2];
             p.out = g1.c, p.out_row = g1.sc[1];
-            const PlanTensor* result = &steps[c.last].operands[2];
-            if (c.last + 1 < steps.size() && steps[c.last + 1].kind == StepKind::Softmax && read_next_only(c.last)) {
-                const RowParams& r = steps[c.last + 1].row;
-                if (r.in0 == g1.c && !r.in1 && !r.half && r.rows == g1.m && r.len == g1.n && r.scale == 1.f && (r.len == 1 || (r.in_axis_stride == 1 && r.out_axis_stride == 1)) &&
-                    (r.rows == 1 || (r.outer_rank == 1 && r.in_strides[0] == g1.sc[1]))) {
-                    p.softmax = 1;
-                    p.out = r.out;
-                    p.out_row = r.rows == 1 ? 0 : r.out_strides[0];
-                    c.last++;
-                    result = &steps[c.last].operands[1];
-                }
+            if (r.softmax) {
+                const RowParams& row = plan->steps[r.last].row;
+                p.out = row.out;
+                p.out_row = row.rows == 1 ? 0 : row.out_strides[0];
+                launches -= plan->steps[r.last].launches;
             }
-            // (the result may have been given the memory of what the first layer reads)
-            const auto in = bytes_of(steps[i].operands[0]), out = bytes_of(*result);
-            if (c.last == c.first || (in.first < out.second && out.first < in.second)) continue;
-            dense_chains.push_back(c);
-            i = c.last;
+            launches++;
+            dense_runs.push_back(p);
         }
     }
 
     // Step i of the list, as part of a run of all of them
     void launch_at(size_t i) {
-        for (const DenseChain& c : dense_chains) {
-            if (i < c.first || i > c.last) continue;
-            if (i == c.first) {
-                const int err = launch_dense_chain(c.p, stream);
+        for (size_t r = 0; r < dense_runs.size(); r++) {
+            const DenseRun& run = plan->dense_runs[r];
+            if (i < run.first || i > run.last) continue;
+            if (i == run.first) {
+                const int err = launch_dense_chain(dense_runs[r], stream);
                 if (err != 0) fail(KN_ERR_CUDA, std::string("launch of dense layers failed: ") + cudaGetErrorString((cudaError_t)err));
             }
             return;
@@ -371,7 +320,7 @@ struct Executor {
                 for (auto& e : ev) KN_CUDA(cudaEventCreate(&e));
                 KN_CUDA(cudaEventRecord(ev[0], stream));
                 for (size_t i = 0; i < plan->steps.size(); i++) {
-                    launch_step(plan->steps[i]);
+                    launch_at(i);
                     KN_CUDA(cudaEventRecord(ev[i + 1], stream));
                 }
                 KN_CUDA(cudaStreamSynchronize(stream));
@@ -993,7 +942,10 @@ int kn_executor_last_profile(kn_executor* exec, char* buf, size_t cap, size_t* n
         for (size_t i = 0; i < plan.steps.size() && i < us.size(); i++) {
             const kn::Step& s = plan.steps[i];
             os << i << " " << kn::step_kind_name(s.kind) << (s.tensor_core ? "/tc" : "") << " " << us[i] << " "
-               << (uint64_t)s.alg_bytes << " " << (uint64_t)s.flops << " " << s.desc << "\n";
+               << (uint64_t)s.alg_bytes << " " << (uint64_t)s.flops << " " << s.desc;
+            for (const kn::DenseRun& r : plan.dense_runs)   // (all of it in the first step's time)
+                if (i >= r.first && i <= r.last) os << " [launched with steps " << r.first << ".." << r.last << "]";
+            os << "\n";
             total[(int)s.kind] += us[i];
             if (s.tensor_core) total_tc += us[i];
         }

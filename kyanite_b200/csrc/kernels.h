@@ -197,7 +197,7 @@ struct GemmParams {
     uint32_t* status;          // word that a kernel raises when a bounded wait expires
 };
 
-// ---- a run of small dense layers and the softmax behind them in one launch (kernels/dense_chain.cu): the executor's way of
+// ---- a run of small dense layers and the softmax behind them in one launch (kernels/dense_chain.cu; Plan::dense_runs): the way of
 // launching such Gemm and Softmax steps
 constexpr int kDenseChainLayers = 4, kDenseChainMaxK = 256, kDenseChainMaxN = 128, kDenseChainWeights = 7424;
 struct DenseLayer {

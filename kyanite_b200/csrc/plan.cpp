@@ -188,6 +188,7 @@ class Planner {
         fuse_conv_chains();
         drop_unused_constants();
         assign_memory();
+        find_dense_runs();
     }
 
    private:
@@ -3331,6 +3332,76 @@ class Planner {
         }
     }
 
+    // ---------------------------------------------------------------- dense layers that are launched together
+    // Plain f32 matmuls with constant weights, each of which reads what the one before computed and nobody else reads, and a
+    // softmax of the last one's rows.
+    void find_dense_runs() {
+        const std::vector<Step>& steps = plan_.steps;
+        auto constant = [&](const PlanTensor& t) { return plan_.buffers[t.buf].kind == BufKind::Const; };
+        auto is_layer = [&](const Step& s) {
+            if (s.kind != StepKind::Gemm) return false;
+            const GemmParams& g = s.gemm;
+            return g.batch == 1 && !g.half && !g.round_tf32 && g.conv_operand == 0 && g.row_softmax == 0 && !g.a4.enabled && !g.b4.enabled && g.splits <= 1 &&
+                   s.operands.size() <= 4 && constant(s.operands[1]) && (s.operands.size() == 3 || (g.s1[1] == 0 && constant(s.operands[3]))) &&
+                   (g.act == (int32_t)Activation::None || g.act == (int32_t)Activation::Relu) && g.m >= 1 && g.k >= 1 && g.k <= kDenseChainMaxK &&
+                   g.n >= 1 && g.n <= kDenseChainMaxN && (g.n == 1 || g.sc[2] == 1) && s.operands[2].dtype == DType::F32;
+        };
+        // step i's result is read by step i + 1 and by nothing else
+        auto read_next_only = [&](size_t i) {
+            const int buf = steps[i].operands[2].buf;
+            if (plan_.buffers[buf].always_live) return false;
+            for (size_t j = 0; j < steps.size(); j++)
+                for (const PlanTensor& t : steps[j].operands)
+                    if (t.buf == buf && j != i && j != i + 1) return false;
+            return true;
+        };
+        auto same_place = [&](const PlanTensor& a, const PlanTensor& b) { return a.buf == b.buf && a.offset == b.offset; };
+        auto bytes_of = [&](const PlanTensor& t) {   // [first, last) of what it covers, in the arena
+            int64_t low, high;
+            t.ss.extent(&low, &high);
+            const int64_t at = plan_.buffers[t.buf].arena_offset + t.offset * 4;
+            return std::make_pair(at + low * 4, at + (high + 1) * 4);
+        };
+        for (size_t i = 0; i < steps.size(); i++) {
+            if (!is_layer(steps[i])) continue;
+            int weights = 0;
+            size_t end = i;   // behind the last layer
+            for (; end < steps.size() && end - i < (size_t)kDenseChainLayers && is_layer(steps[end]); end++) {
+                const GemmParams& g = steps[end].gemm;
+                if (end > i) {
+                    const GemmParams& before = steps[end - 1].gemm;
+                    if (!same_place(steps[end].operands[0], steps[end - 1].operands[2]) || g.m != before.m || g.k != before.n ||
+                        (g.m > 1 && g.sa[1] != before.sc[1]) || (g.k > 1 && g.sa[2] != 1) || !read_next_only(end - 1))
+                        break;
+                }
+                const int more = dense_chain_weights((int)g.k, (int)g.n);
+                if (weights + more > kDenseChainWeights) break;
+                weights += more;
+            }
+            if (end == i) continue;
+            DenseRun run{i, end - 1, false};
+            const PlanTensor* result = &steps[run.last].operands[2];
+            if (end < steps.size() && steps[end].kind == StepKind::Softmax && read_next_only(run.last)) {
+                const RowParams& r = steps[end].row;
+                const GemmParams& g = steps[run.last].gemm;
+                if (same_place(steps[end].operands[0], *result) && steps[end].operands.size() == 2 && !r.half && r.rows == g.m && r.len == g.n && r.scale == 1.f &&
+                    (r.len == 1 || (r.in_axis_stride == 1 && r.out_axis_stride == 1)) && (r.rows == 1 || (r.outer_rank == 1 && r.in_strides[0] == g.sc[1]))) {
+                    run.softmax = true;
+                    run.last = end;
+                    result = &steps[end].operands[1];
+                }
+            }
+            if (run.last == run.first) continue;
+            // (the result may have been given the memory of what the first layer reads)
+            if (!constant(steps[i].operands[0])) {
+                const auto in = bytes_of(steps[i].operands[0]), out = bytes_of(*result);
+                if (in.first < out.second && out.first < in.second) continue;
+            }
+            plan_.dense_runs.push_back(run);
+            i = run.last;
+        }
+    }
+
     // ---------------------------------------------------------------- memory
     // Live ranges over step indices, then offsets inside one arena: buffers are placed largest
     // first at the lowest offset that does not collide with an already placed buffer whose live
@@ -3490,6 +3561,7 @@ std::string Plan::describe() const {
         for (size_t o = 0; o < s.operands.size(); o++) os << (o ? " " : "") << (s.writes[o] ? "w:" : "r:") << s.operands[o].str();
         os << "]\n";
     }
+    for (const DenseRun& r : dense_runs) os << "together " << r.first << ".." << r.last << ": dense layers" << (r.softmax ? " and softmax" : "") << ", one launch\n";
     for (size_t i = 0; i < inputs.size(); i++) os << "input " << i << " " << inputs[i].str() << "\n";
     for (size_t i = 0; i < outputs.size(); i++) os << "output " << i << " " << outputs[i].str() << "\n";
     return os.str();

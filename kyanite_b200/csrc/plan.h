@@ -77,11 +77,18 @@ struct Step {
     GroupNormParams group_norm{};
 };
 
+// Steps that are launched together: a run of small dense layers and the softmax behind them, if there is one (kernels/dense_chain.cu)
+struct DenseRun {
+    size_t first, last;   // steps
+    bool softmax;         // the last one is
+};
+
 struct Plan {
     int64_t batch = 0;
     kn_options opts{};
     std::vector<BufferInfo> buffers;
     std::vector<Step> steps;
+    std::vector<DenseRun> dense_runs;  // in order
     std::vector<PlanTensor> inputs;    // dense, one per graph input
     std::vector<PlanTensor> outputs;   // dense, one per graph output
     std::vector<std::vector<int64_t>> input_shapes, output_shapes;

@@ -1,10 +1,9 @@
 """Small dense layers that follow one another, and a softmax behind them, in one launch (kernels/dense_chain.cu): the executor's way
-of running such steps, which the plan still lists one by one.  It computes in f32 whatever the mode, so in the default mode, where
-64 rows and more would have their operands rounded to 11 bits, results at f32's precision also show that it ran."""
+of running such steps, which the plan lists one by one, with a line that says which are launched together."""
 import numpy as np
 import pytest
 
-from kyanite_b200.executor import MATH_F32, MATH_TF32
+from kyanite_b200.executor import MATH_F32, MATH_TF32, plan_describe
 from kyanite_b200.graph import BATCH, Graph, UnaryOp, shape
 
 
@@ -43,6 +42,22 @@ def want(x, weights, softmax):
     return y
 
 
+def together(g, rows, mode=MATH_F32):
+    """(first, last) of the steps that are launched together"""
+    lines = [l.split(":")[0].split(" ")[1].split("..") for l in plan_describe(g, rows, mode).splitlines() if l.startswith("together")]
+    return [(int(a), int(b)) for a, b in lines]
+
+
+def test_runs():
+    def runs(widths, softmax, rows=8, **more):
+        return together(layers(widths, softmax, **more)[0], rows)
+    assert runs([16, 32, 32, 4], True) == [(0, 3)] and runs([16, 32, 32, 4], False) == [(0, 2)] and runs([256, 3], True) == [(0, 1)]
+    assert runs([256, 3], False) == [] and runs([300, 3], True) == [] and runs([20, 129, 3], False) == []      # one layer; too long; too wide
+    assert runs([8] * 7, True) == [(0, 3), (4, 6)]                                                             # four layers at most
+    assert runs([64, 64, 64, 8], True) == [(1, 3)]                                                             # weights of 7424 floats
+    assert runs([16, 32, 32, 4], True, probe=1) == [(0, 1), (3, 4)]                                            # a result that is read elsewhere
+
+
 CASES = [  # widths of the layers, softmax, bias
     ([16, 32, 32, 4], True, True), ([256, 3], True, True), ([5, 9, 8, 1], False, True), ([1, 96, 33], True, False), ([7, 31, 64, 8, 2], True, True),
     ([20, 8, 40], False, True), ([33, 100], True, True),
@@ -62,10 +77,13 @@ def test_values(rows, widths, softmax, bias, mode):
         got, = ex.evaluate([x])
         # a few layers of f32 sums of at most 256 terms
         assert np.abs(got - expected).max() <= 4e-6 * np.abs(expected).max()
-        ex.set_profile(True)                       # (one by one: the steps themselves)
-        alone, = ex.evaluate([x])
+        steps, launches = ex.step_count()
+        assert launches == steps - sum(last - first for first, last in together(g, rows, mode))
+        ex.set_profile(True)                       # (the same launches, timed)
+        np.testing.assert_array_equal(got, ex.evaluate([x])[0])
+        profile = [l for l in ex.last_profile().splitlines() if not l.startswith("total")]
+        assert len(profile) == steps and sum("launched with" in l for l in profile) == sum(last - first + 1 for first, last in together(g, rows, mode))
         ex.set_profile(False)
-        assert np.abs(alone - expected).max() <= 4e-3 * np.abs(expected).max()
         np.testing.assert_array_equal(got, ex.evaluate([x])[0])
 
 
