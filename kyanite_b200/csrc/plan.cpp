@@ -581,7 +581,7 @@ class Planner {
                 // (of an image whose channels are contiguous: kept so where that can be viewed, as in the enlargements of an
                 // image by broadcasting along new axes)
                 PlanTensor dense;
-                if (in.ss.rank() >= 4 && in.ss.shape[1] > 1 && in.ss.strides[1] == 1) {
+                if (in.ss.rank() >= 4 && in.ss.shape[1] > 1 && in.ss.strides[1] == 1 && wanted_channels_last(v)) {
                     std::vector<int64_t> memory{in.ss.shape[0]};
                     std::vector<int> back{0, in.ss.rank() - 1};
                     for (int d = 2; d < in.ss.rank(); d++) memory.push_back(in.ss.shape[d]), back.push_back(d - 1);
@@ -663,13 +663,13 @@ class Planner {
     }
 
     // Where a concatenation goes: channels-last if it joins the channels of images that all are (each part is a copy of whole
-    // rows then, and so is what a convolution or a group norm reads), else plain
+    // rows then) and what becomes of it is read so, else plain
     PlanTensor alloc_concat(int v, const std::vector<PlanTensor>& parts) {
         const ValueInfo& info = g_.values[v];
         const std::vector<int64_t> sh = shape_of(v);
         bool last = info.dtype == DType::F32 && info.axis == 1 && sh.size() == 4 && sh[1] % 4 == 0 && sh[2] * sh[3] > 1;
         for (const PlanTensor& t : parts) last = last && t.ss.strides[1] == 1 && t.ss.shape[1] % 4 == 0 && t.ss.strides[3] != 1;
-        if (!last) return alloc_shared(sh, info.dtype, v);
+        if (!last || !wanted_channels_last(v)) return alloc_shared(sh, info.dtype, v);
         PlanTensor out = alloc_shared({sh[0], sh[2], sh[3], sh[1]}, info.dtype, v);
         return out.with(out.ss.permute({0, 3, 1, 2}));
     }
@@ -2036,7 +2036,13 @@ class Planner {
     // Group normalisation: view [N, groups, rest] -> layernorm -> view -> * scale -> + shift (-> times its own sigmoid), scale and
     // shift one value per channel.  One launch that reads and writes plain or channels-last memory, where the
     // nodes by themselves need plain memory, an elementwise step and a transposing copy on either side.
-    std::optional<PlanTensor> try_fused_group_norm(int root) {
+    struct GroupNormMatch {
+        int x = -1, norm = -1;
+        bool silu = false;
+        bool convolutions = false;   // what reads the result wants its channels contiguous
+        PlanTensor scale, shift;
+    };
+    std::optional<GroupNormMatch> match_group_norm(int root) {
         auto is_binary = [&](int v, BinaryOp op) { return g_.values[v].op == OpKind::Binary && g_.values[v].binary_op == op; };
         if (g_.values[root].dtype != DType::F32 || shape_of(root).size() != 4) return std::nullopt;
         int sum = root;
@@ -2083,8 +2089,24 @@ class Planner {
             *t = visit(v);
             return per_channel(*t);
         };
-        PlanTensor st, ht;
-        if (!channel_value(scale, &st) || !channel_value(shift, &ht)) return std::nullopt;
+        GroupNormMatch m;
+        if (!channel_value(scale, &m.scale) || !channel_value(shift, &m.shift)) return std::nullopt;
+        m.x = x;
+        m.norm = norm;
+        m.silu = silu;
+        m.convolutions = !users_[root].empty();
+        for (int u : users_[root]) m.convolutions = m.convolutions && g_.values[u].op == OpKind::Conv && g_.values[u].inputs[0] == root;
+        return m;
+    }
+
+    std::optional<PlanTensor> try_fused_group_norm(int root) {
+        const auto match = match_group_norm(root);
+        if (!match) return std::nullopt;
+        const bool silu = match->silu, convolutions = match->convolutions;
+        const int x = match->x, norm = match->norm;
+        const PlanTensor &st = match->scale, &ht = match->shift;
+        const std::vector<int64_t> sh = shape_of(root);
+        const int64_t N = sh[0], C = sh[1], hw = sh[2] * sh[3], groups = shape_of(norm)[1];
 
         // from here on steps are emitted
         PlanTensor in = visit(x);
@@ -2096,8 +2118,6 @@ class Planner {
             const auto& s = t.ss.strides;
             return s[1] == 1 && s[3] > 0 && s[3] % 4 == 0 && s[3] < (1ll << 31) && (sh[2] == 1 || s[2] == sh[3] * s[3]) && (N == 1 || s[0] % 4 == 0) && t.offset % 4 == 0;
         };
-        bool convolutions = !users_[root].empty();   // what reads the result wants its channels contiguous
-        for (int u : users_[root]) convolutions = convolutions && g_.values[u].op == OpKind::Conv && g_.values[u].inputs[0] == root;
         const bool in_last = !plain(in) && last(in) && convolutions;
         if (!in_last && !plain(in)) in = ensure_simple_copy(in, x);
         const bool out_last = in_last || convolutions;
@@ -2495,7 +2515,14 @@ class Planner {
         // tensor-core convolution wants.  If the value the graph asks for (a view of the result, say the
         // [N, groups, ...] view a group norm takes) cannot be expressed on that layout, channels x positions:
         // the filter is the A operand (shared by the batch), the result is plain NCHW.
-        const bool nchw = narrow || !StridedShape({N, K, OH, OW}, {OH * OW * K, 1, OW * K, K}).view(shape_of(root)).has_value();
+        const StridedShape turned({N, K, OH, OW}, {OH * OW * K, 1, OW * K, K});
+        // A group norm behind it reads it plain as its view does, or either way (try_fused_group_norm): then as the windows need not be
+        // materialised (below; 2 images of 24 x 24, 640 channels, convolution, norm, convolution 78.9 us with windows, 75.0 without).
+        const auto norm = group_norm_of(root);
+        auto windows_read_in_place = [&](int64_t rows) { return !strided && !pointwise && C % 32 == 0 && OW <= 256 && rows % OW == 0; };
+        const bool plain_norm = norm && !turned.view(shape_of(norm->norm)).has_value() && K >= 64 && OH * OW % 4 == 0 &&
+                                (!norm->convolutions || (N * OH * OW > 512 && !windows_read_in_place(128) && windows_read_in_place(gemm_persistent_bn(OH * OW))));
+        const bool nchw = narrow || !turned.view(shape_of(root)).has_value() || plain_norm;
         if (nchw && ((K < 64 && !narrow) || OH * OW < 16 || (OH * OW) % 4 != 0)) return std::nullopt;
         // addends as [N, OH*OW, K] or [N, K, OH*OW]
         ConvGemm g;
@@ -2633,12 +2660,34 @@ class Planner {
         std::vector<int64_t> o = shape_of(conv);
         return o[0] * o[2] * o[3] >= kConvTilePositions && o[1] >= 4;
     }
-    // is it read by a group norm that a convolution follows (try_fused_group_norm), which takes it channels-last as well?
-    bool feeds_group_norm(int v) {
+    // the group norm that reads it (try_fused_group_norm), if there is one
+    std::optional<GroupNormMatch> group_norm_of(int v) {
         for (int u : users_[v]) {
-            if (g_.values[u].op != OpKind::View || users_[u].size() != 1 || shape_of(u).size() != 3) continue;
-            const int norm = users_[u][0];
-            if (g_.values[norm].op == OpKind::Layernorm && g_.values[norm].axis == 2 && users_[norm].size() == 1 && g_.values[users_[norm][0]].op == OpKind::View) return true;
+            int root = u;   // view, layernorm, view, * scale, + shift, each read by the next alone
+            for (int depth = 0; depth < 4 && root >= 0; depth++) root = users_[root].size() == 1 ? users_[root][0] : -1;
+            if (root < 0) continue;
+            std::vector<int> ends = users_[root];   // (times its own sigmoid, or as it is)
+            ends.push_back(root);
+            for (int end : ends) {
+                auto match = match_group_norm(end);
+                if (match && match->x == v) return match;
+            }
+        }
+        return std::nullopt;
+    }
+    // does it take it channels-last?
+    bool feeds_group_norm(int v) {
+        const auto match = group_norm_of(v);
+        return match && match->convolutions;
+    }
+    // does a convolution or a group norm read it, or what views, broadcasts, concatenations and elementwise operations make of it,
+    // channels-last?
+    bool wanted_channels_last(int v, int depth = 0) {
+        if (feeds_tensor_core_conv(v) || feeds_group_norm(v)) return true;
+        for (int u : users_[v]) {
+            const OpKind op = g_.values[u].op;
+            const bool follows = op == OpKind::View || op == OpKind::Broadcast || op == OpKind::Concat || op == OpKind::Unary || op == OpKind::Binary;
+            if (follows && depth < 8 && wanted_channels_last(u, depth + 1)) return true;
         }
         return false;
     }

@@ -68,6 +68,40 @@ def test_no_turning_copies():
         assert len([l for l in lines if " vec4 acc" in l]) == 2, lines
 
 
+def group_norm(g, t, c, groups, h, w, scale=True):
+    y = g.view(g.layernorm(g.view(t, shape(BATCH, groups, c // groups * h * w)), 2, 1e-5), shape(BATCH, c, h, w))
+    one = lambda: g.constant_tensor(np.ones((1, c, 1, 1), np.float32))  # noqa: E731
+    return g.add(g.mul(y, one()), one()) if scale else g.add(y, one())
+
+
+@pytest.mark.parametrize("h,w,scale,view", [(9, 10, True, False), (16, 16, False, False), (16, 16, True, True), (7, 7, False, True)])
+def test_convolutions_before_a_norm_that_reads_plain_memory(h, w, scale, view):
+    """Planes that are no multiple of four, a norm without a scale, a result that is viewed: no copy between convolution and norm."""
+    c, g = 64, Graph()
+    x = conv(g, g.input(shape(BATCH, c, h, w)), c, c, 1)
+    g.output(g.unary(UnaryOp.TANH, x))
+    y = group_norm(g, x, c, 16, h, w, scale)
+    g.output(conv(g, y, c, c, 2))
+    if view:
+        g.output(g.view(y, shape(BATCH, c, h * w)))
+    lines = [l.split()[2] for l in plan_describe(g, 4, MATH_TF32).splitlines() if l.startswith("step")]
+    # the input turned, the convolution, its tanh, the norm [and its scale and shift], turned for the second convolution
+    assert lines.count("Scalar") == (4 if "Layernorm" in lines else 3 if view else 2), lines
+
+
+def test_copies_that_nobody_wants_channels_last():
+    """Concatenated and enlarged images that a softmax, a plain norm or the caller reads are written in plain memory at once."""
+    c, h, w, g = 256, 8, 16, Graph()
+    x = g.input(shape(BATCH, c, h, w))
+    a = conv(g, x, c, c, 1)
+    b = conv(g, a, c, c, 2)                    # (channels-last, both)
+    g.output(conv(g, b, c, 64, 3))
+    g.output(g.concat([a, b], 1))
+    g.output(enlarge(g, a, c, h, w))
+    copies = [l for l in plan_describe(g, 2, MATH_TF32).splitlines() if l.startswith("step") and " copy " in l]
+    assert len(copies) == 1 + 2 + 2, copies    # the input, the two parts, two enlargements
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("batch", [1, 3])
 @pytest.mark.parametrize("name", NAMES)
