@@ -183,8 +183,12 @@ int dense_chain_weights(int k, int n) {
 
 int launch_dense_chain(const DenseChainParams& p, cudaStream_t stream) {
     if (p.rows == 0) return 0;
-    // a row per warp until the chip has several blocks an SM, then four, which share the reads of the weights
-    const bool four = p.rows > 148 * 4 * kWarps;
+    // A row per warp until the chip has several blocks an SM, then four, which share the reads of the weights; the fewer those are, the
+    // later.  f32, one row -> four: 100-3 + softmax, 4096 rows 8.9 -> 12.3 us, 9000 13.7 -> 13.0; 200-8-8 3000 10.2 -> 18.4, 6000 19.1 -> 20.1;
+    // 64-64 3000 17.7 -> 12.2.
+    int weights = 0;
+    for (int l = 0; l < p.n_layers; l++) weights += dense_chain_weights(p.layer[l].k, p.layer[l].n);
+    const bool four = p.rows > 148 * kWarps * (weights <= 512 ? 15 : weights <= 2048 ? 7 : 4);
     const int64_t per_block = kWarps * (four ? 4 : 1), blocks = (p.rows + per_block - 1) / per_block;
     if (four) launch_pdl(dense_chain_kernel<4>, dim3((unsigned)blocks), dim3(kThreads), (size_t)0, stream, p);
     else launch_pdl(dense_chain_kernel<1>, dim3((unsigned)blocks), dim3(kThreads), (size_t)0, stream, p);

@@ -3382,6 +3382,27 @@ class Planner {
     }
 
     // ---------------------------------------------------------------- dense layers that are launched together
+    // Is one launch shorter than those of its steps?  Microseconds, fitted to 38 shapes at 64 to 65 536 rows: what a launch takes at least,
+    // and what a row adds.  In one launch: a row of the input, the weights from shared memory (every block fetches them).  One by
+    // one: on tensor cores hardly anything, on CUDA cores more, with few columns (a warp per row) most.  TF32, one by one -> one
+    // launch: 16-32-32-4 + softmax 10.6 -> 4.4 us at 64 rows, 138 -> 109 at 65 536; 64-64-8 + softmax 7.7 -> 7.1 at 64 rows, 8.8 -> 11.3 at 1500,
+    // 69 -> 160 at 65 536; 96-64 + softmax 5.0 -> 6.1 at 64.  f32: 96-64 + softmax 11.6 -> 6.1 at 64, 12.3 -> 14.7 at 1500, 68 -> 199 at 65 536.
+    bool dense_run_pays(const DenseRun& run, int weights) const {
+        double single = 0, single_rows = 0;   // all steps; what 65 536 rows add
+        const size_t end = run.last + (run.softmax ? 0 : 1);
+        for (size_t i = run.first; i < end; i++) {
+            const Step& s = plan_.steps[i];
+            const double k = (double)s.gemm.k, n = (double)s.gemm.n;
+            single += s.tensor_core ? 2.6 : n > 8 ? 7.5 : 3.5;
+            single_rows += s.tensor_core ? 16 : n > 8 ? 30 + 0.25 * k : k >= 32 ? 60 + 9 * n + 0.3 * k : 35;
+        }
+        if (run.softmax) single += 2.6, single_rows += 12;
+        const GemmParams& first = plan_.steps[run.first].gemm;
+        const double layers = (double)(end - run.first), rows = (double)first.m / 65536;
+        const double together = 2.7 + 0.4 * layers + 0.0005 * weights, together_rows = std::max(60.0, 25 + 10 * layers + 0.4 * (double)first.k + 0.016 * weights);
+        return together + 1.1 * rows * together_rows < std::max(single, single / 2 + rows * single_rows);
+    }
+
     // Plain f32 matmuls with constant weights, each of which reads what the one before computed and nobody else reads, and a
     // softmax of the last one's rows.
     void find_dense_runs() {
@@ -3440,7 +3461,7 @@ class Planner {
                     result = &steps[end].operands[1];
                 }
             }
-            if (run.last == run.first) continue;
+            if (run.last == run.first || !dense_run_pays(run, weights)) continue;
             // (the result may have been given the memory of what the first layer reads)
             if (!constant(steps[i].operands[0])) {
                 const auto in = bytes_of(steps[i].operands[0]), out = bytes_of(*result);

@@ -55,6 +55,11 @@ def test_runs():
     assert runs([256, 3], False) == [] and runs([300, 3], True) == [] and runs([20, 129, 3], False) == []      # one layer; too long; too wide
     assert runs([8] * 7, True) == [(0, 3), (4, 6)]                                                             # four layers at most
     assert runs([64, 64, 64, 8], True) == [(1, 3)]                                                             # weights of 7424 floats
+    assert runs([64, 64, 8], True, 500) and runs([96, 64], True) and not runs([96, 64], True, 2000)
+    g = layers([64, 64, 8], True)[0]                                                                           # on tensor cores from 64 rows on
+    assert together(g, 63, MATH_TF32) and together(g, 500, MATH_TF32) and together(g, 1500, MATH_TF32) == [(1, 2)]
+    assert not together(layers([96, 64], True)[0], 64, MATH_TF32)
+    assert together(layers([16, 32, 32, 4], True)[0], 65536, MATH_TF32) == [(0, 3)]
     assert runs([16, 32, 32, 4], True, probe=1) == [(0, 1), (3, 4)]                                            # a result that is read elsewhere
 
 
@@ -75,8 +80,9 @@ def test_values(rows, widths, softmax, bias, mode):
     expected = want(x, weights, softmax)
     with CudaExecutor(0, g, rows, math_mode=mode) as ex:
         got, = ex.evaluate([x])
-        # a few layers of f32 sums of at most 256 terms
-        assert np.abs(got - expected).max() <= 4e-6 * np.abs(expected).max()
+        # a few layers of f32 sums of at most 256 terms; steps that stay by themselves may round their operands to 11 bits
+        rounded = "/tc" in "".join(l for i, l in enumerate(plan_describe(g, rows, mode).splitlines()[1:]) if not any(a <= i <= b for a, b in together(g, rows, mode)))
+        assert np.abs(got - expected).max() <= (4e-3 if rounded else 4e-6) * np.abs(expected).max()
         steps, launches = ex.step_count()
         assert launches == steps - sum(last - first for first, last in together(g, rows, mode))
         ex.set_profile(True)                       # (the same launches, timed)
