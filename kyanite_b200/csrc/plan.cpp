@@ -2497,18 +2497,21 @@ class Planner {
         const bool may_be_implicit = !strided && C % 32 == 0 && OW <= 256 && 128 % OW == 0 && OH * OW >= 64 &&
                                      !(opts_.flags & KN_FLAG_NO_PERSISTENT_GEMM);
         const bool long_k = C * R * S >= 2048 && (may_be_implicit || N * OH * OW * R * S * C * 4 <= (256ll << 20));
-        if (!strided && !few_positions && !pointwise && !long_k && (C > 8 || OH * OW < 784)) return std::nullopt;
+        const double flops = 2.0 * (double)N * OH * OW * K * C * R * S;
+        // An image of few channels (a network's first convolution; boards, whose convolutions chain, have fewer positions): the
+        // convolution kernel loads 32 channels per tap whatever there are.  With the copy that turns the image, windows and matmul: 4 ->
+        // 320 channels of 64 x 64 31.6 -> 9.5 us, 64 images 3 -> 64 of 32 x 32 95 -> 17, 3 -> 64 of 224 x 224 86 -> 15; at 77, 116 and 105 MB of windows 64
+        // images 3 -> 64 of 64 x 64 258 -> 82, 16 of 224 x 224 816 -> 252, 1 -> 32, 5 x 5, of 128 x 128 981 -> 343.
+        const bool shallow = C <= 8 && OH * OW >= 784 && R * S > 1 && (C * R * S <= 256 || flops >= 2e8) && !strided && K >= 16 &&
+                             N * OH * OW * R * S * C * 4 <= (256ll << 20);
+        if (!strided && !few_positions && !pointwise && !long_k && !shallow) return std::nullopt;
         if (pointwise && !strided && py == 0 && px == 0 && becomes_chain_head(ci, x)) return std::nullopt;
         if (N < 1 || N > 65535 || OH * OW < 64 || K % 4 != 0 || C < 1 || R * S > 64) return std::nullopt;
         // Few channels of a long reduction (an image's last convolution): the convolution kernel has a CTA per 128 positions that goes
         // through all of K; where that leaves half of the SMs idle, slices of K over clusters.  320 -> 4 channels of 64 x 64 39.4 -> 11.3
         // us, 512 -> 12 of 16 x 16 59.9 -> 8.1; at the line, 256 -> 12 of 74 x 128, 33.5 -> 19.5.
         const bool narrow = K < 16 && !pointwise && long_k && may_be_implicit && OH * OW % 128 == 0 && N * OH * OW <= 74 * 128;
-        // An image of few channels (a network's first convolution; boards, whose convolutions chain, have fewer positions): the
-        // convolution kernel loads 32 channels per tap whatever there are.  With the copy that turns the image, windows and matmul: 4 ->
-        // 320 channels of 64 x 64 31.6 -> 9.5 us, 64 images 3 -> 64 of 32 x 32 95 -> 17, 3 -> 64 of 224 x 224 86 -> 15.
-        const bool shallow = C <= 8 && OH * OW >= 784 && R * S > 1 && C * R * S <= 256 && !strided && N * OH * OW * R * S * ((C + 3) / 4 * 4) * 4 <= (64ll << 20);
-        if (!narrow && !(shallow && K >= 16) && (K < 16 || 2.0 * (double)N * OH * OW * K * C * R * S < 2e8)) return std::nullopt;
+        if (!narrow && !shallow && (K < 16 || flops < 2e8)) return std::nullopt;
         const ValueInfo& wi = g_.values[ci.inputs[1]];
         if (wi.op != OpKind::Constant || !w.ss.has_simple_strides() || w.offset != 0) return std::nullopt;
         // Two orientations.  positions x channels: the result is channels-last in memory, which the next

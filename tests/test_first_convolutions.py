@@ -31,7 +31,8 @@ def test_route():
     assert not windows(8, 64, 32, 32, 7, 7, (3, 3))     # windows of more than 256 elements
     assert not windows(4, 12, 64, 64) and not windows(4, 30, 64, 64)
     assert not windows(4, 64, 64, 64, mode=MATH_F32)
-    assert not windows(4, 64, 512, 512, batch=8)
+    assert windows(3, 64, 224, 224, batch=16) and windows(8, 64, 64, 64, 7, 7, (3, 3), batch=8)   # 87 and 51 MB of windows
+    assert not windows(4, 64, 512, 512, batch=8)        # 302 MB: the limit is 256
 
 
 CASES = [(4, 320, 64, 64, 3, 3, (1, 1), False, False, 1), (3, 64, 32, 32, 3, 3, (1, 1), False, True, 3), (1, 32, 28, 28, 5, 5, (2, 2), False, False, 2),
