@@ -345,6 +345,12 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     }
                 }
             };
+            if (TERM && plain && __any_sync(0xffffffffu, !(fabsf(ref) < 1e30f))) {
+                // (a row masked by the lowest value so far: its reference times log2(e) would overflow)
+#pragma unroll
+                for (int i = 0; i < 64; i++) v[i >> 5][i & 31] = __float_as_uint(p.scale * __uint_as_float(v[i >> 5][i & 31]));
+                plain = false;
+            }
             const float shift = -ref * unit, factor = plain ? p.scale * unit : unit;
             if (TERM && !plain) exponentials([&](float x) { return (x - ref) * unit; });   // (the lowest finite value times log2(e) would overflow)
             else exponentials([&](float x) { return fmaf(x, factor, shift); });
