@@ -9,7 +9,7 @@
 // rescaled (once the block before has been added), which after the first few blocks hardly ever happens; the quotient does
 // not depend on the reference.
 //
-//   warps 0..3      softmax: a row per thread, all 64 columns of it, so nothing is exchanged
+//   warps 0..3      softmax: a row per thread, all 64 columns of it, so nothing is exchanged (few blocks on few CTAs: eight warps, PAIRED)
 //   warp 4, a lane  producer: Q once, keys and values of a block through two buffers each (one where two do not fit)
 //   warp 5, a lane  MMA issuer: the next block's score MMAs go ahead of this block's context MMAs, under its exponentials
 //
@@ -44,11 +44,11 @@ namespace {
 
 using namespace tcp;
 
-constexpr int kFlThreads = 192;
 constexpr int kFlRows = 128, kFlKeys = 64;
 constexpr int kFlTableKeys = 128;          // keys of a block in the planner's table of a constant term
 constexpr int kFlQBytes = kFlRows * 128, kFlKeyBytes = kFlKeys * 128;   // a panel: rows of 128 bytes
 constexpr int kFlTmemCols = 256, kFlOutCol = 128;
+constexpr int kFlExchangeBytes = 2 * 2 * kFlRows * 4;   // (PAIRED)
 constexpr float kLog2e = 1.44269504088896340736f;
 constexpr float kRiseLimit = 8.0f;
 constexpr float kHalfSumBelow = -1024.f;   // f16 values are one apart here
@@ -88,12 +88,15 @@ __device__ __forceinline__ void arrive_one(uint32_t bar) {
 __device__ __forceinline__ void tmem_loads_done() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_stores_done() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-template <bool HALF, bool TERM>
-__global__ void __launch_bounds__(kFlThreads, 2)
+// PAIRED: eight softmax warps, of which four take the even blocks and four the odd ones; of a pair of blocks they exchange the rows'
+// maxima, so that both go by one reference.  For grids that leave an SM one CTA, whose blocks would follow one another.
+template <bool HALF, bool TERM, bool PAIRED>
+__global__ void __launch_bounds__(PAIRED ? 320 : 192, PAIRED ? 1 : 2)
 flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ FlashParams p) {
     extern __shared__ uint8_t smem_raw[];
     constexpr int kElems = HALF ? 64 : 32;   // elements per 128 bytes
+    constexpr int kSoftmaxWarps = PAIRED ? 8 : 4;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
     const uint32_t k_bytes = (uint32_t)(p.qk_blocks * kFlKeyBytes), v_bytes = (uint32_t)(p.v_panels * kFlKeyBytes);
@@ -113,12 +116,12 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             mbar_init(k_full + b, 1);
             mbar_init(v_full + b, 1);
             mbar_init(s_full + b, 1);
-            mbar_init(p_ready + b, 4);
+            mbar_init(p_ready + b, kSoftmaxWarps);
         }
         *abandon = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 4) {
+    if (warp == kSoftmaxWarps) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_addr), "r"((uint32_t)kFlTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -143,7 +146,7 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
     const int n_blocks = min(n_table * kTableStep, p.key_blocks);
 
-    if (warp == 4) {
+    if (warp == kSoftmaxWarps) {
         if (elect_one()) {
             // ---------------- producer
             const uint32_t q_bytes = (uint32_t)(p.qk_blocks * kFlQBytes);
@@ -171,7 +174,7 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     tma_load_4d(to + (uint32_t)(b * kFlKeyBytes), &map_v, v_full + 8u * (j & 1), b * kElems, j * kFlKeys, v2, v3);
             }
         }
-    } else if (warp == 5) {
+    } else if (warp == kSoftmaxWarps + 1) {
         if (elect_one()) {
             // ---------------- MMA issuer: f32 accumulate, M = 128; Q and the keys K-major, V with its columns contiguous
             // (bit 16: the MN-major B operand)
@@ -220,7 +223,8 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
     } else {
         // ---------------- softmax
-        const int quarter = warp, row_in_tile = quarter * 32 + lane, row = mt * kFlRows + row_in_tile;
+        const int quarter = PAIRED ? warp & 3 : warp, group = warp >> 2, row_in_tile = quarter * 32 + lane, row = mt * kFlRows + row_in_tile;
+        float* exchange = (float*)(gen_base + (bars + 128u - base));   // [2][group][row]
         const uint32_t lane_bits = (uint32_t)(quarter * 32) << 16;
         const uint32_t my_o = tmem_o + lane_bits;
         using T = typename std::conditional<HALF, __half, float>::type;
@@ -232,78 +236,109 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             tc_fence_after();
             return good != 0;
         };
+        // one value a row against the other group's, if everybody goes on; `turn` alternates from call to call
+        auto meet = [&](bool good, int turn, float& mine_, float& others) -> bool {
+            exchange[((turn & 1) * 2 + group) * kFlRows + row_in_tile] = mine_;
+            uint32_t all;
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\t"
+                "setp.ne.u32 p, %1, 0;\n\t"
+                "bar.red.and.pred q, 1, 256, p;\n\t"
+                "selp.u32 %0, 1, 0, q;\n\t}"
+                : "=r"(all)
+                : "r"((uint32_t)good)
+                : "memory");
+            others = exchange[((turn & 1) * 2 + (group ^ 1)) * kFlRows + row_in_tile];
+            return all != 0;
+        };
         // x in units of its exponent: with a term  x = scale * s + term, exponent (x - ref) * log2(e); without one x = s
         const float unit = TERM ? kLog2e : p.scale * kLog2e;
         float seen = -INFINITY, ref = 0.f, sum = 0.f;
-        bool ok = true;
-        for (int j = 0; j < n_blocks; j++) {
+        bool ok = true, far = false;   // far: a row of the warp has a reference of the lowest values' size
+        constexpr int kStep = PAIRED ? 2 : 1;
+        for (int first_j = 0; first_j < n_blocks; first_j += kStep) {
+            const int j = first_j + (PAIRED ? group : 0);
+            const bool mine = !PAIRED || j < n_blocks;
             const uint32_t b = (uint32_t)(j & 1);
             const uint32_t my_s = tmem_s + lane_bits + b * kFlKeys;
-            if (!wait(s_full + 8u * b, (uint32_t)((j >> 1) & 1), 58)) { ok = false; break; }
+            bool good = true;
+            if constexpr (PAIRED) {   // (nobody leaves alone: see `meet`)
+                good = ok && (!mine || wait(s_full + 8u * b, (uint32_t)((j >> 1) & 1), 58));
+            } else {
+                if (!wait(s_full + 8u * b, (uint32_t)((j >> 1) & 1), 58)) { ok = false; break; }
+            }
             uint32_t v[2][32];
-            tmem_load_32_nowait(my_s, v[0]);
-            tmem_load_32_nowait(my_s + 32u, v[1]);
-            tmem_loads_done();
-            const int col0 = j * kFlKeys;
+            float top = -INFINITY;
             bool plain = false;   // a block whose term is zero throughout: scores as without a term
-            if (TERM) {
-                const int kind = blocks_of == nullptr ? 1 : (int)blocks_of[1 + j / kTableStep];
-                if (kind == 0 && p.scale > 0.f) {
-                    plain = true;
-                } else if (kind != 1) {
-                    const float same = kind == 2 ? -INFINITY : 0.f;
+            if (!PAIRED || (mine && good)) {
+                tmem_load_32_nowait(my_s, v[0]);
+                tmem_load_32_nowait(my_s + 32u, v[1]);
+                tmem_loads_done();
+                const int col0 = j * kFlKeys;
+                if (TERM) {
+                    const int kind = blocks_of == nullptr ? 1 : (int)blocks_of[1 + j / kTableStep];
+                    if (kind == 0 && p.scale > 0.f) {
+                        plain = true;
+                    } else if (kind != 1) {
+                        const float same = kind == 2 ? -INFINITY : 0.f;
 #pragma unroll
-                    for (int i = 0; i < 64; i++) v[i >> 5][i & 31] = __float_as_uint(fmaf(p.scale, __uint_as_float(v[i >> 5][i & 31]), same));
-                } else {
-                    const T* t = term_row + (int64_t)col0 * p.term_s[2];
-                    const bool vec = p.term_s[2] == 1 && col0 + 64 <= p.term_cols && ((uintptr_t)t & 15) == 0;
+                        for (int i = 0; i < 64; i++) v[i >> 5][i & 31] = __float_as_uint(fmaf(p.scale, __uint_as_float(v[i >> 5][i & 31]), same));
+                    } else {
+                        const T* t = term_row + (int64_t)col0 * p.term_s[2];
+                        const bool vec = p.term_s[2] == 1 && col0 + 64 <= p.term_cols && ((uintptr_t)t & 15) == 0;
 #pragma unroll
-                    for (int c = 0; c < 2; c++) {
+                        for (int c = 0; c < 2; c++) {
 #pragma unroll
-                        for (int i = 0; i < 32; i += 8) {
-                            float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                            if (vec) {
-                                if (HALF) {
-                                    const uint4 u = __ldg((const uint4*)(t + c * 32 + i));
-                                    const __half2* h = (const __half2*)&u;
+                            for (int i = 0; i < 32; i += 8) {
+                                float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                                if (vec) {
+                                    if (HALF) {
+                                        const uint4 u = __ldg((const uint4*)(t + c * 32 + i));
+                                        const __half2* h = (const __half2*)&u;
 #pragma unroll
-                                    for (int q = 0; q < 4; q++) {
-                                        const float2 f = __half22float2(h[q]);
-                                        a[2 * q] = f.x, a[2 * q + 1] = f.y;
+                                        for (int q = 0; q < 4; q++) {
+                                            const float2 f = __half22float2(h[q]);
+                                            a[2 * q] = f.x, a[2 * q + 1] = f.y;
+                                        }
+                                    } else {
+#pragma unroll
+                                        for (int q = 0; q < 2; q++) {
+                                            const float4 f = __ldg((const float4*)(t + c * 32 + i) + q);
+                                            a[4 * q] = f.x, a[4 * q + 1] = f.y, a[4 * q + 2] = f.z, a[4 * q + 3] = f.w;
+                                        }
                                     }
                                 } else {
 #pragma unroll
-                                    for (int q = 0; q < 2; q++) {
-                                        const float4 f = __ldg((const float4*)(t + c * 32 + i) + q);
-                                        a[4 * q] = f.x, a[4 * q + 1] = f.y, a[4 * q + 2] = f.z, a[4 * q + 3] = f.w;
-                                    }
+                                    for (int q = 0; q < 8; q++)
+                                        if (col0 + c * 32 + i + q < p.n) a[q] = (float)t[(int64_t)(c * 32 + i + q) * p.term_s[2]];
                                 }
-                            } else {
 #pragma unroll
-                                for (int q = 0; q < 8; q++)
-                                    if (col0 + c * 32 + i + q < p.n) a[q] = (float)t[(int64_t)(c * 32 + i + q) * p.term_s[2]];
-                            }
-#pragma unroll
-                            for (int q = 0; q < 8; q++) {
-                                float x = fmaf(p.scale, __uint_as_float(v[c][i + q]), a[q]);
-                                // Far below anything a row with an unmasked key looks at, f16 sums are rounded as such: a row
-                                // that is masked by f16's lowest value throughout has the same sum, or -infinity, everywhere.
-                                if (HALF && x < kHalfSumBelow) x = __half2float(__float2half_rn(x));
-                                v[c][i + q] = __float_as_uint(x);
+                                for (int q = 0; q < 8; q++) {
+                                    float x = fmaf(p.scale, __uint_as_float(v[c][i + q]), a[q]);
+                                    // Far below anything a row with an unmasked key looks at, f16 sums are rounded as such: a row
+                                    // that is masked by f16's lowest value throughout has the same sum, or -infinity, everywhere.
+                                    if (HALF && x < kHalfSumBelow) x = __half2float(__float2half_rn(x));
+                                    v[c][i + q] = __float_as_uint(x);
+                                }
                             }
                         }
                     }
                 }
-            }
-            if (col0 + 64 > p.n) {   // columns past the last key
+                if (col0 + 64 > p.n) {   // columns past the last key
 #pragma unroll
-                for (int i = 0; i < 64; i++)
-                    if (col0 + i >= p.n) v[i >> 5][i & 31] = 0xFF800000u;
-            }
-            float top = -INFINITY;
+                    for (int i = 0; i < 64; i++)
+                        if (col0 + i >= p.n) v[i >> 5][i & 31] = 0xFF800000u;
+                }
 #pragma unroll
-            for (int i = 0; i < 64; i++) top = fmaxf(top, __uint_as_float(v[i >> 5][i & 31]));
-            if (plain) top *= p.scale;
+                for (int i = 0; i < 64; i++) top = fmaxf(top, __uint_as_float(v[i >> 5][i & 31]));
+                if (plain) top *= p.scale;
+            }
+            if (PAIRED) {
+                float other;
+                ok = meet(good, first_j >> 1, top, other);
+                if (!ok) break;
+                top = fmaxf(top, other);
+            }
             // a row whose scores were all -infinity so far has no reference yet (and zeros in its sum and output)
             const bool first = seen == -INFINITY;
             seen = fmaxf(seen, top);
@@ -312,10 +347,18 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 const float next = rise && seen > -INFINITY ? seen : ref;
                 const float factor = rise && !first ? exp2_approx((ref - next) * unit) : 1.f;
                 ref = next;
+                if (TERM) far = __any_sync(0xffffffffu, !(fabsf(ref) < 1e30f));
                 sum *= factor;
-                if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
-                    if (!wait(pv_done + 8u * (b ^ 1u), (uint32_t)(((j - 1) >> 1) & 1), 59)) { ok = false; break; }   // (the block before is still being added)
-                    for (int c = 0; c < (p.out_cols + 31) >> 5; c++) {
+                if (first_j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
+                    const int before = first_j - 1;   // (is still being added)
+                    int chunks = (p.out_cols + 31) >> 5;
+                    if constexpr (PAIRED) {
+                        ok = wait(pv_done + 8u * (before & 1), (uint32_t)((before >> 1) & 1), 59);
+                        chunks = ok ? chunks : 0;
+                    } else {
+                        if (!wait(pv_done + 8u * (b ^ 1u), (uint32_t)((before >> 1) & 1), 59)) { ok = false; break; }
+                    }
+                    for (int c = PAIRED ? group : 0; c < chunks; c += kStep) {
                         uint32_t o[32];
                         tmem_load_32(my_o + (uint32_t)(c * 32), o);
 #pragma unroll
@@ -323,6 +366,13 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                         tmem_store_32(my_o + (uint32_t)(c * 32), o);
                     }
                 }
+            }
+            if (PAIRED) {   // (a group's half of the output is rescaled before the other's block is added)
+                tmem_stores_done();
+                tc_fence_before();
+                __syncwarp();
+                if (ok && lane == 0 && first_j + (group ^ 1) < n_blocks) arrive_one(p_ready + 8u * (b ^ 1u));
+                if (!ok || !mine) continue;
             }
             auto exponentials = [&](auto exponent) {
 #pragma unroll
@@ -345,7 +395,7 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     }
                 }
             };
-            if (TERM && plain && __any_sync(0xffffffffu, !(fabsf(ref) < 1e30f))) {
+            if (TERM && plain && far) {
                 // (a row masked by the lowest value so far: its reference times log2(e) would overflow)
 #pragma unroll
                 for (int i = 0; i < 64; i++) v[i >> 5][i & 31] = __float_as_uint(p.scale * __uint_as_float(v[i >> 5][i & 31]));
@@ -365,10 +415,16 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             __syncwarp();
             if (lane == 0) arrive_one(p_ready + 8u * b);
         }
-        if (ok && wait(pv_done + 8u * ((n_blocks - 1) & 1), (uint32_t)(((n_blocks - 1) >> 1) & 1), 59)) {
+        ok = ok && wait(pv_done + 8u * ((n_blocks - 1) & 1), (uint32_t)(((n_blocks - 1) >> 1) & 1), 59);
+        if (PAIRED) {
+            float other;
+            ok = meet(ok, (n_blocks + 1) >> 1, sum, other);
+            sum = group == 0 ? sum + other : other + sum;
+        }
+        if (ok) {
             const float inv = 1.f / sum;
             T* dst = (T*)p.out + (bt / p.out_heads) * p.out_s[0] + (bt % p.out_heads) * p.out_s[1] + (int64_t)row * p.out_s[2];
-            for (int c = 0; c < (p.dv + 31) >> 5; c++) {
+            for (int c = PAIRED ? group : 0; c < (p.dv + 31) >> 5; c += kStep) {
                 uint32_t o[32];
                 tmem_load_32(my_o + (uint32_t)(c * 32), o);
 #pragma unroll
@@ -396,7 +452,7 @@ flash_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         tc_fence_before();
     }
     __syncthreads();
-    if (warp == 4) {
+    if (warp == kSoftmaxWarps) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_s), "r"((uint32_t)kFlTmemCols) : "memory");
     }
@@ -446,7 +502,7 @@ struct FlashLaunch {
     FiniteParams finite;
     unsigned grid;
     int smem_bytes;
-    bool half;
+    bool half, paired;
 };
 
 // Shared memory with `key_slots` and `value_slots` buffers
@@ -529,18 +585,31 @@ std::shared_ptr<void> flash_attention_prepare(const GemmParams& g, uint32_t* sta
     if (!operand(g.b4, g.b, kFlKeys, g.n, g.k, g.sb[0], g.sb[2], g.sb[1], false, &l->map_k, &p.b_bi, 0)) return nullptr;
     if (!operand(g.v4, g.values, kFlKeys, g.n, g.values_cols, g.values_strides[0], g.values_strides[1], g.values_strides[2], true, &l->map_v, &p.v_bi, 1))
         return nullptr;
+    l->grid = (unsigned)(g.batch * p.m_tiles);
+    // Two to four blocks with a term where an SM has one CTA.  One group of softmax warps -> two, causal f16: 32 heads of 128 rows, d = 64 9.4 -> 7.9 us, d =
+    // 128 10.6 -> 8.9; 256 rows 11.6 -> 10.6 and 13.2 -> 11.7.  With more blocks the next block's scores under this block's exponentials gain
+    // more (8 heads of 512 rows 14.3 -> 15.7, f32 8 of 1024 rows 18.4 -> 24.2), and without a term the exponentials are short: 2 of 1590 rows,
+    // 157 keys 6.2 -> 7.2.
+    l->paired = p.term != nullptr && l->grid <= 148 && p.key_blocks > 1 && p.key_blocks <= 4 && flash_smem_bytes(g.k, g.values_cols, half, 1, 1) + kFlExchangeBytes <= 227 * 1024;
     // two buffers of each where two CTAs of it share an SM (or none would with one)
-    const int half_sm = 113 * 1024, whole_sm = 227 * 1024;
+    const int half_sm = 113 * 1024, whole_sm = 227 * 1024 - (l->paired ? kFlExchangeBytes : 0);
     p.key_slots = p.value_slots = 1;
-    const int limit = flash_smem_bytes(g.k, g.values_cols, half, 1, 1) <= half_sm ? half_sm : whole_sm;
+    const int limit = !l->paired && flash_smem_bytes(g.k, g.values_cols, half, 1, 1) <= half_sm ? half_sm : whole_sm;
     if (flash_smem_bytes(g.k, g.values_cols, half, 1, 2) <= limit) p.value_slots = 2;
     if (flash_smem_bytes(g.k, g.values_cols, half, 2, p.value_slots) <= limit) p.key_slots = 2;
-    l->smem_bytes = flash_smem_bytes(g.k, g.values_cols, half, p.key_slots, p.value_slots);
-    l->grid = (unsigned)(g.batch * p.m_tiles);
+    l->smem_bytes = flash_smem_bytes(g.k, g.values_cols, half, p.key_slots, p.value_slots) + (l->paired ? kFlExchangeBytes : 0);
     return l;
 }
 
+using FlashKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, FlashParams);
+template <bool PAIRED>
+static FlashKernel flash_kernel(bool half, bool term) {
+    return half ? (term ? flash_attention_kernel<true, true, PAIRED> : flash_attention_kernel<true, false, PAIRED>)
+                : (term ? flash_attention_kernel<false, true, PAIRED> : flash_attention_kernel<false, false, PAIRED>);
+}
+
 int flash_attention_launch(const void* launch, cudaStream_t stream) {
+    auto kernel = [](bool half, bool term, bool paired) { return paired ? flash_kernel<true>(half, term) : flash_kernel<false>(half, term); };
     const FlashLaunch& l = *(const FlashLaunch*)launch;
     static std::mutex mu;
     static bool done[64] = {false};
@@ -549,8 +618,8 @@ int flash_attention_launch(const void* launch, cudaStream_t stream) {
     {
         std::lock_guard<std::mutex> lock(mu);
         if (device >= 0 && device < 64 && !done[device]) {
-            for (const void* v : {(const void*)flash_attention_kernel<false, false>, (const void*)flash_attention_kernel<false, true>,
-                                  (const void*)flash_attention_kernel<true, false>, (const void*)flash_attention_kernel<true, true>}) {
+            for (FlashKernel v : {kernel(false, false, false), kernel(false, true, false), kernel(true, false, false), kernel(true, true, false),
+                                  kernel(false, false, true), kernel(false, true, true), kernel(true, false, true), kernel(true, true, true)}) {
                 cudaError_t e = cudaFuncSetAttribute(v, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
                 if (e != cudaSuccess) return (int)e;
             }
@@ -561,12 +630,7 @@ int flash_attention_launch(const void* launch, cudaStream_t stream) {
         const dim3 blocks((unsigned)l.p.batch * (unsigned)l.p.table_blocks);
         launch_pdl(l.half ? flash_finite_kernel<true> : flash_finite_kernel<false>, blocks, dim3(256), (size_t)0, stream, l.finite);
     }
-    const dim3 grid(l.grid), block(kFlThreads);
-    const size_t smem = (size_t)l.smem_bytes;
-    if (l.half && l.p.term) launch_pdl(flash_attention_kernel<true, true>, grid, block, smem, stream, l.map_q, l.map_k, l.map_v, l.p);
-    else if (l.half) launch_pdl(flash_attention_kernel<true, false>, grid, block, smem, stream, l.map_q, l.map_k, l.map_v, l.p);
-    else if (l.p.term) launch_pdl(flash_attention_kernel<false, true>, grid, block, smem, stream, l.map_q, l.map_k, l.map_v, l.p);
-    else launch_pdl(flash_attention_kernel<false, false>, grid, block, smem, stream, l.map_q, l.map_k, l.map_v, l.p);
+    launch_pdl(kernel(l.half, l.p.term != nullptr, l.paired), dim3(l.grid), dim3(l.paired ? 320 : 192), (size_t)l.smem_bytes, stream, l.map_q, l.map_k, l.map_v, l.p);
     return (int)cudaGetLastError();
 }
 

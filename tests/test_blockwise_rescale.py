@@ -10,11 +10,14 @@ from oracle.cpu_eval import assert_tensors_match, cpu_eval_graph
 
 @pytest.mark.gpu
 # (a wide head in f32 over whole blocks of keys goes another way)
-@pytest.mark.parametrize("n,half,d,dv", [(n, *c) for n in (63, 64, 65, 128, 191, 449) for c in ((False, 40, 40), (False, 128, 96), (True, 128, 128), (True, 24, 72))
-                                         if n % 64 or c != (False, 128, 96)])
-def test_rising_maxima(n, half, d, dv):
+# (f32 goes this way where its matmuls by themselves would round their operands; 20 entries leave an SM one CTA, whose softmax warps
+# take two blocks at a time)
+@pytest.mark.parametrize("n,b,half,d,dv", [(n, *c) for n in (63, 64, 65, 128, 129, 191, 449)
+                                           for c in ((220, False, 40, 40), (220, False, 128, 96), (20, True, 128, 128), (20, True, 24, 72), (100, True, 128, 128), (100, True, 24, 72))
+                                           if n % 64 or c != (220, False, 128, 96)])
+def test_rising_maxima(n, b, half, d, dv):
     from kyanite_b200.executor import CudaExecutor
-    b, m = (20 if half else 220), 200   # (f32 goes this way where its matmuls by themselves would round their operands)
+    m = 200
     dtype = DType.F16 if half else DType.F32
     r = np.random.Generator(np.random.PCG64(n))
     g = Graph()
