@@ -15,8 +15,8 @@
 //   warp 1, a lane  MMA issuer: four tcgen05.mma.kind::tf32 (K = 8) per stage into accumulator `tile & 1`;
 //                   waits for that accumulator to be drained, signals it full with tcgen05.commit
 //   warps 2..9      epilogue: two groups of four, thread <-> accumulator lane <-> output row; the groups take 32 columns each in
-//                   turn.  One group is as fast while the next tile's MMAs hide it; where a CTA has few tiles or the epilogue
-//                   computes (GELU) it is not: 16384 x 768 x 768 + bias 38.8 us with one group and 36.5 with two, 16384 x 3072 x
+//                   turn; f32 results with nothing added or computed have one (gemm_persistent_prepare).  One group is as fast
+//                   while the next tile's MMAs hide it; where a CTA has few tiles or the epilogue adds or computes it is not: 16384 x 768 x 768 + bias 38.8 us with one group and 36.5 with two, 16384 x 3072 x
 //                   768 + GELU 136.9 and 129.8, 2048 x 4096 x 4096 of halves 51.9 and 51.3 (without an epilogue to speak of, 2048 x
 //                   11008 x 4096 of halves, 129.8 and 130.3).  One warp of a group polls for the accumulator, the rest sleep at
 //                   a barrier: with all of them polling, long reductions lost 1% to the power it took.
@@ -1054,10 +1054,12 @@ std::shared_ptr<void> gemm_persistent_prepare(const GemmParams& g, uint32_t* sta
         p.clocks = table;
     }
     const int stage_bytes = kGpATileBytes + (pair ? p.bn / 2 : p.bn) * 128;
-    // One group where a tile has few K blocks and nothing to compute, so that its stores bound it: they leave in the order of the
-    // columns then.  384 x 512 x 512 x 64: one group 85.6 us, two 94.2, two with a staging tile more each 100; one group
-    // chosen in the kernel instead of compiled 92.
-    p.groups = !pair && p.k_iters <= 8 && g.act == 0 ? 1 : 2;
+    // One group where there is nothing to add or compute: stores leave in the order of the columns then, which is what short tiles in
+    // f32 are bound by (f16 stores are half as long), and the power that the second group takes is the MMAs'.  One group -> two:
+    // 384 x 512 x 512 x 64 87.9 -> 94.7 us (with a staging tile more each 100; one group chosen in the kernel instead of compiled 92), 4096 x
+    // 2304 x 64 11.6 -> 13.0, 16384 x 768 x 512 34.0 -> 34.8, x 2048 102.3 -> 102.5.  With a bias 4096 x 2304 x 64 22.0 -> 17.0, x 256 23.9 -> 19.7, x 384
+    // 26.1 -> 21.4; f16 16384 x 768 x 128 17.1 -> 15.7, x 640 24.7 -> 23.9.
+    p.groups = !pair && !half && g.add1 == nullptr && g.act == 0 ? 1 : 2;
     const int fixed = 1024 + 2 * kGpStageTileBytes + 16 * 8 + 64 + 64;
     p.stages = std::max(2, std::min(6, (227 * 1024 - fixed) / stage_bytes));
     l->smem_bytes = fixed + p.stages * stage_bytes;
@@ -1079,7 +1081,7 @@ int gemm_persistent_launch(const void* launch, cudaStream_t stream) {
     {
         std::lock_guard<std::mutex> lock(mu);
         if (device >= 0 && device < 64 && !done[device]) {
-            const void* variants[] = {(const void*)gemm_persistent_kernel<false, false, 1>, (const void*)gemm_persistent_kernel<true, false, 1>,
+            const void* variants[] = {(const void*)gemm_persistent_kernel<false, false, 1>,
                                       (const void*)gemm_persistent_kernel<false, false, 2>, (const void*)gemm_persistent_kernel<true, false, 2>,
                                       (const void*)gemm_persistent_kernel<false, true, 2>, (const void*)gemm_persistent_kernel<true, true, 2>};
             for (const void* v : variants) {
@@ -1111,7 +1113,7 @@ int gemm_persistent_launch(const void* launch, cudaStream_t stream) {
     auto launch_groups = [&](auto kernel) {
         launch_pdl(kernel, dim3(l.grid), dim3(64u + 128u * (unsigned)l.p.groups), (size_t)(l.smem_bytes), stream, l.map_a, l.map_b, l.map_c, l.p);
     };
-    if (l.p.groups == 1) launch_groups(l.half ? gemm_persistent_kernel<true, false, 1> : gemm_persistent_kernel<false, false, 1>);
+    if (l.p.groups == 1) launch_groups(gemm_persistent_kernel<false, false, 1>);
     else launch_groups(l.half ? gemm_persistent_kernel<true, false, 2> : gemm_persistent_kernel<false, false, 2>);
     return (int)cudaGetLastError();
 }
