@@ -87,9 +87,6 @@ struct RowParams {
                              // statistics and the arithmetic stay f32, the result is rounded to f16 once
 };
 
-// ---- root-mean-square norm over the innermost axis:  out = x / sqrt(mean(x^2) + eps) * gain.  The IR has no such
-// operation; the planner recognises the pow / mean / sqrt / div / mul subgraph (with the value casts around it in
-// half-storage graphs) and this one kernel takes the place of five elementwise and reduce steps.
 // ---- group normalisation with scale, shift and SiLU (kernels/group_norm.cu)
 struct GroupNormParams {
     const float* in;
@@ -105,6 +102,9 @@ struct GroupNormParams {
     uint32_t* status;                // word that the kernel raises when a bounded wait expires
 };
 
+// ---- root-mean-square norm over the innermost axis:  out = x / sqrt(mean(x^2) + eps) * gain.  The IR has no such
+// operation; the planner recognises the pow / mean / sqrt / div / mul subgraph (with the value casts around it in
+// half-storage graphs) and this one kernel takes the place of five elementwise and reduce steps.
 struct RmsNormParams {
     const void* in;          // [rows, len], rows `in_row_stride` elements apart, f32 or f16
     void* out;               // [rows, len] dense, f32 or f16

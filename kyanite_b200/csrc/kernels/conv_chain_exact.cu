@@ -55,7 +55,7 @@ struct ExactKernelParams {
     const float* weights;
     int64_t s_in[4], s_out[4];
     int32_t c_in, k, h, w;
-    int32_t n_layers, cluster, cols, col_groups, k_groups, items;   // cols: output channels of a CTA; items = h * col_groups
+    int32_t n_layers, cluster, cols, k_groups, items;   // cols: output channels of a CTA; items: (image row, 8 of them)
     int32_t chunk, slots, channels;      // input channels of a weight chunk; ring slots; input channels that shared memory holds
     int32_t segment;                     // chunks that are summed by themselves, or 0: all of them
     int32_t act_floats;                  // of a channel: (h + 2) * kPitch
@@ -439,7 +439,6 @@ std::shared_ptr<void> chain_exact_prepare(const ConvChainParams& c, uint32_t* st
     p.n_layers = c.n_layers;
     p.cluster = g.cluster;
     p.cols = g.cols;
-    p.col_groups = g.cols / 8;
     p.k_groups = g.k_groups;
     p.items = g.items;
     p.chunk = g.chunk;

@@ -83,13 +83,6 @@ __device__ __forceinline__ uint64_t smem_desc_rows(uint32_t addr, uint32_t pitch
     return (smem_desc_sw128(addr) & ~((uint64_t)0x3FFF << 32)) | ((uint64_t)(pitch * 8u) << 32);
 }
 
-// Arrives on the leader's barrier without a release at cluster scope, which waits for every store of the thread to be visible
-// to the whole GPU (measured: 1000 cycles an arrival, 226 -> 207 us for 33 layers of 256 boards).  What this arrival hands over
-// lies in the SM's own shared memory and is read by that SM's tensor core: `fence.proxy.async` before it has completed it there.
-__device__ __forceinline__ void mbar_arrive_pair_leader(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-
 __device__ __forceinline__ float2 add_pair(float2 a, float2 b) {
     uint64_t d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*(uint64_t*)&a), "l"(*(uint64_t*)&b));
@@ -266,7 +259,9 @@ conv_chain_pair_kernel(const __grid_constant__ CUtensorMap map_trunk, const __gr
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_pair_leader(leader_act + 8u * cb);
+            // (no release at cluster scope, which takes 1000 cycles an arrival, 226 -> 207 us for 33 layers of 256 boards: what is handed
+            // over lies in this SM's own shared memory and is read by its tensor core; the fence has completed it there)
+            if (lane == 0) mbar_arrive_remote(leader_act + 8u * cb);
         };
         // layer 0's input: from global memory into the operand and the held columns
         asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -212,7 +212,8 @@ int launch_pieces(const GroupNormParams& p, cudaStream_t stream) {
 
 }  // namespace
 
-// CTAs of a group: as many as give the chip one each, and as its values need; 0 if eight do not hold them.
+// CTAs of a group: as many as give the chip one each, and as its values need; 0 if eight do not hold them.  (120 and not 148: 32 groups, the
+// usual number, are 128 CTAs of clusters of four; clusters of eight are two rounds of 960 channels of 64 x 64, 36.6 us instead of 18.7.)
 int group_norm_cluster(int64_t groups, int64_t values) {
     for (int c = 1; c <= kMaxCluster; c *= 2)
         if (values <= (int64_t)c * kMaxThreads * kMaxFloats && (groups * c >= 120 || c == kMaxCluster)) return c;
