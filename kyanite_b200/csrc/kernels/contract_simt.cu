@@ -496,11 +496,13 @@ contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int slices = args.slices;
     const int slice = (int)(blockIdx.z % (unsigned)slices);
+    // units of four columns of the result, of which each slice stores `share`
+    int share = 0;
+    if (COUNTED) share = (L::kUnits + slices - 1) / slices;
     const uint32_t arrived = smem_addr(smem + L::kBarrier);
     if (slices > 1) {
         if (COUNTED) {
             if (threadIdx.x == 0) {
-                const int share = (L::kUnits + slices - 1) / slices;
                 tcp::mbar_init(arrived, 1);
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
                 tcp::mbar_expect_tx(arrived, (uint32_t)(max(0, min(share, L::kUnits - slice * share)) * slices) * 16u);
@@ -690,9 +692,8 @@ contract_cols_kernel(const __grid_constant__ Problem prob, const __grid_constant
                 make_float4(acc[i][2 * j].x, acc[i][2 * j].y, acc[i][2 * j + 1].x, acc[i][2 * j + 1].y);
     __syncthreads();
     if (slices > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    // units of four columns, in the order in which the result's contiguous axis comes first; of several slices, each
-    // stores `share` of them
-    const int share = (L::kUnits + slices - 1) / slices;
+    // units, in the order in which the result's contiguous axis comes first
+    if (!COUNTED) share = (L::kUnits + slices - 1) / slices;
     auto place = [&](int u, int& mm, int& nn) {
         mm = args.rows_fast ? u % BM : u / (BN / 4);
         nn = (args.rows_fast ? u / BM : u % (BN / 4)) * 4;
