@@ -184,7 +184,8 @@ KN_API int kn_executor_step_count(const kn_executor* exec, int* steps, int* laun
 /* `set_profile` / `last_profile` (kn-cuda-eval/src/executor.rs:43-58, 208-257, 291-325): with
  * profiling on, the next `run_async`/`evaluate` launches step by step (no graph replay) with a CUDA
  * event pair around each step.  `kn_executor_last_profile` writes one line per step
- * (`index kind microseconds algorithmic_bytes flops description`) followed by per-kind totals. */
+ * (`index kind microseconds algorithmic_bytes flops description`) followed by per-kind totals.  Steps that are launched
+ * together (small dense layers) say so in their descriptions; the first of them has the time of all. */
 KN_API int kn_executor_set_profile(kn_executor* exec, int enable);
 KN_API int kn_executor_last_profile(kn_executor* exec, char* buf, size_t cap, size_t* needed);
 /* Launches step `step` alone `launches` times back to back between one pair of CUDA events on the

@@ -4,8 +4,9 @@
 //
 // A warp takes R rows through all layers; the weights of all layers lie in shared memory (requested ahead of the dependency wait:
 // they are constants).  Layers of more than eight columns give each lane a column of every 32; narrower ones give the lanes the
-// reduction.  f32 multiply-adds throughout; four products are summed by themselves before they join the sum over all (one running
-// sum is 1.1 times as far from 64 bits as the layers launched one by one).
+// reduction.  f32 multiply-adds throughout; four products are summed by themselves before they join one of two sums over every other four
+// (against 64 bits, layers launched one by one 1: one running sum 1.1, of fours 1.02, two of them 1.00; 16-32-32-4, 16 networks of 4000
+// rows; 128-32-8 0.78).
 //
 // What bounds it: one launch, the first loads, and a chain of k multiply-adds per layer.  8 rows of 16 -> 32 -> 32 -> 4 + softmax:
 // four launches of 14.3 us -> one; with its copies and the host's calls 28.6 -> 22.4 us.
@@ -73,12 +74,12 @@ __global__ void __launch_bounds__(kThreads) dense_chain_kernel(const __grid_cons
         const bool last = l == p.n_layers - 1;
         if (d.n > 8) {
             const int cols = (d.n + 31) & ~31, rows = (d.k + 3) & ~3, groups = cols >> 5;
-            float y[R][4];
+            float y[R][4], odd[R][4];   // (every other four products)
 #pragma unroll
             for (int r = 0; r < R; r++)
 #pragma unroll
-                for (int c = 0; c < 4; c++) y[r][c] = 0.f;
-            for (int k = 0; k < rows; k += 4) {
+                for (int c = 0; c < 4; c++) y[r][c] = odd[r][c] = 0.f;
+            auto four = [&](float (&to)[R][4], int k) {
                 float4 x[R];
 #pragma unroll
                 for (int r = 0; r < R; r++) x[r] = *(const float4*)&values[warp][r][k];
@@ -88,9 +89,17 @@ __global__ void __launch_bounds__(kThreads) dense_chain_kernel(const __grid_cons
                     const float* at = w + k * cols + c * 32 + lane;
                     const float w0 = at[0], w1 = at[cols], w2 = at[2 * cols], w3 = at[3 * cols];
 #pragma unroll
-                    for (int r = 0; r < R; r++) y[r][c] += fmaf(x[r].y, w1, x[r].x * w0) + fmaf(x[r].w, w3, x[r].z * w2);
+                    for (int r = 0; r < R; r++) to[r][c] += fmaf(x[r].y, w1, x[r].x * w0) + fmaf(x[r].w, w3, x[r].z * w2);
                 }
+            };
+            for (int k = 0; k < rows; k += 8) {
+                four(y, k);
+                if (k + 4 < rows) four(odd, k + 4);
             }
+#pragma unroll
+            for (int r = 0; r < R; r++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) y[r][c] += odd[r][c];
             __syncwarp();
 #pragma unroll
             for (int r = 0; r < R; r++) {
