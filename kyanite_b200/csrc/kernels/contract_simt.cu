@@ -456,10 +456,10 @@ __global__ void __launch_bounds__(kThreads, KG) contract_simt_kernel(const __gri
 // stages as there are; rows are located once, in a table, and not by divisions in the loop; slices of a tile send their sums to
 // the CTA that stores them (a cluster barrier that the peers have started, waited for at the first remote store; no remote reads).
 // COUNTED: that they have arrived is told by a barrier in the receiver's memory that counts their bytes (`st.async`), not by a
-// second cluster barrier, which has to release what it hands over and takes some 1000 cycles.  Only where a CTA has its SM to itself
-// or tiles are small: where two and more large tiles share an SM another CTA computes meanwhile, and the code with the counter
-// is the slower one even without slices (seven layers of 128 channels: 40 boards 178 -> 186 us with it, 95 373 -> 382,
-// 256 717 -> 723; 34 147.7 -> 147.7; eight boards of 256 channels 104 -> 106).
+// second cluster barrier, which has to release what it hands over and takes some 1000 cycles.  Not where three and more large tiles
+// share an SM, another CTA computing meanwhile, or eight slices do: the code with the counter is the slower one there, even
+// without slices (seven layers of 128 channels: 40 boards 178 -> 186 us with it, 95 373 -> 381, 256 715 -> 722; eight boards of 256
+// channels 102 -> 106; with two tiles an SM two batches of 22 boards at a time 1009 -> 988 for 33 layers).
 // One 8 x 8 board, 128 -> 128 channels, 3 x 3: 12.1 us on contract_simt_kernel, 5.2 us here (5.6 with a second cluster barrier)
 // (in a chain; by itself 7.4, kernel_bench's conv_exact_board); 64 boards 48 -> 36 us, 256 boards 112 us
 // (0.61 of the rate); 12 heads of 120 x 64 x 120 (probabilities . V) 14.1 -> 4.8 us.
@@ -815,7 +815,8 @@ int launch_cols(const Problem& prob, int64_t M, int64_t N, int64_t batch, int64_
     if (tile == kLargeAlone) return launch_cols_tile<Problem, 64, 64, 8, 8, 4, 3, 1, true>(prob, M, N, batch, args, 0, stream);
     // (two CTAs an SM are kept at two by the shared memory they ask for: three on some SMs and one on others took 81 us
     // instead of 57 for 1024 x 1024 x 1024)
-    return launch_cols_tile<Problem, 64, 64, 8, 8, 2, 3, 3, false>(prob, M, N, batch, args, per_sm == 2 ? 80 * 1024 : 0, stream);
+    if (per_sm <= 2 && args.slices < 8) return launch_cols_tile<Problem, 64, 64, 8, 8, 2, 3, 3, true>(prob, M, N, batch, args, 80 * 1024, stream);
+    return launch_cols_tile<Problem, 64, 64, 8, 8, 2, 3, 3, false>(prob, M, N, batch, args, per_sm <= 2 ? 80 * 1024 : 0, stream);
 }
 
 template <class Problem, int BM, int BN, int TN, int KG, class Index = int>
